@@ -28,6 +28,19 @@ def _load():
 
 
 lib = _load()
+
+
+def _load_native():
+    """``_fwp_torch.so``, the host path of the autograd entry points (csrc/binding/fwp_torch.cpp)."""
+    try:
+        from recurrent_fwp_b200 import _fwp_torch
+    except ImportError as e:
+        raise ImportError('recurrent_fwp_b200: the native host path is not usable (%s). Build it with '
+                          '`python recurrent_fwp_b200/build.py`.' % e) from e
+    return _fwp_torch
+
+
+native = _load_native()
 _T = ctypes.POINTER(FwpTensor)
 _T3 = ctypes.POINTER(FwpTensor)   # arrays of three descriptors are passed as pointers
 _i, _vp, _i64 = ctypes.c_int, ctypes.c_void_p, ctypes.c_int64
@@ -165,6 +178,24 @@ def unit_inner(t):
     return t.contiguous()
 
 
+def entry_point(name, normalise):
+    """The public callable of one op.  ``native.<name>`` takes arguments that are already in the form the kernels
+    read and answers NotImplemented for anything else; then ``normalise`` raises the error that fits, or returns the
+    arguments with unit inner strides."""
+    native_op = getattr(native, name)
+
+    def op(*args):
+        out = native_op(*args)
+        if out is NotImplemented:
+            out = native_op(*normalise(*args))
+            if out is NotImplemented:
+                raise RuntimeError('%s: unsupported arguments' % name)
+        return out
+
+    op.__name__ = op.__qualname__ = name
+    return op
+
+
 def stream_and_device(t):
     return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream), t.device.index
 
@@ -182,16 +213,11 @@ def device_fault():
     return int(lib.fwp_delta_device_fault())
 
 
-def raise_on_device_fault(what):
-    """With FWP_CHECK_DEVICE_FAULT=1 in the environment the delta-rule wrappers call this after every launch: it
-    synchronises the device and raises if a bounded wait inside a kernel ran out (the launch then produced wrong
-    numbers instead of hanging).  Off by default because of the synchronisation; a trainer can instead poll
-    ``device_fault()`` at step or epoch boundaries."""
-    if _CHECK_FAULT and device_fault() != 0:
-        raise RuntimeError('%s: a bounded wait inside the kernel ran out; its results are invalid' % what)
-
-
-_CHECK_FAULT = os.environ.get('FWP_CHECK_DEVICE_FAULT', '0') == '1'
+# With FWP_CHECK_DEVICE_FAULT=1 in the environment the delta-rule ops ask after every launch: that synchronises the
+# device and raises if a bounded wait inside a kernel ran out (the launch then produced wrong numbers instead of
+# hanging).  Off by default because of the synchronisation; a trainer can instead poll ``device_fault()`` at step or
+# epoch boundaries.
+native.check_device_fault(os.environ.get('FWP_CHECK_DEVICE_FAULT', '0') == '1')
 
 
 def launch_count():

@@ -1,4 +1,5 @@
-"""Build ``libfwp.so`` (the C-ABI library) in-tree with nvcc for sm_100a.
+"""Build ``libfwp.so`` (the C-ABI library) in-tree with nvcc for sm_100a, and ``_fwp_torch.so`` (the host path of
+the autograd entry points, plain C++ against PyTorch) beside it.
 
     python recurrent_fwp_b200/build.py [--force] [--verbose]
 
@@ -12,11 +13,14 @@ import glob
 import os
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, 'csrc')
 OBJ = os.path.join(PKG, 'build')
 LIB = os.path.join(PKG, 'libfwp.so')
+BINDING_SRC = os.path.join(CSRC, 'binding', 'fwp_torch.cpp')
+BINDING = os.path.join(PKG, '_fwp_torch.so')
 NVCC = os.environ.get('NVCC', '/usr/local/cuda/bin/nvcc')
 FLAGS = ['-gencode', 'arch=compute_100a,code=sm_100a', '-lineinfo', '-O3', '-std=c++17',
          '-Xcompiler', '-fPIC', '-Xcompiler', '-fvisibility=hidden']
@@ -34,6 +38,23 @@ def _compile(args):
     cmd = [NVCC] + FLAGS + (['-Xptxas', '-v'] if verbose else []) + ['-c', src, '-o', obj]
     r = subprocess.run(cmd, capture_output=True, text=True)
     return src, r.returncode, r.stdout + r.stderr
+
+
+def _compile_binding():
+    """_fwp_torch.so: links libfwp.so (found beside it at run time) and the PyTorch libraries already loaded."""
+    import torch
+    from torch.utils import cpp_extension
+    cmd = [os.environ.get('CXX', 'g++'), '-O2', '-std=c++17', '-fPIC', '-shared', '-fvisibility=hidden',
+           '-D_GLIBCXX_USE_CXX11_ABI=%d' % torch._C._GLIBCXX_USE_CXX11_ABI,
+           '-I' + sysconfig.get_paths()['include'], '-I' + os.path.join(os.path.dirname(os.path.dirname(NVCC)), 'include')]
+    cmd += ['-isystem' + d for d in cpp_extension.include_paths()]
+    cmd += [BINDING_SRC, '-o', BINDING, '-L' + PKG, '-l:libfwp.so', '-Wl,-rpath,$ORIGIN']
+    cmd += ['-L' + d for d in cpp_extension.library_paths()]
+    cmd += ['-lc10', '-lc10_cuda', '-ltorch_cpu', '-ltorch_cuda', '-ltorch', '-ltorch_python']
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError('the compiler failed on %s' % BINDING_SRC)
 
 
 def build(force=False, verbose=False):
@@ -60,6 +81,8 @@ def build(force=False, verbose=False):
         if r.returncode:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError('link failed')
+    if force or _newer([BINDING_SRC] + glob.glob(os.path.join(PKG, '..', 'include', '*.h')), BINDING):
+        _compile_binding()
     return LIB
 
 

@@ -4,7 +4,7 @@ The reference's layers (language_modeling/src/utils/cuda_fast_weight_layer.py:10
 algorithmic/layers.py:110-137) turn the fused projection ``qkvb`` of shape (len, B, H, 3d+1) into the op's
 arguments with a chain of split / sigmoid / permute / elu+1 / sum-normalise launches, and turn the op's
 output back into (len, B, H*d) with a scale, a transpose and a reshape.  The two autograd Functions here do
-each direction in one launch; ``delta_attention`` strings them around ``fast_weight_delta``:
+each direction in one launch; ``delta_attention`` runs them around the delta rule in one autograd node:
 
     out = delta_attention(qkvb.view(len, B, H, 3*d + 1), W, scale)      # (len, B, H*d); W updated in place
 
@@ -15,7 +15,6 @@ import ctypes
 import torch
 
 from recurrent_fwp_b200 import _lib
-from recurrent_fwp_b200.fast_weight import fast_weight_delta
 
 
 def _p(t):
@@ -87,7 +86,21 @@ delta_layer_prologue = DeltaLayerPrologue.apply
 delta_layer_epilogue = DeltaLayerEpilogue.apply
 
 
+def _normalise(qkvb, W, scale):
+    _lib.require_cuda(qkvb)
+    if qkvb.dtype != torch.float32 or qkvb.dim() != 4 or (qkvb.shape[3] - 1) % 3:
+        raise RuntimeError('qkvb must be float32 of shape (len, B, H, 3*d + 1)')
+    _, B, H, w = qkvb.shape
+    D = (w - 1) // 3
+    _lib.require_f32(qkvb, {'W': (W, (B, H, D, D))})
+    if W.stride(3) != 1:
+        raise RuntimeError('W must have a unit innermost stride (it is updated in place)')
+    return qkvb.contiguous(), W, float(scale)
+
+
+_delta_attention = _lib.entry_point('delta_attention', _normalise)
+
+
 def delta_attention(qkvb, W, scale):
     """Prologue, delta-rule fast weight memory, epilogue.  qkvb: (len, B, H, 3d+1); W: (B, H, d, d), updated in place."""
-    q, k, v, beta = delta_layer_prologue(qkvb)
-    return delta_layer_epilogue(fast_weight_delta(q, k, v, beta, W), scale)
+    return _delta_attention(qkvb, W, scale)

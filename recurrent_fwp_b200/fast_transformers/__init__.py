@@ -11,41 +11,22 @@ import torch
 from recurrent_fwp_b200 import _lib
 
 
+def _normalise(Q, K, V, W):
+    N, H, L, E = Q.shape
+    M = V.shape[3]
+    _lib.io_dtype(Q)
+    _lib.require_streams(Q, {'K': (K, (N, H, L, E)), 'V': (V, (N, H, L, M))})
+    _lib.require_f32(Q, {'W': (W, (N, H, E, M))})
+    _lib.require_cuda(Q, K, V, W)
+    if M > 1 and W.stride(3) != 1:
+        raise RuntimeError('W must have a unit innermost stride (it is updated in place)')
+    return [_lib.unit_inner(t) for t in (Q, K, V)] + [W]
+
+
 class FastWeightSum(torch.autograd.Function):
-    """Fast weight using the purely additive (sum) update rule."""
+    """Fast weight using the purely additive (sum) update rule; native like the delta rule's."""
 
-    @staticmethod
-    def forward(ctx, Q, K, V, W):
-        N, H, L, E = Q.shape
-        M = V.shape[3]
-        _lib.io_dtype(Q)
-        _lib.require_streams(Q, {'K': (K, (N, H, L, E)), 'V': (V, (N, H, L, M))})
-        _lib.require_f32(Q, {'W': (W, (N, H, E, M))})
-        _lib.require_cuda(Q, K, V, W)
-        Qc, Kc, Vc = (_lib.unit_inner(t.detach()) for t in (Q, K, V))
-        out = torch.empty((N, H, L, M), device=Q.device, dtype=Q.dtype)
-        stream, dev = _lib.stream_and_device(Q)
-        _lib.check(_lib.lib.fwp_causal_dot_product(
-            N, H, L, E, M, _lib.desc(Qc), _lib.desc(Kc), _lib.desc(Vc), _lib.desc(W.detach()),
-            _lib.desc(out), _lib.io_dtype(Q), stream, dev), 'causal_dot_product')
-        ctx.save_for_backward(Qc, Kc, Vc)
-        return out
-
-    @staticmethod
-    def backward(ctx, grad_out):
-        Q, K, V = ctx.saved_tensors
-        N, H, L, E = Q.shape
-        M = V.shape[3]
-        grad_out = _lib.grad_like(grad_out, Q, (N, H, L, M))
-        grad_Q = torch.empty_like(Q, memory_format=torch.contiguous_format)
-        grad_K = torch.empty_like(K, memory_format=torch.contiguous_format)
-        grad_V = torch.empty_like(V, memory_format=torch.contiguous_format)
-        stream, dev = _lib.stream_and_device(Q)
-        _lib.check(_lib.lib.fwp_causal_dot_backward(
-            N, H, L, E, M, _lib.desc(Q), _lib.desc(K), _lib.desc(V), _lib.desc(grad_out),
-            _lib.desc(grad_Q), _lib.desc(grad_K), _lib.desc(grad_V),
-            _lib.io_dtype(Q), stream, dev), 'causal_dot_backward')
-        return grad_Q, grad_K, grad_V, None
+    apply = staticmethod(_lib.entry_point('fast_weight_sum', _normalise))
 
 
 fast_weight_sum = FastWeightSum.apply
