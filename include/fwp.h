@@ -91,7 +91,9 @@ unsigned long long fwp_launch_count(void);
  * "launch.dependent" (1 / 0: the register-resident delta-rule kernels are launched with programmatic stream serialisation, so that
  * their prologue overlaps the tail of the kernel before them in the stream, or plainly),
  * "delta.pipe64" (1 / 2 / 0: chunkwise bf16 kernels with a preparing warp one chunk ahead in both directions,
- * in the forward only, or not at all).  Returns 0 if accepted, FWP_ERR_UNSUPPORTED for an unknown key. */
+ * in the forward only, or not at all),
+ * "delta.wy" (-1 automatic / 1 / 0: the chunkwise split-product plan wherever it is the faster one, wherever it has an
+ * instance, or never), "delta.wy.helpers" (0 automatic / 4 / 2: preparing warps per sequence of that plan).  Returns 0 if accepted, FWP_ERR_UNSUPPORTED for an unknown key. */
 int fwp_tune(const char* key, int value);
 /* Name of the kernel this host thread launched last through the library ("" before the
  * first launch): lets a benchmark label its numbers with the plan the dispatch picked. */

@@ -66,6 +66,8 @@ enum TuneKey {
     T_SUM_BWD_ROLES,        // "sum_bwd.roles": 1 the three gradients of the sum rule in warps of their own, side by side; 0 one after the other
     T_LAUNCH_DEPENDENT,     // "launch.dependent": 1 the register-resident delta-rule kernels (blocked and per-step) are launched with programmatic stream serialisation (their prologue overlaps the tail of the kernel before), 0 plain launches
     T_STEP_SPREAD,          // "step.spread": 1 the per-step forward packs fewer sequences into a CTA while that puts CTAs on more SMs, 0 always four warps per CTA
+    T_DELTA_WY,             // "delta.wy": -1 automatic, 1 / 0 the chunkwise split-product plan (fwp_delta_wy.cuh) wherever it has an instance, or never
+    T_DELTA_WY_HELPERS,     // "delta.wy.helpers": preparing warps per sequence of that plan (2 or 4), 0 automatic
     T_COUNT
 };
 int tune_get(TuneKey key, int fallback);

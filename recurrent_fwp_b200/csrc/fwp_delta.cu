@@ -517,10 +517,31 @@ static int launch_sum_bwd_generic(const SumBwdParams& p, int nseq, cudaStream_t 
 // 12-15 us per launch (32 x 8 sequences), and the d=64 fp32 backward only pays off beyond 64 steps.
 // "delta.blocked" = 0 / 1 forces the per-step / blocked plan (tests cross-check one against the other).
 constexpr int kShortSeq = 16;
+// Where the chunkwise split-product plan (fwp_delta_wy.cuh) is the faster forward, from measurements on B200 with fp32
+// streams (sequences x steps; before -> with it, us):
+//   d = 16: 16 x 256 19.6 -> 11.6, 256 x 256 19.8 -> 15.4, 1536 x 64 21.2 -> 19.4, but 512 x 256 20.4 -> 27.8: with more than
+//           two sequences per SM the blocked kernel's four short chains per CTA win unless the sequences are short;
+//   d = 32: 128 x 256 44.7 -> 20.9, 256 x 512 88 -> 50, 512 x 256 47 -> 42;   d = 48: 512 x 256 154 -> 90;
+//   d = 64: 64 x 256 65.7 -> 34.9, 512 x 256 148 -> 117, but 256 x 20 10.2 -> 11.0 (two chunks are all start-up);
+//   E, M = 96, 32: 128 x 256 692 -> 68;   128, 128: 1655 -> 98 (the shared-memory kernels).
+template <typename T, bool SUM>
+static bool fwd_wy_pays(const DeltaFwdParams& p, int nseq) {
+    const int d = p.E > p.M ? p.E : p.M;
+    if (p.L <= kShortSeq) return d > 64 && p.L > 4;
+    if (d <= 16) return nseq <= 2 * sm_count() || p.L <= 4 * kShortSeq;
+    return d <= 32 || d > 64 || p.L > 2 * kShortSeq;
+}
 template <typename T, bool SUM>
 static int dispatch_fwd(const DeltaFwdParams& p, int nseq, cudaStream_t st) {
     const int D = pad_dim(p.E > p.M ? p.E : p.M);
     const int force = tune_get(T_DELTA_BLOCKED, -1);
+    const int wy = force == -1 ? tune_get(T_DELTA_WY, -1) : 0;
+    bool tensor_plan = false;       // bf16 streams at E = M = 64 keep their own chunkwise kernels
+    if constexpr (!SUM && sizeof(T) == 2) tensor_plan = p.L > kShortSeq && tune_get(T_DELTA_CHUNK64, 1) == 1 && chunk_bf16_applies(p);
+    if (wy == 1 || (wy == -1 && !tensor_plan && fwd_wy_pays<T, SUM>(p, nseq))) {
+        const int rc = launch_fwd_wy<T, SUM>(p, nseq, st);
+        if (rc >= 0) return rc;
+    }
     if (D == 0) return launch_fwd_generic<T, SUM>(p, nseq, st);
     switch (D) {
         case 16: {
@@ -753,7 +774,7 @@ FWP_API int fwp_delta_device_fault(void) {
         const int zero = 0;
         cudaMemcpyToSymbol(fwp::g_delta_fault, &zero, sizeof zero);
     }
-    const int t = fwp::tc_fault_read_clear();
-    if (t < 0) return -1;
-    return (v || t) ? 1 : 0;
+    const int t = fwp::tc_fault_read_clear(), w = fwp::wy_fault_read_clear();
+    if (t < 0 || w < 0) return -1;
+    return (v || t || w) ? 1 : 0;
 }

@@ -68,6 +68,9 @@ bool chunk_bf16_applies(const DeltaFwdParams& p);
 int launch_fwd_chunk_bf16(const DeltaFwdParams& p, int nseq, cudaStream_t st);
 bool chunk_bf16_applies(const DeltaBwdParams& p);
 int launch_bwd_chunk_bf16(const DeltaBwdParams& p, int nseq, cudaStream_t st);
+// chunkwise plan on split fp32 products (fwp_delta_wy.cuh); -1 when the sizes have no instance
+int wy_fault_read_clear();
+template <typename T, bool SUM> int launch_fwd_wy(const DeltaFwdParams& p, int nseq, cudaStream_t st);
 int tc_fault_read_clear();
 int launch_wait_probe(int polls, cudaStream_t st);
 

@@ -1,0 +1,69 @@
+"""The chunkwise split-product plan of the delta and sum rules (csrc/fwp_delta_wy.cuh): every instance, at chunk remainders,
+padded head sizes, layer-sliced streams with rows at odd offsets, and both ways of sharing the work between warps."""
+import pytest
+import torch
+
+from tests import util
+
+pytestmark = pytest.mark.gpu
+DEV = 'cuda:0'
+
+
+def run(fwp, rule, x, W, plan):
+    from recurrent_fwp_b200 import _lib
+    try:
+        for key, value in plan.items():
+            _lib.tune(key, value)
+        f = fwp.fast_weight_delta if rule == 'delta' else fwp.fast_weight_sum
+        W = W.clone()
+        with torch.no_grad():
+            y = f(*x, W)
+        return y, W, _lib.last_kernel()
+    finally:
+        _lib.tune('delta.wy', -1)
+        _lib.tune('delta.wy.helpers', 0)
+
+
+def sliced(x):
+    """The same streams as transposed views of one (L, B, H, width) tensor, rows at odd element offsets."""
+    p = torch.cat([t.permute(2, 0, 1, 3) for t in x], -1)
+    return [t.permute(1, 2, 0, 3) for t in torch.split(p, [t.shape[3] for t in x], -1)]
+
+
+@pytest.mark.parametrize('E,M', [(16, 16), (9, 14), (32, 32), (20, 31), (48, 48), (64, 64), (50, 33), (32, 97), (96, 16),
+                                 (70, 32), (96, 64), (128, 16), (128, 20), (101, 64), (128, 128)])
+@pytest.mark.parametrize('L', [1, 17, 130])
+def test_forward_meets_the_oracle(fwp, E, M, L):
+    B, H = 2, 3
+    q, k, v, b, _ = util.delta_inputs(7, B, H, L, E, M)
+    W0 = torch.randn(B, H, E, M, generator=util.gen(8)) * 0.1
+    for rule in ('delta', 'sum'):
+        x = [q, k, v] + ([b] if rule == 'delta' else [])
+        S = W0.double().clone()
+        ref = torch.empty(B, H, L, M, dtype=torch.float64)
+        for t in range(L):
+            kt, u = k[:, :, t].double(), v[:, :, t].double()
+            if rule == 'delta':
+                u = b[:, :, t].double() * (u - torch.einsum('bhem,bhe->bhm', S, kt))
+            S = S + kt[..., None] * u[:, :, None]
+            ref[:, :, t] = torch.einsum('bhem,bhe->bhm', S, q[:, :, t].double())
+        dev = [t.to(DEV) for t in x]
+        for streams in (dev, sliced(dev)):
+            for helpers in (2, 4):
+                y, W, kernel = run(fwp, rule, streams, W0.to(DEV), {'delta.wy': 1, 'delta.wy.helpers': helpers})
+                assert kernel.startswith('delta_fwd_wy')
+                # fp32 accuracy: three-part products keep every bit of the operands
+                assert util.max_abs(y, ref) <= 2e-6 * max(1., ref.abs().max().item()), (rule, helpers)
+                assert util.max_abs(W, S) <= 2e-6 * max(1., S.abs().max().item()), (rule, helpers)
+
+
+@pytest.mark.parametrize('B,H,L,d', [(300, 1, 70, 16), (40, 8, 33, 32), (150, 2, 50, 64)])
+def test_forward_with_more_sequences_than_the_gpu_holds(fwp, B, H, L, d):
+    q, k, v, b, _ = (t.to(DEV) for t in util.delta_inputs(9, B, H, L, d))
+    W0 = torch.randn(B, H, d, d, generator=util.gen(10)).to(DEV) * 0.1
+    y, W, _ = run(fwp, 'delta', [q, k, v, b], W0, {'delta.wy': 0})
+    for helpers in (0, 2, 4):
+        y2, W2, _ = run(fwp, 'delta', [q, k, v, b], W0, {'delta.wy': 1, 'delta.wy.helpers': helpers})
+        assert util.max_abs(y, y2) <= 5e-6 and util.max_abs(W, W2) <= 5e-6
+    from recurrent_fwp_b200 import _lib
+    assert _lib.device_fault() == 0
