@@ -93,7 +93,8 @@ unsigned long long fwp_launch_count(void);
  * "delta.pipe64" (1 / 2 / 0: chunkwise bf16 kernels with a preparing warp one chunk ahead in both directions,
  * in the forward only, or not at all),
  * "delta.wy" (-1 automatic / 1 / 0: the chunkwise split-product plan wherever it is the faster one, wherever it has an
- * instance, or never), "delta.wy.helpers" (0 automatic / 4 / 2: preparing warps per sequence of that plan).  Returns 0 if accepted, FWP_ERR_UNSUPPORTED for an unknown key. */
+ * instance, or never), "delta.wy.helpers" (0 automatic / 4 / 2: preparing warps per sequence of that plan),
+ * "delta_bwd.phases" (-1 automatic / 1 / 0: the three-launch backward over scratch, see below).  Returns 0 if accepted, FWP_ERR_UNSUPPORTED for an unknown key. */
 int fwp_tune(const char* key, int value);
 /* Name of the kernel this host thread launched last through the library ("" before the
  * first launch): lets a benchmark label its numbers with the plan the dispatch picked. */
@@ -121,6 +122,20 @@ int fwp_fast_weight_backward(int N, int H, int L, int E, int M,
                              const fwp_tensor* fw_mem,
                              const fwp_tensor* grad_Q, const fwp_tensor* grad_K,
                              const fwp_tensor* grad_V, const fwp_tensor* grad_beta,
+                             int io_dtype, void* stream, int device);
+
+/* The same backward for callers that can lend device memory: with at least fwp_fast_weight_backward_scratch_floats(...)
+ * floats of it (16-byte aligned, contents undefined before and after), shapes that gain from it run as three launches that
+ * work on all chunks of all sequences at once.  0 floats, or scratch == NULL: the plain backward.  The pointer is not kept.
+ * The answer depends on the sizes and the execution-plan switches only. */
+int64_t fwp_fast_weight_backward_scratch_floats(int N, int H, int L, int E, int M, int io_dtype);
+int fwp_fast_weight_backward_with_scratch(int N, int H, int L, int E, int M,
+                             const fwp_tensor* Q, const fwp_tensor* K, const fwp_tensor* V,
+                             const fwp_tensor* beta, const fwp_tensor* v_old, const fwp_tensor* grad_out,
+                             const fwp_tensor* fw_mem,
+                             const fwp_tensor* grad_Q, const fwp_tensor* grad_K,
+                             const fwp_tensor* grad_V, const fwp_tensor* grad_beta,
+                             float* scratch, int64_t scratch_floats,
                              int io_dtype, void* stream, int device);
 
 /* The delta-rule kernels move contiguous chunks with bulk asynchronous copies (in the tcgen05 plan also TMA

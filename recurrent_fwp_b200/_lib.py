@@ -49,6 +49,7 @@ _i, _vp, _i64 = ctypes.c_int, ctypes.c_void_p, ctypes.c_int64
 SIGNATURES = {
     'fwp_fast_weight_forward': [_i] * 5 + [_T] * 8 + [_i, _vp, _i],
     'fwp_fast_weight_backward': [_i] * 5 + [_T] * 12 + [_i, _vp, _i],
+    'fwp_fast_weight_backward_with_scratch': [_i] * 5 + [_T] * 11 + [ctypes.POINTER(ctypes.c_float), _i64, _i, _vp, _i],
     'fwp_causal_dot_product': [_i] * 5 + [_T] * 5 + [_i, _vp, _i],
     'fwp_causal_dot_backward': [_i] * 5 + [_T] * 7 + [_i, _vp, _i],
     'fwp_rec_update_fwm_tanh_forward': [_i] * 4 + [_T] * 16 + [_i, _vp, _i],
@@ -68,7 +69,7 @@ SIGNATURES = {
 }
 OTHER_SYMBOLS = ['fwp_status_string', 'fwp_last_cuda_error', 'fwp_version', 'fwp_max_head_dim',
                  'fwp_launch_count', 'fwp_tune', 'fwp_rec_update_fwm_tanh_scratch_floats', 'fwp_delta_device_fault',
-                 'fwp_last_kernel']
+                 'fwp_last_kernel', 'fwp_fast_weight_backward_scratch_floats']
 
 for _name, _args in SIGNATURES.items():
     _f = getattr(lib, _name)
@@ -80,6 +81,8 @@ lib.fwp_launch_count.restype = ctypes.c_ulonglong
 lib.fwp_tune.argtypes = [ctypes.c_char_p, _i]
 lib.fwp_rec_update_fwm_tanh_scratch_floats.argtypes = [_i, _i, _i]
 lib.fwp_rec_update_fwm_tanh_scratch_floats.restype = _i64
+lib.fwp_fast_weight_backward_scratch_floats.argtypes = [_i] * 6
+lib.fwp_fast_weight_backward_scratch_floats.restype = _i64
 lib.fwp_last_kernel.restype = ctypes.c_char_p
 
 

@@ -162,6 +162,18 @@ std::shared_ptr<NodeT> make_node(const std::array<const Tensor*, K>& in, const D
 }
 
 // ------------------------------------------------------------------ delta rule
+// the backward with the scratch memory it asks for
+void delta_backward(const Dims& d, const Tensor& Q, const Tensor& K, const Tensor& V, const Tensor& beta, const Tensor& v_old, const Tensor& gy,
+                    const Tensor& W, const Tensor& gQ, const Tensor& gK, const Tensor& gV, const Tensor& gb) {
+    const int64_t need = fwp_fast_weight_backward_scratch_floats(d.N, d.H, d.L, d.E, d.M, dtype_code(Q));
+    Tensor scratch;
+    if (need > 0) scratch = empty({need}, at::kFloat, Q);
+    check_delta(fwp_fast_weight_backward_with_scratch(d.N, d.H, d.L, d.E, d.M, Desc(Q), Desc(K), Desc(V), Desc(beta), Desc(v_old), Desc(gy),
+                                                      Desc(W), Desc(gQ), Desc(gK), Desc(gV), Desc(gb),
+                                                      need > 0 ? scratch.data_ptr<float>() : nullptr, need, dtype_code(Q), stream_of(Q),
+                                                      Q.device().index()), "fast_weight_backward");
+}
+
 struct DeltaNode final : public OpNode {
     std::string name() const override { return "DeltaFastWeightBackward"; }
     variable_list apply(variable_list&& g) override {
@@ -171,9 +183,7 @@ struct DeltaNode final : public OpNode {
         const Tensor &Q = t[0], &K = t[1], &V = t[2], &beta = t[3], &W = t[4];
         const Tensor gy = incoming(g[0], Q, {d.N, d.H, d.L, d.M});
         Tensor gQ = like_stream(d.E, Q), gK = like_stream(d.E, Q), gV = like_stream(d.M, Q), gb = like_stream(1, Q);
-        check_delta(fwp_fast_weight_backward(d.N, d.H, d.L, d.E, d.M, Desc(Q), Desc(K), Desc(V), Desc(beta), Desc(own[0]),
-                                             Desc(Tensor()), Desc(gy), Desc(W), Desc(gQ), Desc(gK), Desc(gV), Desc(gb),
-                                             dtype_code(Q), stream_of(Q), Q.device().index()), "fast_weight_backward");
+        delta_backward(d, Q, K, V, beta, own[0], gy, W, gQ, gK, gV, gb);
         return {gQ, gK, gV, gb, Tensor()};
     }
 };
@@ -225,9 +235,7 @@ struct DeltaLayerNode final : public OpNode {
         Tensor gy = empty(d, d.M, x), gq = empty(d, d.E, x), gk = empty(d, d.E, x), gv = empty(d, d.M, x), gb = empty(d, 1, x);
         check(fwp_delta_layer_transpose(d.L, d.N, d.H, d.M, gout.data_ptr<float>(), gy.data_ptr<float>(), (float)scale, 0, st, dev),
               "delta_layer_transpose");
-        check_delta(fwp_fast_weight_backward(d.N, d.H, d.L, d.E, d.M, Desc(q), Desc(k), Desc(v), Desc(beta), Desc(v_old),
-                                             Desc(Tensor()), Desc(gy), Desc(W), Desc(gq), Desc(gk), Desc(gv), Desc(gb),
-                                             FWP_F32, st, dev), "fast_weight_backward");
+        delta_backward(d, q, k, v, beta, v_old, gy, W, gq, gk, gv, gb);
         Tensor gx = empty({d.L, d.N, d.H, 3 * d.E + 1}, at::kFloat, x);
         check(fwp_delta_layer_prologue_backward(d.L, d.N, d.H, d.E, x.data_ptr<float>(), gq.data_ptr<float>(), gk.data_ptr<float>(),
                                                 gv.data_ptr<float>(), gb.data_ptr<float>(), gx.data_ptr<float>(), st, dev),

@@ -68,6 +68,7 @@ enum TuneKey {
     T_STEP_SPREAD,          // "step.spread": 1 the per-step forward packs fewer sequences into a CTA while that puts CTAs on more SMs, 0 always four warps per CTA
     T_DELTA_WY,             // "delta.wy": -1 automatic, 1 / 0 the chunkwise split-product plan (fwp_delta_wy.cuh) wherever it has an instance, or never
     T_DELTA_WY_HELPERS,     // "delta.wy.helpers": preparing warps per sequence of that plan (2 or 4), 0 automatic
+    T_DELTA_PHASES,         // "delta_bwd.phases": -1 automatic, 1 / 0 the three-launch backward wherever it has an instance and scratch, or never
     T_COUNT
 };
 int tune_get(TuneKey key, int fallback);

@@ -571,6 +571,26 @@ static int dispatch_fwd(const DeltaFwdParams& p, int nseq, cudaStream_t st) {
     return FWP_ERR_UNSUPPORTED;
 }
 
+// Where the three-launch backward is the faster one, from measurements on B200 (fp32, 256 steps, us, one-launch kernel ->
+// three launches):
+//   d = 16: 16 sequences 37 -> 13, 128 37 -> 25, 256 38 -> 37, 512 38 -> 65; with rows of 12 128 65 -> 27, 256 66 -> 52, 512 67 -> 76
+//   d = 32: 128 63 -> 48, 256 64 -> 92; with rows of 20 128 139 -> 51, 512 283 -> 174
+//   d = 64: 64 114 -> 76, 128 116 -> 125; with rows of 55 512 1789 -> 557;  d = 48: 512 1128 -> 354
+//   E, M = 96, 32: 128 1152 -> 113, 1024 2783 -> 1233
+// The four-step blocked kernels are at their best with rows of exactly 16, 32 or 64 elements and a sequence for every SM;
+// short rows cost them a division per copied piece, and states above 64 have no register-resident kernel at all.
+template <typename T>
+static bool bwd_phases_pay(const DeltaBwdParams& p, int nseq) {
+    if (sizeof(T) != 4 || tune_get(T_DELTA_BLOCKED, -1) != -1) return false;
+    const int force = tune_get(T_DELTA_PHASES, -1);
+    if (force != -1) return force == 1;
+    const int d = p.E > p.M ? p.E : p.M;
+    if (d > 64) return p.L > 4;
+    if (p.L <= kShortSeq) return false;
+    const bool full = p.E == p.M && (d == 16 || d == 32 || d == 64);
+    if (d <= 16) return nseq <= (full ? 1 : 2) * sm_count();
+    return !full || nseq <= (d == 64 ? sm_count() / 2 : sm_count());
+}
 template <typename T>
 static int dispatch_bwd(const DeltaBwdParams& p0, int nseq, cudaStream_t st) {
     DeltaBwdParams p = p0;
@@ -674,7 +694,7 @@ static int fast_weight_backward_impl(int N, int H, int L, int E, int M,
                                         const fwp_tensor* fw_mem,
                                         const fwp_tensor* grad_Q, const fwp_tensor* grad_K,
                                         const fwp_tensor* grad_V, const fwp_tensor* grad_beta,
-                                        int io_dtype, void* stream, int device) {
+                                        float* scratch, int64_t scratch_floats, int io_dtype, void* stream, int device) {
     (void)v_insert;
     if (int rc = check_common(N, H, L, E, M, io_dtype)) return rc;
     const int eb = io_dtype == FWP_F32 ? 4 : 2;
@@ -693,6 +713,11 @@ static int fast_weight_backward_impl(int N, int H, int L, int E, int M,
     p.W = (float*)fw_mem->data; p.wN = fw_mem->stride[0]; p.wH = fw_mem->stride[1]; p.wE = fw_mem->stride[2];
     p.H = H; p.L = L; p.E = E; p.M = M; p.NH = N * H;
     cudaStream_t st = (cudaStream_t)stream;
+    if (scratch && io_dtype == FWP_F32 && bwd_phases_pay<float>(p, N * H)) {
+        if (reinterpret_cast<uintptr_t>(scratch) & 15) return FWP_ERR_SCRATCH;
+        const int64_t need = bwd_phases<float>(false, p, N * H, nullptr, st);
+        if (need > 0) return scratch_floats < need ? FWP_ERR_SCRATCH : (int)bwd_phases<float>(true, p, N * H, scratch, st);
+    }
     if (io_dtype == FWP_F32) return dispatch_bwd<float>(p, N * H, st);
     return dispatch_bwd<__nv_bfloat16>(p, N * H, st);
 }
@@ -706,7 +731,27 @@ FWP_API int fwp_fast_weight_backward(int N, int H, int L, int E, int M,
                                         const fwp_tensor* grad_V, const fwp_tensor* grad_beta,
                                         int io_dtype, void* stream, int device) {
     return fast_weight_backward_impl(N, H, L, E, M, Q, K, V, beta, v_old, v_insert, grad_out, fw_mem, grad_Q, grad_K, grad_V,
-                                     grad_beta, io_dtype, stream, device);
+                                     grad_beta, nullptr, 0, io_dtype, stream, device);
+}
+
+FWP_API int64_t fwp_fast_weight_backward_scratch_floats(int N, int H, int L, int E, int M, int io_dtype) {
+    if (check_common(N, H, L, E, M, io_dtype) || io_dtype != FWP_F32) return 0;
+    DeltaBwdParams p;
+    p.H = H; p.L = L; p.E = E; p.M = M; p.NH = N * H;
+    if (!bwd_phases_pay<float>(p, N * H)) return 0;
+    const int64_t need = bwd_phases<float>(false, p, N * H, nullptr, nullptr);
+    return need > 0 ? need : 0;
+}
+
+FWP_API int fwp_fast_weight_backward_with_scratch(int N, int H, int L, int E, int M,
+                                        const fwp_tensor* Q, const fwp_tensor* K, const fwp_tensor* V,
+                                        const fwp_tensor* beta, const fwp_tensor* v_old,
+                                        const fwp_tensor* grad_out, const fwp_tensor* fw_mem,
+                                        const fwp_tensor* grad_Q, const fwp_tensor* grad_K,
+                                        const fwp_tensor* grad_V, const fwp_tensor* grad_beta,
+                                        float* scratch, int64_t scratch_floats, int io_dtype, void* stream, int device) {
+    return fast_weight_backward_impl(N, H, L, E, M, Q, K, V, beta, v_old, nullptr, grad_out, fw_mem, grad_Q, grad_K, grad_V,
+                                     grad_beta, scratch, scratch_floats, io_dtype, stream, device);
 }
 
 FWP_API int fwp_causal_dot_product(int N, int H, int L, int E, int M,

@@ -71,6 +71,9 @@ int launch_bwd_chunk_bf16(const DeltaBwdParams& p, int nseq, cudaStream_t st);
 // chunkwise plan on split fp32 products (fwp_delta_wy.cuh); -1 when the sizes have no instance
 int wy_fault_read_clear();
 template <typename T, bool SUM> int launch_fwd_wy(const DeltaFwdParams& p, int nseq, cudaStream_t st);
+// three-launch backward over a workspace (fwp_delta_phases.cuh): floats of scratch it needs (run = false) or the launches; -1
+// when the sizes have no instance
+template <typename T> int64_t bwd_phases(bool run, const DeltaBwdParams& p, int nseq, float* scratch, cudaStream_t st);
 int tc_fault_read_clear();
 int launch_wait_probe(int polls, cudaStream_t st);
 

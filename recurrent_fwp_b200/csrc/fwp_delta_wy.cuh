@@ -18,15 +18,10 @@
 // The two sides meet at two mbarriers per buffer.  With many sequences of a large state the copies of S would fill
 // shared memory, so there (OUT = false) the chain warps form the outputs themselves.
 #pragma once
-#include "fwp_delta_params.cuh"
-#include "fwp_split3.cuh"
+#include "fwp_wy_common.cuh"
 
 namespace fwp {
 namespace wy {
-
-using namespace s3;
-constexpr int C = 16;                   // steps per chunk
-constexpr int PC = C + 8;               // pitch of the 16 x 16 operand tiles
 
 static __device__ int g_wy_fault;       // a bounded wait ran out (read by fwp_delta_device_fault)
 
@@ -41,8 +36,6 @@ __device__ __forceinline__ void warp_arrive(unsigned long long* bar, int lane) {
 __device__ __forceinline__ void wait(unsigned long long* bar, unsigned parity) {
     if (!mbar_wait_bounded(bar, parity)) atomicExch(&g_wy_fault, 1);
 }
-
-template <typename T> __host__ __device__ constexpr int stream_parts() { return sizeof(T) == 4 ? 3 : 1; }
 
 // One stream of one sequence as a warp copies it, sixteen rows at a time, into an fp32 tile of pitch P floats.  fp32 rows
 // go by cp.async (16-byte pieces where the rows allow it, else 4-byte: the layers' value slices start at odd offsets);
@@ -147,129 +140,6 @@ __device__ __forceinline__ void put_block_t(const float (&x)[2][4], float* at) {
         for (int i = 0; i < 4; i++) at[block_t_at<P>(n, i)] = x[n][i];
 }
 
-// 16 x 16 block of rows [0, nt) of a stream straight from global memory as C fragments: element (row, col) =
-// p[row * sL + col].  `at` = p + g * sL + 2t.
-template <typename T>
-__device__ __forceinline__ void load_block(float (&x)[2][4], const T* at, long long sL, int nt, int width, bool pairs, int g, int t) {
-    if (pairs && nt == C) {
-#pragma unroll
-        for (int hi = 0; hi < 2; hi++)
-#pragma unroll
-            for (int n = 0; n < 2; n++) {
-                const T* q = at + (hi ? 8 * sL : 0) + 8 * n;
-                if constexpr (sizeof(T) == 4) {
-                    const float2 v = *reinterpret_cast<const float2*>(q);
-                    x[n][2 * hi] = v.x;
-                    x[n][2 * hi + 1] = v.y;
-                } else {
-                    const unsigned v = *reinterpret_cast<const unsigned*>(q);
-                    x[n][2 * hi] = __uint_as_float(v << 16);
-                    x[n][2 * hi + 1] = __uint_as_float(v & 0xffff0000u);
-                }
-            }
-    } else {
-#pragma unroll
-        for (int hi = 0; hi < 2; hi++)
-#pragma unroll
-            for (int n = 0; n < 2; n++)
-#pragma unroll
-                for (int i = 0; i < 2; i++) {
-                    const int r = g + 8 * hi, c = 8 * n + 2 * t + i;
-                    x[n][2 * hi + i] = r < nt && c < width ? to_f32(at[8 * hi * sL + 8 * n + i]) : 0.f;
-                }
-    }
-}
-// the same block transposed: element (m, step) = p[step * sL + m].  `at` = p + 2t * sL + g: the four rows a lane touches
-// hold 8 consecutive elements each of 8 lanes, whole sectors at any alignment.
-template <typename T>
-__device__ __forceinline__ void load_block_t(float (&x)[2][4], const T* at, long long sL, int nt, int width, int g, int t) {
-    const bool whole = nt == C && width >= 16;
-#pragma unroll
-    for (int n = 0; n < 2; n++)
-#pragma unroll
-        for (int i = 0; i < 2; i++) {
-            const T* q = at + (8 * n + i) * sL;
-            if (whole) {
-                x[n][i] = to_f32(q[0]);
-                x[n][2 + i] = to_f32(q[8]);
-            } else {
-                const bool row = 8 * n + 2 * t + i < nt;
-                x[n][i] = row && g < width ? to_f32(q[0]) : 0.f;
-                x[n][2 + i] = row && g + 8 < width ? to_f32(q[8]) : 0.f;
-            }
-        }
-}
-template <typename T>
-__device__ __forceinline__ void store_block_t(const float (&x)[2][4], T* at, long long sL, int nt, int width, int g, int t) {
-    if (nt == C && width >= 16) {
-#pragma unroll
-        for (int n = 0; n < 2; n++)
-#pragma unroll
-            for (int i = 0; i < 2; i++) {
-                T* q = at + (8 * n + i) * sL;
-                q[0] = from_f32<T>(x[n][i]);
-                q[8] = from_f32<T>(x[n][2 + i]);
-            }
-    } else {
-#pragma unroll
-        for (int n = 0; n < 2; n++)
-#pragma unroll
-            for (int i = 0; i < 2; i++) {
-                if (8 * n + 2 * t + i >= nt) continue;
-                T* q = at + (8 * n + i) * sL;
-                if (g < width) q[0] = from_f32<T>(x[n][i]);
-                if (g + 8 < width) q[8] = from_f32<T>(x[n][2 + i]);
-            }
-    }
-}
-
-// T = (I + A)^-1, A strictly lower triangular in rows of pitch PA floats; lane c (mod 16) finds column c and leaves it
-// as row c of the operand tile `Tt` (T^T), its two copies sharing the splitting.
-template <int PA>
-__device__ __forceinline__ void invert_lower(const float* A, __nv_bfloat16* Tt, int lane) {
-    const int c = lane & 15;
-    float x[C];
-    f2 xp[C / 2];
-#pragma unroll
-    for (int p = 0; p < C / 2; p++) xp[p] = 0ull;
-#pragma unroll
-    for (int i = 0; i < C; i++) {
-        f2 acc = 0ull;
-#pragma unroll
-        for (int q = 0; 4 * q < i; q++) {
-            const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(A + i * PA + 4 * q);
-            acc = ffma2(a.x, xp[2 * q], acc);
-            if (4 * q + 2 < i) acc = ffma2(a.y, xp[2 * q + 1], acc);
-        }
-        x[i] = (i == c ? 1.f : 0.f) - f2_hsum(acc);
-        xp[i >> 1] = (i & 1) ? f2_pack(x[i - 1], x[i]) : f2_pack(x[i], 0.f);
-    }
-    const bool upper = lane >= 16;
-    unsigned o[3][4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        unsigned s[3];
-        split<3>(upper ? x[2 * j + 8] : x[2 * j], upper ? x[2 * j + 9] : x[2 * j + 1], s);
-#pragma unroll
-        for (int i = 0; i < 3; i++) o[i][j] = s[i];
-    }
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-        *reinterpret_cast<uint4*>(Tt + (i * C + c) * PC + (upper ? 8 : 0)) = make_uint4(o[i][0], o[i][1], o[i][2], o[i][3]);
-}
-
-__device__ __forceinline__ void add_to(float (&x)[2][4], const float (&d)[2][4]) {
-#pragma unroll
-    for (int i = 0; i < 8; i++) x[i >> 2][i & 3] += d[i >> 2][i & 3];
-}
-// x += A B, the product formed from zero
-template <Right R, int NA, int NB>
-__device__ __forceinline__ void add_product(float (&x)[2][4], const Frag<NA>& a, const Frag<NB>& b) {
-    float d[2][4] = {};
-    product<R>(d, a, b);
-    add_to(x, d);
-}
-
 // ---------------------------------------------------------------------------------- forward, few sequences
 template <int E, int M, int NP>
 struct FewBuf {
@@ -368,8 +238,7 @@ __global__ void __launch_bounds__((M / 16 + NB) * 32) delta_fwd_wy_few_kernel(co
                 if constexpr (!SUM) {
                     Frag<3> r;
                     load_rows(r, aX + 32 * k, kPart);
-                    if (k == 0) product<BY_ROWS>(xs, s, r);
-                    else add_product<BY_ROWS>(xs, s, r);
+                    sum_product<BY_ROWS>(k, xs, s, r);
                 }
 #pragma unroll
                 for (int i = 0; i < 3; i++) buf.s[warp][k][i][lane] = make_uint4(s.r[i][0], s.r[i][1], s.r[i][2], s.r[i][3]);
@@ -449,8 +318,8 @@ __global__ void __launch_bounds__((M / 16 + NB) * 32) delta_fwd_wy_few_kernel(co
             tile_block<PR>(x, &buf.qraw[g][2 * t + 16 * k]);
             from_c(fq, x[0], x[1]);
             store(aQ + 32 * k, kPart, fq);
-            if (!SUM) add_product<BY_ROWS>(kk, fk, fk);
-            add_product<BY_ROWS>(qk, fq, fk);
+            if (!SUM) sum_product<BY_ROWS>(k, kk, fk, fk);
+            sum_product<BY_ROWS>(k, qk, fq, fk);
         }
 #pragma unroll
         for (int nn = 0; nn < 2; nn++) {
@@ -618,10 +487,10 @@ __global__ void __launch_bounds__((M / 16 + NB) * 32, CTAS) delta_fwd_wy_kernel(
                 from_c(s, S[2 * k], S[2 * k + 1]);
                 if (!SUM) {
                     load_rows(r, aK + 32 * k, kPart);
-                    add_product<BY_ROWS>(u, s, r);
+                    sum_product<BY_ROWS>(k, u, s, r);
                 }
                 load_rows(r, aQ + 32 * k, kPart);
-                add_product<BY_ROWS>(y, s, r);
+                sum_product<BY_ROWS>(k, y, s, r);
             }
             if constexpr (SUM) {
 #pragma unroll
@@ -720,8 +589,8 @@ __global__ void __launch_bounds__((M / 16 + NB) * 32, CTAS) delta_fwd_wy_kernel(
             from_c(fq, qf[f][0], qf[f][1]);
             store(aK + 32 * k, kPart, fk);
             store(aQ + 32 * k, kPart, fq);
-            if (!SUM) add_product<BY_ROWS>(kk, fk, fk);
-            add_product<BY_ROWS>(qk, fq, fk);
+            if (!SUM) sum_product<BY_ROWS>(k, kk, fk, fk);
+            sum_product<BY_ROWS>(k, qk, fq, fk);
         }
         __syncwarp();
 #pragma unroll

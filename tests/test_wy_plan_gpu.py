@@ -67,3 +67,58 @@ def test_forward_with_more_sequences_than_the_gpu_holds(fwp, B, H, L, d):
         assert util.max_abs(y, y2) <= 5e-6 and util.max_abs(W, W2) <= 5e-6
     from recurrent_fwp_b200 import _lib
     assert _lib.device_fault() == 0
+
+
+@pytest.mark.parametrize('E,M', [(16, 16), (9, 14), (32, 32), (20, 31), (48, 48), (64, 64), (50, 33), (32, 97), (96, 16),
+                                 (70, 32), (96, 64), (128, 16), (128, 20), (101, 64), (128, 128)])
+@pytest.mark.parametrize('L', [5, 17, 130])
+def test_three_launch_backward_meets_the_oracle(fwp, E, M, L):
+    """csrc/fwp_delta_phases.cuh against autograd through the recurrence in fp64, packed and layer-sliced streams."""
+    from recurrent_fwp_b200 import _lib
+    B, H = 2, 3
+    q, k, v, b, gy = util.delta_inputs(17, B, H, L, E, M)
+    W0 = torch.randn(B, H, E, M, generator=util.gen(18)) * 0.1
+    leaves = [t.double().requires_grad_() for t in (q, k, v, b)]
+    S, ys = W0.double(), []
+    for t in range(L):
+        kt = leaves[1][:, :, t]
+        u = leaves[3][:, :, t] * (leaves[2][:, :, t] - torch.einsum('bhem,bhe->bhm', S, kt))
+        S = S + kt[..., None] * u[:, :, None]
+        ys.append(torch.einsum('bhem,bhe->bhm', S, leaves[0][:, :, t]))
+    torch.stack(ys, 2).backward(gy.double())
+    dev = [t.to(DEV) for t in (q, k, v, b)]
+    seen = []
+    try:
+        _lib.tune('delta_bwd.phases', 1)
+        for streams in (dev, sliced(dev)):
+            x = [t.detach().requires_grad_() for t in streams]
+            W = W0.to(DEV)
+            y = fwp.fast_weight_delta(*x, W)
+            x[0].register_hook(lambda g: seen.append(_lib.last_kernel()))
+            y.backward(gy.to(DEV))
+            for got, ref in zip(x, leaves):
+                assert util.max_abs(got.grad, ref.grad) <= 3e-6 * max(1., ref.grad.abs().max().item())
+            assert util.max_abs(W, W0) <= 2e-6
+    finally:
+        _lib.tune('delta_bwd.phases', -1)
+    assert seen == ['delta_bwd_finish_kernel'] * 2
+
+
+def test_three_launch_backward_in_segments(fwp):
+    """More chunks than one segment's workspace holds: G and the rewound state cross the segment borders."""
+    from recurrent_fwp_b200 import _lib
+    B, H, L, d = 160, 8, 100, 64
+    q, k, v, b, gy = (t.to(DEV) for t in util.delta_inputs(23, B, H, L, d))
+    W0 = torch.randn(B, H, d, d, generator=util.gen(24)).to(DEV) * 0.1
+    res = {}
+    try:
+        for plan in (0, 1):
+            _lib.tune('delta_bwd.phases', plan)
+            x = [t.clone().requires_grad_() for t in (q, k, v, b)]
+            W = W0.clone()
+            fwp.fast_weight_delta(*x, W).backward(gy)
+            res[plan] = [t.grad for t in x] + [W]
+    finally:
+        _lib.tune('delta_bwd.phases', -1)
+    for a, c in zip(res[0], res[1]):
+        assert util.max_abs(a, c) <= 5e-6 * max(1., a.abs().max().item())
