@@ -80,7 +80,7 @@ unsigned long long fwp_launch_count(void);
  * "delta.tc64" (-1 / 1 / 0: tcgen05 forward of that plan when the call has no more sequences than the device has SMs
  * and at least 128 steps, always, or never), "<op>.<D>.split", "delta_bwd.bulk",
  * "delta_bwd.16.chunk", "rec_fwd.32.warp" (1 / 0: short-chain forward of the recurrent delta net),
- * "rnn_bwd.32.roles" (1 / 2 / 0: chain-warp + trailing-warp backward of the delta RNN, 16 or 8 steps per chunk, or off),
+ * "rnn_bwd.32.roles" (1 / 2 / 0: chain-warp + trailing-warps backward of the delta RNN, 8 or 4 steps per chunk, or off),
  * "lstm_bwd.32.roles" (1 / 0: chain-warp + per-gate trailing-warp backward of the delta LSTM),
  * "lstm_fwd.32.gates" (1 / 0: one-warp-per-gate forward of the delta LSTM),
  * "rec_bwd.32.roles" (1 / 0: chain-warp + trailing-warp backward of the recurrent delta net),
@@ -104,7 +104,7 @@ const char* fwp_last_kernel(void);
  * replaces fast_weight_forward(Q,K,V,beta,v_old,v_insert,kv,out),
  *   algorithmic/fast_weight/fast_weight_cuda.cu:182-240
  * Q,K [N,H,L,E]; V,v_old,v_insert,out [N,H,L,M]; beta [N,H,L,1]; kv [N,H,E,M].
- * v_insert may have data == NULL (the backward recomputes it). */
+ * v_insert may have data == NULL (the backward recomputes it), and so may v_old when no backward follows. */
 int fwp_fast_weight_forward(int N, int H, int L, int E, int M,
                             const fwp_tensor* Q, const fwp_tensor* K, const fwp_tensor* V,
                             const fwp_tensor* beta, const fwp_tensor* v_old,

@@ -203,12 +203,14 @@ PyObject* fast_weight_delta(PyObject*, PyObject* const* args, Py_ssize_t n) {
     Tensor out;
     {
         pybind11::gil_scoped_release no_gil;
+        const bool grad = needs_grad(in);
         out = empty({d.N, d.H, d.L, d.M}, ty, Q);
-        Tensor v_old = empty(d, d.M, Q);
+        Tensor v_old;
+        if (grad) v_old = empty(d, d.M, Q);
         check_delta(fwp_fast_weight_forward(d.N, d.H, d.L, d.E, d.M, Desc(Q), Desc(K), Desc(V), Desc(beta), Desc(v_old),
                                             Desc(Tensor()), Desc(W), Desc(out), dtype_code(Q), stream_of(Q), dev.index()),
                     "fast_weight_forward");
-        if (needs_grad(in)) {
+        if (grad) {
             auto node = make_node<DeltaNode>(in, d);
             for (auto* t : in) node->save(*t);
             node->own = {v_old};
@@ -260,7 +262,9 @@ PyObject* delta_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
         pybind11::gil_scoped_release no_gil;
         void* st = stream_of(x);
         const int dev = x.device().index();
-        Tensor q = empty(d, D, x), k = empty(d, D, x), v = empty(d, D, x), beta = empty(d, 1, x), y = empty(d, D, x), v_old = empty(d, D, x);
+        Tensor q = empty(d, D, x), k = empty(d, D, x), v = empty(d, D, x), beta = empty(d, 1, x), y = empty(d, D, x), v_old;
+        const bool grad = needs_grad(in);
+        if (grad) v_old = empty(d, D, x);
         check(fwp_delta_layer_prologue_forward(d.L, d.N, d.H, D, x.data_ptr<float>(), q.data_ptr<float>(), k.data_ptr<float>(),
                                                v.data_ptr<float>(), beta.data_ptr<float>(), st, dev), "delta_layer_prologue_forward");
         check_delta(fwp_fast_weight_forward(d.N, d.H, d.L, D, D, Desc(q), Desc(k), Desc(v), Desc(beta), Desc(v_old), Desc(Tensor()),
@@ -268,7 +272,7 @@ PyObject* delta_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
         out = empty({d.L, d.N, d.H * D}, at::kFloat, x);
         check(fwp_delta_layer_transpose(d.L, d.N, d.H, D, y.data_ptr<float>(), out.data_ptr<float>(), (float)scale, 1, st, dev),
               "delta_layer_transpose");
-        if (needs_grad(in)) {
+        if (grad) {
             auto node = make_node<DeltaLayerNode>(in, d);
             node->save(x);
             node->save(W);

@@ -93,7 +93,7 @@ delta_fwd_step_kernel(const DeltaFwdParams p) {
             if (col_ok && g.s == 0) {
                 put<T>(p.out, n, h, t0 + t, g.idx, y);
                 if constexpr (!SUM) {
-                    put<float>(p.v_old, n, h, t0 + t, g.idx, vo);
+                    if (p.v_old.p) put<float>(p.v_old, n, h, t0 + t, g.idx, vo);
                     if (p.v_ins.p) put<float>(p.v_ins, n, h, t0 + t, g.idx, u);
                 }
             }
@@ -663,7 +663,7 @@ static int fast_weight_forward_impl(int N, int H, int L, int E, int M,
     const int eb = io_dtype == FWP_F32 ? 4 : 2;
     int rc;
     if ((rc = check_tensor(Q, eb, true)) || (rc = check_tensor(K, eb, true)) || (rc = check_tensor(V, eb, true)) ||
-        (rc = check_tensor(beta, eb, true)) || (rc = check_tensor(v_old, 4, true)) ||
+        (rc = check_tensor(beta, eb, true)) || (rc = check_tensor(v_old, 4, false)) ||
         (rc = check_tensor(v_insert, 4, false)) || (rc = check_tensor(kv, 4, true)) ||
         (rc = check_tensor(out, eb, true)))
         return rc;

@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(slots_for(D * SPLIT) * (D * SPLIT + 32)) delta
             const int t0 = c * TC, nt = min(TC, p.L - t0);
             flush_rows<D, 32, T, TC>(o, p.out, n, h, t0, nt, p.M, ptid);
             if constexpr (!SUM) {
-                flush_rows<D, 32, float, TC>(o + TC * D, p.v_old, n, h, t0, nt, p.M, ptid);
+                if (p.v_old.p) flush_rows<D, 32, float, TC>(o + TC * D, p.v_old, n, h, t0, nt, p.M, ptid);
                 if (p.v_ins.p) flush_rows<D, 32, float, TC>(o + 2 * TC * D, p.v_ins, n, h, t0, nt, p.M, ptid);
             }
         };

@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(cb::NT, 4) delta_fwd_chunk_bf16_inv_kernel(con
     const bf16* vb = reinterpret_cast<const bf16*>(p.v.p) + n * p.v.sN + h * p.v.sH;
     const bf16* bb = reinterpret_cast<const bf16*>(p.beta.p) + n * p.beta.sN + h * p.beta.sH;
     bf16* yb = reinterpret_cast<bf16*>(p.out.p) + n * p.out.sN + h * p.out.sH;
-    float* vob = reinterpret_cast<float*>(p.v_old.p) + n * p.v_old.sN + h * p.v_old.sH;
+    float* vob = p.v_old.p ? reinterpret_cast<float*>(p.v_old.p) + n * p.v_old.sN + h * p.v_old.sH : nullptr;
     float* uib = p.v_ins.p ? reinterpret_cast<float*>(p.v_ins.p) + n * p.v_ins.sN + h * p.v_ins.sH : nullptr;
     float* W = p.W + n * p.wN + h * p.wH;
     const int m0 = 16 * warp;
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(cb::NT, 4) delta_fwd_chunk_bf16_inv_kernel(con
                     const int m = m0 + g + 8 * (i >> 1), t = 8 * j + 2 * t4 + (i & 1);
                     u[j][i] = bs[t] * (cv[j][i] - P[j][i]);
                     if (t < nt) {
-                        vob[(long long)(t0 + t) * p.v_old.sL + m] = P[j][i] - py[j][i];
+                        if (vob) vob[(long long)(t0 + t) * p.v_old.sL + m] = P[j][i] - py[j][i];
                         if (uib) uib[(long long)(t0 + t) * p.v_ins.sL + m] = u[j][i];
                     }
                 }
@@ -603,7 +603,7 @@ __global__ void __launch_bounds__(cb::NTP, 4) delta_fwd_chunk_bf16_pipe_kernel(c
 
     // ---------------------------------------------------------------- the chain warps
     bf16* yb = reinterpret_cast<bf16*>(p.out.p) + n * p.out.sN + h * p.out.sH;
-    float* vob = reinterpret_cast<float*>(p.v_old.p) + n * p.v_old.sN + h * p.v_old.sH;
+    float* vob = p.v_old.p ? reinterpret_cast<float*>(p.v_old.p) + n * p.v_old.sN + h * p.v_old.sH : nullptr;
     float* uib = p.v_ins.p ? reinterpret_cast<float*>(p.v_ins.p) + n * p.v_ins.sN + h * p.v_ins.sH : nullptr;
     float* W = p.W + n * p.wN + h * p.wH;
     const int m0 = 16 * warp;
@@ -666,7 +666,7 @@ __global__ void __launch_bounds__(cb::NTP, 4) delta_fwd_chunk_bf16_pipe_kernel(c
                 const int m = m0 + g + 8 * (i >> 1), t = 8 * j + 2 * t4 + (i & 1);
                 u[j][i] = bs[t] * (cv[j][i] - P[j][i]);
                 if (t < nt) {
-                    vob[(long long)(t0 + t) * p.v_old.sL + m] = P[j][i] - py[j][i];
+                    if (vob) vob[(long long)(t0 + t) * p.v_old.sL + m] = P[j][i] - py[j][i];
                     if (uib) uib[(long long)(t0 + t) * p.v_ins.sL + m] = u[j][i];
                 }
             }

@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(kGenThreads) delta_fwd_generic_kernel(const De
             const float u = SUM ? vs[m] : sc[0] * (vs[m] - vo);
             us[m] = u;
             if (!SUM) {
-                put<float>(p.v_old, n, h, t, m, vo);
+                if (p.v_old.p) put<float>(p.v_old, n, h, t, m, vo);
                 if (p.v_ins.p) put<float>(p.v_ins, n, h, t, m, u);
             }
         }

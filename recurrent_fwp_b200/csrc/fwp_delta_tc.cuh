@@ -128,7 +128,7 @@ delta_fwd_tc_kernel(const DeltaFwdParams p, const __grid_constant__ CUtensorMap 
     const int seq = blockIdx.x, n = seq / p.H, h = seq - n * p.H;
     const bf16* bb = reinterpret_cast<const bf16*>(p.beta.p) + n * p.beta.sN + h * p.beta.sH;
     bf16* yb = reinterpret_cast<bf16*>(p.out.p) + n * p.out.sN + h * p.out.sH;
-    float* vob = reinterpret_cast<float*>(p.v_old.p) + n * p.v_old.sN + h * p.v_old.sH;
+    float* vob = p.v_old.p ? reinterpret_cast<float*>(p.v_old.p) + n * p.v_old.sN + h * p.v_old.sH : nullptr;
     float* W = p.W + n * p.wN + h * p.wH;
     const int nchunks = (p.L + CH - 1) / CH;
     const int row0 = 16 * gw, r0 = row0 + g, r1 = r0 + 8;      // the chunk rows (and state rows) this thread holds
@@ -529,10 +529,10 @@ delta_fwd_tc_kernel(const DeltaFwdParams p, const __grid_constant__ CUtensorMap 
                     const int c0 = 8 * j + 2 * t4;
                     const __nv_bfloat162 v0 = *reinterpret_cast<const __nv_bfloat162*>(&vp[2 * j]);
                     const __nv_bfloat162 v1 = *reinterpret_cast<const __nv_bfloat162*>(&vp[2 * j + 1]);
-                    if (r0 < nt)
+                    if (vob && r0 < nt)
                         *reinterpret_cast<float2*>(vob + (long long)(t0 + r0) * p.v_old.sL + c0) =
                             make_float2(__low2float(v0) - w[4 * j], __high2float(v0) - w[4 * j + 1]);
-                    if (r1 < nt)
+                    if (vob && r1 < nt)
                         *reinterpret_cast<float2*>(vob + (long long)(t0 + r1) * p.v_old.sL + c0) =
                             make_float2(__low2float(v1) - w[4 * j + 2], __high2float(v1) - w[4 * j + 3]);
                 }
