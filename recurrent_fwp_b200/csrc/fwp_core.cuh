@@ -58,7 +58,7 @@ enum TuneKey {
     T_DELTA_BWD_CHUNK16,    // "delta_bwd.16.chunk": 32 or 16 steps per staged chunk
     T_LSTM_FWD_SPLIT32, T_LSTM_BWD_SPLIT32, T_RNN_FWD_SPLIT32, T_RNN_BWD_SPLIT32, T_REC_FWD_SPLIT32, T_REC_BWD_SPLIT32,
     T_REC_FWD_WARP32,       // "rec_fwd.32.warp": 1 short-chain one-warp forward of the recurrent delta net at d <= 32, 0 the general kernel
-    T_RNN_BWD_ROLES32,      // "rnn_bwd.32.roles": 1 / 2 chain-warp + trailing-warp backward of the delta RNN at d <= 32 (16 / 8 steps per chunk), 0 the general kernel
+    T_RNN_BWD_ROLES32,      // "rnn_bwd.32.roles": 1 / 2 chain-warp + trailing-warps backward of the delta RNN at d = 32 (8 / 4 steps per chunk), 0 the general kernel
     T_LSTM_BWD_ROLES32,     // "lstm_bwd.32.roles": 1 chain-warp + three trailing-warp backward of the delta LSTM at d <= 32, 0 the general kernel
     T_LSTM_FWD_GATES32,     // "lstm_fwd.32.gates": 1 one-warp-per-gate forward of the delta LSTM at d = 32, 0 the general kernel
     T_DELTA_PIPE64,         // "delta.pipe64": 1 chunkwise bf16 forward with a preparing warp one chunk ahead, 0 every warp prepares for itself
@@ -526,17 +526,21 @@ __device__ __forceinline__ void stage_rows(T* tile, const Src<T>& src, int t0, i
 // A stage is `ntile` tiles of TC rows x 32 floats laid one after the other, followed by `ncol` columns of r4(TC)
 // floats ([L,1] streams).  The sources sit in a small table in shared memory, so one short loop issues every copy of
 // a chunk: a few instructions per 16-byte piece instead of one inlined copy routine per tile.  Requires full-width
-// rows that start on 16-byte boundaries (the host checks with rows_16B_aligned before choosing such a kernel).
+// rows; a piece of a stream whose rows do not all start on 16-byte boundaries (the layers' slices) goes by four words.
 struct StageTable {
     static constexpr int kMaxTiles = 20, kMaxCols = 4;
     const float* src[kMaxTiles];        // element (n, h, 0, 0) of each tile's stream; nullptr = tile not used
     long long sL[kMaxTiles];
+    int words[kMaxTiles];               // 1: rows are not 16-byte aligned
+    int any_words;                      // 1: some tile is so; the others keep the shorter loop
     const float* csrc[kMaxCols];
     long long csL[kMaxCols];
 };
 __device__ __forceinline__ void stage_table_set(StageTable* tb, int i, const Row4& r, int n, int h) {
     tb->src[i] = r.p ? reinterpret_cast<const float*>(r.p) + n * r.sN + h * r.sH : nullptr;
     tb->sL[i] = r.sL;
+    tb->words[i] = ((reinterpret_cast<uintptr_t>(tb->src[i]) & 15) != 0 || r.sL % 4 != 0) ? 1 : 0;
+    tb->any_words = (i == 0 ? 0 : tb->any_words) | tb->words[i];
 }
 __device__ __forceinline__ void stage_table_set_col(StageTable* tb, int i, const Row4& r, int n, int h) {
     tb->csrc[i] = reinterpret_cast<const float*>(r.p) + n * r.sN + h * r.sH;
@@ -548,11 +552,27 @@ __device__ __forceinline__ void stage_table_issue(float* stage, const StageTable
     static_assert((TC & (TC - 1)) == 0 && TC >= 4, "rows per chunk: a power of two");
     constexpr int D = 32;
     const int total = ntile * TC * 8;
+    if (!tb->any_words) {
 #pragma unroll 1
-    for (int i = tid; i < total; i += NT) {
-        const int piece = i & 7, r = (i >> 3) & (TC - 1), tile = i / (8 * TC);
-        const float* sp = tb->src[tile];
-        if (r < nt && sp) cp_async16(stage + i * 4, sp + (long long)(t0 + r) * tb->sL[tile] + piece * 4);
+        for (int i = tid; i < total; i += NT) {
+            const int piece = i & 7, r = (i >> 3) & (TC - 1), tile = i / (8 * TC);
+            const float* sp = tb->src[tile];
+            if (r < nt && sp) cp_async16(stage + i * 4, sp + (long long)(t0 + r) * tb->sL[tile] + piece * 4);
+        }
+    } else {
+#pragma unroll 1
+        for (int i = tid; i < total; i += NT) {
+            const int piece = i & 7, r = (i >> 3) & (TC - 1), tile = i / (8 * TC);
+            const float* sp = tb->src[tile];
+            if (r >= nt || !sp) continue;
+            sp += (long long)(t0 + r) * tb->sL[tile] + piece * 4;
+            if (!tb->words[tile]) {
+                cp_async16(stage + i * 4, sp);
+                continue;
+            }
+#pragma unroll
+            for (int w = 0; w < 4; w++) cp_async4(stage + i * 4 + w, sp + w);
+        }
     }
     float* cols = stage + ntile * TC * D;
     if (tid < ncol * TC) {

@@ -404,7 +404,8 @@ template <int VAR>
 static int launch_lstm_bwd_roles32(const LstmBwdParams& p, int nseq, cudaStream_t st) {
     constexpr int TC = 8;
     auto kern = lstm_bwd_roles32_kernel<TC, VAR>;
-    const int slots = nseq % 2 ? 1 : 2;
+    int slots = 2;
+    while (nseq % slots) slots >>= 1;          // sequences per CTA must divide the sequence count
     const size_t bytes = (size_t)LstmRolesSmem<TC>::kFloats * sizeof(float) * slots;
     if (int rc = smem_optin(kern, bytes)) return rc;
     kern<<<nseq / slots, 128 * slots, bytes, st>>>(p);
@@ -419,7 +420,7 @@ static int launch_lstm_fwd_gates32(const LstmFwdParams& p, int nseq, cudaStream_
     constexpr int TC = 16;
     auto kern = lstm_fwd_gates32_kernel<TC, VAR>;
     int slots = 4;
-    while (nseq % slots) slots >>= 1;
+    while (nseq % slots) slots >>= 1;          // sequences per CTA must divide the sequence count
     const size_t bytes = (size_t)LstmGatesSmem<TC>::kFloats * sizeof(float) * slots;
     if (int rc = smem_optin(kern, bytes)) return rc;
     kern<<<nseq / slots, 96 * slots, bytes, st>>>(p);
@@ -434,10 +435,11 @@ static int dispatch_lstm_fwd(const LstmFwdParams& p, int nseq, cudaStream_t st) 
     switch (pad_dim(p.D)) {
         case 16: return launch_lstm_fwd<16, 2, 16, VAR>(p, nseq, st);
         case 32: {
-            bool fast = p.D == 32 && tune_get(T_LSTM_FWD_GATES32, 1);       // full width, 16-byte aligned rows
-            for (int a = 0; a < 3 && fast; a++)
-                fast = rows_16B_aligned(p.z[a]) && rows_16B_aligned(p.k[a]) && rows_16B_aligned(p.v[a]);
-            if (fast) return launch_lstm_fwd_gates32<VAR>(p, nseq, st);
+            // full rows; rows at odd offsets (the layers' slices) go word by word, which a short call does not earn back
+            bool aligned = true;
+            for (int a = 0; a < 3; a++)
+                aligned = aligned && rows_16B_aligned(p.z[a]) && rows_16B_aligned(p.k[a]) && rows_16B_aligned(p.v[a]);
+            if (p.D == 32 && tune_get(T_LSTM_FWD_GATES32, 1) && (aligned || p.L >= 64)) return launch_lstm_fwd_gates32<VAR>(p, nseq, st);
             const int sp = tune_get(T_LSTM_FWD_SPLIT32, 1);
             // measured (512 sequences x 512 steps): 1 -> 0.78 ms, 4 -> 0.83 ms, 2 -> 0.85 ms
             if (sp == 2) return launch_lstm_fwd<32, 2, 8, VAR>(p, nseq, st);
@@ -454,13 +456,12 @@ static int dispatch_lstm_bwd(const LstmBwdParams& p, int nseq, cudaStream_t st) 
     switch (pad_dim(p.D)) {
         case 16: return launch_lstm_bwd<16, 2, 8, VAR>(p, nseq, st);
         case 32: {
-            bool fast = p.D == 32 && tune_get(T_LSTM_BWD_ROLES32, 1);      // full width, 16-byte aligned rows
-            for (int a = 0; a < 3 && fast; a++)
-                fast = rows_16B_aligned(p.k[a]) && rows_16B_aligned(p.v[a]) && rows_16B_aligned(p.v_old[a]) &&
-                       rows_16B_aligned(p.gate[a]);
-            fast = fast && rows_16B_aligned(p.gy) && rows_16B_aligned(p.od) && rows_16B_aligned(p.cell) &&
-                   rows_16B_aligned(p.umc) && (VAR != 1 || rows_16B_aligned(p.out));
-            if (fast) return launch_lstm_bwd_roles32<VAR>(p, nseq, st);
+            bool aligned = rows_16B_aligned(p.gy) && rows_16B_aligned(p.od) && rows_16B_aligned(p.cell) &&
+                           rows_16B_aligned(p.umc) && (VAR != 1 || rows_16B_aligned(p.out));
+            for (int a = 0; a < 3; a++)
+                aligned = aligned && rows_16B_aligned(p.k[a]) && rows_16B_aligned(p.v[a]) && rows_16B_aligned(p.v_old[a]) &&
+                          rows_16B_aligned(p.gate[a]);
+            if (p.D == 32 && tune_get(T_LSTM_BWD_ROLES32, 1) && (aligned || p.L >= 64)) return launch_lstm_bwd_roles32<VAR>(p, nseq, st);
             const int sp = tune_get(T_LSTM_BWD_SPLIT32, 2);
             // measured: 2 -> 1.37 ms, 4 -> 2.14 ms
             if (sp == 4) return launch_lstm_bwd<32, 4, 4, VAR>(p, nseq, st);

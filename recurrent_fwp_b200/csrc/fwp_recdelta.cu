@@ -524,7 +524,7 @@ static int launch_rec_fwd_warp32(const RecFwdParams& p, int nseq, cudaStream_t s
     auto kern = p.D == 32 ? rec_fwd_warp32_kernel<TC, true> : rec_fwd_warp32_kernel<TC, false>;
     const size_t bytes = (2 * RecFwdStage<32, TC>::kFloats + 3 * 32) * sizeof(float);
     int slots = 4;
-    while (nseq % slots) slots >>= 1;
+    while (nseq % slots) slots >>= 1;          // sequences per CTA must divide the sequence count
     if (int rc = smem_optin(kern, bytes * slots)) return rc;
     kern<<<nseq / slots, 32 * slots, bytes * slots, st>>>(p);
     count_launch();
@@ -551,7 +551,7 @@ static int launch_rec_bwd_roles32(const RecBwdParams& p, int nseq, cudaStream_t 
     constexpr int TC = 8;
     auto kern = rec_bwd_roles32_kernel<TC>;
     int slots = 4;
-    while (nseq % slots) slots >>= 1;
+    while (nseq % slots) slots >>= 1;          // sequences per CTA must divide the sequence count
     const size_t bytes = (size_t)RecRolesSmem<TC>::kFloats * sizeof(float) * slots;
     if (int rc = smem_optin(kern, bytes)) return rc;
     kern<<<nseq / slots, 64 * slots, bytes, st>>>(p);
@@ -677,8 +677,9 @@ FWP_API int fwp_rec_update_fwm_tanh_backward(int N, int H, int L, int D,
     switch (DP) {
         case 16: rc = launch_rec_bwd<16, 2, 16>(p, N * H, st); break;
         case 32: {
-            if (p.D == 32 && tune_get(T_REC_BWD_ROLES32, 1) && rows_16B_aligned(p.q) && rows_16B_aligned(p.k) &&
-                rows_16B_aligned(p.v) && rows_16B_aligned(p.v_old) && rows_16B_aligned(p.od) && rows_16B_aligned(p.gy)) {
+            const bool aligned = rows_16B_aligned(p.q) && rows_16B_aligned(p.k) && rows_16B_aligned(p.v) && rows_16B_aligned(p.v_old) &&
+                                 rows_16B_aligned(p.od) && rows_16B_aligned(p.gy);
+            if (p.D == 32 && tune_get(T_REC_BWD_ROLES32, 1) && (aligned || p.L >= 64)) {
                 rc = launch_rec_bwd_roles32(p, N * H, st);
                 break;
             }

@@ -327,10 +327,10 @@ template <int TC, bool V1>
 static int launch_rnn_bwd_roles32(const RnnBwdParams& p, int nseq, cudaStream_t st) {
     auto kern = rnn_bwd_roles32_kernel<TC, V1>;
     int slots = 4;
-    while (nseq % slots) slots >>= 1;
+    while (nseq % slots) slots >>= 1;          // sequences per CTA must divide the sequence count
     const size_t bytes = (size_t)RnnRolesSmem<TC, V1>::kFloats * sizeof(float) * slots;
     if (int rc = smem_optin(kern, bytes)) return rc;
-    kern<<<nseq / slots, 64 * slots, bytes, st>>>(p);
+    kern<<<nseq / slots, 96 * slots, bytes, st>>>(p);
     count_launch();
     note_kernel("rnn_bwd_roles32_kernel");
     cudaError_t e = cudaGetLastError();
@@ -409,11 +409,13 @@ static int rnn_backward(int N, int H, int L, int D,
         case 16: return launch_rnn_bwd<16, 2, 16, V1>(p, N * H, st);
         case 32: {
             int roles = tune_get(T_RNN_BWD_ROLES32, 1);
-            if (p.D != 32 || !rows_16B_aligned(p.k) || !rows_16B_aligned(p.v) || !rows_16B_aligned(p.gy) ||
-                !rows_16B_aligned(p.v_old) || !rows_16B_aligned(p.od) || (V1 && !rows_16B_aligned(p.out)))
-                roles = 0;              // the two-warp kernel wants full width and 16-byte aligned rows
-            if (roles == 1) return launch_rnn_bwd_roles32<16, V1>(p, N * H, st);
-            if (roles == 2) return launch_rnn_bwd_roles32<8, V1>(p, N * H, st);
+            // the role kernel wants full rows; rows at odd offsets (the layers' slices) go word by word, which a short call
+            // does not earn back
+            const bool aligned = rows_16B_aligned(p.k) && rows_16B_aligned(p.v) && rows_16B_aligned(p.gy) && rows_16B_aligned(p.v_old) &&
+                                 rows_16B_aligned(p.od) && (!V1 || rows_16B_aligned(p.out));
+            if (p.D != 32 || (!aligned && p.L < 64)) roles = 0;
+            if (roles == 1) return launch_rnn_bwd_roles32<8, V1>(p, N * H, st);
+            if (roles == 2) return launch_rnn_bwd_roles32<4, V1>(p, N * H, st);
             const int sp = tune_get(T_RNN_BWD_SPLIT32, 1);
             // measured (512 sequences x 512 steps): 1 -> 0.34 ms, 2 -> 0.39 ms, 4 -> 0.42 ms
             if (sp == 2) return launch_rnn_bwd<32, 2, 8, V1>(p, N * H, st);
