@@ -376,8 +376,7 @@ template <int D, int SPLIT, int TC, int VAR>
 static int launch_lstm_fwd(const LstmFwdParams& p, int nseq, cudaStream_t st) {
     auto kern = lstm_fwd_kernel<D, SPLIT, TC, VAR>;
     const size_t bytes = (2 * LstmFwdStage<D, TC>::kFloats + 2 * (D + 16)) * sizeof(float);
-    int slots = slots_for(D * SPLIT);
-    while (nseq % slots) slots >>= 1;          // sequences per CTA must divide the sequence count
+    const int slots = spread_slots(slots_for(D * SPLIT), nseq);
     if (int rc = smem_optin(kern, bytes * slots)) return rc;
     kern<<<nseq / slots, D * SPLIT * slots, bytes * slots, st>>>(p);
     count_launch();
@@ -390,8 +389,7 @@ template <int D, int SPLIT, int TC, int VAR>
 static int launch_lstm_bwd(const LstmBwdParams& p, int nseq, cudaStream_t st) {
     auto kern = lstm_bwd_kernel<D, SPLIT, TC, VAR>;
     const size_t bytes = (2 * LstmBwdStage<D, TC>::kFloats + 2 * (9 * D + 48)) * sizeof(float);
-    int slots = slots_for(D * SPLIT);
-    while (nseq % slots) slots >>= 1;          // sequences per CTA must divide the sequence count
+    const int slots = spread_slots(slots_for(D * SPLIT), nseq);
     if (int rc = smem_optin(kern, bytes * slots)) return rc;
     kern<<<nseq / slots, D * SPLIT * slots, bytes * slots, st>>>(p);
     count_launch();
@@ -404,8 +402,7 @@ template <int VAR>
 static int launch_lstm_bwd_roles32(const LstmBwdParams& p, int nseq, cudaStream_t st) {
     constexpr int TC = 8;
     auto kern = lstm_bwd_roles32_kernel<TC, VAR>;
-    int slots = 2;
-    while (nseq % slots) slots >>= 1;          // sequences per CTA must divide the sequence count
+    const int slots = spread_slots(2, nseq);
     const size_t bytes = (size_t)LstmRolesSmem<TC>::kFloats * sizeof(float) * slots;
     if (int rc = smem_optin(kern, bytes)) return rc;
     kern<<<nseq / slots, 128 * slots, bytes, st>>>(p);
@@ -419,8 +416,7 @@ template <int VAR>
 static int launch_lstm_fwd_gates32(const LstmFwdParams& p, int nseq, cudaStream_t st) {
     constexpr int TC = 16;
     auto kern = lstm_fwd_gates32_kernel<TC, VAR>;
-    int slots = 4;
-    while (nseq % slots) slots >>= 1;          // sequences per CTA must divide the sequence count
+    const int slots = spread_slots(4, nseq);
     const size_t bytes = (size_t)LstmGatesSmem<TC>::kFloats * sizeof(float) * slots;
     if (int rc = smem_optin(kern, bytes)) return rc;
     kern<<<nseq / slots, 96 * slots, bytes, st>>>(p);

@@ -509,8 +509,7 @@ template <int D, int SPLIT, int TC>
 static int launch_rec_fwd(const RecFwdParams& p, int nseq, cudaStream_t st) {
     auto kern = rec_fwd_kernel<D, SPLIT, TC>;
     const size_t bytes = (2 * RecFwdStage<D, TC>::kFloats + 2 * (3 * D + 32)) * sizeof(float);
-    int slots = slots_for(D * SPLIT);
-    while (nseq % slots) slots >>= 1;          // sequences per CTA must divide the sequence count
+    const int slots = spread_slots(slots_for(D * SPLIT), nseq);
     if (int rc = smem_optin(kern, bytes * slots)) return rc;
     kern<<<nseq / slots, D * SPLIT * slots, bytes * slots, st>>>(p);
     count_launch();
@@ -523,8 +522,7 @@ template <int TC>
 static int launch_rec_fwd_warp32(const RecFwdParams& p, int nseq, cudaStream_t st) {
     auto kern = p.D == 32 ? rec_fwd_warp32_kernel<TC, true> : rec_fwd_warp32_kernel<TC, false>;
     const size_t bytes = (2 * RecFwdStage<32, TC>::kFloats + 3 * 32) * sizeof(float);
-    int slots = 4;
-    while (nseq % slots) slots >>= 1;          // sequences per CTA must divide the sequence count
+    const int slots = spread_slots(4, nseq);
     if (int rc = smem_optin(kern, bytes * slots)) return rc;
     kern<<<nseq / slots, 32 * slots, bytes * slots, st>>>(p);
     count_launch();
@@ -537,8 +535,7 @@ template <int D, int SPLIT, int TC>
 static int launch_rec_bwd(const RecBwdParams& p, int nseq, cudaStream_t st) {
     auto kern = rec_bwd_kernel<D, SPLIT, TC>;
     const size_t bytes = (2 * RecBwdStage<D, TC>::kFloats + 2 * RecBwdSmem<D>::kXs + RecBwdSmem<D>::kR) * sizeof(float);
-    int slots = slots_for(D * SPLIT);
-    while (nseq % slots) slots >>= 1;          // sequences per CTA must divide the sequence count
+    const int slots = spread_slots(slots_for(D * SPLIT), nseq);
     if (int rc = smem_optin(kern, bytes * slots)) return rc;
     kern<<<nseq / slots, D * SPLIT * slots, bytes * slots, st>>>(p);
     count_launch();
@@ -550,8 +547,7 @@ static int launch_rec_bwd(const RecBwdParams& p, int nseq, cudaStream_t st) {
 static int launch_rec_bwd_roles32(const RecBwdParams& p, int nseq, cudaStream_t st) {
     constexpr int TC = 8;
     auto kern = rec_bwd_roles32_kernel<TC>;
-    int slots = 4;
-    while (nseq % slots) slots >>= 1;          // sequences per CTA must divide the sequence count
+    const int slots = spread_slots(4, nseq);
     const size_t bytes = (size_t)RecRolesSmem<TC>::kFloats * sizeof(float) * slots;
     if (int rc = smem_optin(kern, bytes)) return rc;
     kern<<<nseq / slots, 64 * slots, bytes, st>>>(p);

@@ -299,8 +299,7 @@ template <int D, int SPLIT, int TC, bool V1>
 static int launch_rnn_fwd(const RnnFwdParams& p, int nseq, cudaStream_t st) {
     auto kern = rnn_fwd_kernel<D, SPLIT, TC, V1>;
     const size_t bytes = (2 * RnnFwdStage<D, TC>::kFloats + 2 * (D + 16)) * sizeof(float);
-    int slots = slots_for(D * SPLIT);
-    while (nseq % slots) slots >>= 1;          // sequences per CTA must divide the sequence count
+    const int slots = spread_slots(slots_for(D * SPLIT), nseq);
     if (int rc = smem_optin(kern, bytes * slots)) return rc;
     kern<<<nseq / slots, D * SPLIT * slots, bytes * slots, st>>>(p);
     count_launch();
@@ -313,8 +312,7 @@ template <int D, int SPLIT, int TC, bool V1>
 static int launch_rnn_bwd(const RnnBwdParams& p, int nseq, cudaStream_t st) {
     auto kern = rnn_bwd_kernel<D, SPLIT, TC, V1>;
     const size_t bytes = (2 * RnnBwdStage<D, TC, V1>::kFloats + 2 * (3 * D + 24)) * sizeof(float);
-    int slots = slots_for(D * SPLIT);
-    while (nseq % slots) slots >>= 1;          // sequences per CTA must divide the sequence count
+    const int slots = spread_slots(slots_for(D * SPLIT), nseq);
     if (int rc = smem_optin(kern, bytes * slots)) return rc;
     kern<<<nseq / slots, D * SPLIT * slots, bytes * slots, st>>>(p);
     count_launch();
@@ -326,8 +324,7 @@ static int launch_rnn_bwd(const RnnBwdParams& p, int nseq, cudaStream_t st) {
 template <int TC, bool V1>
 static int launch_rnn_bwd_roles32(const RnnBwdParams& p, int nseq, cudaStream_t st) {
     auto kern = rnn_bwd_roles32_kernel<TC, V1>;
-    int slots = 4;
-    while (nseq % slots) slots >>= 1;          // sequences per CTA must divide the sequence count
+    const int slots = spread_slots(4, nseq);
     const size_t bytes = (size_t)RnnRolesSmem<TC, V1>::kFloats * sizeof(float) * slots;
     if (int rc = smem_optin(kern, bytes)) return rc;
     kern<<<nseq / slots, 96 * slots, bytes, st>>>(p);
