@@ -579,15 +579,22 @@ static int dispatch_fwd(const DeltaFwdParams& p, int nseq, cudaStream_t st) {
 //   E, M = 96, 32: 128 1152 -> 113, 1024 2783 -> 1233
 // The four-step blocked kernels are at their best with rows of exactly 16, 32 or 64 elements and a sequence for every SM;
 // short rows cost them a division per copied piece, and states above 64 have no register-resident kernel at all.
-template <typename T>
-static bool bwd_phases_pay(const DeltaBwdParams& p, int nseq) {
-    if (sizeof(T) != 4 || tune_get(T_DELTA_BLOCKED, -1) != -1) return false;
+// bf16 streams (1024 steps) need a third of the operand parts:
+//   d = 16: 16 sequences 187 -> 37, 128 189 -> 102, 288 190 -> 188, 512 191 -> 270; with rows of 12 (256 steps) 512 166 -> 75
+//   d = 32: 16 653 -> 55, 128 679 -> 215, 512 775 -> 714, 1024 1092 -> 1432;  d = 48 (256 steps): 512 648 -> 306, 1600 1766 -> 1235
+//   rows of 56 (256 steps): 512 651 -> 603.  Rows of 64 have a one-launch kernel on tensor cores.
+static bool bwd_phases_pay(const DeltaBwdParams& p, int nseq, int io_dtype) {
+    if (tune_get(T_DELTA_BLOCKED, -1) != -1) return false;
     const int force = tune_get(T_DELTA_PHASES, -1);
     if (force != -1) return force == 1;
     const int d = p.E > p.M ? p.E : p.M;
     if (d > 64) return p.L > 4;
     if (p.L <= kShortSeq) return false;
     const bool full = p.E == p.M && (d == 16 || d == 32 || d == 64);
+    if (io_dtype == FWP_BF16) {
+        if (full && d == 64) return false;
+        return (d > 32 && d <= 48) || nseq <= (full && d == 16 ? 2 : 4) * sm_count();
+    }
     if (d <= 16) return nseq <= (full ? 1 : 2) * sm_count();
     return !full || nseq <= (d == 64 ? sm_count() / 2 : sm_count());
 }
@@ -713,10 +720,11 @@ static int fast_weight_backward_impl(int N, int H, int L, int E, int M,
     p.W = (float*)fw_mem->data; p.wN = fw_mem->stride[0]; p.wH = fw_mem->stride[1]; p.wE = fw_mem->stride[2];
     p.H = H; p.L = L; p.E = E; p.M = M; p.NH = N * H;
     cudaStream_t st = (cudaStream_t)stream;
-    if (scratch && io_dtype == FWP_F32 && bwd_phases_pay<float>(p, N * H)) {
+    const auto phases = io_dtype == FWP_F32 ? bwd_phases<float> : bwd_phases<__nv_bfloat16>;
+    if (scratch && bwd_phases_pay(p, N * H, io_dtype)) {
         if (reinterpret_cast<uintptr_t>(scratch) & 15) return FWP_ERR_SCRATCH;
-        const int64_t need = bwd_phases<float>(false, p, N * H, nullptr, st);
-        if (need > 0) return scratch_floats < need ? FWP_ERR_SCRATCH : (int)bwd_phases<float>(true, p, N * H, scratch, st);
+        const int64_t need = phases(false, p, N * H, nullptr, st);
+        if (need > 0) return scratch_floats < need ? FWP_ERR_SCRATCH : (int)phases(true, p, N * H, scratch, st);
     }
     if (io_dtype == FWP_F32) return dispatch_bwd<float>(p, N * H, st);
     return dispatch_bwd<__nv_bfloat16>(p, N * H, st);
@@ -735,11 +743,11 @@ FWP_API int fwp_fast_weight_backward(int N, int H, int L, int E, int M,
 }
 
 FWP_API int64_t fwp_fast_weight_backward_scratch_floats(int N, int H, int L, int E, int M, int io_dtype) {
-    if (check_common(N, H, L, E, M, io_dtype) || io_dtype != FWP_F32) return 0;
+    if (check_common(N, H, L, E, M, io_dtype)) return 0;
     DeltaBwdParams p;
     p.H = H; p.L = L; p.E = E; p.M = M; p.NH = N * H;
-    if (!bwd_phases_pay<float>(p, N * H)) return 0;
-    const int64_t need = bwd_phases<float>(false, p, N * H, nullptr, nullptr);
+    if (!bwd_phases_pay(p, N * H, io_dtype)) return 0;
+    const int64_t need = (io_dtype == FWP_F32 ? bwd_phases<float> : bwd_phases<__nv_bfloat16>)(false, p, N * H, nullptr, nullptr);
     return need > 0 ? need : 0;
 }
 

@@ -76,5 +76,6 @@ int64_t bwd_phases(bool run, const DeltaBwdParams& p, int nseq, float* scratch, 
     return -1;
 }
 template int64_t bwd_phases<float>(bool, const DeltaBwdParams&, int, float*, cudaStream_t);
+template int64_t bwd_phases<__nv_bfloat16>(bool, const DeltaBwdParams&, int, float*, cudaStream_t);
 
 }  // namespace fwp

@@ -122,3 +122,29 @@ def test_three_launch_backward_in_segments(fwp):
         _lib.tune('delta_bwd.phases', -1)
     for a, c in zip(res[0], res[1]):
         assert util.max_abs(a, c) <= 5e-6 * max(1., a.abs().max().item())
+
+
+@pytest.mark.parametrize('E,M', [(16, 16), (9, 14), (32, 32), (21, 30), (48, 48), (56, 33), (96, 64), (128, 128)])
+@pytest.mark.parametrize('L', [17, 130])
+def test_three_launch_backward_of_bf16_streams(fwp, E, M, L):
+    """The gradients are the fp32 ones of the same bf16 values, rounded once."""
+    from recurrent_fwp_b200 import _lib
+    B, H = 2, 3
+    x16 = [t.to(DEV).bfloat16() for t in util.delta_inputs(27, B, H, L, E, M)]
+    W0 = torch.randn(B, H, E, M, generator=util.gen(28)).to(DEV) * 0.1
+    res, seen = [], []
+    try:
+        _lib.tune('delta_bwd.phases', 1)
+        for streams in (x16, sliced(x16[:4]) + x16[4:], [t.float() for t in x16]):
+            x = [t.detach().requires_grad_() for t in streams[:4]]
+            W = W0.clone()
+            y = fwp.fast_weight_delta(*x, W)
+            x[0].register_hook(lambda g: seen.append(_lib.last_kernel()))
+            y.backward(streams[4])
+            res.append([t.grad.float() for t in x] + [W])
+    finally:
+        _lib.tune('delta_bwd.phases', -1)
+    assert seen == ['delta_bwd_finish_kernel'] * 3
+    for got in res[:2]:
+        for a, r in zip(got, res[2]):
+            assert ((a - r).abs() <= 2 ** -8 * r.abs() + 1e-5 * r.abs().max()).all()
