@@ -2,6 +2,7 @@
 // applicability test and launches here.  One fused launch per direction, no workspace.
 #include <atomic>
 #include "fwp_delta_chunk_bf16.cuh"
+#include "fwp_delta_chunk_bf16_bwd.cuh"
 #include "fwp_delta_tc.cuh"
 
 namespace fwp {
@@ -99,8 +100,10 @@ bool chunk_bf16_applies(const DeltaBwdParams& p) {
 
 int launch_bwd_chunk_bf16(const DeltaBwdParams& p, int nseq, cudaStream_t st) {
     // "delta.pipe64": 1 both directions with a preparing warp, 2 the forward only, 0 neither
+    constexpr int PW = 3, R = 7;        // measured, 128 sequences x 1024 steps: 3 preparing warps 86 us, 2 106, 4 97; 7 to 10 stages alike
     if (tune_get(T_DELTA_PIPE64, 1) == 1)
-        return launch(delta_bwd_chunk_bf16_pipe_kernel, p, nseq, cb::NTP, sizeof(cb::SmemBP), st, "delta_bwd_chunk_bf16_pipe_kernel");
+        return launch_dependent(delta_bwd_chunk_bf16_pipe_kernel<PW, R>, p, nseq, (12 + PW) * 32, sizeof(cb::BwdSmem<R>), st,
+                                "delta_bwd_chunk_bf16_pipe_kernel");
     return launch(delta_bwd_chunk_bf16_inv_kernel, p, nseq, cb::NT, sizeof(cb::SmemB2), st, "delta_bwd_chunk_bf16_inv_kernel");
 }
 
