@@ -268,6 +268,8 @@ struct SumStage {
 
 template <int D, int SPLIT, int TC, typename T>
 __global__ void __launch_bounds__(D * SPLIT * slots_for(D * SPLIT)) sum_bwd_kernel(const SumBwdParams p) {
+    griddep_wait();               // launched as a dependent: global memory is touched from here on
+    griddep_launch_dependents();
     using G = Geo<D, SPLIT>;
     const G g;
     const int n = g.seq / p.H, h = g.seq - n * p.H;
@@ -355,6 +357,8 @@ template <int D, int TC, typename T>
 __host__ __device__ constexpr int sum_roles_floats() { return sum_stages<T>() * 3 * r4(Tile<D, TC, T>::kFloats) + 2 * TC * D; }   // per role and sequence
 template <int D, int SPLIT, int TC, typename T>
 __global__ void __launch_bounds__(3 * D * SPLIT * slots_for(D * SPLIT)) sum_bwd_roles_kernel(const SumBwdParams p) {
+    griddep_wait();               // launched as a dependent: global memory is touched from here on
+    griddep_launch_dependents();
     using G = Geo<D, SPLIT>;
     using Tl = Tile<D, TC, T>;
     constexpr int TT = r4(Tl::kFloats), NST = sum_stages<T>(), PER = sum_roles_floats<D, TC, T>();
@@ -479,9 +483,9 @@ static int launch_sum_bwd(const SumBwdParams& p, int nseq, cudaStream_t st) {
     int slots = slots_for(D * SPLIT);
     while (nseq % slots) slots >>= 1;          // sequences per CTA must divide the sequence count
     if (tune_get(T_SUM_BWD_ROLES, 1))
-        return launch(sum_bwd_roles_kernel<D, SPLIT, TC, T>, p, nseq / slots, 3 * D * SPLIT * slots,
+        return launch_dependent(sum_bwd_roles_kernel<D, SPLIT, TC, T>, p, nseq / slots, 3 * D * SPLIT * slots,
                       slots * 3 * sum_roles_floats<D, TC, T>() * sizeof(float), st, "sum_bwd_roles_kernel");
-    return launch(sum_bwd_kernel<D, SPLIT, TC, T>, p, nseq / slots, D * SPLIT * slots,
+    return launch_dependent(sum_bwd_kernel<D, SPLIT, TC, T>, p, nseq / slots, D * SPLIT * slots,
                   slots * 2 * SumStage<D, TC, T>::kFloats * sizeof(float), st, "sum_bwd_kernel");
 }
 

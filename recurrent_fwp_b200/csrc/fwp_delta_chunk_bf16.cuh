@@ -449,6 +449,8 @@ __device__ __forceinline__ void nbar_arrive(int id, int n) { asm volatile("bar.a
 }  // namespace cb
 
 __global__ void __launch_bounds__(cb::NTP, 4) delta_fwd_chunk_bf16_pipe_kernel(const DeltaFwdParams p) {
+    griddep_wait();               // launched as a dependent: global memory is touched from here on
+    griddep_launch_dependents();
     using namespace cb;
     using bf16 = __nv_bfloat16;
     extern __shared__ __align__(16) unsigned char cb_smem[];

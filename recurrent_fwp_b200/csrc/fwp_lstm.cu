@@ -44,6 +44,8 @@ struct LstmFwdStage {
 
 template <int D, int SPLIT, int TC, int VAR>
 __global__ void __launch_bounds__(D * SPLIT * slots_for(D * SPLIT)) lstm_fwd_kernel(const LstmFwdParams p) {
+    griddep_wait();               // launched as a dependent: global memory is touched from here on
+    griddep_launch_dependents();
     using G = Geo<D, SPLIT>;
     const G g;
     const int n = g.seq / p.H, h = g.seq - n * p.H;
@@ -205,6 +207,8 @@ struct LstmBwdStage {
 
 template <int D, int SPLIT, int TC, int VAR>
 __global__ void __launch_bounds__(D * SPLIT * slots_for(D * SPLIT)) lstm_bwd_kernel(const LstmBwdParams p) {
+    griddep_wait();               // launched as a dependent: global memory is touched from here on
+    griddep_launch_dependents();
     using G = Geo<D, SPLIT>;
     const G g;
     const int n = g.seq / p.H, h = g.seq - n * p.H;
@@ -363,26 +367,12 @@ __global__ void __launch_bounds__(D * SPLIT * slots_for(D * SPLIT)) lstm_bwd_ker
 namespace fwp {
 
 // ------------------------------------------------------------------ launchers
-template <typename K>
-static int smem_optin(K kernel, size_t bytes) {
-    if (bytes > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        if (e != cudaSuccess) return set_cuda_error(e);
-    }
-    return FWP_OK;
-}
-
 template <int D, int SPLIT, int TC, int VAR>
 static int launch_lstm_fwd(const LstmFwdParams& p, int nseq, cudaStream_t st) {
     auto kern = lstm_fwd_kernel<D, SPLIT, TC, VAR>;
     const size_t bytes = (2 * LstmFwdStage<D, TC>::kFloats + 2 * (D + 16)) * sizeof(float);
     const int slots = spread_slots(slots_for(D * SPLIT), nseq);
-    if (int rc = smem_optin(kern, bytes * slots)) return rc;
-    kern<<<nseq / slots, D * SPLIT * slots, bytes * slots, st>>>(p);
-    count_launch();
-    note_kernel("lstm_fwd_kernel");
-    cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? FWP_OK : set_cuda_error(e);
+    return launch_dependent(kern, p, nseq / slots, D * SPLIT * slots, bytes * slots, st, "lstm_fwd_kernel");
 }
 
 template <int D, int SPLIT, int TC, int VAR>
@@ -390,12 +380,7 @@ static int launch_lstm_bwd(const LstmBwdParams& p, int nseq, cudaStream_t st) {
     auto kern = lstm_bwd_kernel<D, SPLIT, TC, VAR>;
     const size_t bytes = (2 * LstmBwdStage<D, TC>::kFloats + 2 * (9 * D + 48)) * sizeof(float);
     const int slots = spread_slots(slots_for(D * SPLIT), nseq);
-    if (int rc = smem_optin(kern, bytes * slots)) return rc;
-    kern<<<nseq / slots, D * SPLIT * slots, bytes * slots, st>>>(p);
-    count_launch();
-    note_kernel("lstm_bwd_kernel");
-    cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? FWP_OK : set_cuda_error(e);
+    return launch_dependent(kern, p, nseq / slots, D * SPLIT * slots, bytes * slots, st, "lstm_bwd_kernel");
 }
 
 template <int VAR>
@@ -404,12 +389,7 @@ static int launch_lstm_bwd_roles32(const LstmBwdParams& p, int nseq, cudaStream_
     auto kern = lstm_bwd_roles32_kernel<TC, VAR>;
     const int slots = spread_slots(2, nseq);
     const size_t bytes = (size_t)LstmRolesSmem<TC>::kFloats * sizeof(float) * slots;
-    if (int rc = smem_optin(kern, bytes)) return rc;
-    kern<<<nseq / slots, 128 * slots, bytes, st>>>(p);
-    count_launch();
-    note_kernel("lstm_bwd_roles32_kernel");
-    cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? FWP_OK : set_cuda_error(e);
+    return launch_dependent(kern, p, nseq / slots, 128 * slots, bytes, st, "lstm_bwd_roles32_kernel");
 }
 
 template <int VAR>
@@ -418,12 +398,7 @@ static int launch_lstm_fwd_gates32(const LstmFwdParams& p, int nseq, cudaStream_
     auto kern = lstm_fwd_gates32_kernel<TC, VAR>;
     const int slots = spread_slots(4, nseq);
     const size_t bytes = (size_t)LstmGatesSmem<TC>::kFloats * sizeof(float) * slots;
-    if (int rc = smem_optin(kern, bytes)) return rc;
-    kern<<<nseq / slots, 96 * slots, bytes, st>>>(p);
-    count_launch();
-    note_kernel("lstm_fwd_gates32_kernel");
-    cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? FWP_OK : set_cuda_error(e);
+    return launch_dependent(kern, p, nseq / slots, 96 * slots, bytes, st, "lstm_fwd_gates32_kernel");
 }
 
 template <int VAR>

@@ -29,6 +29,8 @@ struct LstmRolesSmem {
 
 template <int TC, int VAR>
 __global__ void __launch_bounds__(256, 1) lstm_bwd_roles32_kernel(const LstmBwdParams p) {
+    griddep_wait();               // launched as a dependent: global memory is touched from here on
+    griddep_launch_dependents();
     constexpr int D = 32, NP = 16, NT = 128;
     using SM = LstmRolesSmem<TC>;
     using Stage = typename SM::Stage;
@@ -256,6 +258,8 @@ struct LstmGatesSmem {
 
 template <int TC, int VAR>
 __global__ void __launch_bounds__(384, 1) lstm_fwd_gates32_kernel(const LstmFwdParams p) {
+    griddep_wait();               // launched as a dependent: global memory is touched from here on
+    griddep_launch_dependents();
     constexpr int D = 32, NP = 16, NT = 96;
     using SM = LstmGatesSmem<TC>;
     using Stage = typename SM::Stage;

@@ -31,6 +31,8 @@ struct RecRolesSmem {
 
 template <int TC>
 __global__ void __launch_bounds__(256, 1) rec_bwd_roles32_kernel(const RecBwdParams p) {
+    griddep_wait();               // launched as a dependent: global memory is touched from here on
+    griddep_launch_dependents();
     constexpr int D = 32, NP = 16, NT = 64;
     using SM = RecRolesSmem<TC>;
     using Stage = typename SM::Stage;

@@ -36,6 +36,8 @@ struct RnnFwdStage {
 
 template <int D, int SPLIT, int TC, bool V1>
 __global__ void __launch_bounds__(D * SPLIT * slots_for(D * SPLIT)) rnn_fwd_kernel(const RnnFwdParams p) {
+    griddep_wait();               // launched as a dependent: global memory is touched from here on
+    griddep_launch_dependents();
     using G = Geo<D, SPLIT>;
     const G g;
     const int n = g.seq / p.H, h = g.seq - n * p.H;
@@ -166,6 +168,8 @@ struct RnnBwdStage {
 // v1 step:                 g = gy + g_h ; dz = h_t .* (g - <h_t, g>) ; G += h_{t-1} (x) dz ; g_h = S_t dz ; delta block
 template <int D, int SPLIT, int TC, bool V1>
 __global__ void __launch_bounds__(D * SPLIT * slots_for(D * SPLIT)) rnn_bwd_kernel(const RnnBwdParams p) {
+    griddep_wait();               // launched as a dependent: global memory is touched from here on
+    griddep_launch_dependents();
     using G = Geo<D, SPLIT>;
     const G g;
     const int n = g.seq / p.H, h = g.seq - n * p.H;
@@ -286,26 +290,12 @@ __global__ void __launch_bounds__(D * SPLIT * slots_for(D * SPLIT)) rnn_bwd_kern
 namespace fwp {
 
 // ------------------------------------------------------------------ launchers
-template <typename K>
-static int smem_optin(K kernel, size_t bytes) {
-    if (bytes > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        if (e != cudaSuccess) return set_cuda_error(e);
-    }
-    return FWP_OK;
-}
-
 template <int D, int SPLIT, int TC, bool V1>
 static int launch_rnn_fwd(const RnnFwdParams& p, int nseq, cudaStream_t st) {
     auto kern = rnn_fwd_kernel<D, SPLIT, TC, V1>;
     const size_t bytes = (2 * RnnFwdStage<D, TC>::kFloats + 2 * (D + 16)) * sizeof(float);
     const int slots = spread_slots(slots_for(D * SPLIT), nseq);
-    if (int rc = smem_optin(kern, bytes * slots)) return rc;
-    kern<<<nseq / slots, D * SPLIT * slots, bytes * slots, st>>>(p);
-    count_launch();
-    note_kernel("rnn_fwd_kernel");
-    cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? FWP_OK : set_cuda_error(e);
+    return launch_dependent(kern, p, nseq / slots, D * SPLIT * slots, bytes * slots, st, "rnn_fwd_kernel");
 }
 
 template <int D, int SPLIT, int TC, bool V1>
@@ -313,12 +303,7 @@ static int launch_rnn_bwd(const RnnBwdParams& p, int nseq, cudaStream_t st) {
     auto kern = rnn_bwd_kernel<D, SPLIT, TC, V1>;
     const size_t bytes = (2 * RnnBwdStage<D, TC, V1>::kFloats + 2 * (3 * D + 24)) * sizeof(float);
     const int slots = spread_slots(slots_for(D * SPLIT), nseq);
-    if (int rc = smem_optin(kern, bytes * slots)) return rc;
-    kern<<<nseq / slots, D * SPLIT * slots, bytes * slots, st>>>(p);
-    count_launch();
-    note_kernel("rnn_bwd_kernel");
-    cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? FWP_OK : set_cuda_error(e);
+    return launch_dependent(kern, p, nseq / slots, D * SPLIT * slots, bytes * slots, st, "rnn_bwd_kernel");
 }
 
 template <int TC, bool V1>
@@ -326,12 +311,7 @@ static int launch_rnn_bwd_roles32(const RnnBwdParams& p, int nseq, cudaStream_t 
     auto kern = rnn_bwd_roles32_kernel<TC, V1>;
     const int slots = spread_slots(4, nseq);
     const size_t bytes = (size_t)RnnRolesSmem<TC, V1>::kFloats * sizeof(float) * slots;
-    if (int rc = smem_optin(kern, bytes)) return rc;
-    kern<<<nseq / slots, 96 * slots, bytes, st>>>(p);
-    count_launch();
-    note_kernel("rnn_bwd_roles32_kernel");
-    cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? FWP_OK : set_cuda_error(e);
+    return launch_dependent(kern, p, nseq / slots, 96 * slots, bytes, st, "rnn_bwd_roles32_kernel");
 }
 
 template <bool V1>

@@ -30,6 +30,8 @@ struct RnnRolesSmem {
 
 template <int TC, bool V1>
 __global__ void __launch_bounds__(384, 1) rnn_bwd_roles32_kernel(const RnnBwdParams p) {
+    griddep_wait();               // launched as a dependent: global memory is touched from here on
+    griddep_launch_dependents();
     constexpr int D = 32, NP = 16, NT = 96;
     using SM = RnnRolesSmem<TC, V1>;
     using Stage = typename SM::Stage;
