@@ -169,6 +169,13 @@ int fwp_delta_layer_prologue_forward(int L, int B, int H, int D, const float* qk
 int fwp_delta_layer_prologue_backward(int L, int B, int H, int D, const float* qkvb,
                                       const float* grad_q, const float* grad_k, const float* grad_v,
                                       const float* grad_beta, float* grad_qkvb, void* stream, int device);
+/* the same with queries q_scale * q, and their gradient: a layer that scales its output can scale the queries instead, and let
+ * the delta rule write and read (L,B,H,D) tensors through strides */
+int fwp_delta_layer_prologue_forward_scaled(int L, int B, int H, int D, const float* qkvb,
+                                            float* q, float* k, float* v, float* beta, float q_scale, void* stream, int device);
+int fwp_delta_layer_prologue_backward_scaled(int L, int B, int H, int D, const float* qkvb,
+                                             const float* grad_q, const float* grad_k, const float* grad_v,
+                                             const float* grad_beta, float* grad_qkvb, float q_scale, void* stream, int device);
 int fwp_delta_layer_transpose(int L, int B, int H, int D, const float* src, float* dst, float scale,
                               int to_len_major, void* stream, int device);
 

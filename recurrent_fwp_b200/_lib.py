@@ -62,6 +62,8 @@ SIGNATURES = {
     'fwp_fast_lstm_forward': [_i] * 5 + [_T3] * 4 + [_T, _T, _T3, _T, _T, _T, _T3, _T3] + [_i, _vp, _i],
     'fwp_delta_layer_prologue_forward': [_i] * 4 + [ctypes.c_void_p] * 5 + [_vp, _i],
     'fwp_delta_layer_prologue_backward': [_i] * 4 + [ctypes.c_void_p] * 6 + [_vp, _i],
+    'fwp_delta_layer_prologue_forward_scaled': [_i] * 4 + [ctypes.c_void_p] * 5 + [ctypes.c_float, _vp, _i],
+    'fwp_delta_layer_prologue_backward_scaled': [_i] * 4 + [ctypes.c_void_p] * 6 + [ctypes.c_float, _vp, _i],
     'fwp_delta_layer_transpose': [_i] * 4 + [ctypes.c_void_p] * 2 + [ctypes.c_float, _i, _vp, _i],
     'fwp_debug_bounded_wait_probe': [_i, _vp, _i],
     'fwp_delayed': [_i] * 4 + [_T] * 4 + [_i, _vp, _i],

@@ -163,12 +163,12 @@ std::shared_ptr<NodeT> make_node(const std::array<const Tensor*, K>& in, const D
 
 // ------------------------------------------------------------------ delta rule
 // the backward with the scratch memory it asks for
-void delta_backward(const Dims& d, const Tensor& Q, const Tensor& K, const Tensor& V, const Tensor& beta, const Tensor& v_old, const Tensor& gy,
+void delta_backward(const Dims& d, const Tensor& Q, const Tensor& K, const Tensor& V, const Tensor& beta, const Tensor& v_old, const Desc& gy,
                     const Tensor& W, const Tensor& gQ, const Tensor& gK, const Tensor& gV, const Tensor& gb) {
     const int64_t need = fwp_fast_weight_backward_scratch_floats(d.N, d.H, d.L, d.E, d.M, dtype_code(Q));
     Tensor scratch;
     if (need > 0) scratch = empty({need}, at::kFloat, Q);
-    check_delta(fwp_fast_weight_backward_with_scratch(d.N, d.H, d.L, d.E, d.M, Desc(Q), Desc(K), Desc(V), Desc(beta), Desc(v_old), Desc(gy),
+    check_delta(fwp_fast_weight_backward_with_scratch(d.N, d.H, d.L, d.E, d.M, Desc(Q), Desc(K), Desc(V), Desc(beta), Desc(v_old), gy,
                                                       Desc(W), Desc(gQ), Desc(gK), Desc(gV), Desc(gb),
                                                       need > 0 ? scratch.data_ptr<float>() : nullptr, need, dtype_code(Q), stream_of(Q),
                                                       Q.device().index()), "fast_weight_backward");
@@ -183,7 +183,7 @@ struct DeltaNode final : public OpNode {
         const Tensor &Q = t[0], &K = t[1], &V = t[2], &beta = t[3], &W = t[4];
         const Tensor gy = incoming(g[0], Q, {d.N, d.H, d.L, d.M});
         Tensor gQ = like_stream(d.E, Q), gK = like_stream(d.E, Q), gV = like_stream(d.M, Q), gb = like_stream(1, Q);
-        delta_backward(d, Q, K, V, beta, own[0], gy, W, gQ, gK, gV, gb);
+        delta_backward(d, Q, K, V, beta, own[0], Desc(gy), W, gQ, gK, gV, gb);
         return {gQ, gK, gV, gb, Tensor()};
     }
 };
@@ -222,6 +222,17 @@ PyObject* fast_weight_delta(PyObject*, PyObject* const* args, Py_ssize_t n) {
 }
 
 // ------------------------------------- delta-rule attention layer: prologue, delta rule, epilogue in one node
+// The layer's scale goes into the queries, and the delta rule writes its output (and reads the incoming gradient) as the
+// (len, B, H, D) tensor it is: no transposing pass on either side (two of 8 us each at 256 sequences x 512 steps, D = 32).
+Desc heads_first(const Tensor& t, const Dims& d) {
+    Desc r(Tensor{});
+    r.d.data = t.data_ptr();
+    r.d.stride[0] = d.H * d.M;
+    r.d.stride[1] = d.M;
+    r.d.stride[2] = d.N * d.H * d.M;
+    r.d.stride[3] = 1;
+    return r;
+}
 struct DeltaLayerNode final : public OpNode {
     double scale = 1;
     std::string name() const override { return "DeltaAttentionBackward"; }
@@ -234,13 +245,12 @@ struct DeltaLayerNode final : public OpNode {
         const Tensor gout = g[0].contiguous();
         void* st = stream_of(x);
         const int dev = x.device().index();
-        Tensor gy = empty(d, d.M, x), gq = empty(d, d.E, x), gk = empty(d, d.E, x), gv = empty(d, d.M, x), gb = empty(d, 1, x);
-        check(fwp_delta_layer_transpose(d.L, d.N, d.H, d.M, gout.data_ptr<float>(), gy.data_ptr<float>(), (float)scale, 0, st, dev),
-              "delta_layer_transpose");
+        const Desc gy = heads_first(gout, d);
+        Tensor gq = empty(d, d.E, x), gk = empty(d, d.E, x), gv = empty(d, d.M, x), gb = empty(d, 1, x);
         delta_backward(d, q, k, v, beta, v_old, gy, W, gq, gk, gv, gb);
         Tensor gx = empty({d.L, d.N, d.H, 3 * d.E + 1}, at::kFloat, x);
-        check(fwp_delta_layer_prologue_backward(d.L, d.N, d.H, d.E, x.data_ptr<float>(), gq.data_ptr<float>(), gk.data_ptr<float>(),
-                                                gv.data_ptr<float>(), gb.data_ptr<float>(), gx.data_ptr<float>(), st, dev),
+        check(fwp_delta_layer_prologue_backward_scaled(d.L, d.N, d.H, d.E, x.data_ptr<float>(), gq.data_ptr<float>(), gk.data_ptr<float>(),
+                                                       gv.data_ptr<float>(), gb.data_ptr<float>(), gx.data_ptr<float>(), (float)scale, st, dev),
               "delta_layer_prologue_backward");
         return {gx, Tensor()};
     }
@@ -262,16 +272,15 @@ PyObject* delta_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
         pybind11::gil_scoped_release no_gil;
         void* st = stream_of(x);
         const int dev = x.device().index();
-        Tensor q = empty(d, D, x), k = empty(d, D, x), v = empty(d, D, x), beta = empty(d, 1, x), y = empty(d, D, x), v_old;
+        Tensor q = empty(d, D, x), k = empty(d, D, x), v = empty(d, D, x), beta = empty(d, 1, x), v_old;
+        out = empty({d.L, d.N, d.H * D}, at::kFloat, x);
         const bool grad = needs_grad(in);
         if (grad) v_old = empty(d, D, x);
-        check(fwp_delta_layer_prologue_forward(d.L, d.N, d.H, D, x.data_ptr<float>(), q.data_ptr<float>(), k.data_ptr<float>(),
-                                               v.data_ptr<float>(), beta.data_ptr<float>(), st, dev), "delta_layer_prologue_forward");
+        check(fwp_delta_layer_prologue_forward_scaled(d.L, d.N, d.H, D, x.data_ptr<float>(), q.data_ptr<float>(), k.data_ptr<float>(),
+                                                      v.data_ptr<float>(), beta.data_ptr<float>(), (float)scale, st, dev),
+              "delta_layer_prologue_forward");
         check_delta(fwp_fast_weight_forward(d.N, d.H, d.L, D, D, Desc(q), Desc(k), Desc(v), Desc(beta), Desc(v_old), Desc(Tensor()),
-                                            Desc(W), Desc(y), FWP_F32, st, dev), "fast_weight_forward");
-        out = empty({d.L, d.N, d.H * D}, at::kFloat, x);
-        check(fwp_delta_layer_transpose(d.L, d.N, d.H, D, y.data_ptr<float>(), out.data_ptr<float>(), (float)scale, 1, st, dev),
-              "delta_layer_transpose");
+                                            Desc(W), heads_first(out, d), FWP_F32, st, dev), "fast_weight_forward");
         if (grad) {
             auto node = make_node<DeltaLayerNode>(in, d);
             node->save(x);

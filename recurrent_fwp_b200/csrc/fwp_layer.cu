@@ -23,6 +23,26 @@ struct LayerDims {
     int L, B, H, D;
     long long rows;     // L * B * H
 };
+struct PrologueParams {
+    const float* qkvb;
+    float *q, *k, *v, *beta;
+    float scale;        // of the queries
+    LayerDims d;
+};
+struct PrologueGradParams {
+    const float *qkvb, *gq, *gk, *gv, *gbeta;
+    float* gx;
+    float scale;
+    LayerDims d;
+};
+struct TransposeParams {
+    const float* src;
+    float* dst;
+    LayerDims d;
+    int per_row;
+    float scale;
+    int to_len_major;
+};
 
 // elu(x) + 1 = x + 1 for x > 0, exp(x) otherwise
 __device__ __forceinline__ float elu_p1(float x) { return x > 0.f ? x + 1.f : expf(x); }
@@ -48,9 +68,12 @@ __device__ __forceinline__ float row_sum(float x) {
 constexpr int kLayerPer = 4;
 
 template <int LPR, int PASSES>
-__global__ void __launch_bounds__(kLayerWarps * 32) layer_prologue_fwd_kernel(const float* __restrict__ qkvb, float* __restrict__ q,
-                                                                               float* __restrict__ k, float* __restrict__ v,
-                                                                               float* __restrict__ beta, const LayerDims d) {
+__global__ void __launch_bounds__(kLayerWarps * 32) layer_prologue_fwd_kernel(const PrologueParams p) {
+    griddep_wait();
+    griddep_launch_dependents();
+    const LayerDims& d = p.d;
+    const float* __restrict__ qkvb = p.qkvb;
+    float *__restrict__ q = p.q, *__restrict__ k = p.k, *__restrict__ v = p.v, *__restrict__ beta = p.beta;
     constexpr int RPW = 32 / LPR;       // rows per warp and pass
     const int lane = threadIdx.x & 31, sub = lane % LPR, D = d.D;
     const long long r0 = ((long long)blockIdx.x * kLayerWarps + (threadIdx.x >> 5)) * (RPW * PASSES) + lane / LPR;
@@ -84,7 +107,7 @@ __global__ void __launch_bounds__(kLayerWarps * 32) layer_prologue_fwd_kernel(co
             sq += xq[a][j];
             sk += xk[a][j];
         }
-        const float iq = 1.f / row_sum<LPR>(sq), ik = 1.f / row_sum<LPR>(sk);
+        const float iq = p.scale / row_sum<LPR>(sq), ik = 1.f / row_sum<LPR>(sk);
         if (!live) continue;
 #pragma unroll
         for (int j = 0; j < kLayerPer; j++) {
@@ -99,12 +122,15 @@ __global__ void __launch_bounds__(kLayerWarps * 32) layer_prologue_fwd_kernel(co
     }
 }
 
-// y = p / s with p = elu(x)+1:  dL/dx_i = (g_i - sum_j g_j y_j) / s * (x_i > 0 ? 1 : p_i);  sigmoid: g * b * (1 - b)
+// y = p / s with p = elu(x)+1:  dL/dx_i = (g_i - sum_j g_j y_j) / s * (x_i > 0 ? 1 : p_i);  sigmoid: g * b * (1 - b).  The
+// queries are scale * y, so their gradient comes in as g / scale.
 template <int LPR>
-__global__ void __launch_bounds__(kLayerWarps * 32) layer_prologue_bwd_kernel(const float* __restrict__ qkvb, const float* __restrict__ gq,
-                                                                               const float* __restrict__ gk, const float* __restrict__ gv,
-                                                                               const float* __restrict__ gbeta, float* __restrict__ gx,
-                                                                               const LayerDims d) {
+__global__ void __launch_bounds__(kLayerWarps * 32) layer_prologue_bwd_kernel(const PrologueGradParams p) {
+    griddep_wait();
+    griddep_launch_dependents();
+    const LayerDims& d = p.d;
+    const float *__restrict__ qkvb = p.qkvb, *__restrict__ gq = p.gq, *__restrict__ gk = p.gk, *__restrict__ gv = p.gv, *__restrict__ gbeta = p.gbeta;
+    float* __restrict__ gx = p.gx;
     constexpr int RPW = 32 / LPR;
     const int lane = threadIdx.x & 31, sub = lane % LPR, D = d.D;
     const long long r = ((long long)blockIdx.x * kLayerWarps + (threadIdx.x >> 5)) * RPW + lane / LPR;
@@ -118,7 +144,7 @@ __global__ void __launch_bounds__(kLayerWarps * 32) layer_prologue_bwd_kernel(co
         const bool ok = live && i < D;
         xq[j] = ok ? x[i] : 0.f;
         xk[j] = ok ? x[D + i] : 0.f;
-        aq[j] = ok ? gq[o * D + i] : 0.f;
+        aq[j] = ok ? p.scale * gq[o * D + i] : 0.f;
         ak[j] = ok ? gk[o * D + i] : 0.f;
         av[j] = ok ? gv[o * D + i] : 0.f;
     }
@@ -159,8 +185,14 @@ __global__ void __launch_bounds__(kLayerWarps * 32) layer_prologue_bwd_kernel(co
 // (B, H, len, D) <-> (len, B, H, D) with a scale: dst row of one side = scale * src row of the other.
 // One thread per 16-byte piece (4-byte piece when D is not a multiple of 4), kLayerRows pieces per thread.
 template <typename V>
-__global__ void __launch_bounds__(kLayerWarps * 32) layer_transpose_kernel(const V* __restrict__ src, V* __restrict__ dst,
-                                                                            const LayerDims d, int per_row, float scale, int to_len_major) {
+__global__ void __launch_bounds__(kLayerWarps * 32) layer_transpose_kernel(const TransposeParams p) {
+    griddep_wait();
+    griddep_launch_dependents();
+    const V* __restrict__ src = reinterpret_cast<const V*>(p.src);
+    V* __restrict__ dst = reinterpret_cast<V*>(p.dst);
+    const LayerDims& d = p.d;
+    const int per_row = p.per_row, to_len_major = p.to_len_major;
+    const float scale = p.scale;
     const long long total = d.rows * per_row;
     const long long i0 = ((long long)blockIdx.x * kLayerRows) * (kLayerWarps * 32) + threadIdx.x;
     V x[kLayerRows];
@@ -209,6 +241,8 @@ struct DelayedParams {
 };
 template <typename V>
 __global__ void __launch_bounds__(256) delayed_kernel(const DelayedParams p) {
+    griddep_wait();
+    griddep_launch_dependents();
     const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
     if (i >= p.total) return;
     constexpr int W = sizeof(V) / 4;
@@ -243,38 +277,36 @@ static int layer_dims(int L, int B, int H, int D, LayerDims& d) {
     return FWP_OK;
 }
 
-static int finish_launch() {
-    count_launch();
-    cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? FWP_OK : set_cuda_error(e);
-}
-
 }  // namespace fwp
 
 using namespace fwp;
 
-FWP_API int fwp_delta_layer_prologue_forward(int L, int B, int H, int D, const float* qkvb,
-                                             float* q, float* k, float* v, float* beta, void* stream, int device) {
-    LayerDims d;
-    if (int rc = layer_dims(L, B, H, D, d)) return rc;
+FWP_API int fwp_delta_layer_prologue_forward_scaled(int L, int B, int H, int D, const float* qkvb, float* q, float* k, float* v,
+                                                    float* beta, float q_scale, void* stream, int device) {
+    PrologueParams p = {qkvb, q, k, v, beta, q_scale, {}};
+    if (int rc = layer_dims(L, B, H, D, p.d)) return rc;
     if (!qkvb || !q || !k || !v || !beta) return FWP_ERR_NULL;
     if ((reinterpret_cast<uintptr_t>(qkvb) | reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) |
          reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(beta)) & 3) return FWP_ERR_ALIGN;
     DeviceGuard guard(device);
     if (guard.status) return guard.status;
     cudaStream_t st = (cudaStream_t)stream;
-    auto grid = [&](int rows_per_warp) { return (int)((d.rows + kLayerWarps * rows_per_warp - 1) / (kLayerWarps * rows_per_warp)); };
-    if (D <= 32) layer_prologue_fwd_kernel<8, 2><<<grid(8), kLayerWarps * 32, 0, st>>>(qkvb, q, k, v, beta, d);
-    else if (D <= 64) layer_prologue_fwd_kernel<16, 2><<<grid(4), kLayerWarps * 32, 0, st>>>(qkvb, q, k, v, beta, d);
-    else layer_prologue_fwd_kernel<32, 2><<<grid(2), kLayerWarps * 32, 0, st>>>(qkvb, q, k, v, beta, d);
-    return finish_launch();
+    auto grid = [&](int rows_per_warp) { return (int)((p.d.rows + kLayerWarps * rows_per_warp - 1) / (kLayerWarps * rows_per_warp)); };
+    if (D <= 32) return launch_dependent(layer_prologue_fwd_kernel<8, 2>, p, grid(8), kLayerWarps * 32, 0, st, nullptr);
+    if (D <= 64) return launch_dependent(layer_prologue_fwd_kernel<16, 2>, p, grid(4), kLayerWarps * 32, 0, st, nullptr);
+    return launch_dependent(layer_prologue_fwd_kernel<32, 2>, p, grid(2), kLayerWarps * 32, 0, st, nullptr);
 }
 
-FWP_API int fwp_delta_layer_prologue_backward(int L, int B, int H, int D, const float* qkvb,
-                                              const float* grad_q, const float* grad_k, const float* grad_v,
-                                              const float* grad_beta, float* grad_qkvb, void* stream, int device) {
-    LayerDims d;
-    if (int rc = layer_dims(L, B, H, D, d)) return rc;
+FWP_API int fwp_delta_layer_prologue_forward(int L, int B, int H, int D, const float* qkvb,
+                                             float* q, float* k, float* v, float* beta, void* stream, int device) {
+    return fwp_delta_layer_prologue_forward_scaled(L, B, H, D, qkvb, q, k, v, beta, 1.f, stream, device);
+}
+
+FWP_API int fwp_delta_layer_prologue_backward_scaled(int L, int B, int H, int D, const float* qkvb,
+                                                     const float* grad_q, const float* grad_k, const float* grad_v,
+                                                     const float* grad_beta, float* grad_qkvb, float q_scale, void* stream, int device) {
+    PrologueGradParams p = {qkvb, grad_q, grad_k, grad_v, grad_beta, grad_qkvb, q_scale, {}};
+    if (int rc = layer_dims(L, B, H, D, p.d)) return rc;
     if (!qkvb || !grad_q || !grad_k || !grad_v || !grad_beta || !grad_qkvb) return FWP_ERR_NULL;
     if ((reinterpret_cast<uintptr_t>(qkvb) | reinterpret_cast<uintptr_t>(grad_q) | reinterpret_cast<uintptr_t>(grad_k) |
          reinterpret_cast<uintptr_t>(grad_v) | reinterpret_cast<uintptr_t>(grad_beta) | reinterpret_cast<uintptr_t>(grad_qkvb)) & 3)
@@ -282,11 +314,16 @@ FWP_API int fwp_delta_layer_prologue_backward(int L, int B, int H, int D, const 
     DeviceGuard guard(device);
     if (guard.status) return guard.status;
     cudaStream_t st = (cudaStream_t)stream;
-    auto grid = [&](int rows_per_warp) { return (int)((d.rows + kLayerWarps * rows_per_warp - 1) / (kLayerWarps * rows_per_warp)); };
-    if (D <= 32) layer_prologue_bwd_kernel<8><<<grid(4), kLayerWarps * 32, 0, st>>>(qkvb, grad_q, grad_k, grad_v, grad_beta, grad_qkvb, d);
-    else if (D <= 64) layer_prologue_bwd_kernel<16><<<grid(2), kLayerWarps * 32, 0, st>>>(qkvb, grad_q, grad_k, grad_v, grad_beta, grad_qkvb, d);
-    else layer_prologue_bwd_kernel<32><<<grid(1), kLayerWarps * 32, 0, st>>>(qkvb, grad_q, grad_k, grad_v, grad_beta, grad_qkvb, d);
-    return finish_launch();
+    auto grid = [&](int rows_per_warp) { return (int)((p.d.rows + kLayerWarps * rows_per_warp - 1) / (kLayerWarps * rows_per_warp)); };
+    if (D <= 32) return launch_dependent(layer_prologue_bwd_kernel<8>, p, grid(4), kLayerWarps * 32, 0, st, nullptr);
+    if (D <= 64) return launch_dependent(layer_prologue_bwd_kernel<16>, p, grid(2), kLayerWarps * 32, 0, st, nullptr);
+    return launch_dependent(layer_prologue_bwd_kernel<32>, p, grid(1), kLayerWarps * 32, 0, st, nullptr);
+}
+
+FWP_API int fwp_delta_layer_prologue_backward(int L, int B, int H, int D, const float* qkvb,
+                                              const float* grad_q, const float* grad_k, const float* grad_v,
+                                              const float* grad_beta, float* grad_qkvb, void* stream, int device) {
+    return fwp_delta_layer_prologue_backward_scaled(L, B, H, D, qkvb, grad_q, grad_k, grad_v, grad_beta, grad_qkvb, 1.f, stream, device);
 }
 
 FWP_API int fwp_delta_layer_transpose(int L, int B, int H, int D, const float* src, float* dst, float scale,
@@ -303,12 +340,9 @@ FWP_API int fwp_delta_layer_transpose(int L, int B, int H, int D, const float* s
     const long long ctas = (d.rows * per_row + per_cta - 1) / per_cta;
     if (ctas > 0x7fffffffLL) return FWP_ERR_SHAPE;
     cudaStream_t st = (cudaStream_t)stream;
-    if ((D & 3) == 0)
-        layer_transpose_kernel<float4><<<(int)ctas, kLayerWarps * 32, 0, st>>>(reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst),
-                                                                              d, per_row, scale, to_len_major ? 1 : 0);
-    else
-        layer_transpose_kernel<float><<<(int)ctas, kLayerWarps * 32, 0, st>>>(src, dst, d, per_row, scale, to_len_major ? 1 : 0);
-    return finish_launch();
+    const TransposeParams p = {src, dst, d, per_row, scale, to_len_major ? 1 : 0};
+    if ((D & 3) == 0) return launch_dependent(layer_transpose_kernel<float4>, p, (int)ctas, kLayerWarps * 32, 0, st, nullptr);
+    return launch_dependent(layer_transpose_kernel<float>, p, (int)ctas, kLayerWarps * 32, 0, st, nullptr);
 }
 
 FWP_API int fwp_delayed(int N, int H, int L, int D, const fwp_tensor* src, const fwp_tensor* first,
@@ -339,7 +373,6 @@ FWP_API int fwp_delayed(int N, int H, int L, int D, const fwp_tensor* src, const
     const long long ctas = (p.total + 255) / 256;
     if (ctas > 0x7fffffffLL) return FWP_ERR_SHAPE;
     cudaStream_t st = (cudaStream_t)stream;
-    if (vec) delayed_kernel<float4><<<(int)ctas, 256, 0, st>>>(p);
-    else delayed_kernel<float><<<(int)ctas, 256, 0, st>>>(p);
-    return finish_launch();
+    return vec ? launch_dependent(delayed_kernel<float4>, p, (int)ctas, 256, 0, st, nullptr)
+               : launch_dependent(delayed_kernel<float>, p, (int)ctas, 256, 0, st, nullptr);
 }
