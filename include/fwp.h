@@ -84,7 +84,7 @@ unsigned long long fwp_launch_count(void);
  * "lstm_bwd.32.roles" (1 / 0: chain-warp + per-gate trailing-warp backward of the delta LSTM),
  * "lstm_fwd.32.gates" (1 / 0: one-warp-per-gate forward of the delta LSTM),
  * "rec_bwd.32.roles" (1 / 0: chain-warp + trailing-warp backward of the recurrent delta net),
- * "sum_bwd.roles" (1 / 0: the three gradients of the sum rule computed side by side by warps of their own, or one
+ * "sum_bwd.roles" (-1 automatic; 2: three chunkwise forwards in one launch, up to head size 64; 1 / 0: the three gradients of the sum rule computed side by side by warps of their own, or one
  * after the other by the same warps),
  * "step.spread" (1 / 0: the per-step forward packs fewer sequences into a CTA while that puts CTAs on more SMs, or
  * always four warps per CTA),

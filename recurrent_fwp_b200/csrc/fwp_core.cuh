@@ -63,7 +63,7 @@ enum TuneKey {
     T_LSTM_FWD_GATES32,     // "lstm_fwd.32.gates": 1 one-warp-per-gate forward of the delta LSTM at d = 32, 0 the general kernel
     T_DELTA_PIPE64,         // "delta.pipe64": 1 chunkwise bf16 forward with a preparing warp one chunk ahead, 0 every warp prepares for itself
     T_REC_BWD_ROLES32,      // "rec_bwd.32.roles": 1 chain-warp + trailing-warp backward of the recurrent delta net at d = 32, 0 the general kernel
-    T_SUM_BWD_ROLES,        // "sum_bwd.roles": 1 the three gradients of the sum rule in warps of their own, side by side; 0 one after the other
+    T_SUM_BWD_ROLES,        // "sum_bwd.roles": -1 automatic, 2 three chunkwise forwards in one launch, 1 the three gradients of the sum rule in warps of their own, side by side; 0 one after the other
     T_LAUNCH_DEPENDENT,     // "launch.dependent": 1 the register-resident delta-rule kernels (blocked and per-step) are launched with programmatic stream serialisation (their prologue overlaps the tail of the kernel before), 0 plain launches
     T_STEP_SPREAD,          // "step.spread": 1 the per-step forward packs fewer sequences into a CTA while that puts CTAs on more SMs, 0 always four warps per CTA
     T_DELTA_WY,             // "delta.wy": -1 automatic, 1 / 0 the chunkwise split-product plan (fwp_delta_wy.cuh) wherever it has an instance, or never
@@ -760,7 +760,7 @@ static int set_smem(K kernel, size_t bytes) {
 
 // `name` (a string literal) is what fwp_last_kernel() reports for the calling thread afterwards; nullptr leaves that as it is.
 template <typename K, typename P>
-static int launch(K kern, const P& p, int grid, int threads, size_t bytes, cudaStream_t st, const char* name) {
+static int launch(K kern, const P& p, dim3 grid, int threads, size_t bytes, cudaStream_t st, const char* name) {
     if (int rc = set_smem(kern, bytes)) return rc;
     kern<<<grid, threads, bytes, st>>>(p);
     count_launch();
@@ -773,11 +773,11 @@ static int launch(K kern, const P& p, int grid, int threads, size_t bytes, cudaS
 // may be scheduled while the kernel before them in the stream drains ("launch.dependent" = 0: a plain launch).  The
 // call itself is cheaper too: 2.4 us of host time against 4.
 template <typename K, typename P>
-static int launch_dependent(K kern, const P& p, int grid, int threads, size_t bytes, cudaStream_t st, const char* name) {
+static int launch_dependent(K kern, const P& p, dim3 grid, int threads, size_t bytes, cudaStream_t st, const char* name) {
     if (!tune_get(T_LAUNCH_DEPENDENT, 1)) return launch(kern, p, grid, threads, bytes, st, name);
     if (int rc = set_smem(kern, bytes)) return rc;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = bytes;
     cfg.stream = st;

@@ -248,12 +248,6 @@ __global__ void __launch_bounds__(D * SPLIT * slots_for(D * SPLIT)) delta_bwd_st
 
 // sum-rule backward: dq_t = S_t gy_t with S accumulated forwards from zero,
 // dk_t = G_t v_t, dv_t = G_t^T k_t with G accumulated backwards (causal_product_cuda.cu:369-445).
-struct SumBwdParams {
-    Row4 q, k, v, gy, gq, gk, gv;
-    int H, L, E, M;
-    int NH;     // number of sequences (N*H)
-};
-
 template <int D, int TC, typename T>
 struct SumStage {
     Tile<D, TC, T> q, k, v, gy;
@@ -640,9 +634,26 @@ static int dispatch_bwd(const DeltaBwdParams& p0, int nseq, cudaStream_t st) {
     return FWP_ERR_UNSUPPORTED;
 }
 
+// Where the sum rule's backward is faster as three chunkwise forwards in one launch, from measurements on B200 (256 steps, us,
+// three roles on vector units -> three forwards on split products):
+//   d = 16: 16 sequences 34 -> 7, 144 34 -> 16, 256 34 -> 24, 512 35 -> 39;  rows of 12: 512 53 -> 44, 1536 155 -> 110
+//   d = 32: 16 62 -> 14, 512 105 -> 67, 1536 296 -> 186;  d = 64: 16 143 -> 21, 512 565 -> 190;  d = 48: 512 635 -> 151
+//   bf16: d = 16 16 52 -> 19, 512 53 -> 64; d = 64 512 645 -> 226
+//   20 steps: d = 32 64 7.4 -> 3.6, 512 11 -> 13; d = 64 512 51 -> 36;  17 steps: d = 16 512 6.1 -> 7.2
+static bool sum_bwd_wy_pays(const SumBwdParams& p, int nseq) {
+    const int d = p.E > p.M ? p.E : p.M;
+    if (d > 64 || p.L <= kShortSeq) return false;
+    if (nseq <= 2 * sm_count()) return true;
+    return d > 32 || (p.L > 2 * kShortSeq && !(p.E == 16 && p.M == 16));
+}
 template <typename T>
 static int dispatch_sum_bwd(const SumBwdParams& p, int nseq, cudaStream_t st) {
     const int D = pad_dim(p.E > p.M ? p.E : p.M);
+    const int roles = tune_get(T_SUM_BWD_ROLES, -1);
+    if (roles == 2 || (roles == -1 && sum_bwd_wy_pays(p, nseq))) {
+        const int rc = launch_sum_bwd_wy<T>(p, nseq, st);
+        if (rc >= 0) return rc;
+    }
     if (D == 0) return launch_sum_bwd_generic<T>(p, nseq, st);
     switch (D) {
         case 16: return launch_sum_bwd<16, 2, 16, T>(p, nseq, st);
@@ -831,7 +842,7 @@ FWP_API int fwp_delta_device_fault(void) {
         const int zero = 0;
         cudaMemcpyToSymbol(fwp::g_delta_fault, &zero, sizeof zero);
     }
-    const int t = fwp::tc_fault_read_clear(), w = fwp::wy_fault_read_clear();
-    if (t < 0 || w < 0) return -1;
-    return (v || t || w) ? 1 : 0;
+    const int t = fwp::tc_fault_read_clear(), w = fwp::wy_fault_read_clear(), u = fwp::sum_wy_fault_read_clear();
+    if (t < 0 || w < 0 || u < 0) return -1;
+    return (v || t || w || u) ? 1 : 0;
 }

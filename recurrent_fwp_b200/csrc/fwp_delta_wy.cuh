@@ -23,6 +23,13 @@
 namespace fwp {
 namespace wy {
 
+// The sum rule's three gradients are sum-rule forwards of other streams, two of them backwards in time (negative strides):
+//   dq_t = sum_{i<=t} (gy_t . v_i) k_i,   dv_t = sum_{i>=t} (k_t . q_i) gy_i,   dk_t = sum_{i>=t} (v_t . gy_i) q_i
+// from states that start at zero.  One launch runs the three side by side.
+struct SumBwdForwards {
+    DeltaFwdParams p[3];
+};
+
 static __device__ int g_wy_fault;       // a bounded wait ran out (read by fwp_delta_device_fault)
 
 __device__ __forceinline__ void arrive(unsigned long long* bar) {
@@ -158,7 +165,7 @@ struct FewBuf {
 };
 
 template <int E, int M, int NB, typename T, bool SUM>
-__global__ void __launch_bounds__((M / 16 + NB) * 32) delta_fwd_wy_few_kernel(const DeltaFwdParams p) {
+__device__ __forceinline__ void fwd_few(const DeltaFwdParams& p) {
     constexpr int NCW = M / 16, KS = E / 16, NP = stream_parts<T>();
     using Buf = FewBuf<E, M, NP>;
     constexpr int P = Buf::P, PR = Buf::PR, PV = Buf::PV, kPart = C * P * 2, kPartC = C * PC * 2;
@@ -210,14 +217,14 @@ __global__ void __launch_bounds__((M / 16 + NB) * 32) delta_fwd_wy_few_kernel(co
 
     if (warp < NCW) {
         const int m0 = warp * 16, width = p.M - m0;
-        float* W = p.W + n * p.wN + h * p.wH + m0;
+        float* W = p.W ? p.W + n * p.wN + h * p.wH + m0 : nullptr;    // none: a state that starts at zero and is not asked for
         float S[2 * KS][4];             // S[j]: state rows e = 8j + 2t, 8j + 2t + 1 of columns m = g, g + 8
 #pragma unroll
         for (int j = 0; j < 2 * KS; j++)
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 const int e = 8 * j + 2 * t + (i & 1), m = g + 8 * (i >> 1);
-                S[j][i] = e < p.E && m < width ? W[(long long)e * p.wE + m] : 0.f;
+                S[j][i] = W && e < p.E && m < width ? W[(long long)e * p.wE + m] : 0.f;
             }
         int b = 0, st = 0;
         unsigned phase = 0;
@@ -272,7 +279,7 @@ __global__ void __launch_bounds__((M / 16 + NB) * 32) delta_fwd_wy_few_kernel(co
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 const int e = 8 * j + 2 * t + (i & 1), m = g + 8 * (i >> 1);
-                if (e < p.E && m < width) W[(long long)e * p.wE + m] = S[j][i];
+                if (W && e < p.E && m < width) W[(long long)e * p.wE + m] = S[j][i];
             }
         return;
     }
@@ -418,6 +425,14 @@ __global__ void __launch_bounds__((M / 16 + NB) * 32) delta_fwd_wy_few_kernel(co
         __syncwarp();
     }
 }
+template <int E, int M, int NB, typename T, bool SUM>
+__global__ void __launch_bounds__((M / 16 + NB) * 32) delta_fwd_wy_few_kernel(const DeltaFwdParams p) {
+    fwd_few<E, M, NB, T, SUM>(p);
+}
+template <int E, int M, int NB, typename T, bool SUM>
+__global__ void __launch_bounds__((M / 16 + NB) * 32) sum_bwd_wy_few_kernel(const __grid_constant__ SumBwdForwards a) {
+    fwd_few<E, M, NB, T, SUM>(a.p[blockIdx.y]);
+}
 
 // --------------------------------------------------------------------------------- forward, many sequences
 // The same for many sequences: what counts is the number of resident warps, so the helpers keep nothing but operand
@@ -433,7 +448,7 @@ struct FwdBuf {
 };
 
 template <int E, int M, int NB, int CTAS, typename T, bool SUM>
-__global__ void __launch_bounds__((M / 16 + NB) * 32, CTAS) delta_fwd_wy_kernel(const DeltaFwdParams p) {
+__device__ __forceinline__ void fwd(const DeltaFwdParams& p) {
     constexpr int NCW = M / 16, KS = E / 16, NP = stream_parts<T>();
     using Buf = FwdBuf<E, NP>;
     constexpr int P = Buf::P, kPart = C * P * 2, kPartC = C * PC * 2;
@@ -456,14 +471,14 @@ __global__ void __launch_bounds__((M / 16 + NB) * 32, CTAS) delta_fwd_wy_kernel(
 
     if (warp < NCW) {
         const int m0 = warp * 16, width = p.M - m0;
-        float* W = p.W + n * p.wN + h * p.wH + m0;
+        float* W = p.W ? p.W + n * p.wN + h * p.wH + m0 : nullptr;    // none: a state that starts at zero and is not asked for
         float S[2 * KS][4];             // S[j]: state rows e = 8j + 2t, 8j + 2t + 1 of columns m = g, g + 8
 #pragma unroll
         for (int j = 0; j < 2 * KS; j++)
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 const int e = 8 * j + 2 * t + (i & 1), m = g + 8 * (i >> 1);
-                S[j][i] = e < p.E && m < width ? W[(long long)e * p.wE + m] : 0.f;
+                S[j][i] = W && e < p.E && m < width ? W[(long long)e * p.wE + m] : 0.f;
             }
         const T* vp = reinterpret_cast<const T*>(p.v.p) + n * p.v.sN + h * p.v.sH + m0 + 2 * t * p.v.sL + g;
         T* yp = reinterpret_cast<T*>(p.out.p) + n * p.out.sN + h * p.out.sH + m0 + 2 * t * p.out.sL + g;
@@ -540,7 +555,7 @@ __global__ void __launch_bounds__((M / 16 + NB) * 32, CTAS) delta_fwd_wy_kernel(
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 const int e = 8 * j + 2 * t + (i & 1), m = g + 8 * (i >> 1);
-                if (e < p.E && m < width) W[(long long)e * p.wE + m] = S[j][i];
+                if (W && e < p.E && m < width) W[(long long)e * p.wE + m] = S[j][i];
             }
         return;
     }
@@ -625,6 +640,14 @@ __global__ void __launch_bounds__((M / 16 + NB) * 32, CTAS) delta_fwd_wy_kernel(
         }
         warp_arrive(&filled[b], lane);
     }
+}
+template <int E, int M, int NB, int CTAS, typename T, bool SUM>
+__global__ void __launch_bounds__((M / 16 + NB) * 32, CTAS) delta_fwd_wy_kernel(const DeltaFwdParams p) {
+    fwd<E, M, NB, CTAS, T, SUM>(p);
+}
+template <int E, int M, int NB, int CTAS, typename T, bool SUM>
+__global__ void __launch_bounds__((M / 16 + NB) * 32, CTAS) sum_bwd_wy_kernel(const __grid_constant__ SumBwdForwards a) {
+    fwd<E, M, NB, CTAS, T, SUM>(a.p[blockIdx.y]);
 }
 
 }  // namespace wy

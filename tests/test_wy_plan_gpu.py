@@ -148,3 +148,33 @@ def test_three_launch_backward_of_bf16_streams(fwp, E, M, L):
     for got in res[:2]:
         for a, r in zip(got, res[2]):
             assert ((a - r).abs() <= 2 ** -8 * r.abs() + 1e-5 * r.abs().max()).all()
+
+
+@pytest.mark.parametrize('E,M', [(16, 16), (9, 14), (32, 32), (20, 31), (48, 48), (64, 64), (50, 33)])
+@pytest.mark.parametrize('B,H,L', [(2, 3, 1), (2, 3, 17), (2, 3, 130), (75, 2, 130)])
+def test_sum_rule_backward_as_three_forwards(fwp, E, M, B, H, L):
+    """csrc/fwp_sum_wy.cu: gradients against the sums they stand for in fp64, packed and layer-sliced streams."""
+    from recurrent_fwp_b200 import _lib
+    q, k, v, _, gy = util.delta_inputs(37, B, H, L, E, M)
+    Q, K, V, G = (t.double().to(DEV) for t in (q, k, v, gy))
+    lower = torch.tril(torch.ones(L, L, dtype=torch.float64, device=DEV))
+    A = (G @ V.transpose(-1, -2)) * lower                     # gy_t . v_i
+    P = (Q @ K.transpose(-1, -2)) * lower                     # q_t . k_i
+    refs = [A @ K, A.transpose(-1, -2) @ Q, P.transpose(-1, -2) @ G]
+    dev = [t.to(DEV) for t in (q, k, v)]
+    seen = []
+    try:
+        _lib.tune('sum_bwd.roles', 2)
+        for streams in (dev, sliced(dev)):
+            for dtype in (torch.float32, torch.bfloat16):
+                x = [t.detach().to(dtype).requires_grad_() for t in streams]
+                y = fwp.fast_weight_sum(*x, torch.zeros(B, H, E, M, device=DEV))
+                x[0].register_hook(lambda g: seen.append(_lib.last_kernel()))
+                y.backward(gy.to(DEV).to(dtype))
+                for got, ref in zip(x, refs):
+                    tol = 3e-6 if dtype == torch.float32 else 2e-2
+                    assert util.max_abs(got.grad.float(), ref) <= tol * max(1., ref.abs().max().item())
+    finally:
+        _lib.tune('sum_bwd.roles', -1)
+    assert len(seen) == 4 and all(s.startswith('sum_bwd_wy') for s in seen)
+    assert _lib.device_fault() == 0
