@@ -515,19 +515,38 @@ static int launch_sum_bwd_generic(const SumBwdParams& p, int nseq, cudaStream_t 
 // 12-15 us per launch (32 x 8 sequences), and the d=64 fp32 backward only pays off beyond 64 steps.
 // "delta.blocked" = 0 / 1 forces the per-step / blocked plan (tests cross-check one against the other).
 constexpr int kShortSeq = 16;
-// Where the chunkwise split-product plan (fwp_delta_wy.cuh) is the faster forward, from measurements on B200 with fp32
-// streams (sequences x steps; before -> with it, us):
-//   d = 16: 16 x 256 19.6 -> 11.6, 256 x 256 19.8 -> 15.4, 1536 x 64 21.2 -> 19.4, but 512 x 256 20.4 -> 27.8: with more than
-//           two sequences per SM the blocked kernel's four short chains per CTA win unless the sequences are short;
-//   d = 32: 128 x 256 44.7 -> 20.9, 256 x 512 88 -> 50, 512 x 256 47 -> 42;   d = 48: 512 x 256 154 -> 90;
-//   d = 64: 64 x 256 65.7 -> 34.9, 512 x 256 148 -> 117, but 256 x 20 10.2 -> 11.0 (two chunks are all start-up);
-//   E, M = 96, 32: 128 x 256 692 -> 68;   128, 128: 1655 -> 98 (the shared-memory kernels).
+// How full the last wave of a kernel that holds `per_sm` sequences per SM is with `nseq` of them, over its waves: a call that
+// just spills into another wave takes a whole one longer.
+static float wave_fill(int nseq, int per_sm) {
+    const int wave = per_sm * sm_count();
+    return (float)nseq / (float)((nseq + wave - 1) / wave * wave);
+}
+// Where the chunkwise split-product plan (fwp_delta_wy.cuh) is the faster forward, from measurements on B200 (time of the
+// kernel it replaces over its own, delta rule / sum rule, 20 to 250 steps, 160 to 1536 sequences).  What it costs grows with
+// chunks times sequences; the vector kernels are chains of steps that many sequences share, at their best with rows of
+// exactly 16, 32 or 64 elements.
+//   d = 16, fp32 (the blocked kernel holds four sequences per SM): 160 to 320 1.0-1.2 / 1.3-1.5, 480 0.8-1.0 / 1.0-1.2, 736
+//           (a second wave) 1.4-1.7 / 1.7-2.0, 1536 1.0-1.1 / 1.1-1.6;  bf16: the same from 250 steps on, better below;  rows of 12:
+//           1.2-2.5, bf16 2.0-4.4;
+//   d = 32, fp32: 160 1.1-1.9, 320 and 480 0.9 below 64 steps, 1.0-1.2 from there, 736 0.6-1.0, 1536 0.6-0.8; sum rule: 480
+//           1.0-1.4, 736 0.8-1.2, 1536 0.7-1.0;  rows of 24: up to 480 1.0-2.2, then as full rows;  bf16: 1.3-2.1, rows of 24 1.9-3.2;
+//   d = 48: 1.0-2.3 but for 0.8 at 1536 x 20, bf16 1.2-2.8;
+//   d = 64, fp32: 160 1.0 (20 steps) to 1.7, 320 0.9 (20) to 1.5, 736 0.7 (20), 0.9 (40), 1.1 (64) to 1.2;
+//   E, M = 96, 32: 128 x 256 692 -> 68 us;   128, 128: 1655 -> 98 us (the shared-memory kernels).
 template <typename T, bool SUM>
 static bool fwd_wy_pays(const DeltaFwdParams& p, int nseq) {
-    const int d = p.E > p.M ? p.E : p.M;
+    const int d = p.E > p.M ? p.E : p.M, sms = sm_count();
+    const bool full = p.E == p.M && (d == 16 || d == 32 || d == 64), fp32 = sizeof(T) == 4;
     if (p.L <= kShortSeq) return d > 64 && p.L > 4;
-    if (d <= 16) return nseq <= 2 * sm_count() || p.L <= 4 * kShortSeq;
-    return d <= 32 || d > 64 || p.L > 2 * kShortSeq;
+    if (d > 64) return true;
+    if (d <= 16) return !full || wave_fill(nseq, 4) < 0.75f || ((SUM || !fp32) && p.L <= 10 * kShortSeq);
+    if (d <= 32) {
+        if (!fp32 || nseq <= 2 * sms) return true;
+        if (nseq <= 4 * sms) return SUM || !full || p.L >= 4 * kShortSeq;
+        return SUM && nseq <= 6 * sms && p.L >= 4 * kShortSeq;
+    }
+    if (d <= 48 || !fp32) return p.L > 2 * kShortSeq || nseq <= 4 * sms;
+    return p.L >= 4 * kShortSeq || (p.L > 2 * kShortSeq && nseq <= 3 * sms) || nseq <= sms;
 }
 template <typename T, bool SUM>
 static int dispatch_fwd(const DeltaFwdParams& p, int nseq, cudaStream_t st) {
@@ -575,6 +594,11 @@ static int dispatch_fwd(const DeltaFwdParams& p, int nseq, cudaStream_t st) {
 //   d = 32: 128 63 -> 48, 256 64 -> 92; with rows of 20 128 139 -> 51, 512 283 -> 174
 //   d = 64: 64 114 -> 76, 128 116 -> 125; with rows of 55 512 1789 -> 557;  d = 48: 512 1128 -> 354
 //   E, M = 96, 32: 128 1152 -> 113, 1024 2783 -> 1233
+// and by length (time of the one-launch kernel over that of the three): d = 16, 80 sequences: 0.9 at 24 steps, 1.1 at 40, 1.8 at 250;
+//   d = 32: 80 0.7 (24), 0.9 (40), 1.2 (64), 1.4 (500), 144 0.9 (100), 1.1 (250), 304 (a second wave of the blocked kernel, which
+//   holds two sequences per SM) 1.1 (40), 1.2 (100), 400 0.9;
+//   d = 64: 80 0.8 (24), 1.2 (40), 1.6 (64); from there on against the blocked kernel (one per SM) 1.0, 144 0.8, 160 1.3, 208 1.0;
+//   rows of 55: 736 0.8 up to 64 steps, then 2.1;  304 1.1 (24), 1.5, 3.3
 // The four-step blocked kernels are at their best with rows of exactly 16, 32 or 64 elements and a sequence for every SM;
 // short rows cost them a division per copied piece, and states above 64 have no register-resident kernel at all.
 // bf16 streams (1024 steps) need a third of the operand parts:
@@ -585,16 +609,27 @@ static bool bwd_phases_pay(const DeltaBwdParams& p, int nseq, int io_dtype) {
     if (tune_get(T_DELTA_BLOCKED, -1) != -1) return false;
     const int force = tune_get(T_DELTA_PHASES, -1);
     if (force != -1) return force == 1;
-    const int d = p.E > p.M ? p.E : p.M;
+    const int d = p.E > p.M ? p.E : p.M, sms = sm_count();
     if (d > 64) return p.L > 4;
     if (p.L <= kShortSeq) return false;
     const bool full = p.E == p.M && (d == 16 || d == 32 || d == 64);
     if (io_dtype == FWP_BF16) {
         if (full && d == 64) return false;
-        return (d > 32 && d <= 48) || nseq <= (full && d == 16 ? 2 : 4) * sm_count();
+        return (d > 32 && d <= 48) || nseq <= (full && d == 16 ? 2 : 4) * sms;
     }
-    if (d <= 16) return nseq <= (full ? 1 : 2) * sm_count();
-    return !full || nseq <= (d == 64 ? sm_count() / 2 : sm_count());
+    if (!full) {
+        if (d <= 16) return nseq <= 2 * sms;
+        return d <= 48 || p.L > 4 * kShortSeq || (p.L > 2 * kShortSeq && nseq <= 3 * sms);
+    }
+    if (p.L <= 2 * kShortSeq) return false;
+    if (d == 16) return nseq <= sms;
+    if (d == 32) {
+        if (nseq > 2 * sms) return wave_fill(nseq, 2) < 0.6f && nseq <= 4 * sms;
+        return nseq <= sms && p.L >= (nseq <= sms * 3 / 4 ? 4 : 10) * kShortSeq;
+    }
+    if (p.L <= 3 * kShortSeq) return nseq <= sms * 3 / 4;
+    if (p.L <= 4 * kShortSeq) return nseq <= 3 * sms;
+    return nseq <= sms / 2 || (nseq > sms && nseq <= sms * 5 / 4);
 }
 template <typename T>
 static int dispatch_bwd(const DeltaBwdParams& p0, int nseq, cudaStream_t st) {

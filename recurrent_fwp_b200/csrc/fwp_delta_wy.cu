@@ -40,10 +40,11 @@ int launch_fwd_wy(const DeltaFwdParams& p, int nseq, cudaStream_t st) {
     const int d = p.E > p.M ? p.E : p.M;
     if (d <= 16) {
         // at d = 16 a chain waits more than it works: up to two sequences per SM the form with the short chain wins once
-        // its longer start (about 5 us) is paid for: 11.6 against 14.5 us at 16 sequences of 256 steps, 7.7 against 3.9 at 20 steps
+        // its longer start (about 5 us) is paid for: 11.6 against 14.5 us at 16 sequences of 256 steps, 7.7 against 3.9 at 20 steps.
+        // Rows shorter than 16 cost its staging copies a loop per row: 20.6 us, where the other form takes 17
         if constexpr (sizeof(T) == 4) {
             const int force = tune_get(T_DELTA_WY_HELPERS, 0);
-            const bool few = force ? force == 4 : p.L >= 7 * wy::C;
+            const bool few = force ? force == 4 : p.E == 16 && p.M == 16 && p.L >= 7 * wy::C;
             if (few && nseq <= sm_count()) return run_fwd_few<16, 16, 6, T, SUM>(p, nseq, st);
             if (few && (force || nseq <= 2 * sm_count())) return run_fwd_few<16, 16, 4, T, SUM>(p, nseq, st);
         }

@@ -47,7 +47,7 @@ int launch_sum_bwd_wy(const SumBwdParams& p, int nseq, cudaStream_t st) {
     const int d = p.E > p.M ? p.E : p.M, chains = 3 * nseq, sms = sm_count();
     if (d <= 16) {
         if constexpr (sizeof(T) == 4) {
-            const bool few = p.L >= 7 * wy::C;
+            const bool few = p.E == 16 && p.M == 16 && p.L >= 7 * wy::C;
             if (few && chains <= sms) return run_few<6, T>(a, nseq, st);
             if (few && chains <= 2 * sms) return run_few<4, T>(a, nseq, st);
         }
