@@ -24,6 +24,15 @@
  * Output buffers are overwritten (the reference accumulates into zeros).
  * State tensors are in/out: the forward leaves the end-of-segment state in
  * them, the backward rewinds them in place to the start-of-segment state.
+ * Output buffers must not overlap inputs, states or each other.
+ *
+ * Values that are not finite follow the recurrence: a NaN or Inf reaches the
+ * steps, value columns and sequences that depend on it and no others, with one
+ * exception.  The tensor-core kernels for bf16 streams of exactly E = M = 64
+ * (fast_weight_forward / _backward, more than 16 steps, every row 16-byte
+ * aligned) form whole chunks of 16 steps (64 in the tcgen05 forward), and there
+ * a bad step may show in any step of its own chunk and sequence.  "delta.chunk64"
+ * = 0 (fwp_tune) selects kernels without that exception.
  *
  * Ownership: the caller allocates everything, including scratch; the library
  * allocates nothing and keeps no pointer after a call returns.  Calls may be made

@@ -31,6 +31,7 @@ static int run_bwd(const DeltaBwdParams& p, int nseq, float* scratch, cudaStream
     a.p = p;
     a.ws = reinterpret_cast<uint4*>(scratch);
     a.carry = a.ws + (size_t)nseq * sg.nc * (sg.chunk / 16);
+    a.again = reinterpret_cast<int*>(a.carry + (size_t)nseq * (sg.carry / 16));
     const int nchunks = (p.L + wy::C - 1) / wy::C;
     for (int end = nchunks; end > 0; end -= sg.nc) {
         a.c0 = end > sg.nc ? end - sg.nc : 0;
@@ -56,7 +57,7 @@ template <int E, int M, int KG, typename T>
 static int64_t one(bool run, const DeltaBwdParams& p, int nseq, float* scratch, cudaStream_t st) {
     if (run) return run_bwd<E, M, KG, T>(p, nseq, scratch, st);
     const Segments sg = segments<E, M, T>(nseq, p.L);
-    return (int64_t)((sg.chunk * sg.nc + sg.carry) / 4 * (size_t)nseq);
+    return (int64_t)((sg.chunk * sg.nc + sg.carry + sizeof(int)) / 4 * (size_t)nseq);
 }
 template <typename T>
 int64_t bwd_phases(bool run, const DeltaBwdParams& p, int nseq, float* scratch, cudaStream_t st) {

@@ -15,6 +15,12 @@
 // lane, so that every access to it is a coalesced 512-byte line per warp; it is meant to stay in the L2 cache, and long
 // calls are cut into segments that do.  Each kernel is short enough to stay in the instruction cache (one kernel with a
 // role per phase was not: instruction fetch was its largest stall, and two sequences per SM took twice as long as one).
+//
+// Values that are not finite.  As in the forward (fwp_delta_wy.cuh), a chunk's products would carry a NaN or Inf to steps of
+// the chunk that do not depend on it: here to gradients of later steps.  What can do so ends up in G or in the rewound
+// state, and stays there (both are running sums), so the chain kernel looks at the two when it is through with a segment
+// and marks the sequence; finish writes nothing for marked sequences, and in the last segment the warp of chunk 0 does
+// the sequence again step by step (stepwise_backward).
 #pragma once
 #include "fwp_wy_common.cuh"
 
@@ -38,6 +44,7 @@ struct BwdPhase {
     DeltaBwdParams p;
     uint4* ws;                          // [sequence][chunk of the segment]
     uint4* carry;                       // [sequence][MS][KS][2][32]: G^T between segments
+    int* again;                         // [sequence]: something that is not finite turned up
     int c0, nc;                         // the segment: chunks [c0, c0 + nc)
     int first;                          // 1: the last chunks of the sequence, G starts from zero
 };
@@ -77,8 +84,8 @@ __device__ __forceinline__ void scale_steps(float (&x)[2][4], const float (&b)[2
     for (int i = 0; i < 8; i++) x[i >> 2][i & 3] *= b[i >> 2][i & 1];
 }
 template <typename T>
-__device__ __forceinline__ const T* stream_at(const Row4& r, int n, int h) {
-    return reinterpret_cast<const T*>(r.p) + n * r.sN + h * r.sH;
+__device__ __forceinline__ T* stream_at(const Row4& r, int n, int h) {
+    return reinterpret_cast<T*>(r.p) + n * r.sN + h * r.sH;
 }
 // beta of the steps a lane's columns stand for (2t, 2t+1, 2t+8, 2t+9); 0 past the end
 template <typename T>
@@ -87,6 +94,82 @@ __device__ __forceinline__ void load_beta(float (&b)[2][2], const T* p, long lon
     for (int i = 0; i < 4; i++) {
         const int s = 8 * (i >> 1) + 2 * t + (i & 1);
         b[i >> 1][i & 1] = s < nt ? to_f32(p[s * sL]) : 0.f;
+    }
+}
+
+template <int K>
+__device__ __forceinline__ bool finite(const float (&x)[K][2][4]) {
+    float acc = 0.f;
+#pragma unroll
+    for (int k = 0; k < K; k++)
+#pragma unroll
+        for (int i = 0; i < 8; i++) acc = fmaf(x[k][i >> 2][i & 3], 0.f, acc);
+    return acc == 0.f;
+}
+
+// The recurrence of one sequence backwards as it stands, by one warp: lanes own columns of G for r, then rows for dQ and dK.
+// W holds the rewound state; S is brought forward from it with the u of the forward first.  `G` and `S` hold E x M floats
+// each and `vec` 2 M, all of them this warp's own.  Inlined, for the reason stepwise_forward is.
+template <typename T>
+__device__ __forceinline__ void stepwise_backward(const DeltaBwdParams& p, int seq, float* G, float* S, float* vec) {
+    const int lane = threadIdx.x & 31, n = seq / p.H, h = seq - n * p.H, E = p.E, M = p.M;
+    const T *qp = stream_at<T>(p.q, n, h), *kp = stream_at<T>(p.k, n, h), *vp = stream_at<T>(p.v, n, h), *bp = stream_at<T>(p.beta, n, h);
+    const T* yp = stream_at<T>(p.gy, n, h);
+    const float* op = stream_at<float>(p.v_old, n, h);
+    T *gqp = stream_at<T>(p.gq, n, h), *gkp = stream_at<T>(p.gk, n, h), *gvp = stream_at<T>(p.gv, n, h), *gbp = stream_at<T>(p.gb, n, h);
+    const float* W = p.W + n * p.wN + h * p.wH;
+    float *us = vec, *bs = vec + M;
+    for (int m = lane; m < M; m += 32) {
+#pragma unroll 1
+        for (int e = 0; e < E; e++) {
+            S[e * M + m] = W[(long long)e * p.wE + m];
+            G[e * M + m] = 0.f;
+        }
+        for (long long t = 0; t < p.L; t++) {
+            const float u = to_f32(bp[t * p.beta.sL]) * (to_f32(vp[t * p.v.sL + m]) - op[t * p.v_old.sL + m]);
+#pragma unroll 1
+            for (int e = 0; e < E; e++) S[e * M + m] = fmaf(to_f32(kp[t * p.k.sL + e]), u, S[e * M + m]);
+        }
+    }
+    __syncwarp();
+    for (long long t = p.L - 1; t >= 0; t--) {
+        const T *q = qp + t * p.q.sL, *k = kp + t * p.k.sL, *y = yp + t * p.gy.sL;
+        const float beta = to_f32(bp[t * p.beta.sL]);
+        float db = 0.f;
+        for (int m = lane; m < M; m += 32) {
+            const float gy = to_f32(y[m]), w = to_f32(vp[t * p.v.sL + m]) - op[t * p.v_old.sL + m];
+            float r = 0.f;
+#pragma unroll 1
+            for (int e = 0; e < E; e++) {
+                const float x = fmaf(to_f32(q[e]), gy, G[e * M + m]);
+                G[e * M + m] = x;
+                r = fmaf(x, to_f32(k[e]), r);
+            }
+            db = fmaf(r, w, db);
+            us[m] = beta * w;
+            bs[m] = beta * r;
+            gvp[t * p.gv.sL + m] = from_f32<T>(beta * r);
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) db += __shfl_xor_sync(0xffffffffu, db, o);
+        if (lane == 0) gbp[t * p.gb.sL] = from_f32<T>(db);
+        __syncwarp();
+        for (int e = lane; e < E; e += 32) {
+            const float ke = to_f32(k[e]);
+            float dq = 0.f, dk = 0.f, sb = 0.f;
+#pragma unroll 1
+            for (int m = 0; m < M; m++) {
+                const float s = S[e * M + m], x = G[e * M + m], u = us[m], b = bs[m], s0 = fmaf(-ke, u, s);
+                dq = fmaf(s, to_f32(y[m]), dq);
+                dk = fmaf(x, u, dk);
+                sb = fmaf(s0, b, sb);
+                S[e * M + m] = s0;
+                G[e * M + m] = fmaf(-ke, b, x);
+            }
+            gqp[t * p.gq.sL + e] = from_f32<T>(dq);
+            gkp[t * p.gk.sL + e] = from_f32<T>(dk - sb);
+        }
+        __syncwarp();
     }
 }
 
@@ -99,7 +182,7 @@ struct PrepareSmem {                    // per warp
 };
 
 template <int E, int M, int WARPS, typename T>
-__global__ void __launch_bounds__(WARPS * 32) delta_bwd_prepare_kernel(const BwdPhase a) {
+__global__ void __launch_bounds__(WARPS * 32) delta_bwd_prepare_kernel(const __grid_constant__ BwdPhase a) {
     constexpr int KS = E / 16, MS = M / 16, NP = stream_parts<T>();
     using Sp = BwdSpace<E, M, NP>;
     using Sm = PrepareSmem<E, NP>;
@@ -114,6 +197,7 @@ __global__ void __launch_bounds__(WARPS * 32) delta_bwd_prepare_kernel(const Bwd
     if (seq >= p.NH) return;
     Sm& sm = reinterpret_cast<Sm*>(smem_raw)[threadIdx.x >> 5];
     const int n = seq / p.H, h = seq - n * p.H, t0 = c * C, nt = min(C, p.L - t0);
+    if (a.first && c == a.c0 && lane == 0) a.again[seq] = 0;
     uint4* const ws = a.ws + unit * Sp::kSize;
     const unsigned at = 2 * lane_at(lane, P), atC = 2 * lane_at(lane, PC);
     const unsigned aK = smem_u32(&sm.K[0][0][0]) + at, aQ = smem_u32(&sm.Q[0][0][0]) + at;
@@ -234,7 +318,7 @@ struct ChainRing {                      // pieces of 16 bytes per lane
     static constexpr size_t kBytes = (size_t)DEPTH * kPieces * 512;
 };
 template <int E, int M, int DEPTH, typename T>
-__global__ void __launch_bounds__(64) delta_bwd_chain_kernel(const BwdPhase a) {
+__global__ void __launch_bounds__(64) delta_bwd_chain_kernel(const __grid_constant__ BwdPhase a) {
     constexpr int KS = E / 16, MS = M / 16, NP = stream_parts<T>();
     using Sp = BwdSpace<E, M, NP>;
     using Rg = ChainRing<E, M, DEPTH, T>;
@@ -249,10 +333,11 @@ __global__ void __launch_bounds__(64) delta_bwd_chain_kernel(const BwdPhase a) {
         const int n = seq / p.H, h = seq - n * p.H;
         float* W = p.W + n * p.wN + h * p.wH;
         constexpr int AHEAD = 4;
+        bool good = true;
 #pragma unroll 1
         for (int k = 0; k < KS; k++) {
             uint4* at = ws + Sp::S + (k * MS + j) * 64;
-            float s[2][4], d[AHEAD][2][4];
+            float s1[1][2][4], (&s)[2][4] = s1[0], d[AHEAD][2][4];
 #pragma unroll
             for (int i = 0; i < 8; i++) {
                 const int e = 16 * k + g + 8 * ((i >> 1) & 1), m = 16 * j + 8 * (i >> 2) + 2 * t + (i & 1);
@@ -276,7 +361,9 @@ __global__ void __launch_bounds__(64) delta_bwd_chain_kernel(const BwdPhase a) {
                 const int e = 16 * k + g + 8 * ((i >> 1) & 1), m = 16 * j + 8 * (i >> 2) + 2 * t + (i & 1);
                 if (e < p.E && m < p.M) W[(long long)e * p.wE + m] = s[i >> 2][i & 3];
             }
+            good &= finite(s1);
         }
+        if (!good) a.again[seq] = 1;
         return;
     }
     uint4* const carry = a.carry + ((long long)seq * MS + j) * KS * 64;
@@ -342,12 +429,13 @@ __global__ void __launch_bounds__(64) delta_bwd_chain_kernel(const BwdPhase a) {
     }
 #pragma unroll
     for (int k = 0; k < KS; k++) put_block(carry + k * 64, G[k], lane);
+    if (!finite(G)) a.again[seq] = 1;
 }
 
 // ------------------------------------------------------------------------------------------------------- finish
 // One warp per chunk and group of KG row blocks of the state.
 template <int E, int M, int KG, int WARPS, typename T>
-__global__ void __launch_bounds__(WARPS * 32) delta_bwd_finish_kernel(const BwdPhase a) {
+__global__ void __launch_bounds__(WARPS * 32, M == 16 ? (E > 64 ? 5 : 4) : 0) delta_bwd_finish_kernel(const __grid_constant__ BwdPhase a) {
     constexpr int KS = E / 16, MS = M / 16, NP = stream_parts<T>(), GROUPS = (KS + KG - 1) / KG;
     using Sp = BwdSpace<E, M, NP>;
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -366,7 +454,7 @@ __global__ void __launch_bounds__(WARPS * 32) delta_bwd_finish_kernel(const BwdP
     const T* vp = stream_at<T>(p.v, n, h) + (t0 + 2 * t) * p.v.sL + g;
     const T* yp = stream_at<T>(p.gy, n, h) + (t0 + 2 * t) * p.gy.sL + g;
     const float* op = stream_at<float>(p.v_old, n, h) + (t0 + 2 * t) * p.v_old.sL + g;
-    T* gvp = const_cast<T*>(stream_at<T>(p.gv, n, h)) + (t0 + 2 * t) * p.gv.sL + g;
+    T* gvp = stream_at<T>(p.gv, n, h) + (t0 + 2 * t) * p.gv.sL + g;
     float dq[KG][2][4], dk[KG][2][4], hh[2][4] = {}, pp[2][4] = {}, db[2][2] = {};
 #pragma unroll
     for (int k = 0; k < KG; k++) {
@@ -387,6 +475,13 @@ __global__ void __launch_bounds__(WARPS * 32) delta_bwd_finish_kernel(const BwdP
     };
     streams(0);
     states(0, 0);
+    if (__builtin_expect(a.again[seq] != 0, 0)) {
+        if (c == 0 && k0 == 0) {                        // the last segment: nobody else writes to this chunk's part of the workspace
+            float* const own = reinterpret_cast<float*>(a.ws + unit * Sp::kSize);
+            stepwise_backward<T>(p, seq, own + 4 * Sp::G, own + 4 * Sp::S, own + 4 * Sp::R);
+        }
+        return;
+    }
     const int kn = KS % KG ? min(KG, KS - k0) : KG;
 #pragma unroll 1
     for (int j = 0; j < MS; j++) {
@@ -451,8 +546,8 @@ __global__ void __launch_bounds__(WARPS * 32) delta_bwd_finish_kernel(const BwdP
         fr.r[i][1] = transpose8(fr.r[i][2]);
         fr.r[i][3] |= transpose8(fr.r[i][3]);
     }
-    T* gqp = const_cast<T*>(stream_at<T>(p.gq, n, h)) + (t0 + g) * p.gq.sL + 2 * t;
-    T* gkp = const_cast<T*>(stream_at<T>(p.gk, n, h)) + (t0 + g) * p.gk.sL + 2 * t;
+    T* gqp = stream_at<T>(p.gq, n, h) + (t0 + g) * p.gq.sL + 2 * t;
+    T* gkp = stream_at<T>(p.gk, n, h) + (t0 + g) * p.gk.sL + 2 * t;
     auto even = [&](const T* q, long long sL) { return (reinterpret_cast<uintptr_t>(q) & (2 * sizeof(T) - 1)) == 0 && (sL & 1) == 0; };
     const bool qpair = even(gqp, p.gq.sL), kpair = even(gkp, p.gk.sL);
 #pragma unroll
@@ -468,7 +563,7 @@ __global__ void __launch_bounds__(WARPS * 32) delta_bwd_finish_kernel(const BwdP
         store_block<T>(dk[k], gkp + 16 * (k0 + k), p.gk.sL, nt, p.E - 16 * (k0 + k), kpair, g, t);
     }
     if (k0 == 0) {
-        T* gbp = const_cast<T*>(stream_at<T>(p.gb, n, h)) + t0 * p.gb.sL;
+        T* gbp = stream_at<T>(p.gb, n, h) + t0 * p.gb.sL;
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             float d = db[i >> 1][i & 1];

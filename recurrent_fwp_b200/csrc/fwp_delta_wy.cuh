@@ -17,6 +17,14 @@
 //     T V and tril(Q K^T).  After it (OUT): the outputs, from the parts of S and u the chain left behind.
 // The two sides meet at two mbarriers per buffer.  With many sequences of a large state the copies of S would fill
 // shared memory, so there (OUT = false) the chain warps form the outputs themselves.
+//
+// Values that are not finite.  A chunk's products run over all sixteen steps: above the diagonal a zero meets the value of
+// a later step, and zero times NaN or Inf is NaN, so one bad step would reach up to fifteen outputs before it (and a split
+// Inf is Inf, NaN, NaN).  Whatever goes wrong this way -- in an input, or by overflow -- stays in the state to the end of
+// the sequence (S only ever gets K^T u added); a query alone shows in its row of tril(Q K^T).  So a CTA that ends with a
+// state, or meets a product of queries and keys, that is not finite does its sequence again, step by step from the state
+// it started from (stepwise_forward): what a caller sees is the recurrence itself, for any value.  The end state is
+// therefore stored behind a barrier of the CTA.
 #pragma once
 #include "fwp_wy_common.cuh"
 
@@ -117,6 +125,60 @@ __device__ __forceinline__ bool rows_vec(const T* base, long long sL) {
     return (reinterpret_cast<uintptr_t>(base) & 15) == 0 && sL % (16 / (int)sizeof(T)) == 0;
 }
 
+// the CTA's flag: something that is not finite turned up
+__device__ __forceinline__ int& redo() {
+    __shared__ int flag;
+    return flag;
+}
+// raises it when one of a block's values is not finite: their sum times zero is NaN then
+template <int K>
+__device__ __forceinline__ void note(const float (&x)[K][4]) {
+    f2 acc = 0ull;
+#pragma unroll
+    for (int i = 0; i < 2 * K; i++) acc = ffma2(f2_pack(x[i >> 1][2 * (i & 1)], x[i >> 1][2 * (i & 1) + 1]), 0ull, acc);
+    if (!(f2_hsum(acc) == 0.f)) redo() = 1;
+}
+
+// The recurrence of one sequence as it stands, a thread per state column; W in place, or a zeroed E x M array of the
+// caller's where the parameters name none.  It stands once at the end of a kernel, inlined: a call would cost every launch
+// 0.5 to 0.9 us (the kernel then has a stack).
+template <typename T, bool SUM>
+__device__ __forceinline__ void stepwise_forward(const DeltaFwdParams& p, float* own) {
+    const int n = blockIdx.x / p.H, h = blockIdx.x - n * p.H;
+    const T* const qp = reinterpret_cast<const T*>(p.q.p) + n * p.q.sN + h * p.q.sH;
+    const T* const kp = reinterpret_cast<const T*>(p.k.p) + n * p.k.sN + h * p.k.sH;
+    const T* const vp = reinterpret_cast<const T*>(p.v.p) + n * p.v.sN + h * p.v.sH;
+    const T* const bp = SUM ? nullptr : reinterpret_cast<const T*>(p.beta.p) + n * p.beta.sN + h * p.beta.sH;
+    T* const yp = reinterpret_cast<T*>(p.out.p) + n * p.out.sN + h * p.out.sH;
+    float* const vop = SUM || !p.v_old.p ? nullptr : reinterpret_cast<float*>(p.v_old.p) + n * p.v_old.sN + h * p.v_old.sH;
+    float* const vip = SUM || !p.v_ins.p ? nullptr : reinterpret_cast<float*>(p.v_ins.p) + n * p.v_ins.sN + h * p.v_ins.sH;
+    const long long sE = p.W ? p.wE : p.M;
+    for (int m = threadIdx.x; m < p.M; m += blockDim.x) {
+        float* const S = (p.W ? p.W + n * p.wN + h * p.wH : own) + m;
+        if (!p.W)
+            for (int e = 0; e < p.E; e++) S[e * sE] = 0.f;
+        for (long long t = 0; t < p.L; t++) {
+            const T *k = kp + t * p.k.sL, *q = qp + t * p.q.sL;
+            float u = to_f32(vp[t * p.v.sL + m]), y = 0.f;
+            if constexpr (!SUM) {
+                float vo = 0.f;
+#pragma unroll 1
+                for (int e = 0; e < p.E; e++) vo = fmaf(S[e * sE], to_f32(k[e]), vo);
+                u = to_f32(bp[t * p.beta.sL]) * (u - vo);
+                if (vop) vop[t * p.v_old.sL + m] = vo;
+                if (vip) vip[t * p.v_ins.sL + m] = u;
+            }
+#pragma unroll 1
+            for (int e = 0; e < p.E; e++) {
+                const float s = fmaf(to_f32(k[e]), u, S[e * sE]);
+                S[e * sE] = s;
+                y = fmaf(s, to_f32(q[e]), y);
+            }
+            yp[t * p.out.sL + m] = from_f32<T>(y);
+        }
+    }
+}
+
 // 16 x 16 block of a tile as C fragments: `at` is this lane's (g, 2t)
 template <int P>
 __device__ __forceinline__ void tile_block(float (&x)[2][4], const float* at) {
@@ -180,6 +242,7 @@ __device__ __forceinline__ void fwd_few(const DeltaFwdParams& p) {
             mbar_init(&filled[i], 1);
             mbar_init(&done[i], NCW);
         }
+        redo() = 0;
         mbar_fence_init();
     }
     if (warp >= NCW && (p.E < E || p.M < M)) {      // columns that no copy writes
@@ -274,6 +337,9 @@ __device__ __forceinline__ void fwd_few(const DeltaFwdParams& p) {
             warp_arrive(&done[b], lane);
             if (++b == NB) { b = 0; phase ^= 1; st ^= 1; }
         }
+        note(S);
+        slot_barrier(0, (NCW + NB) * 32);           // the other warps have written what they have to write
+        if (redo()) return;
 #pragma unroll
         for (int j = 0; j < 2 * KS; j++)
 #pragma unroll
@@ -345,6 +411,7 @@ __device__ __forceinline__ void fwd_few(const DeltaFwdParams& p) {
                 *reinterpret_cast<float2*>(&buf.inv.A[g + 8][8 * nn + 2 * t]) = make_float2(kk[nn][2], kk[nn][3]);
             }
         }
+        note(qk);
         Frag<3> f;
         from_c(f, qk[0], qk[1]);
         store(aA, kPartC, f);
@@ -424,14 +491,19 @@ __device__ __forceinline__ void fwd_few(const DeltaFwdParams& p) {
         if (vop) flush<M, PV, float>(&buf.v[st][0][0], vop + t0 * p.v_old.sL, p.v_old.sL, nt, p.M, vovec && p.M == M, lane);
         __syncwarp();
     }
+    slot_barrier(0, (NCW + NB) * 32);
 }
 template <int E, int M, int NB, typename T, bool SUM>
-__global__ void __launch_bounds__((M / 16 + NB) * 32) delta_fwd_wy_few_kernel(const DeltaFwdParams p) {
+__global__ void __launch_bounds__((M / 16 + NB) * 32, 2) delta_fwd_wy_few_kernel(const __grid_constant__ DeltaFwdParams p) {
     fwd_few<E, M, NB, T, SUM>(p);
+    if (redo()) stepwise_forward<T, SUM>(p, nullptr);
 }
 template <int E, int M, int NB, typename T, bool SUM>
-__global__ void __launch_bounds__((M / 16 + NB) * 32) sum_bwd_wy_few_kernel(const __grid_constant__ SumBwdForwards a) {
+__global__ void __launch_bounds__((M / 16 + NB) * 32, 2) sum_bwd_wy_few_kernel(const __grid_constant__ SumBwdForwards a) {
+    static_assert(E * M * sizeof(float) <= NB * sizeof(FewBuf<E, M, stream_parts<T>()>), "room for the state of stepwise_forward");
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     fwd_few<E, M, NB, T, SUM>(a.p[blockIdx.y]);
+    if (redo()) stepwise_forward<T, SUM>(a.p[blockIdx.y], reinterpret_cast<float*>(smem_raw));
 }
 
 // --------------------------------------------------------------------------------- forward, many sequences
@@ -463,6 +535,7 @@ __device__ __forceinline__ void fwd(const DeltaFwdParams& p) {
             mbar_init(&filled[i], 1);
             mbar_init(&freed[i], NCW);
         }
+        redo() = 0;
         mbar_fence_init();
     }
     __syncthreads();
@@ -550,6 +623,9 @@ __device__ __forceinline__ void fwd(const DeltaFwdParams& p) {
             store_block_t<T>(y, yp + c * C * p.out.sL, p.out.sL, nt, width, g, t);
             if (++b == NB) { b = 0; phase ^= 1; }
         }
+        note(S);
+        slot_barrier(0, (NCW + NB) * 32);           // the other warps have written what they have to write
+        if (redo()) return;
 #pragma unroll
         for (int j = 0; j < 2 * KS; j++)
 #pragma unroll
@@ -625,6 +701,7 @@ __device__ __forceinline__ void fwd(const DeltaFwdParams& p) {
                 *reinterpret_cast<float2*>(&buf.A[g + 8][8 * nn + 2 * t]) = make_float2(kk[nn][2], kk[nn][3]);
             }
         }
+        note(qk);
         Frag<3> f;
         from_c(f, qk[0], qk[1]);
         store(aA, kPartC, f);
@@ -640,14 +717,19 @@ __device__ __forceinline__ void fwd(const DeltaFwdParams& p) {
         }
         warp_arrive(&filled[b], lane);
     }
+    slot_barrier(0, (NCW + NB) * 32);
 }
 template <int E, int M, int NB, int CTAS, typename T, bool SUM>
-__global__ void __launch_bounds__((M / 16 + NB) * 32, CTAS) delta_fwd_wy_kernel(const DeltaFwdParams p) {
+__global__ void __launch_bounds__((M / 16 + NB) * 32, CTAS) delta_fwd_wy_kernel(const __grid_constant__ DeltaFwdParams p) {
     fwd<E, M, NB, CTAS, T, SUM>(p);
+    if (redo()) stepwise_forward<T, SUM>(p, nullptr);
 }
 template <int E, int M, int NB, int CTAS, typename T, bool SUM>
 __global__ void __launch_bounds__((M / 16 + NB) * 32, CTAS) sum_bwd_wy_kernel(const __grid_constant__ SumBwdForwards a) {
+    static_assert(E * M * sizeof(float) <= NB * sizeof(FwdBuf<E, stream_parts<T>()>), "room for the state of stepwise_forward");
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     fwd<E, M, NB, CTAS, T, SUM>(a.p[blockIdx.y]);
+    if (redo()) stepwise_forward<T, SUM>(a.p[blockIdx.y], reinterpret_cast<float*>(smem_raw));
 }
 
 }  // namespace wy
