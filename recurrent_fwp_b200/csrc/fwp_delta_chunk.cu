@@ -88,7 +88,8 @@ int launch_fwd_chunk_bf16(const DeltaFwdParams& p, int nseq, cudaStream_t st) {
     }
     // "delta.pipe64" = 1 (default): the state-independent part of every chunk is prepared one chunk ahead by a fifth warp
     if (tune_get(T_DELTA_PIPE64, 1) >= 1)
-        return launch_dependent(delta_fwd_chunk_bf16_pipe_kernel, p, nseq, cb::NTP, sizeof(cb::SmemP), st, "delta_fwd_chunk_bf16_pipe_kernel");
+        return launch_dependent(p.v_old.p ? delta_fwd_chunk_bf16_pipe_kernel<true> : delta_fwd_chunk_bf16_pipe_kernel<false>, p, nseq,
+                                cb::NTP, sizeof(cb::SmemP), st, "delta_fwd_chunk_bf16_pipe_kernel");
     return launch(delta_fwd_chunk_bf16_inv_kernel, p, nseq, cb::NT, sizeof(cb::SmemI), st, "delta_fwd_chunk_bf16_inv_kernel");
 }
 
