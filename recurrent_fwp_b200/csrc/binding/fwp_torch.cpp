@@ -120,23 +120,28 @@ bool needs_grad(const std::array<const Tensor*, K>& in) {
 }
 
 // ------------------------------------------------------------- autograd nodes
-// `user` holds what the caller can also reach (inputs, states, outputs; version-checked on unpack), `own` the buffers
-// only this call knows.  Gradients are returned in the order of the forward's arguments, undefined for the states.
+// What a backward needs is saved as torch's own nodes save it, so that saved-tensor hooks (activation checkpointing,
+// offloading) see all of it: `user` holds what the caller can also reach (inputs, states, outputs; version-checked on
+// unpack), `own` the buffers only this call knows.  Gradients are returned in the order of the forward's arguments,
+// undefined for the states.
 struct OpNode : public Node {
     Dims d;
-    std::vector<SavedVariable> user;
-    std::vector<Tensor> own;
+    std::vector<SavedVariable> user, own;
     void save(const Tensor& t) { user.emplace_back(t, false); }
     void save_output(const Tensor& t) { user.emplace_back(t, true); }
+    void keep(std::initializer_list<Tensor> l) {
+        own.reserve(l.size());
+        for (auto& t : l) own.emplace_back(t, false);
+    }
     void release_variables() override {
         std::lock_guard<std::mutex> lock(mutex_);
         for (auto& s : user) s.reset_data();
-        own.clear();
+        for (auto& s : own) s.reset_data();
     }
-    std::vector<Tensor> unpack() {
+    std::vector<Tensor> unpack(std::vector<SavedVariable>& saved) {
         std::vector<Tensor> t;
-        t.reserve(user.size());
-        for (auto& s : user) t.push_back(s.unpack(shared_from_this()));
+        t.reserve(saved.size());
+        for (auto& s : saved) t.push_back(s.unpack(shared_from_this()));
         return t;
     }
     // the incoming gradient in the streams' element type with a unit inner stride
@@ -179,11 +184,11 @@ struct DeltaNode final : public OpNode {
     variable_list apply(variable_list&& g) override {
         std::lock_guard<std::mutex> lock(mutex_);
         at::NoGradGuard no_grad;
-        const auto t = unpack();
+        const auto t = unpack(user), o = unpack(own);
         const Tensor &Q = t[0], &K = t[1], &V = t[2], &beta = t[3], &W = t[4];
         const Tensor gy = incoming(g[0], Q, {d.N, d.H, d.L, d.M});
         Tensor gQ = like_stream(d.E, Q), gK = like_stream(d.E, Q), gV = like_stream(d.M, Q), gb = like_stream(1, Q);
-        delta_backward(d, Q, K, V, beta, own[0], Desc(gy), W, gQ, gK, gV, gb);
+        delta_backward(d, Q, K, V, beta, o[0], Desc(gy), W, gQ, gK, gV, gb);
         return {gQ, gK, gV, gb, Tensor()};
     }
 };
@@ -213,7 +218,7 @@ PyObject* fast_weight_delta(PyObject*, PyObject* const* args, Py_ssize_t n) {
         if (grad) {
             auto node = make_node<DeltaNode>(in, d);
             for (auto* t : in) node->save(*t);
-            node->own = {v_old};
+            node->keep({v_old});
             torch::autograd::create_gradient_edge(out, node);
         }
     }
@@ -239,8 +244,8 @@ struct DeltaLayerNode final : public OpNode {
     variable_list apply(variable_list&& g) override {
         std::lock_guard<std::mutex> lock(mutex_);
         at::NoGradGuard no_grad;
-        const auto t = unpack();
-        const Tensor &x = t[0], &W = t[1], &q = own[0], &k = own[1], &v = own[2], &beta = own[3], &v_old = own[4];
+        const auto t = unpack(user), o = unpack(own);
+        const Tensor &x = t[0], &W = t[1], &q = o[0], &k = o[1], &v = o[2], &beta = o[3], &v_old = o[4];
         TORCH_CHECK(g[0].defined() && g[0].scalar_type() == at::kFloat, "the incoming gradient must be float32");
         const Tensor gout = g[0].contiguous();
         void* st = stream_of(x);
@@ -285,7 +290,7 @@ PyObject* delta_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
             auto node = make_node<DeltaLayerNode>(in, d);
             node->save(x);
             node->save(W);
-            node->own = {q, k, v, beta, v_old};
+            node->keep({q, k, v, beta, v_old});
             node->scale = scale;
             torch::autograd::create_gradient_edge(out, node);
         }
@@ -300,7 +305,7 @@ struct SumNode final : public OpNode {
     variable_list apply(variable_list&& g) override {
         std::lock_guard<std::mutex> lock(mutex_);
         at::NoGradGuard no_grad;
-        const auto t = unpack();
+        const auto t = unpack(user);
         const Tensor &Q = t[0], &K = t[1], &V = t[2];
         const Tensor gy = incoming(g[0], Q, {d.N, d.H, d.L, d.M});
         Tensor gQ = like_stream(d.E, Q), gK = like_stream(d.E, Q), gV = like_stream(d.M, Q);
@@ -344,9 +349,9 @@ struct RecNode final : public OpNode {
     variable_list apply(variable_list&& g) override {
         std::lock_guard<std::mutex> lock(mutex_);
         at::NoGradGuard no_grad;
-        const auto t = unpack();
+        const auto t = unpack(user), o = unpack(own);
         const Tensor *R = &t[0], &W = t[4], &out = t[5];
-        const Tensor &q = own[0], &k = own[1], &v = own[2], &beta = own[3], &v_old = own[4], &h0 = own[5];
+        const Tensor &q = o[0], &k = o[1], &v = o[2], &beta = o[3], &v_old = o[4], &h0 = o[5];
         const Tensor gy = incoming(g[0], out, {d.N, d.H, d.L, d.M});
         Tensor gq = empty(d, d.M, out), gk = empty(d, d.M, out), gv = empty(d, d.M, out), gb = empty(d, 1, out);
         Tensor gR[3], delayed = empty(d, d.M, out);
@@ -395,7 +400,7 @@ PyObject* rec_update_fwm_tanh(PyObject*, PyObject* const* args, Py_ssize_t n) {
             torch::autograd::create_gradient_edge(out, node);
             for (int i = 4; i < 9; i++) node->save(*in[i]);
             node->save_output(out);
-            node->own = {q, k, v, beta, v_old, h_init};
+            node->keep({q, k, v, beta, v_old, h_init});
         }
     }
     return THPVariable_Wrap(std::move(out));
@@ -409,16 +414,16 @@ struct RnnNode final : public OpNode {
     variable_list apply(variable_list&& g) override {
         std::lock_guard<std::mutex> lock(mutex_);
         at::NoGradGuard no_grad;
-        const auto t = unpack();
-        const Tensor &K = t[0], &V = t[1], &beta = t[2], &W = t[3], &out = t[4], &v_old = own[0];
+        const auto t = unpack(user), o = unpack(own);
+        const Tensor &K = t[0], &V = t[1], &beta = t[2], &W = t[3], &out = t[4], &v_old = o[0];
         const Tensor gy = incoming(g[0], out, {d.N, d.H, d.L, d.M});
         Tensor gZ = empty(d, d.M, out), gK = empty(d, d.M, out), gV = empty(d, d.M, out), gb = empty(d, 1, out);
-        Tensor delayed = own[1];        // v2: the normalised delayed outputs of the forward; v1: the start vector
+        Tensor delayed = o[1];        // v2: the normalised delayed outputs of the forward; v1: the start vector
         void* st = stream_of(out);
         const int dev = out.device().index();
         if (VERSION == 1) {
             delayed = empty(d, d.M, out);
-            check(fwp_delayed(d.N, d.H, d.L, d.M, Desc(out), Desc(own[1]), Desc(Tensor()), Desc(delayed), 0, st, dev), "delayed");
+            check(fwp_delayed(d.N, d.H, d.L, d.M, Desc(out), Desc(o[1]), Desc(Tensor()), Desc(delayed), 0, st, dev), "delayed");
         }
         const auto backward = VERSION == 1 ? fwp_fast_rnn_backward : fwp_fast_rnn_v2_backward;
         check(backward(d.N, d.H, d.L, d.M, Desc(K), Desc(V), Desc(beta), Desc(v_old), Desc(gy), Desc(out), Desc(delayed), Desc(W),
@@ -462,7 +467,7 @@ PyObject* fast_rnn(PyObject*, PyObject* const* args, Py_ssize_t n) {
             torch::autograd::create_gradient_edge(out, node);
             for (auto* t : {&K, &V, &beta, &W}) node->save(*t);
             node->save_output(out);
-            node->own = {v_old, aux};
+            node->keep({v_old, aux});
         }
     }
     return THPVariable_Wrap(std::move(out));
@@ -478,18 +483,18 @@ struct LstmNode final : public OpNode {
     variable_list apply(variable_list&& g) override {
         std::lock_guard<std::mutex> lock(mutex_);
         at::NoGradGuard no_grad;
-        const auto t = unpack();        // K[3], V[3], beta[3], W[3], out, cell
+        const auto t = unpack(user), o = unpack(own);       // K[3], V[3], beta[3], W[3], out, cell
         const Tensor &out = t[12], &cell = t[13];
-        const Tensor *gates = &own[0], *v_old = &own[3];
+        const Tensor *gates = &o[0], *v_old = &o[3];
         const Tensor gy = incoming(g[0], out, {d.N, d.H, d.L, d.M});        // the cell's gradient is ignored, as in the reference
         void* st = stream_of(out);
         const int dev = out.device().index();
-        Tensor delayed = own[6], u_minus_c = empty(d, d.M, out);            // v1: h0, v2-v4: the normalised delayed outputs
+        Tensor delayed = o[6], u_minus_c = empty(d, d.M, out);            // v1: h0, v2-v4: the normalised delayed outputs
         if (variant == 1) {
             delayed = empty(d, d.M, out);
-            check(fwp_delayed(d.N, d.H, d.L, d.M, Desc(out), Desc(own[6]), Desc(Tensor()), Desc(delayed), 0, st, dev), "delayed");
+            check(fwp_delayed(d.N, d.H, d.L, d.M, Desc(out), Desc(o[6]), Desc(Tensor()), Desc(delayed), 0, st, dev), "delayed");
         }
-        check(fwp_delayed(d.N, d.H, d.L, d.M, Desc(cell), Desc(own[7]), Desc(gates[1]), Desc(u_minus_c), 0, st, dev), "delayed");
+        check(fwp_delayed(d.N, d.H, d.L, d.M, Desc(cell), Desc(o[7]), Desc(gates[1]), Desc(u_minus_c), 0, st, dev), "delayed");
         Tensor gZ[3], gK[3], gV[3], gb[3];
         for (int i = 0; i < 3; i++) {
             gZ[i] = empty(d, d.M, out);
@@ -553,7 +558,7 @@ PyObject* fast_lstm(PyObject*, PyObject* const* args, Py_ssize_t n) {
                 for (int i = 0; i < 3; i++) node->save(*in[5 * i + s]);
             node->save_output(out);
             node->save_output(cell);
-            node->own = {gates[0], gates[1], gates[2], v_old[0], v_old[1], v_old[2], VARIANT == 1 ? h_init : aux, c_init};
+            node->keep({gates[0], gates[1], gates[2], v_old[0], v_old[1], v_old[2], VARIANT == 1 ? h_init : aux, c_init});
         }
     }
     PyObject* pair = PyTuple_New(2);

@@ -1,0 +1,63 @@
+"""Saved-tensor hooks reach everything the native autograd nodes keep for their backward: activation checkpointing and
+offloading free it all, and give the gradients of the plain call."""
+import pytest
+import torch
+from torch.utils.checkpoint import checkpoint
+
+from tests import util
+
+pytestmark = pytest.mark.gpu
+DEV = 'cuda:0'
+B, H, L, d = 2, 4, 130, 16
+STEP = B * H * L * d * 4        # bytes of one (B, H, L, d) tensor
+
+
+def cases(fwp):
+    """name -> (leaves, call, how many (B, H, L, d) tensors the node keeps besides inputs and outputs)"""
+    from recurrent_fwp_b200.delta_layer_io import delta_attention
+    z = lambda *s: torch.zeros(*s, device=DEV)
+    W, h = lambda: z(B, H, d, d), lambda: z(B, H, 1, d)
+    q, k, v, b, _ = (t.to(DEV) for t in util.delta_inputs(81, B, H, L, d))
+    qkvb = torch.randn(L, B, H, 3 * d + 1, generator=util.gen(82)).to(DEV)
+    rec = [t.to(DEV) for t in util.rec_inputs(83, B, H, L, d)[:8]]
+    rnn = [t.to(DEV) for t in util.rnn_inputs(84, B, H, L, d)[:4]]
+    lstm = [t.to(DEV) for g in util.lstm_inputs(85, B, H, L, d)[0] for t in g]
+    call_lstm = lambda f: lambda *x: f(*x[0:4], W(), *x[4:8], W(), *x[8:12], W(), h(), h())[0]
+    return {'delta': ([q, k, v, b], lambda *x: fwp.fast_weight_delta(*x, W()), 1),
+            'layer': ([qkvb], lambda x: delta_attention(x, W(), 0.25), 4),
+            'sum': ([q, k, v], lambda *x: fwp.fast_weight_sum(*x, W()), 0),
+            'rec': (rec, lambda *x: fwp.rec_update_fwm_tanh(*x, W(), h()), 4),
+            'rnn1': (rnn, lambda z_, k_, v_, b_: fwp.fast_rnn(z_, k_, v_, W(), b_, h()), 1),
+            'rnn2': (rnn, lambda z_, k_, v_, b_: fwp.fast_rnn_v2(z_, k_, v_, W(), b_, h()), 2),
+            'lstm1': (lstm, call_lstm(fwp.fast_lstm), 6),
+            'lstm4': (lstm, call_lstm(fwp.fast_lstm_v4), 7)}
+
+
+@pytest.mark.parametrize('name', ['delta', 'layer', 'sum', 'rec', 'rnn1', 'rnn2', 'lstm1', 'lstm4'])
+def test_hooks_see_every_kept_buffer(fwp, name):
+    leaves, call, kept = cases(fwp)[name]
+    plain = [t.clone().requires_grad_() for t in leaves]
+    y = call(*plain)
+    gy = torch.randn(y.shape, generator=util.gen(86)).to(DEV)
+    y.backward(gy)
+
+    def run(wrapped):
+        x = [t.clone().requires_grad_() for t in leaves]
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        out = wrapped(*x)
+        held = torch.cuda.memory_allocated() - before - out.numel() * 4
+        out.backward(gy)
+        for a, r in zip(x, plain):
+            assert torch.equal(a.grad, r.grad)
+        return held
+
+    def offloaded(*x):
+        with torch.autograd.graph.save_on_cpu():
+            return call(*x)
+
+    own = run(call)
+    assert own >= kept * STEP
+    # with its tensors elsewhere a call holds no more than small change (states and the like)
+    assert run(offloaded) < STEP
+    assert run(lambda *x: checkpoint(call, *x, use_reentrant=False)) < STEP
