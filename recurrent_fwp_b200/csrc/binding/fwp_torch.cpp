@@ -150,7 +150,7 @@ struct OpNode : public Node {
         TORCH_CHECK(g.device() == like.device() && g.sizes() == shape, "grad_out is ", g.sizes(), " on ", g.device(),
                     ", expected ", shape, " on ", like.device());
         Tensor r = g.scalar_type() == like.scalar_type() ? g : g.to(like.scalar_type());
-        return r.size(3) == 1 || r.stride(3) == 1 ? r : r.contiguous();
+        return r.size(-1) == 1 || r.stride(-1) == 1 ? r : r.contiguous();
     }
     Tensor like_stream(int64_t width, const Tensor& like) const { return empty({d.N, d.H, d.L, width}, like.scalar_type(), like); }
 };
@@ -246,8 +246,7 @@ struct DeltaLayerNode final : public OpNode {
         at::NoGradGuard no_grad;
         const auto t = unpack(user), o = unpack(own);
         const Tensor &x = t[0], &W = t[1], &q = o[0], &k = o[1], &v = o[2], &beta = o[3], &v_old = o[4];
-        TORCH_CHECK(g[0].defined() && g[0].scalar_type() == at::kFloat, "the incoming gradient must be float32");
-        const Tensor gout = g[0].contiguous();
+        const Tensor gout = incoming(g[0], x, {d.L, d.N, d.H * d.M}).contiguous();
         void* st = stream_of(x);
         const int dev = x.device().index();
         const Desc gy = heads_first(gout, d);

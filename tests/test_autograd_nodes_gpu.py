@@ -1,5 +1,5 @@
-"""Saved-tensor hooks reach everything the native autograd nodes keep for their backward: activation checkpointing and
-offloading free it all, and give the gradients of the plain call."""
+"""The native autograd nodes among torch's own: saved-tensor hooks reach everything they keep for their backward (activation
+checkpointing and offloading free it all, and give the gradients of the plain call), and undefined gradients are zeros."""
 import pytest
 import torch
 from torch.utils.checkpoint import checkpoint
@@ -61,3 +61,24 @@ def test_hooks_see_every_kept_buffer(fwp, name):
     # with its tensors elsewhere a call holds no more than small change (states and the like)
     assert run(offloaded) < STEP
     assert run(lambda *x: checkpoint(call, *x, use_reentrant=False)) < STEP
+
+
+class Cut(torch.autograd.Function):
+    """Passes a tensor on and hands no gradient back: the node before it gets an undefined one."""
+
+    @staticmethod
+    def forward(ctx, x):
+        return x.clone()
+
+    @staticmethod
+    def backward(ctx, g):
+        return None
+
+
+@pytest.mark.parametrize('name', ['delta', 'layer', 'sum', 'rec', 'rnn1', 'rnn2', 'lstm1', 'lstm4'])
+def test_an_undefined_incoming_gradient_counts_as_zeros(fwp, name):
+    leaves, call, _ = cases(fwp)[name]
+    x = [t.clone().requires_grad_() for t in leaves]
+    Cut.apply(call(*x)).sum().backward()
+    for t in x:
+        assert t.grad is not None and not t.grad.any()
