@@ -147,10 +147,10 @@ int fwp_fast_weight_backward_with_scratch(int N, int H, int L, int E, int M,
                              float* scratch, int64_t scratch_floats,
                              int io_dtype, void* stream, int device);
 
-/* The delta-rule kernels move contiguous chunks with bulk asynchronous copies (in the tcgen05 plan also TMA
- * tile loads and tensor-core products) whose completion waits are bounded.  Returns 1 if such a wait ever ran out on the current device since the last
- * call (that launch then produced wrong numbers instead of hanging the GPU), 0 if not, -1 on a
- * CUDA error.  Synchronises the device; reading clears the flag.  No counterpart in the reference. */
+/* The kernels of the delta and sum rules wait for bulk copies, for tensor-core products and for one another's warps at
+ * barriers; these waits are bounded.  Returns 1 if such a wait ever ran out on the current device since the last call
+ * (that launch then produced wrong numbers instead of hanging the GPU), 0 if not, -1 on a CUDA error.  Synchronises the
+ * device; reading clears the flag.  No counterpart in the reference. */
 int fwp_delta_device_fault(void);
 /* Test hook for that mechanism: launches one CTA that waits, with a limit of `polls` (1..65536) polls, on a
  * barrier nothing completes; the wait runs out, the kernel returns, and the next fwp_delta_device_fault() reads 1.

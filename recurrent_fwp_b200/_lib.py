@@ -214,11 +214,11 @@ def check(rc, what):
 
 
 def device_fault():
-    """1 if a bounded wait inside a delta-rule kernel ran out since the last call (synchronises the device)."""
+    """1 if a bounded wait inside a kernel of the delta or sum rule ran out since the last call (synchronises the device)."""
     return int(lib.fwp_delta_device_fault())
 
 
-# With FWP_CHECK_DEVICE_FAULT=1 in the environment the delta-rule ops ask after every launch: that synchronises the
+# With FWP_CHECK_DEVICE_FAULT=1 in the environment the delta-rule and sum-rule ops ask after every launch: that synchronises the
 # device and raises if a bounded wait inside a kernel ran out (the launch then produced wrong numbers instead of
 # hanging).  Off by default because of the synchronisation; a trainer can instead poll ``device_fault()`` at step or
 # epoch boundaries.

@@ -33,7 +33,7 @@ using torch::autograd::variable_list;
 
 namespace {
 
-bool g_check_fault = false;     // FWP_CHECK_DEVICE_FAULT: ask for a device fault after every delta-rule launch
+bool g_check_fault = false;     // FWP_CHECK_DEVICE_FAULT: ask for a device fault after every launch of the delta and sum rules
 
 struct Dims {
     int64_t N, H, L, E, M;
@@ -70,7 +70,8 @@ void check(int rc, const char* what) {
         TORCH_CHECK(false, what, " failed: ", fwp_status_string(rc), " [cudaError ", fwp_last_cuda_error(), "]");
     TORCH_CHECK(false, what, " failed: ", fwp_status_string(rc));
 }
-void check_delta(int rc, const char* what) {
+// for the ops whose kernels have bounded waits
+void check_waits(int rc, const char* what) {
     check(rc, what);
     if (g_check_fault)
         TORCH_CHECK(fwp_delta_device_fault() == 0, what, ": a bounded wait inside the kernel ran out; its results are invalid");
@@ -173,7 +174,7 @@ void delta_backward(const Dims& d, const Tensor& Q, const Tensor& K, const Tenso
     const int64_t need = fwp_fast_weight_backward_scratch_floats(d.N, d.H, d.L, d.E, d.M, dtype_code(Q));
     Tensor scratch;
     if (need > 0) scratch = empty({need}, at::kFloat, Q);
-    check_delta(fwp_fast_weight_backward_with_scratch(d.N, d.H, d.L, d.E, d.M, Desc(Q), Desc(K), Desc(V), Desc(beta), Desc(v_old), gy,
+    check_waits(fwp_fast_weight_backward_with_scratch(d.N, d.H, d.L, d.E, d.M, Desc(Q), Desc(K), Desc(V), Desc(beta), Desc(v_old), gy,
                                                       Desc(W), Desc(gQ), Desc(gK), Desc(gV), Desc(gb),
                                                       need > 0 ? scratch.data_ptr<float>() : nullptr, need, dtype_code(Q), stream_of(Q),
                                                       Q.device().index()), "fast_weight_backward");
@@ -212,7 +213,7 @@ PyObject* fast_weight_delta(PyObject*, PyObject* const* args, Py_ssize_t n) {
         out = empty({d.N, d.H, d.L, d.M}, ty, Q);
         Tensor v_old;
         if (grad) v_old = empty(d, d.M, Q);
-        check_delta(fwp_fast_weight_forward(d.N, d.H, d.L, d.E, d.M, Desc(Q), Desc(K), Desc(V), Desc(beta), Desc(v_old),
+        check_waits(fwp_fast_weight_forward(d.N, d.H, d.L, d.E, d.M, Desc(Q), Desc(K), Desc(V), Desc(beta), Desc(v_old),
                                             Desc(Tensor()), Desc(W), Desc(out), dtype_code(Q), stream_of(Q), dev.index()),
                     "fast_weight_forward");
         if (grad) {
@@ -283,7 +284,7 @@ PyObject* delta_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
         check(fwp_delta_layer_prologue_forward_scaled(d.L, d.N, d.H, D, x.data_ptr<float>(), q.data_ptr<float>(), k.data_ptr<float>(),
                                                       v.data_ptr<float>(), beta.data_ptr<float>(), (float)scale, st, dev),
               "delta_layer_prologue_forward");
-        check_delta(fwp_fast_weight_forward(d.N, d.H, d.L, D, D, Desc(q), Desc(k), Desc(v), Desc(beta), Desc(v_old), Desc(Tensor()),
+        check_waits(fwp_fast_weight_forward(d.N, d.H, d.L, D, D, Desc(q), Desc(k), Desc(v), Desc(beta), Desc(v_old), Desc(Tensor()),
                                             Desc(W), heads_first(out, d), FWP_F32, st, dev), "fast_weight_forward");
         if (grad) {
             auto node = make_node<DeltaLayerNode>(in, d);
@@ -308,8 +309,8 @@ struct SumNode final : public OpNode {
         const Tensor &Q = t[0], &K = t[1], &V = t[2];
         const Tensor gy = incoming(g[0], Q, {d.N, d.H, d.L, d.M});
         Tensor gQ = like_stream(d.E, Q), gK = like_stream(d.E, Q), gV = like_stream(d.M, Q);
-        check(fwp_causal_dot_backward(d.N, d.H, d.L, d.E, d.M, Desc(Q), Desc(K), Desc(V), Desc(gy), Desc(gQ), Desc(gK), Desc(gV),
-                                      dtype_code(Q), stream_of(Q), Q.device().index()), "causal_dot_backward");
+        check_waits(fwp_causal_dot_backward(d.N, d.H, d.L, d.E, d.M, Desc(Q), Desc(K), Desc(V), Desc(gy), Desc(gQ), Desc(gK), Desc(gV),
+                                            dtype_code(Q), stream_of(Q), Q.device().index()), "causal_dot_backward");
         return {gQ, gK, gV, Tensor()};
     }
 };
@@ -330,8 +331,8 @@ PyObject* fast_weight_sum(PyObject*, PyObject* const* args, Py_ssize_t n) {
     {
         pybind11::gil_scoped_release no_gil;
         out = empty({d.N, d.H, d.L, d.M}, ty, Q);
-        check(fwp_causal_dot_product(d.N, d.H, d.L, d.E, d.M, Desc(Q), Desc(K), Desc(V), Desc(W), Desc(out), dtype_code(Q),
-                                     stream_of(Q), dev.index()), "causal_dot_product");
+        check_waits(fwp_causal_dot_product(d.N, d.H, d.L, d.E, d.M, Desc(Q), Desc(K), Desc(V), Desc(W), Desc(out), dtype_code(Q),
+                                           stream_of(Q), dev.index()), "causal_dot_product");
         if (needs_grad(in)) {
             auto node = make_node<SumNode>(in, d);
             for (int i = 0; i < 3; i++) node->save(*in[i]);

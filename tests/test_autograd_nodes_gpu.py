@@ -82,3 +82,28 @@ def test_an_undefined_incoming_gradient_counts_as_zeros(fwp, name):
     Cut.apply(call(*x)).sum().backward()
     for t in x:
         assert t.grad is not None and not t.grad.any()
+
+
+def test_fault_check_covers_both_rules_and_directions(fwp):
+    """With the check on, a wait that ran out (the library's bounded probe raises the flag) fails the next call."""
+    from recurrent_fwp_b200 import _lib
+
+    def ran_out():
+        stream, dev = _lib.stream_and_device(torch.zeros(1, device=DEV))
+        _lib.check(_lib.lib.fwp_debug_bounded_wait_probe(64, stream, dev), 'probe')
+
+    try:
+        _lib.native.check_device_fault(True)
+        for name in ('delta', 'layer', 'sum'):
+            leaves, call, _ = cases(fwp)[name]
+            x = [t.clone().requires_grad_() for t in leaves]
+            y = call(*x)
+            ran_out()
+            with pytest.raises(RuntimeError, match='bounded wait'):
+                call(*x)
+            ran_out()
+            with pytest.raises(RuntimeError, match='bounded wait'):
+                y.sum().backward()
+    finally:
+        _lib.native.check_device_fault(False)
+        _lib.device_fault()
