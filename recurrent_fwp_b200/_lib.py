@@ -183,6 +183,35 @@ def unit_inner(t):
     return t.contiguous()
 
 
+class _Recorded(torch.autograd.Function):
+    """An op as an autograd.Function around the native call, for callers that have to see one: torch.jit.trace records it,
+    forward-mode differentiation and function transforms refuse it."""
+
+    @staticmethod
+    def forward(ctx, name, *args):
+        tracing = torch._C._get_tracing_state()
+        torch._C._set_tracing_state(None)
+        try:
+            with torch.enable_grad():
+                inner = [a.detach().requires_grad_(a.requires_grad) if isinstance(a, torch.Tensor) else a for a in args]
+                out = getattr(native, name)(*inner)
+        finally:
+            torch._C._set_tracing_state(tracing)
+        if out is NotImplemented:
+            raise RuntimeError('%s: unsupported arguments' % name)
+        ctx.inner, ctx.out = inner, out if isinstance(out, tuple) else (out,)
+        return tuple(t.detach() for t in out) if isinstance(out, tuple) else out.detach()
+
+    @staticmethod
+    def backward(ctx, *grads):
+        want = [i for i, a in enumerate(ctx.inner) if isinstance(a, torch.Tensor) and a.requires_grad]
+        got = torch.autograd.grad(ctx.out, [ctx.inner[i] for i in want], grads, allow_unused=True)
+        res = [None] * len(ctx.inner)
+        for i, g in zip(want, got):
+            res[i] = g
+        return (None, *res)
+
+
 def entry_point(name, normalise):
     """The public callable of one op.  ``native.<name>`` takes arguments that are already in the form the kernels
     read and answers NotImplemented for anything else; then ``normalise`` raises the error that fits, or returns the
@@ -192,9 +221,10 @@ def entry_point(name, normalise):
     def op(*args):
         out = native_op(*args)
         if out is NotImplemented:
-            out = native_op(*normalise(*args))
+            args = normalise(*args)
+            out = native_op(*args)
             if out is NotImplemented:
-                raise RuntimeError('%s: unsupported arguments' % name)
+                out = _Recorded.apply(name, *args)
         return out
 
     op.__name__ = op.__qualname__ = name

@@ -15,6 +15,7 @@
 #include <mutex>
 #include <vector>
 #include <ATen/ATen.h>
+#include <ATen/TracerMode.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -100,13 +101,19 @@ bool first_stream(const Tensor& t, bool bf16) {
            (t.size(3) == 1 || t.stride(3) == 1);
 }
 
-// Borrowed tensor arguments of a METH_FASTCALL function; false when one of them is not a tensor.
+// Borrowed tensor arguments of a METH_FASTCALL function; false when one of them is not a plain tensor.  A tensor with a
+// forward-mode tangent or a wrapper of a function transform is not, and nothing is while torch.jit traces: a call from here
+// would drop the tangent, or leave its result in the trace as a constant.  The module has an autograd.Function for those.
 template <size_t K>
 bool tensors(PyObject* const* args, Py_ssize_t n, std::array<const Tensor*, K>& out) {
-    if (n < (Py_ssize_t)K) return false;
+    if (n < (Py_ssize_t)K || at::tracer::impl::is_dispatch_enabled()) return false;
+    constexpr c10::DispatchKeySet wrappers({c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper});
     for (size_t i = 0; i < K; i++) {
         if (!THPVariable_Check(args[i])) return false;
-        out[i] = &THPVariable_Unpack(args[i]);
+        const Tensor& t = THPVariable_Unpack(args[i]);
+        const auto* impl = t.unsafeGetTensorImpl();
+        if (impl->key_set().has_any(wrappers) || (impl->autograd_meta() && torch::autograd::isFwGradDefined(t))) return false;
+        out[i] = &t;
     }
     return true;
 }

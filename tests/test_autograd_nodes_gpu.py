@@ -12,17 +12,20 @@ B, H, L, d = 2, 4, 130, 16
 STEP = B * H * L * d * 4        # bytes of one (B, H, L, d) tensor
 
 
-def cases(fwp):
-    """name -> (leaves, call, how many (B, H, L, d) tensors the node keeps besides inputs and outputs)"""
+def cases(fwp, start=None):
+    """name -> (leaves, call, how many (B, H, L, d) tensors the node keeps besides inputs and outputs); every call starts
+    from multiples of start['W'], start['h']"""
     from recurrent_fwp_b200.delta_layer_io import delta_attention
-    z = lambda *s: torch.zeros(*s, device=DEV)
-    W, h = lambda: z(B, H, d, d), lambda: z(B, H, 1, d)
+    if start is None:
+        start = {'W': torch.zeros(B, H, d, d, device=DEV), 'h': torch.zeros(B, H, 1, d, device=DEV)}
+    # factors, none of them 1: tensors of their own, also for a tracer that merges equal nodes
+    W, h = lambda f=3: start['W'] * f, lambda f=3: start['h'] * f
     q, k, v, b, _ = (t.to(DEV) for t in util.delta_inputs(81, B, H, L, d))
     qkvb = torch.randn(L, B, H, 3 * d + 1, generator=util.gen(82)).to(DEV)
     rec = [t.to(DEV) for t in util.rec_inputs(83, B, H, L, d)[:8]]
     rnn = [t.to(DEV) for t in util.rnn_inputs(84, B, H, L, d)[:4]]
     lstm = [t.to(DEV) for g in util.lstm_inputs(85, B, H, L, d)[0] for t in g]
-    call_lstm = lambda f: lambda *x: f(*x[0:4], W(), *x[4:8], W(), *x[8:12], W(), h(), h())[0]
+    call_lstm = lambda f: lambda *x: f(*x[0:4], W(), *x[4:8], W(2), *x[8:12], W(4), h(), h(2))[0]
     return {'delta': ([q, k, v, b], lambda *x: fwp.fast_weight_delta(*x, W()), 1),
             'layer': ([qkvb], lambda x: delta_attention(x, W(), 0.25), 4),
             'sum': ([q, k, v], lambda *x: fwp.fast_weight_sum(*x, W()), 0),
@@ -107,3 +110,41 @@ def test_fault_check_covers_both_rules_and_directions(fwp):
     finally:
         _lib.native.check_device_fault(False)
         _lib.device_fault()
+
+
+@pytest.mark.parametrize('name', ['delta', 'layer', 'sum', 'rec', 'rnn1', 'rnn2', 'lstm1', 'lstm4'])
+def test_tracing_records_the_call(fwp, name):
+    """torch.jit.trace: the traced function computes, and differentiates, on new inputs what the plain one does."""
+    W, h = torch.full((B, H, d, d), 0.1, device=DEV), torch.full((B, H, 1, d), 0.1, device=DEV)
+    start = {}
+    leaves, call, _ = cases(fwp, start)[name]
+
+    def f(W0, h0, *x):
+        start.update(W=W0, h=h0)
+        return call(*x) * 2
+
+    traced = torch.jit.trace(f, (W * 0, h * 0, *(t.flip(0) for t in leaves)))
+    x, r = ([t.clone().requires_grad_() for t in leaves] for _ in range(2))
+    y, ref = traced(W, h, *x), f(W, h, *r)
+    assert torch.equal(y, ref)
+    gy = torch.randn(y.shape, generator=util.gen(87)).to(DEV)
+    y.backward(gy)
+    ref.backward(gy)
+    for a, b in zip(x, r):
+        assert torch.equal(a.grad, b.grad)
+
+
+@pytest.mark.parametrize('name', ['delta', 'layer', 'sum', 'rec', 'rnn1', 'lstm1'])
+def test_forward_mode_and_function_transforms_are_refused(fwp, name):
+    """The ops have a backward only: a tangent or a transform raises, as from any autograd.Function without them."""
+    import torch.autograd.forward_ad as fw
+    leaves, call, _ = cases(fwp)[name]
+    with fw.dual_level():
+        x = [fw.make_dual(leaves[0], torch.ones_like(leaves[0]))] + leaves[1:]
+        with pytest.raises(RuntimeError):
+            call(*x)
+    with pytest.raises(RuntimeError):
+        torch.func.vmap(lambda t: call(t, *leaves[1:]))(torch.stack([leaves[0]] * 2))
+    with pytest.raises(RuntimeError):
+        torch.func.grad(lambda t: call(t, *leaves[1:]).sum())(leaves[0])
+    assert call(*leaves).isfinite().all()
