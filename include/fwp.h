@@ -135,7 +135,8 @@ int fwp_fast_weight_backward(int N, int H, int L, int E, int M,
 
 /* The same backward for callers that can lend device memory: with at least fwp_fast_weight_backward_scratch_floats(...)
  * floats of it (16-byte aligned, contents undefined before and after), shapes that gain from it run as three launches that
- * work on all chunks of all sequences at once.  0 floats, or scratch == NULL: the plain backward.  The pointer is not kept.
+ * work on all chunks of all sequences at once (larger calls part by part: it is never more than 64 MB).  0 floats, or
+ * scratch == NULL: the plain backward.  The pointer is not kept.
  * The answer depends on the sizes and the execution-plan switches only. */
 int64_t fwp_fast_weight_backward_scratch_floats(int N, int H, int L, int E, int M, int io_dtype);
 int fwp_fast_weight_backward_with_scratch(int N, int H, int L, int E, int M,

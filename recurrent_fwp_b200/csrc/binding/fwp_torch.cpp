@@ -18,6 +18,7 @@
 #include <ATen/TracerMode.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAStream.h>
+#include <c10/util/Exception.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
@@ -175,12 +176,16 @@ std::shared_ptr<NodeT> make_node(const std::array<const Tensor*, K>& in, const D
 }
 
 // ------------------------------------------------------------------ delta rule
-// the backward with the scratch memory it asks for
+// the backward with the scratch memory it asks for; where the device has none left, without
 void delta_backward(const Dims& d, const Tensor& Q, const Tensor& K, const Tensor& V, const Tensor& beta, const Tensor& v_old, const Desc& gy,
                     const Tensor& W, const Tensor& gQ, const Tensor& gK, const Tensor& gV, const Tensor& gb) {
-    const int64_t need = fwp_fast_weight_backward_scratch_floats(d.N, d.H, d.L, d.E, d.M, dtype_code(Q));
+    int64_t need = fwp_fast_weight_backward_scratch_floats(d.N, d.H, d.L, d.E, d.M, dtype_code(Q));
     Tensor scratch;
-    if (need > 0) scratch = empty({need}, at::kFloat, Q);
+    if (need > 0) try {
+        scratch = empty({need}, at::kFloat, Q);
+    } catch (const c10::OutOfMemoryError&) {
+        need = 0;
+    }
     check_waits(fwp_fast_weight_backward_with_scratch(d.N, d.H, d.L, d.E, d.M, Desc(Q), Desc(K), Desc(V), Desc(beta), Desc(v_old), gy,
                                                       Desc(W), Desc(gQ), Desc(gK), Desc(gV), Desc(gb),
                                                       need > 0 ? scratch.data_ptr<float>() : nullptr, need, dtype_code(Q), stream_of(Q),

@@ -12,8 +12,8 @@
 //   b = diag(beta) r = dV,   dbeta_i = r_i . w_i,   dQ = gY S0^T + H K,   H = tril(gY U^T)
 //   dK = U G^T - b S0^T + H^T Q - R K,  R_ij = u_min(i,j) . b_max(i,j)  (i != j)               (finish)
 // All products are split fp32 products (fwp_split3.cuh).  The workspace holds operands as ready fragments, 16 bytes per
-// lane, so that every access to it is a coalesced 512-byte line per warp; it is meant to stay in the L2 cache, and long
-// calls are cut into segments that do.  Each kernel is short enough to stay in the instruction cache (one kernel with a
+// lane, so that every access to it is a coalesced 512-byte line per warp; it is meant to stay in the L2 cache, and larger
+// calls are cut into segments of time, then into groups of sequences, that do.  Each kernel is short enough to stay in the instruction cache (one kernel with a
 // role per phase was not: instruction fetch was its largest stall, and two sequences per SM took twice as long as one).
 //
 // Values that are not finite.  As in the forward (fwp_delta_wy.cuh), a chunk's products would carry a NaN or Inf to steps of
@@ -42,9 +42,10 @@ struct BwdSpace {                       // one chunk, in uint4
 
 struct BwdPhase {
     DeltaBwdParams p;
-    uint4* ws;                          // [sequence][chunk of the segment]
-    uint4* carry;                       // [sequence][MS][KS][2][32]: G^T between segments
-    int* again;                         // [sequence]: something that is not finite turned up
+    uint4* ws;                          // [sequence of the group][chunk of the segment]
+    uint4* carry;                       // [sequence of the group][MS][KS][2][32]: G^T between segments
+    int* again;                         // [sequence of the group]: something that is not finite turned up
+    int s0, ns;                         // the group: sequences [s0, s0 + ns)
     int c0, nc;                         // the segment: chunks [c0, c0 + nc)
     int first;                          // 1: the last chunks of the sequence, G starts from zero
 };
@@ -111,8 +112,8 @@ __device__ __forceinline__ bool finite(const float (&x)[K][2][4]) {
 // W holds the rewound state; S is brought forward from it with the u of the forward first.  `G` and `S` hold E x M floats
 // each and `vec` 2 M, all of them this warp's own.  Inlined, for the reason stepwise_forward is.
 template <typename T>
-__device__ __forceinline__ void stepwise_backward(const DeltaBwdParams& p, int seq, float* G, float* S, float* vec) {
-    const int lane = threadIdx.x & 31, n = seq / p.H, h = seq - n * p.H, E = p.E, M = p.M;
+__device__ __forceinline__ void stepwise_backward(const DeltaBwdParams& p, int n, int h, float* G, float* S, float* vec) {
+    const int lane = threadIdx.x & 31, E = p.E, M = p.M;
     const T *qp = stream_at<T>(p.q, n, h), *kp = stream_at<T>(p.k, n, h), *vp = stream_at<T>(p.v, n, h), *bp = stream_at<T>(p.beta, n, h);
     const T* yp = stream_at<T>(p.gy, n, h);
     const float* op = stream_at<float>(p.v_old, n, h);
@@ -194,9 +195,9 @@ __global__ void __launch_bounds__(WARPS * 32) delta_bwd_prepare_kernel(const __g
     const int seq = (int)(unit / a.nc), c = a.c0 + (int)(unit - (long long)seq * a.nc);
     griddep_wait();
     griddep_launch_dependents();
-    if (seq >= p.NH) return;
+    if (seq >= a.ns) return;
     Sm& sm = reinterpret_cast<Sm*>(smem_raw)[threadIdx.x >> 5];
-    const int n = seq / p.H, h = seq - n * p.H, t0 = c * C, nt = min(C, p.L - t0);
+    const int n = (a.s0 + seq) / p.H, h = a.s0 + seq - n * p.H, t0 = c * C, nt = min(C, p.L - t0);
     if (a.first && c == a.c0 && lane == 0) a.again[seq] = 0;
     uint4* const ws = a.ws + unit * Sp::kSize;
     const unsigned at = 2 * lane_at(lane, P), atC = 2 * lane_at(lane, PC);
@@ -330,7 +331,7 @@ __global__ void __launch_bounds__(64) delta_bwd_chain_kernel(const __grid_consta
     griddep_launch_dependents();
     uint4* const ws = a.ws + (long long)seq * a.nc * Sp::kSize;
     if (threadIdx.x >= 32) {
-        const int n = seq / p.H, h = seq - n * p.H;
+        const int n = (a.s0 + seq) / p.H, h = a.s0 + seq - n * p.H;
         float* W = p.W + n * p.wN + h * p.wH;
         constexpr int AHEAD = 4;
         bool good = true;
@@ -446,8 +447,8 @@ __global__ void __launch_bounds__(WARPS * 32, M == 16 ? (E > 64 ? 5 : 4) : 0) de
     const int seq = (int)(unit / a.nc), c = a.c0 + (int)(unit - (long long)seq * a.nc);
     griddep_wait();
     griddep_launch_dependents();
-    if (seq >= p.NH) return;
-    const int n = seq / p.H, h = seq - n * p.H, t0 = c * C, nt = min(C, p.L - t0);
+    if (seq >= a.ns) return;
+    const int n = (a.s0 + seq) / p.H, h = a.s0 + seq - n * p.H, t0 = c * C, nt = min(C, p.L - t0);
     const uint4* const ws = a.ws + unit * Sp::kSize;
     float bt[2][2];
     load_beta(bt, stream_at<T>(p.beta, n, h) + t0 * p.beta.sL, p.beta.sL, nt, t);
@@ -478,7 +479,7 @@ __global__ void __launch_bounds__(WARPS * 32, M == 16 ? (E > 64 ? 5 : 4) : 0) de
     if (__builtin_expect(a.again[seq] != 0, 0)) {
         if (c == 0 && k0 == 0) {                        // the last segment: nobody else writes to this chunk's part of the workspace
             float* const own = reinterpret_cast<float*>(a.ws + unit * Sp::kSize);
-            stepwise_backward<T>(p, seq, own + 4 * Sp::G, own + 4 * Sp::S, own + 4 * Sp::R);
+            stepwise_backward<T>(p, n, h, own + 4 * Sp::G, own + 4 * Sp::S, own + 4 * Sp::R);
         }
         return;
     }
