@@ -260,6 +260,10 @@ class DeltaStep:
         self.d_none = D(None)     # u_t ("v_insert") is rebuilt by the backward: not stored
         self.d_g = [[D(t) for t in seg] for seg in self.g]
         self.dev_index = device.index
+        # the backward a user gets: with the scratch memory the library asks for at this shape (none at many)
+        self.n_scratch = _lib.lib.fwp_fast_weight_backward_scratch_floats(B, H, L, d, d, self.code) if rule == 'delta' else 0
+        self.scratch = torch.empty(self.n_scratch, **f32)
+        self.p_scratch = ctypes.cast(self.scratch.data_ptr(), ctypes.POINTER(ctypes.c_float)) if self.n_scratch else None
         self.kernels = {}
 
     def fwd(self, s, stream):
@@ -284,9 +288,9 @@ class DeltaStep:
                 B, H, L, d, d, q, k, v, gy, gq, gk, gv, self.code, stream, self.dev_index), 'sum bwd')
             self.kernels['bwd'] = self.L_.last_kernel()
             return
-        self.L_.check(self.L_.lib.fwp_fast_weight_backward(
-            B, H, L, d, d, q, k, v, b, self.d_vo[s], self.d_none, gy, self.d_Ws[s], gq, gk, gv, gb,
-            self.code, stream, self.dev_index), 'bwd')
+        self.L_.check(self.L_.lib.fwp_fast_weight_backward_with_scratch(
+            B, H, L, d, d, q, k, v, b, self.d_vo[s], gy, self.d_Ws[s], gq, gk, gv, gb,
+            self.p_scratch, self.n_scratch, self.code, stream, self.dev_index), 'bwd')
         self.kernels['bwd'] = self.L_.last_kernel()
 
     def step(self):
