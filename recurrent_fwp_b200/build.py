@@ -6,7 +6,8 @@ the autograd entry points, plain C++ against PyTorch) beside it.
 Each ``csrc/*.cu`` is compiled to an object file (in parallel) and linked into
 ``recurrent_fwp_b200/libfwp.so`` with the CUDA runtime linked statically, so the
 library has no dependency beyond the driver.  Objects are rebuilt only when a
-source or header is newer.  nvcc cross-compiles without a GPU.
+source or header is newer, ``_fwp_torch.so`` also when it was built against another
+PyTorch or Python or by another command.  nvcc cross-compiles without a GPU.
 """
 import concurrent.futures
 import glob
@@ -21,6 +22,7 @@ OBJ = os.path.join(PKG, 'build')
 LIB = os.path.join(PKG, 'libfwp.so')
 BINDING_SRC = os.path.join(CSRC, 'binding', 'fwp_torch.cpp')
 BINDING = os.path.join(PKG, '_fwp_torch.so')
+BINDING_STAMP = os.path.join(OBJ, '_fwp_torch.built')
 NVCC = os.environ.get('NVCC', '/usr/local/cuda/bin/nvcc')
 FLAGS = ['-gencode', 'arch=compute_100a,code=sm_100a', '-lineinfo', '-O3', '-std=c++17',
          '-Xcompiler', '-fPIC', '-Xcompiler', '-fvisibility=hidden']
@@ -40,7 +42,7 @@ def _compile(args):
     return src, r.returncode, r.stdout + r.stderr
 
 
-def _compile_binding():
+def _binding_command():
     """_fwp_torch.so: links libfwp.so (found beside it at run time) and the PyTorch libraries already loaded."""
     import torch
     from torch.utils import cpp_extension
@@ -50,11 +52,32 @@ def _compile_binding():
     cmd += ['-isystem' + d for d in cpp_extension.include_paths()]
     cmd += [BINDING_SRC, '-o', BINDING, '-L' + PKG, '-l:libfwp.so', '-Wl,-rpath,$ORIGIN']
     cmd += ['-L' + d for d in cpp_extension.library_paths()]
-    cmd += ['-lc10', '-lc10_cuda', '-ltorch_cpu', '-ltorch_cuda', '-ltorch', '-ltorch_python']
-    r = subprocess.run(cmd, capture_output=True, text=True)
+    return cmd + ['-lc10', '-lc10_cuda', '-ltorch_cpu', '-ltorch_cuda', '-ltorch', '-ltorch_python']
+
+
+def _binding_stamp():
+    """What the extension depends on besides its source: it uses PyTorch's C++ interface, which changes with the version."""
+    import torch
+    return '\n'.join([torch.__version__, str(torch.version.git_version), sys.version] + _binding_command())
+
+
+def _binding_stale():
+    if _newer([BINDING_SRC] + glob.glob(os.path.join(PKG, '..', 'include', '*.h')), BINDING):
+        return True
+    try:
+        with open(BINDING_STAMP) as f:
+            return f.read() != _binding_stamp()
+    except OSError:
+        return True
+
+
+def _compile_binding():
+    r = subprocess.run(_binding_command(), capture_output=True, text=True)
     if r.returncode:
         sys.stderr.write(r.stdout + r.stderr)
         raise RuntimeError('the compiler failed on %s' % BINDING_SRC)
+    with open(BINDING_STAMP, 'w') as f:
+        f.write(_binding_stamp())
 
 
 def build(force=False, verbose=False):
@@ -81,7 +104,7 @@ def build(force=False, verbose=False):
         if r.returncode:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError('link failed')
-    if force or _newer([BINDING_SRC] + glob.glob(os.path.join(PKG, '..', 'include', '*.h')), BINDING):
+    if force or _binding_stale():
         _compile_binding()
     return LIB
 
