@@ -84,7 +84,8 @@ int fwp_max_head_dim(void);
 /* Number of kernels this library has launched in this process (all threads). */
 unsigned long long fwp_launch_count(void);
 /* Execution-plan switch for experiments and cross-checks (process-wide, atomic):
- * "delta.blocked" (-1 automatic, 0 per-step kernels, 1 four-step blocked kernels),
+ * "delta.blocked" (-1 automatic, 0 per-step kernels, 1 four-step blocked kernels: the forward at D = 16, the
+ * backward at D = 16 and, for fp32 streams, 32 and 64),
  * "delta.chunk64" (1 / 0: chunkwise tensor-core plan for bf16 streams at E = M = 64),
  * "delta.tc64" (-1 / 1 / 0: tcgen05 forward of that plan when the call has no more sequences than the device has SMs
  * and at least 128 steps, always, or never), "<op>.<D>.split", "delta_bwd.bulk",

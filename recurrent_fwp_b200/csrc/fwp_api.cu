@@ -14,8 +14,7 @@ static thread_local const char* g_last_kernel = "";
 // Process-wide execution-plan switches: one atomic per key, INT_MIN = not set.
 static const char* const kTuneNames[T_COUNT] = {
     "delta.blocked", "delta.chunk64", "delta.tc64",
-    "delta_fwd.16.split", "delta_fwd.32.split", "delta_fwd.64.split",
-    "sum_fwd.16.split", "sum_fwd.32.split", "sum_fwd.64.split",
+    "delta_fwd.16.split", "sum_fwd.16.split",
     "delta_bwd.16.split", "delta_bwd.32.split", "delta_bwd.64.split",
     "delta_bwd.bulk", "delta_bwd.16.chunk",
     "lstm_fwd.32.split", "lstm_bwd.32.split", "rnn_fwd.32.split", "rnn_bwd.32.split", "rec_fwd.32.split", "rec_bwd.32.split",

@@ -48,11 +48,10 @@ void note_kernel(const char* name);     // remembers, per host thread, the kerne
 // Execution-plan switches (fwp_tune).  Each is one atomic integer looked up by index, so the dispatch of a
 // call reads a few relaxed atomics: no string handling, no lock.
 enum TuneKey {
-    T_DELTA_BLOCKED,        // "delta.blocked": -1 automatic, 0 per-step kernels, 1 four-step blocked kernels
+    T_DELTA_BLOCKED,        // "delta.blocked": -1 automatic, 0 per-step kernels, 1 four-step blocked kernels (forward d = 16; backward d = 16, fp32 also 32 and 64)
     T_DELTA_CHUNK64,        // "delta.chunk64": 1 chunkwise tensor-core plan for bf16 streams at E = M = 64, 0 off
     T_DELTA_TC64,           // "delta.tc64": -1 automatic (tcgen05 forward when the call has no more sequences than the device has SMs and at least 128 steps), 1 tcgen05 forward of that plan, 0 the warp-level mma forward
-    T_DELTA_FWD_SPLIT16, T_DELTA_FWD_SPLIT32, T_DELTA_FWD_SPLIT64,      // "delta_fwd.<D>.split"
-    T_SUM_FWD_SPLIT16, T_SUM_FWD_SPLIT32, T_SUM_FWD_SPLIT64,            // "sum_fwd.<D>.split"
+    T_DELTA_FWD_SPLIT16, T_SUM_FWD_SPLIT16,                             // "delta_fwd.16.split", "sum_fwd.16.split"
     T_DELTA_BWD_SPLIT16, T_DELTA_BWD_SPLIT32, T_DELTA_BWD_SPLIT64,      // "delta_bwd.<D>.split"
     T_DELTA_BWD_BULK,       // "delta_bwd.bulk": 1 bulk-copy staging in the d = 16 backward, 0 cp.async
     T_DELTA_BWD_CHUNK16,    // "delta_bwd.16.chunk": 32 or 16 steps per staged chunk
@@ -746,6 +745,17 @@ __device__ __forceinline__ float warp_sum4_idx(float p0, float p1, float p2, flo
 #pragma unroll
     for (int o = H2 / 2; o >= 1; o >>= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
     return k;
+}
+
+// a device flag of the current device: 1 if it was raised since the last call, which clears it, -1 on a CUDA error
+static inline int flag_read_clear(const int& symbol) {
+    int v = 0;
+    if (cudaMemcpyFromSymbol(&v, symbol, sizeof v) != cudaSuccess) return -1;
+    if (v) {
+        const int zero = 0;
+        cudaMemcpyToSymbol(symbol, &zero, sizeof zero);
+    }
+    return v;
 }
 
 #endif  // __CUDACC__

@@ -511,8 +511,8 @@ static int launch_sum_bwd_generic(const SumBwdParams& p, int nseq, cudaStream_t 
 // Which execution plan runs by default was picked per head dimension from measurements on B200
 // (forward / backward device time, 512 sequences):
 //   D=16: blocked + warp-specialised wins both ways (28.3 / 48.5 us vs 41.7 / 103.7 us per-step);
-//   D=32: forward per-step 55 us vs blocked 56-71 us, backward blocked 138 us vs per-step 175 us;
-//   D=64: forward per-step 161 us vs blocked 208 us; backward fp32 blocked 479 us vs per-step 584 us,
+//   D=32: forward per-step 55 us (a blocked form took 56-71), backward blocked 138 us vs per-step 175 us;
+//   D=64: forward per-step 161 us (a blocked form took 208); backward fp32 blocked 479 us vs per-step 584 us,
 //         bf16 streams (1024 steps) per-step 2.35 ms vs blocked 3.12 ms (the producer warp's widening pass).
 // Short segments (the reinforcement-learning callers step the op with L = 1, reinforcement_learning/torchbeast/
 // layer.py:143-186) take the per-step plan, whose CTAs start faster: at L <= 16 it measures 10-12 us against
@@ -570,23 +570,14 @@ static int dispatch_fwd(const DeltaFwdParams& p, int nseq, cudaStream_t st) {
             if (tune_get(SUM ? T_SUM_FWD_SPLIT16 : T_DELTA_FWD_SPLIT16, 2) == 4) return launch_fwd<16, 4, 32, T, SUM>(p, nseq, st);
             return launch_fwd<16, 2, 32, T, SUM>(p, nseq, st);
         }
-        case 32: {
-            // fp32 streams: per-step 55 us vs blocked 56 us; bf16 streams: blocked 80 us vs per-step 87 us
-            if (force == 0 || (force == -1 && (sizeof(T) == 4 || p.L <= kShortSeq))) return launch_fwd_step<32, 1, 16, T, SUM>(p, nseq, st);
-            const int sp = tune_get(SUM ? T_SUM_FWD_SPLIT32 : T_DELTA_FWD_SPLIT32, 1);
-            if (sp == 2) return launch_fwd<32, 2, 16, T, SUM>(p, nseq, st);
-            if (sp == 4) return launch_fwd<32, 4, 16, T, SUM>(p, nseq, st);
-            return launch_fwd<32, 1, 16, T, SUM>(p, nseq, st);
-        }
+        case 32: return launch_fwd_step<32, 1, 16, T, SUM>(p, nseq, st);
         case 64: {
             if constexpr (!SUM && sizeof(T) == 2) {
                 // chunkwise tensor-core form for bf16 streams ("delta.chunk64" = 0 switches it off)
                 if (force == -1 && p.L > kShortSeq && tune_get(T_DELTA_CHUNK64, 1) == 1 && chunk_bf16_applies(p))
                     return launch_fwd_chunk_bf16(p, nseq, st);
             }
-            if (force != 1) return launch_fwd_step<64, 2, 8, T, SUM>(p, nseq, st);
-            if (tune_get(SUM ? T_SUM_FWD_SPLIT64 : T_DELTA_FWD_SPLIT64, 2) == 4) return launch_fwd<64, 4, 8, T, SUM>(p, nseq, st);
-            return launch_fwd<64, 2, 8, T, SUM>(p, nseq, st);
+            return launch_fwd_step<64, 2, 8, T, SUM>(p, nseq, st);
         }
     }
     return FWP_ERR_UNSUPPORTED;
@@ -654,20 +645,22 @@ static int dispatch_bwd(const DeltaBwdParams& p0, int nseq, cudaStream_t st) {
         }
         case 32: {
             // fp32 streams: blocked 138 us vs per-step 175 us; bf16 streams: per-step 201 us vs blocked 207 us
-            if (force == 0 || (force == -1 && (p.L <= kShortSeq || sizeof(T) != 4))) return launch_bwd_step<32, 2, 8, T>(p, nseq, st);
-            if (tune_get(T_DELTA_BWD_SPLIT32, 2) == 4) return launch_bwd<32, 4, 8, T>(p, nseq, st);
-            return launch_bwd<32, 2, 8, T>(p, nseq, st);
+            if constexpr (sizeof(T) == 4) {
+                if (force == 1 || (force == -1 && p.L > kShortSeq))
+                    return tune_get(T_DELTA_BWD_SPLIT32, 2) == 4 ? launch_bwd<32, 4, 8, T>(p, nseq, st) : launch_bwd<32, 2, 8, T>(p, nseq, st);
+            }
+            return launch_bwd_step<32, 2, 8, T>(p, nseq, st);
         }
         case 64: {
             if constexpr (sizeof(T) == 2) {
                 // chunkwise tensor-core form for bf16 streams ("delta.chunk64" = 0 switches it off)
                 if (force == -1 && p.L > kShortSeq && tune_get(T_DELTA_CHUNK64, 1) == 1 && chunk_bf16_applies(p))
                     return launch_bwd_chunk_bf16(p, nseq, st);
+            } else {
+                if (force == 1 || (force == -1 && p.L > 4 * kShortSeq))
+                    return tune_get(T_DELTA_BWD_SPLIT64, 2) == 4 ? launch_bwd<64, 4, 4, T>(p, nseq, st) : launch_bwd<64, 2, 4, T>(p, nseq, st);
             }
-            const bool blocked = force == 1 || (force == -1 && sizeof(T) == 4 && p.L > 4 * kShortSeq);
-            if (!blocked) return launch_bwd_step<64, 4, 4, T>(p, nseq, st);
-            if (tune_get(T_DELTA_BWD_SPLIT64, 2) == 4) return launch_bwd<64, 4, 4, T>(p, nseq, st);
-            return launch_bwd<64, 2, 4, T>(p, nseq, st);
+            return launch_bwd_step<64, 4, 4, T>(p, nseq, st);
         }
     }
     return FWP_ERR_UNSUPPORTED;
@@ -875,13 +868,7 @@ FWP_API int fwp_debug_bounded_wait_probe(int polls, void* stream, int device) {
 // (the affected launch produced wrong numbers instead of hanging), 0 if not, -1 on a CUDA error.
 // Synchronises the device; reading clears the flag.
 FWP_API int fwp_delta_device_fault(void) {
-    int v = 0;
-    if (cudaMemcpyFromSymbol(&v, fwp::g_delta_fault, sizeof v) != cudaSuccess) return -1;
-    if (v) {
-        const int zero = 0;
-        cudaMemcpyToSymbol(fwp::g_delta_fault, &zero, sizeof zero);
-    }
-    const int t = fwp::tc_fault_read_clear(), w = fwp::wy_fault_read_clear(), u = fwp::sum_wy_fault_read_clear();
-    if (t < 0 || w < 0 || u < 0) return -1;
+    const int v = fwp::flag_read_clear(fwp::g_delta_fault), t = fwp::tc_fault_read_clear(), w = fwp::wy_fault_read_clear(), u = fwp::sum_wy_fault_read_clear();
+    if (v < 0 || t < 0 || w < 0 || u < 0) return -1;
     return (v || t || w || u) ? 1 : 0;
 }

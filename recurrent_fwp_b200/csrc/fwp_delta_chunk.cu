@@ -40,16 +40,7 @@ static int launch_fwd_tc(const DeltaFwdParams& p, int nseq, cudaStream_t st) {
 }
 
 // 1 if a bounded wait of the tcgen05 kernel ran out on the current device since the last call (reading clears it)
-int tc_fault_read_clear() {
-    int v = 0;
-    if (cudaMemcpyFromSymbol(&v, g_tc_fault, sizeof v) != cudaSuccess) return -1;
-    if (v) {
-        const int zero = 0;
-        cudaMemcpyToSymbol(g_tc_fault, &zero, sizeof zero);
-    }
-    return v;
-}
-
+int tc_fault_read_clear() { return flag_read_clear(g_tc_fault); }
 
 // Test hook for the bounded waits: one CTA waits, with the given poll limit, on an mbarrier that nothing ever
 // completes.  The wait runs out, the kernel returns and the device flag is raised, exactly what a kernel of this file

@@ -4,15 +4,7 @@
 namespace fwp {
 
 // 1 if a bounded wait of these kernels ran out on the current device since the last call (reading clears it)
-int sum_wy_fault_read_clear() {
-    int v = 0;
-    if (cudaMemcpyFromSymbol(&v, wy::g_wy_fault, sizeof v) != cudaSuccess) return -1;
-    if (v) {
-        const int zero = 0;
-        cudaMemcpyToSymbol(wy::g_wy_fault, &zero, sizeof zero);
-    }
-    return v;
-}
+int sum_wy_fault_read_clear() { return flag_read_clear(wy::g_wy_fault); }
 
 template <int E, int NB, int CTAS, typename T>
 static int run(const wy::SumBwdForwards& a, int nseq, cudaStream_t st) {
