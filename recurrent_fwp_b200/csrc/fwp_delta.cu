@@ -536,7 +536,7 @@ static float wave_fill(int nseq, int per_sm) {
 //           1.0-1.4, 736 0.8-1.2, 1536 0.7-1.0;  rows of 24: up to 480 1.0-2.2, then as full rows;  bf16: 1.3-2.1, rows of 24 1.9-3.2;
 //   d = 48: 1.0-2.3 but for 0.8 at 1536 x 20, bf16 1.2-2.8;
 //   d = 64, fp32: 160 1.0 (20 steps) to 1.7, 320 0.9 (20) to 1.5, 736 0.7 (20), 0.9 (40), 1.1 (64) to 1.2;
-//   E, M = 96, 32: 128 x 256 692 -> 68 us;   128, 128: 1655 -> 98 us (the shared-memory kernels).
+//   E, M = 96, 32: 128 x 256 545 -> 65 us;   128, 128: 1730 -> 98 us (the shared-memory kernels).
 template <typename T, bool SUM>
 static bool fwd_wy_pays(const DeltaFwdParams& p, int nseq) {
     const int d = p.E > p.M ? p.E : p.M, sms = sm_count();
@@ -588,7 +588,7 @@ static int dispatch_fwd(const DeltaFwdParams& p, int nseq, cudaStream_t st) {
 //   d = 16: 16 sequences 37 -> 13, 128 37 -> 25, 256 38 -> 37, 512 38 -> 65; with rows of 12 128 65 -> 27, 256 66 -> 52, 512 67 -> 76
 //   d = 32: 128 63 -> 48, 256 64 -> 92; with rows of 20 128 139 -> 51, 512 283 -> 174
 //   d = 64: 64 114 -> 76, 128 116 -> 125; with rows of 55 512 1789 -> 557;  d = 48: 512 1128 -> 354
-//   E, M = 96, 32: 128 1152 -> 113, 1024 2783 -> 1233
+//   E, M = 96, 32: 128 951 -> 120, 1024 2777 -> 930;  128, 128: 128 2826 -> 676
 // and by length (time of the one-launch kernel over that of the three): d = 16, 80 sequences: 0.9 at 24 steps, 1.1 at 40, 1.8 at 250;
 //   d = 32: 80 0.7 (24), 0.9 (40), 1.2 (64), 1.4 (500), 144 0.9 (100), 1.1 (250), 304 (a second wave of the blocked kernel, which
 //   holds two sequences per SM) 1.1 (40), 1.2 (100), 400 0.9;

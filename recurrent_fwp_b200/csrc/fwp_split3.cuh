@@ -3,11 +3,14 @@
 // A float is the exact sum of three bf16 numbers (8 significand bits each, 24 together, same exponent range), so a
 // product of two floats is the sum of nine bf16 products, all exact in the fp32 accumulator.  The three smallest
 // (middle x low, low x middle, low x low) are below 2^-24 of the product and are left out, like the rounding of an fp32
-// multiply; six mma.m16n8k16 per tile remain.  Measured on B200 per SM: one such mma every 2.06 cycles, i.e. 166
+// multiply; six mma.m16n8k16 per tile remain.  (G. Henry, P. Tang, A. Heinecke, "Leveraging the bfloat16 artificial
+// intelligence datatype for higher-precision computations", ARITH 2019.)  Measured on B200 per SM: one such mma every 2.06 cycles, i.e. 166
 // fp32-accurate multiply-adds per cycle against 128 on the fp32 pipe -- and the operands come from registers as
 // fragments instead of one shared-memory broadcast per two packed multiply-adds, which is what bounds the fp32 form.
 // The tensor pipe truncates when it accumulates, so sums that run through a whole sequence are kept outside: every
-// product starts from zero, smallest terms first, and is added to the running fp32 value with a rounded add.
+// product starts from zero, smallest terms first, and is added to the running fp32 value with a rounded add (H. Ootomo,
+// R. Yokota, "Recovering single precision accuracy from tensor cores while surpassing the FP32 theoretical peak
+// performance", 2022).
 //
 // Fragments of mma.m16n8k16 (lane = 4 g + t): A holds rows g, g+8 and columns 2t, 2t+1, 2t+8, 2t+9; B rows (k)
 // 2t, 2t+1, 2t+8, 2t+9 of column g; C rows g, g+8 and columns 2t, 2t+1.  So the C fragments of a 16 x 16 matrix Z, packed
