@@ -108,9 +108,10 @@ __device__ __forceinline__ bool finite(const float (&x)[K][2][4]) {
     return acc == 0.f;
 }
 
-// The recurrence of one sequence backwards as it stands, by one warp: lanes own columns of G for r, then rows for dQ and dK.
-// W holds the rewound state; S is brought forward from it with the u of the forward first.  `G` and `S` hold E x M floats
-// each and `vec` 2 M, all of them this warp's own.  Inlined, for the reason stepwise_forward is.
+// The recurrence of one sequence backwards as it stands, by one warp whose lanes own state columns.  W holds the rewound
+// state; S is brought forward from it with the u of the forward first.  `G` and `S` hold E x M floats each and `vec` 2 M, all
+// of them this warp's own (the arrays hold whole blocks of rows, so BT of them can be in flight at a time: the loop is nothing
+// but latency).  Inlined, for the reason stepwise_forward is.
 template <typename T>
 __device__ __forceinline__ void stepwise_backward(const DeltaBwdParams& p, int n, int h, float* G, float* S, float* vec) {
     const int lane = threadIdx.x & 31, E = p.E, M = p.M;
@@ -120,6 +121,8 @@ __device__ __forceinline__ void stepwise_backward(const DeltaBwdParams& p, int n
     T *gqp = stream_at<T>(p.gq, n, h), *gkp = stream_at<T>(p.gk, n, h), *gvp = stream_at<T>(p.gv, n, h), *gbp = stream_at<T>(p.gb, n, h);
     const float* W = p.W + n * p.wN + h * p.wH;
     float *us = vec, *bs = vec + M;
+    constexpr int BT = 8;
+    auto at = [&](const T* row, int e) { return e < E ? to_f32(row[e]) : 0.f; };
     for (int m = lane; m < M; m += 32) {
 #pragma unroll 1
         for (int e = 0; e < E; e++) {
@@ -129,10 +132,15 @@ __device__ __forceinline__ void stepwise_backward(const DeltaBwdParams& p, int n
         for (long long t = 0; t < p.L; t++) {
             const float u = to_f32(bp[t * p.beta.sL]) * (to_f32(vp[t * p.v.sL + m]) - op[t * p.v_old.sL + m]);
 #pragma unroll 1
-            for (int e = 0; e < E; e++) S[e * M + m] = fmaf(to_f32(kp[t * p.k.sL + e]), u, S[e * M + m]);
+            for (int e = 0; e < E; e += BT) {
+                float s[BT];
+#pragma unroll
+                for (int i = 0; i < BT; i++) s[i] = fmaf(at(kp + t * p.k.sL, e + i), u, S[(e + i) * M + m]);
+#pragma unroll
+                for (int i = 0; i < BT; i++) S[(e + i) * M + m] = s[i];
+            }
         }
     }
-    __syncwarp();
     for (long long t = p.L - 1; t >= 0; t--) {
         const T *q = qp + t * p.q.sL, *k = kp + t * p.k.sL, *y = yp + t * p.gy.sL;
         const float beta = to_f32(bp[t * p.beta.sL]);
@@ -141,10 +149,15 @@ __device__ __forceinline__ void stepwise_backward(const DeltaBwdParams& p, int n
             const float gy = to_f32(y[m]), w = to_f32(vp[t * p.v.sL + m]) - op[t * p.v_old.sL + m];
             float r = 0.f;
 #pragma unroll 1
-            for (int e = 0; e < E; e++) {
-                const float x = fmaf(to_f32(q[e]), gy, G[e * M + m]);
-                G[e * M + m] = x;
-                r = fmaf(x, to_f32(k[e]), r);
+            for (int e = 0; e < E; e += BT) {
+                float x[BT];
+#pragma unroll
+                for (int i = 0; i < BT; i++) x[i] = fmaf(at(q, e + i), gy, G[(e + i) * M + m]);
+#pragma unroll
+                for (int i = 0; i < BT; i++) {
+                    G[(e + i) * M + m] = x[i];
+                    if (e + i < E) r = fmaf(x[i], to_f32(k[e + i]), r);
+                }
             }
             db = fmaf(r, w, db);
             us[m] = beta * w;
@@ -154,23 +167,40 @@ __device__ __forceinline__ void stepwise_backward(const DeltaBwdParams& p, int n
 #pragma unroll
         for (int o = 16; o; o >>= 1) db += __shfl_xor_sync(0xffffffffu, db, o);
         if (lane == 0) gbp[t * p.gb.sL] = from_f32<T>(db);
-        __syncwarp();
-        for (int e = lane; e < E; e += 32) {
-            const float ke = to_f32(k[e]);
-            float dq = 0.f, dk = 0.f, sb = 0.f;
 #pragma unroll 1
-            for (int m = 0; m < M; m++) {
-                const float s = S[e * M + m], x = G[e * M + m], u = us[m], b = bs[m], s0 = fmaf(-ke, u, s);
-                dq = fmaf(s, to_f32(y[m]), dq);
-                dk = fmaf(x, u, dk);
-                sb = fmaf(s0, b, sb);
-                S[e * M + m] = s0;
-                G[e * M + m] = fmaf(-ke, b, x);
+        for (int e = 0; e < E; e += BT) {
+            float dq[BT] = {}, dk[BT] = {};
+#pragma unroll 1
+            for (int m = lane; m < M; m += 32) {
+                const float u = us[m], b = bs[m], gy = to_f32(y[m]);
+                float s[BT], x[BT];
+#pragma unroll
+                for (int i = 0; i < BT; i++) {
+                    s[i] = S[(e + i) * M + m];
+                    x[i] = G[(e + i) * M + m];
+                }
+#pragma unroll
+                for (int i = 0; i < BT; i++) {
+                    const float ke = at(k, e + i), s0 = fmaf(-ke, u, s[i]);
+                    dq[i] = fmaf(s[i], gy, dq[i]);
+                    dk[i] = fmaf(x[i], u, fmaf(-s0, b, dk[i]));
+                    S[(e + i) * M + m] = s0;
+                    G[(e + i) * M + m] = fmaf(-ke, b, x[i]);
+                }
             }
-            gqp[t * p.gq.sL + e] = from_f32<T>(dq);
-            gkp[t * p.gk.sL + e] = from_f32<T>(dk - sb);
+#pragma unroll
+            for (int i = 0; i < BT; i++) {
+#pragma unroll
+                for (int o = 16; o; o >>= 1) {
+                    dq[i] += __shfl_xor_sync(0xffffffffu, dq[i], o);
+                    dk[i] += __shfl_xor_sync(0xffffffffu, dk[i], o);
+                }
+                if (lane == i && e + i < E) {
+                    gqp[t * p.gq.sL + e + i] = from_f32<T>(dq[i]);
+                    gkp[t * p.gk.sL + e + i] = from_f32<T>(dk[i]);
+                }
+            }
         }
-        __syncwarp();
     }
 }
 
