@@ -383,13 +383,17 @@ static int launch_lstm_bwd(const LstmBwdParams& p, int nseq, cudaStream_t st) {
     return launch_dependent(kern, p, nseq / slots, D * SPLIT * slots, bytes * slots, st, "lstm_bwd_kernel");
 }
 
+template <int TC, int VAR, int SLOTS>
+static int launch_lstm_bwd_roles32(const LstmBwdParams& p, int nseq, int slots, cudaStream_t st) {
+    const size_t bytes = (size_t)LstmRolesSmem<TC>::kFloats * sizeof(float) * slots;
+    return launch_dependent(lstm_bwd_roles32_kernel<TC, VAR, SLOTS>, p, nseq / slots, 128 * slots, bytes, st, "lstm_bwd_roles32_kernel");
+}
 template <int VAR>
 static int launch_lstm_bwd_roles32(const LstmBwdParams& p, int nseq, cudaStream_t st) {
-    constexpr int TC = 8;
-    auto kern = lstm_bwd_roles32_kernel<TC, VAR>;
-    const int slots = spread_slots(2, nseq);
-    const size_t bytes = (size_t)LstmRolesSmem<TC>::kFloats * sizeof(float) * slots;
-    return launch_dependent(kern, p, nseq / slots, 128 * slots, bytes, st, "lstm_bwd_roles32_kernel");
+    // four sequences per SM leave shared memory for chunks of four steps; fewer keep chunks of eight and registers to spare
+    const int slots = spread_slots(4, nseq);
+    if (slots == 4) return launch_lstm_bwd_roles32<4, VAR, 4>(p, nseq, 4, st);
+    return launch_lstm_bwd_roles32<8, VAR, 2>(p, nseq, slots, st);
 }
 
 template <int VAR>

@@ -1,18 +1,22 @@
-// Backward of the delta LSTM (v1..v4) at d <= 32: a chain warp and one trailing warp per gate.
+// Backward of the delta LSTM (v1..v4) at d = 32: a chain warp and one trailing warp per gate.
 //
 // Time reversed, the only quantities one step hands to the next are the gradient of the fed-back output g_h and
 // the cell gradient g_c.  The chain is  g_h, g_c -> dz[3] (element-wise) -> sum over the gates of S^q_t dz^q ->
 // (softmax backward) -> g_h;  the value, key and beta gradients of the three delta rules hang off dz but feed
 // nothing back.  So per sequence
-//   warp X      holds S^i, S^u, S^o by rows, runs the chain, rewinds the matrices (that needs inputs only) and
-//               leaves dz[3], u[3] = beta (v - v_old) and the z-gradient of the update gate in a ring;
-//   warp H_q    (q = i, u, o) holds G^q by columns, G^q by rows and its own copy of S^q, runs one chunk of steps
-//               behind X, and produces the gate's value, key, beta and z gradients and their stores.
+//   warp X      holds S^i, S^u, S^o by rows (two rows and half the columns per lane), runs the chain, rewinds the matrices
+//               (that needs inputs only) and leaves dz[3], w[3] = v - v_old and the z-gradient of the update gate in a ring;
+//   warp H_q    (q = i, u, o) runs one chunk of steps behind X and produces the gate's value, key, beta and z gradients
+//               (fwp_trail.cuh).
 // The four warps of a sequence meet once per chunk on a named barrier (that is also where staged input tiles
 // change hands); nothing else crosses warps, because a hand-off costs about 140 cycles on this machine against 33
-// for an exchange inside a warp.  Twelve matrices per sequence do not fit the register file for 512 sequences at
-// once, so a CTA carries two sequences and the grid runs in two waves of a much shorter step.
+// for an exchange inside a warp.  SLOTS sequences share a CTA: four fill an SM with chunks of four steps (152 registers for the
+// X warps, 120 for the others, out of the 128 a thread of the launch), so that 512 sequences are resident at once.  Bound by
+// issue slots and the fp32 pipe (65 and 55 % on an SM with four sequences, 1220 warp instructions per sequence and step).
+// 512 sequences x 512 steps: 543 us against 720 us for the form whose H warps held G twice (by columns and by rows, 208
+// registers a thread), two sequences per SM and so two waves.
 #pragma once
+#include "fwp_trail.cuh"
 
 namespace fwp {
 
@@ -21,20 +25,21 @@ struct LstmRolesSmem {
     static constexpr int D = 32;
     using Stage = LstmBwdStage<D, TC>;
     static constexpr int kStages = 3;                 // X on chunk j, the H warps on chunk j - 1, chunk j + 1 in flight
-    static constexpr int kStep = 7 * D;               // per step: dz[3], u[3], z-gradient of gate u (variant 3)
+    static constexpr int kStep = 7 * D;               // per step: dz[3], w[3], z-gradient of gate u (variant 3)
     static constexpr int kRing = TC * kStep;
+    static constexpr int kOwn = 2 * D + TC * (D + 4); // per H warp: dv of two steps, r w of a chunk
     static constexpr int kTable = (sizeof(StageTable) + 15) / 16 * 4;
-    static constexpr int kFloats = kStages * Stage::kFloats + 2 * kRing + 3 * D + kTable;
+    static constexpr int kFloats = kStages * Stage::kFloats + 2 * kRing + 3 * kOwn + kTable;
 };
 
-template <int TC, int VAR>
-__global__ void __launch_bounds__(256, 1) lstm_bwd_roles32_kernel(const LstmBwdParams p) {
+template <int TC, int VAR, int SLOTS>
+__global__ void __launch_bounds__(128 * SLOTS, 1) lstm_bwd_roles32_kernel(const LstmBwdParams p) {
     griddep_wait();               // launched as a dependent: global memory is touched from here on
     griddep_launch_dependents();
-    constexpr int D = 32, NP = 16, NT = 128;
+    constexpr int D = 32, NT = 128;
     using SM = LstmRolesSmem<TC>;
     using Stage = typename SM::Stage;
-    const int nslots = blockDim.x / NT;
+    const int nslots = SLOTS == 4 ? 4 : blockDim.x / NT;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int slot = warp % nslots, role = warp / nslots;       // role 0: X, 1..3: H of gate role - 1
     const int stid = role * 32 + lane;
@@ -44,9 +49,9 @@ __global__ void __launch_bounds__(256, 1) lstm_bwd_roles32_kernel(const LstmBwdP
     float* smem = smem_all + (size_t)slot * SM::kFloats;
     for (int i = stid; i < SM::kFloats - SM::kTable; i += NT) smem[i] = 0.f;
     float* ring = smem + SM::kStages * Stage::kFloats;
-    float* hbuf = ring + 2 * SM::kRing;
+    float* hown = ring + 2 * SM::kRing;
 
-    StageTable* tb = reinterpret_cast<StageTable*>(hbuf + 3 * D);
+    StageTable* tb = reinterpret_cast<StageTable*>(hown + 3 * SM::kOwn);
     if (stid == 0) {                // tile order of LstmBwdStage: k, v, v_old, gate of each gate, then gy, out, od, cell, umc
         for (int a = 0; a < 3; a++) {
             stage_table_set(tb, 4 * a + 0, p.k[a], n, h);
@@ -62,69 +67,52 @@ __global__ void __launch_bounds__(256, 1) lstm_bwd_roles32_kernel(const LstmBwdP
         stage_table_set(tb, 15, p.cell, n, h);
         stage_table_set(tb, 16, p.umc, n, h);
     }
-
-    const int col = lane;           // the head dimension is exactly 32 (the launcher sends other sizes elsewhere)
-    auto load_w_rows = [&](f2 (&S)[NP], int q) {
-        const float* W = p.W[q] + n * p.wN[q] + h * p.wH[q];
-        float v[2];
-#pragma unroll
-        for (int i = 0; i < D; i++) {
-            v[i & 1] = W[(long long)lane * p.wE[q] + i];
-            if (i & 1) S[i >> 1] = f2_pack(v[0], v[1]);
-        }
-    };
-    // X: M0, M1, M2 = S^i, S^u, S^o by rows.  H_q: M0 = G^q by columns, M1 = G^q by rows, M2 = S^q by rows.
-    f2 M0[NP], M1[NP], M2[NP];
-    if (role == 0) {
-        load_w_rows(M0, 0);
-        load_w_rows(M1, 1);
-        load_w_rows(M2, 2);
-    } else {
-#pragma unroll
-        for (int i = 0; i < NP; i++) { M0[i] = 0ull; M1[i] = 0ull; }
-        if (role == 1) load_w_rows(M2, 0);
-        else if (role == 2) load_w_rows(M2, 1);
-        else load_w_rows(M2, 2);
-    }
     slot_barrier(slot, NT);      // the zero fill is complete before the first copies land
 
     const int nchunks = (p.L + TC - 1) / TC;
+    // top of the loop that every warp runs: chunk j's tiles have landed, X is through chunk j - 1, the H warps through j - 2,
+    // and chunk j + 1 goes into the stage the H warps have just left
     auto issue = [&](int j) {
         const int c = nchunks - 1 - j;
         const int t0 = c * TC, nt = min(TC, p.L - t0);
         stage_table_issue<TC, NT>(smem + (j % SM::kStages) * Stage::kFloats, tb, 17, 3, t0, nt, stid);
     };
-    issue(0);
-    float gh = 0.f, gc = 0.f;       // X: gradients handed back through the output and the cell
-    // H_q: this gate's gradient streams, picked once (by value: a reference chosen at run time would make every
-    // later field access an indexed load from the parameter bank)
-    const int gq = role > 0 ? role - 1 : 0;
-    const Row4 rk = gq == 0 ? p.gk[0] : (gq == 1 ? p.gk[1] : p.gk[2]);
-    const Row4 rz = gq == 0 ? p.gz[0] : (gq == 1 ? p.gz[1] : p.gz[2]);
-    const Row4 rv = gq == 0 ? p.gv[0] : (gq == 1 ? p.gv[1] : p.gv[2]);
-    const Row4 rb = gq == 0 ? p.gb[0] : (gq == 1 ? p.gb[1] : p.gb[2]);
-    float* const bgk = reinterpret_cast<float*>(rk.p) + n * rk.sN + h * rk.sH + col;
-    float* const bgz = reinterpret_cast<float*>(rz.p) + n * rz.sN + h * rz.sH + col;
-    float* const bgv = reinterpret_cast<float*>(rv.p) + n * rv.sN + h * rv.sH + col;
-    float* const bgb = reinterpret_cast<float*>(rb.p) + n * rb.sN + h * rb.sH;
-    const long long sgk = rk.sL, sgz = rz.sL, sgv = rv.sL, sgb = rb.sL;
-    for (int j = 0; j <= nchunks; j++) {
+    auto advance = [&](int j) {
         cp_async_wait<0>();
-        slot_barrier(slot, NT);  // chunk j's tiles have landed; X is through chunk j - 1, the H warps through j - 2
-        if (j + 1 < nchunks) issue(j + 1);      // into the stage the H warps have just left
-        if (role == 0 && j < nchunks) {
-            // ------------------------------------------------------------ X: the chain
+        slot_barrier(slot, NT);
+        if (j + 1 < nchunks) issue(j + 1);
+    };
+    issue(0);
+
+    if (role == 0) {
+        // ---------------------------------------------------------------- X: the chain
+        if constexpr (SLOTS == 4) asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
+        // lane (half, lp): rows 2 lp + half (finished here) and 2 lp + 1 - half (given away), columns 16 half .. 16 half + 15
+        const int half = lane >> 4, lp = lane & 15, own = 2 * lp + half, other = 2 * lp + 1 - half;
+        f2 M[3][16];
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            const float* W = p.W[q] + n * p.wN[q] + h * p.wH[q] + 16 * half;
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                const float* w = W + (long long)(i < 8 ? own : other) * p.wE[q] + 2 * (i & 7);
+                M[q][i] = f2_pack(w[0], w[1]);
+            }
+        }
+        float gh = 0.f, gc = 0.f;       // gradients handed back through the output and the cell
+        for (int j = 0; j <= nchunks; j++) {
+            advance(j);
+            if (j == nchunks) break;
             Stage s; s.bind(smem + (j % SM::kStages) * Stage::kFloats);
-            const int c = nchunks - 1 - j;
-            const int nt = min(TC, p.L - c * TC);
+            const int nt = min(TC, p.L - (nchunks - 1 - j) * TC);
             float* rg = ring + (j & 1) * SM::kRing;
 #pragma unroll 1
             for (int t = nt - 1; t >= 0; t--) {
-                const int o = t * D + lane;
+                const int o = t * D + own;
                 float* e = rg + t * SM::kStep;
                 // what the rewind and the trailing warps need and the chain does not
 #pragma unroll
-                for (int q = 0; q < 3; q++) e[(3 + q) * D + lane] = s.b[q].f[t] * (s.v[q].f[o] - s.vo[q].f[o]);
+                for (int q = 0; q < 3; q++) e[(3 + q) * D + own] = s.v[q].f[o] - s.vo[q].f[o];
                 const float gsum = s.gy.f[o] + gh;
                 float a = gsum;
                 if constexpr (VAR == 1) {
@@ -141,19 +129,23 @@ __global__ void __launch_bounds__(256, 1) lstm_bwd_roles32_kernel(const LstmBwdP
                 if constexpr (VAR != 4) dz[1] = dz[1] * (1.f - uu) * uu;
                 gc *= (1.f - gi);
 #pragma unroll
-                for (int q = 0; q < 3; q++) e[q * D + lane] = dz[q];
-                if constexpr (VAR == 3) e[6 * D + lane] = dz[1] + gsum;
+                for (int q = 0; q < 3; q++) e[q * D + own] = dz[q];
+                if constexpr (VAR == 3) e[6 * D + own] = dz[1] + gsum;
                 __syncwarp();
-                // three vectors in three register sets: the loads go out together and the products overlap
-                f2 va[NP], vb[NP], vc[NP];
-                lds_slice<D>(va, e);
-                lds_slice<D>(vb, e + D);
-                lds_slice<D>(vc, e + 2 * D);
-                const float k0 = s.k[0].f[o], k1 = s.k[1].f[o], k2 = s.k[2].f[o];
-                float ghn = dot2<NP>(M0, va) + dot2<NP>(M1, vb) + dot2<NP>(M2, vc);
-                lds_slice<D>(va, e + 3 * D);        // u[3] for the rewind: in flight during the reduction below
-                lds_slice<D>(vb, e + 4 * D);
-                lds_slice<D>(vc, e + 5 * D);
+                f2 a0 = 0ull, a1 = 0ull, b0 = 0ull, b1 = 0ull;
+#pragma unroll
+                for (int q = 0; q < 3; q++) {
+                    f2 x[8];
+                    lds_slice<16>(x, e + q * D + 16 * half);
+#pragma unroll
+                    for (int i = 0; i < 8; i += 2) {
+                        a0 = ffma2(M[q][i], x[i], a0);
+                        b0 = ffma2(M[q][8 + i], x[i], b0);
+                        a1 = ffma2(M[q][i + 1], x[i + 1], a1);
+                        b1 = ffma2(M[q][9 + i], x[i + 1], b1);
+                    }
+                }
+                const float ghn = f2_hsum(fadd2(a0, a1)) + __shfl_xor_sync(0xffffffffu, f2_hsum(fadd2(b0, b1)), 16);
                 if constexpr (VAR != 1) {
                     const float xe = s.od.f[o];
                     const float dotp = warp_sum_idx<1>(xe * ghn);
@@ -161,78 +153,84 @@ __global__ void __launch_bounds__(256, 1) lstm_bwd_roles32_kernel(const LstmBwdP
                 } else {
                     gh = ghn;
                 }
-                axpy2<NP>(M0, va, -k0);             // S^q_{t-1}
-                axpy2<NP>(M1, vb, -k1);
-                axpy2<NP>(M2, vc, -k2);
-            }
-        } else if (role > 0 && j > 0) {
-            // ------------------------------------------------------------ H_q: one chunk behind
-            const int q = role - 1;
-            const int jj = j - 1;
-            Stage s; s.bind(smem + (jj % SM::kStages) * Stage::kFloats);
-            const int c = nchunks - 1 - jj;
-            const int t0 = c * TC, nt = min(TC, p.L - t0);
-            const float* rg = ring + (jj & 1) * SM::kRing;
-            float* hb = hbuf + q * D;
-            const float* ktile = q == 0 ? s.k[0].f : (q == 1 ? s.k[1].f : s.k[2].f);
-            const float* vtile = q == 0 ? s.v[0].f : (q == 1 ? s.v[1].f : s.v[2].f);
-            const float* votile = q == 0 ? s.vo[0].f : (q == 1 ? s.vo[1].f : s.vo[2].f);
-            const float* btile = q == 0 ? s.b[0].f : (q == 1 ? s.b[1].f : s.b[2].f);
-            const long long tl = t0 + nt - 1;
-            float* pgk = bgk + tl * sgk;
-            float* pgz = bgz + tl * sgz;
-            float* pgv = bgv + tl * sgv;
-            float* pgb = bgb + tl * sgb;
-#pragma unroll 1
-            for (int t = nt - 1; t >= 0; t--) {
-                const int o = t * D + lane;
-                const float* e = rg + t * SM::kStep;
-                const float dzl = e[q * D + lane];
-                const float gzl = (VAR == 3 && q == 1) ? e[6 * D + lane] : dzl;
-                const float beta = btile[t];
-                const float w = vtile[o] - votile[o];
-                const float xe = s.od.f[o], ke = ktile[o];
-                // the four vectors that do not wait for this step's br, in four register sets
-                f2 xs[NP], kk[NP], dr[NP], ur[NP];
-                lds_slice<D>(xs, s.od.f + t * D);
-                lds_slice<D>(kk, ktile + t * D);
-                lds_slice<D>(dr, e + q * D);
-                lds_slice<D>(ur, e + (3 + q) * D);
-                // column role
-                axpy2<NP>(M0, xs, dzl);
-                const float r = dot2<NP>(M0, kk);
-                const float br = beta * r;
-                hb[lane] = br;
-                // row role, the part before br
-                axpy2<NP>(M1, dr, xe);
-                float dk = dot2<NP>(M1, ur);
-                axpy2<NP>(M2, ur, -ke);             // S^q_{t-1}
-                axpy2<NP>(M0, kk, -br);
-                const float db = warp_sum_idx<1>(r * w);
-                __syncwarp();
-                lds_slice<D>(xs, hb);
-                dk -= dot2<NP>(M2, xs);
-                axpy2<NP>(M1, xs, -ke);
-                __syncwarp();                       // everyone has read hb before the next step rewrites it
-                *pgk = dk; *pgz = gzl; *pgv = br;
-                if (lane == 0) *pgb = db;
-                pgk -= sgk; pgz -= sgz; pgv -= sgv; pgb -= sgb;
+                // S^q_{t-1} = S^q_t - beta k (x) w, beside the reduction
+#pragma unroll
+                for (int q = 0; q < 3; q++) {
+                    f2 x[8];
+                    lds_slice<16>(x, e + (3 + q) * D + 16 * half);
+                    const float nb = -s.b[q].f[t];
+                    const f2 k0 = f2_dup(nb * s.k[q].f[o]), k1 = f2_dup(nb * s.k[q].f[t * D + other]);
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        M[q][i] = ffma2(x[i], k0, M[q][i]);
+                        M[q][8 + i] = ffma2(x[i], k1, M[q][8 + i]);
+                    }
+                }
             }
         }
-    }
-    if (role == 0) {
-        auto store_w_rows = [&](const f2 (&S)[NP], int q) {
-            float* W = p.W[q] + n * p.wN[q] + h * p.wH[q];
 #pragma unroll
-            for (int i = 0; i < D; i++) {
-                float lo, hi;
-                f2_unpack(S[i >> 1], lo, hi);
-                W[(long long)lane * p.wE[q] + i] = (i & 1) ? hi : lo;
+        for (int q = 0; q < 3; q++) {
+            float* W = p.W[q] + n * p.wN[q] + h * p.wH[q] + 16 * half;
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                float* w = W + (long long)(i < 8 ? own : other) * p.wE[q] + 2 * (i & 7);
+                f2_unpack(M[q][i], w[0], w[1]);
             }
-        };
-        store_w_rows(M0, 0);
-        store_w_rows(M1, 1);
-        store_w_rows(M2, 2);
+        }
+        return;
+    }
+
+    // -------------------------------------------------------------------- H_q: one chunk behind
+    if constexpr (SLOTS == 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 120;");
+    const int q = role - 1;
+    // this gate's gradient streams, picked once (by value: a reference chosen at run time would make every
+    // later field access an indexed load from the parameter bank)
+    const Row4 rk = q == 0 ? p.gk[0] : (q == 1 ? p.gk[1] : p.gk[2]);
+    const Row4 rz = q == 0 ? p.gz[0] : (q == 1 ? p.gz[1] : p.gz[2]);
+    const Row4 rv = q == 0 ? p.gv[0] : (q == 1 ? p.gv[1] : p.gv[2]);
+    const Row4 rb = q == 0 ? p.gb[0] : (q == 1 ? p.gb[1] : p.gb[2]);
+    float* const W = (q == 0 ? p.W[0] : (q == 1 ? p.W[1] : p.W[2])) + n * (q == 0 ? p.wN[0] : (q == 1 ? p.wN[1] : p.wN[2])) +
+                     h * (q == 0 ? p.wH[0] : (q == 1 ? p.wH[1] : p.wH[2]));
+    Trail32 tr;
+    tr.init(lane, W, q == 0 ? p.wE[0] : (q == 1 ? p.wE[1] : p.wE[2]));
+    const long long last = p.L - 1;
+    float* pgk = reinterpret_cast<float*>(rk.p) + n * rk.sN + h * rk.sH + lane + last * rk.sL;
+    float* pgz = reinterpret_cast<float*>(rz.p) + n * rz.sN + h * rz.sH + lane + last * rz.sL;
+    float* pgv = reinterpret_cast<float*>(rv.p) + n * rv.sN + h * rv.sH + tr.own + last * rv.sL;
+    float* const pgb = reinterpret_cast<float*>(rb.p) + n * rb.sN + h * rb.sH;
+    float* const xch = hown + q * SM::kOwn;
+    float* const pw = xch + 2 * D;
+    for (int j = 0; j <= nchunks; j++) {
+        advance(j);
+        if (j == 0) continue;
+        const int jj = j - 1, t0 = (nchunks - 1 - jj) * TC, nt = min(TC, p.L - t0);
+        const float* stage = smem + (jj % SM::kStages) * Stage::kFloats;
+        const float* rg = ring + (jj & 1) * SM::kRing;
+        const float* kt = stage + 4 * q * r4(TC * D);
+        const float* st = stage + 14 * r4(TC * D);
+        const float* bt = stage + 17 * r4(TC * D) + q * r4(TC);
+#pragma unroll 1
+        for (int t = nt - 1; t >= 0; t--) {
+            const float* e = rg + t * SM::kStep;
+            float r, dv, dk;
+            tr.step(st + t * D, kt + t * D, e + q * D, e + (3 + q) * D, bt[t], xch + (t & 1) * D, r, dv, dk);
+            pw[t * (D + 4) + lane] = r * e[(3 + q) * D + tr.own];
+            *pgz = e[((VAR == 3 && q == 1) ? 6 : q) * D + lane];
+            *pgv = dv;
+            *pgk = dk;
+            pgk -= rk.sL; pgz -= rz.sL; pgv -= rv.sL;
+        }
+        // dbeta of the whole chunk at once: 32 / TC lanes share a step
+        __syncwarp();
+        constexpr int SH = 32 / TC;
+        const float* pr = pw + (lane / SH) * (D + 4) + (lane % SH) * (D / SH);
+        float db = 0.f;
+#pragma unroll
+        for (int i = 0; i < D / SH; i++) db += pr[i];
+#pragma unroll
+        for (int o = SH / 2; o > 0; o >>= 1) db += __shfl_xor_sync(0xffffffffu, db, o);
+        if (lane % SH == 0 && lane / SH < nt) pgb[(long long)(t0 + lane / SH) * rb.sL] = db;
+        __syncwarp();
     }
 }
 

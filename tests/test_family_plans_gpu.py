@@ -126,6 +126,27 @@ def test_lstm_plans_agree(fwp, variant, B, H, L):
             assert close(a, r)
 
 
+@pytest.mark.parametrize('variant,L,mis', [(1, 1, False), (2, 4, False), (3, 5, False), (4, 11, False), (1, 66, True), (3, 64, False)])
+def test_lstm_backward_with_four_sequences_per_sm(fwp, variant, L, mis):
+    """111 x 4 sequences fill an SM with four, the form with chunks of four steps; 74 x 4 take two per SM and chunks of eight."""
+    from recurrent_fwp_b200 import _lib
+    for B in (111, 74):
+        H = 4
+        gates, gy = util.lstm_inputs(61, B, H, L, D)
+        Ws = [torch.randn(B, H, D, D, generator=util.gen(62 + i)) * 0.1 for i in range(3)]
+        h0 = torch.randn(B, H, 1, D, generator=util.gen(65))
+        c0 = torch.randn(B, H, 1, D, generator=util.gen(66))
+        fast = run_lstm(variant, gates, Ws, h0, c0, gy, mis=mis)
+        try:
+            _lib.tune('lstm_bwd.32.roles', 0)
+            ref = run_lstm(variant, gates, Ws, h0, c0, gy)
+        finally:
+            _lib.tune('lstm_bwd.32.roles', 1)
+        assert fast['kb'] == 'lstm_bwd_roles32_kernel' and ref['kb'] == 'lstm_bwd_kernel'
+        for a, r in zip(fast['W_back'] + fast['g'], ref['W_back'] + ref['g']):
+            assert close(a, r)
+
+
 @pytest.mark.parametrize('B,H,L', SHAPES)
 def test_recurrent_delta_backward_plans_agree(fwp, B, H, L):
     """The chain-warp + trailing-warp backward against the two-warp split kernel on the same saved tensors:
