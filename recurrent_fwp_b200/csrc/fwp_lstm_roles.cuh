@@ -5,15 +5,15 @@
 // (softmax backward) -> g_h;  the value, key and beta gradients of the three delta rules hang off dz but feed
 // nothing back.  So per sequence
 //   warp X      holds S^i, S^u, S^o by rows (two rows and half the columns per lane), runs the chain, rewinds the matrices
-//               (that needs inputs only) and leaves dz[3], w[3] = v - v_old and the z-gradient of the update gate in a ring;
+//               (that needs inputs only) and leaves dz[3], w[3] = v - v_old, -u[3] = -beta w and the z-gradient of the update gate in a ring;
 //   warp H_q    (q = i, u, o) runs one chunk of steps behind X and produces the gate's value, key, beta and z gradients
 //               (fwp_trail.cuh).
 // The four warps of a sequence meet once per chunk on a named barrier (that is also where staged input tiles
 // change hands); nothing else crosses warps, because a hand-off costs about 140 cycles on this machine against 33
 // for an exchange inside a warp.  SLOTS sequences share a CTA: four fill an SM with chunks of four steps (152 registers for the
 // X warps, 120 for the others, out of the 128 a thread of the launch), so that 512 sequences are resident at once.  Bound by
-// issue slots and the fp32 pipe (65 and 55 % on an SM with four sequences, 1220 warp instructions per sequence and step).
-// 512 sequences x 512 steps: 543 us against 720 us for the form whose H warps held G twice (by columns and by rows, 208
+// issue slots and the fp32 pipe (65 and 55 % on an SM with four sequences, 1200 warp instructions per sequence and step).
+// 512 sequences x 512 steps: 520 us against 720 us for the form whose H warps held G twice (by columns and by rows, 208
 // registers a thread), two sequences per SM and so two waves.
 #pragma once
 #include "fwp_trail.cuh"
@@ -25,7 +25,7 @@ struct LstmRolesSmem {
     static constexpr int D = 32;
     using Stage = LstmBwdStage<D, TC>;
     static constexpr int kStages = 3;                 // X on chunk j, the H warps on chunk j - 1, chunk j + 1 in flight
-    static constexpr int kStep = 7 * D;               // per step: dz[3], w[3], z-gradient of gate u (variant 3)
+    static constexpr int kStep = 10 * D;              // per step: dz[3], -u[3], w[3], z-gradient of gate u (variant 3)
     static constexpr int kRing = TC * kStep;
     static constexpr int kOwn = 2 * D + TC * (D + 4); // per H warp: dv of two steps, r w of a chunk
     static constexpr int kTable = (sizeof(StageTable) + 15) / 16 * 4;
@@ -112,7 +112,11 @@ __global__ void __launch_bounds__(128 * SLOTS, 1) lstm_bwd_roles32_kernel(const 
                 float* e = rg + t * SM::kStep;
                 // what the rewind and the trailing warps need and the chain does not
 #pragma unroll
-                for (int q = 0; q < 3; q++) e[(3 + q) * D + own] = s.v[q].f[o] - s.vo[q].f[o];
+                for (int q = 0; q < 3; q++) {
+                    const float w = s.v[q].f[o] - s.vo[q].f[o];
+                    e[(3 + q) * D + own] = -s.b[q].f[t] * w;
+                    e[(6 + q) * D + own] = w;
+                }
                 const float gsum = s.gy.f[o] + gh;
                 float a = gsum;
                 if constexpr (VAR == 1) {
@@ -130,7 +134,7 @@ __global__ void __launch_bounds__(128 * SLOTS, 1) lstm_bwd_roles32_kernel(const 
                 gc *= (1.f - gi);
 #pragma unroll
                 for (int q = 0; q < 3; q++) e[q * D + own] = dz[q];
-                if constexpr (VAR == 3) e[6 * D + own] = dz[1] + gsum;
+                if constexpr (VAR == 3) e[9 * D + own] = dz[1] + gsum;
                 __syncwarp();
                 f2 a0 = 0ull, a1 = 0ull, b0 = 0ull, b1 = 0ull;
 #pragma unroll
@@ -153,13 +157,12 @@ __global__ void __launch_bounds__(128 * SLOTS, 1) lstm_bwd_roles32_kernel(const 
                 } else {
                     gh = ghn;
                 }
-                // S^q_{t-1} = S^q_t - beta k (x) w, beside the reduction
+                // S^q_{t-1} = S^q_t - k (x) u, beside the reduction
 #pragma unroll
                 for (int q = 0; q < 3; q++) {
                     f2 x[8];
                     lds_slice<16>(x, e + (3 + q) * D + 16 * half);
-                    const float nb = -s.b[q].f[t];
-                    const f2 k0 = f2_dup(nb * s.k[q].f[o]), k1 = f2_dup(nb * s.k[q].f[t * D + other]);
+                    const f2 k0 = f2_dup(s.k[q].f[o]), k1 = f2_dup(s.k[q].f[t * D + other]);
 #pragma unroll
                     for (int i = 0; i < 8; i++) {
                         M[q][i] = ffma2(x[i], k0, M[q][i]);
@@ -191,8 +194,7 @@ __global__ void __launch_bounds__(128 * SLOTS, 1) lstm_bwd_roles32_kernel(const 
     const Row4 rb = q == 0 ? p.gb[0] : (q == 1 ? p.gb[1] : p.gb[2]);
     float* const W = (q == 0 ? p.W[0] : (q == 1 ? p.W[1] : p.W[2])) + n * (q == 0 ? p.wN[0] : (q == 1 ? p.wN[1] : p.wN[2])) +
                      h * (q == 0 ? p.wH[0] : (q == 1 ? p.wH[1] : p.wH[2]));
-    Trail32 tr;
-    tr.init(lane, W, q == 0 ? p.wE[0] : (q == 1 ? p.wE[1] : p.wE[2]));
+    Trail32 tr(lane, W, q == 0 ? p.wE[0] : (q == 1 ? p.wE[1] : p.wE[2]));
     const long long last = p.L - 1;
     float* pgk = reinterpret_cast<float*>(rk.p) + n * rk.sN + h * rk.sH + lane + last * rk.sL;
     float* pgz = reinterpret_cast<float*>(rz.p) + n * rz.sN + h * rz.sH + lane + last * rz.sL;
@@ -214,23 +216,13 @@ __global__ void __launch_bounds__(128 * SLOTS, 1) lstm_bwd_roles32_kernel(const 
             const float* e = rg + t * SM::kStep;
             float r, dv, dk;
             tr.step(st + t * D, kt + t * D, e + q * D, e + (3 + q) * D, bt[t], xch + (t & 1) * D, r, dv, dk);
-            pw[t * (D + 4) + lane] = r * e[(3 + q) * D + tr.own];
-            *pgz = e[((VAR == 3 && q == 1) ? 6 : q) * D + lane];
+            pw[t * (D + 4) + lane] = r * e[(6 + q) * D + tr.own];
+            *pgz = e[((VAR == 3 && q == 1) ? 9 : q) * D + lane];
             *pgv = dv;
             *pgk = dk;
             pgk -= rk.sL; pgz -= rz.sL; pgv -= rv.sL;
         }
-        // dbeta of the whole chunk at once: 32 / TC lanes share a step
-        __syncwarp();
-        constexpr int SH = 32 / TC;
-        const float* pr = pw + (lane / SH) * (D + 4) + (lane % SH) * (D / SH);
-        float db = 0.f;
-#pragma unroll
-        for (int i = 0; i < D / SH; i++) db += pr[i];
-#pragma unroll
-        for (int o = SH / 2; o > 0; o >>= 1) db += __shfl_xor_sync(0xffffffffu, db, o);
-        if (lane % SH == 0 && lane / SH < nt) pgb[(long long)(t0 + lane / SH) * rb.sL] = db;
-        __syncwarp();
+        trail_dbeta<TC>(pw, pgb + t0 * rb.sL, rb.sL, nt, lane);
     }
 }
 

@@ -311,7 +311,7 @@ static int launch_rnn_bwd_roles32(const RnnBwdParams& p, int nseq, cudaStream_t 
     auto kern = rnn_bwd_roles32_kernel<TC, V1>;
     const int slots = spread_slots(4, nseq);
     const size_t bytes = (size_t)RnnRolesSmem<TC, V1>::kFloats * sizeof(float) * slots;
-    return launch_dependent(kern, p, nseq / slots, 96 * slots, bytes, st, "rnn_bwd_roles32_kernel");
+    return launch_dependent(kern, p, nseq / slots, 64 * slots, bytes, st, "rnn_bwd_roles32_kernel");
 }
 
 template <bool V1>

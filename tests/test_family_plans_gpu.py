@@ -80,6 +80,25 @@ def test_rnn_backward_plans_agree(fwp, ver, B, H, L):
             assert close(a, r)
 
 
+@pytest.mark.parametrize('ver,L,mis', [(2, 1, False), (1, 8, False), (2, 9, False), (1, 19, False), (2, 70, True)])
+def test_rnn_backward_with_four_sequences_per_sm(fwp, ver, L, mis):
+    from recurrent_fwp_b200 import _lib
+    B, H = 111, 4
+    z, k, v, b, gy = util.rnn_inputs(51, B, H, L, D)
+    W0 = torch.randn(B, H, D, D, generator=util.gen(52)) * 0.1
+    h0 = torch.randn(B, H, 1, D, generator=util.gen(53))
+    fast = run_rnn(ver, z, k, v, b, W0, h0, gy, mis=mis)
+    try:
+        _lib.tune('rnn_bwd.32.roles', 0)
+        ref = run_rnn(ver, z, k, v, b, W0, h0, gy)
+    finally:
+        _lib.tune('rnn_bwd.32.roles', 1)
+    assert fast['kb'] == 'rnn_bwd_roles32_kernel' and ref['kb'] == 'rnn_bwd_kernel'
+    assert close(fast['W_back'], ref['W_back'])
+    for a, r in zip(fast['g'], ref['g']):
+        assert close(a, r)
+
+
 def run_lstm(variant, gates, Ws, h0, c0, gy, mis=False):
     from recurrent_fwp_b200 import _lib
     name = 'fast_lstm' if variant == 1 else 'fast_lstm_v%d' % variant
