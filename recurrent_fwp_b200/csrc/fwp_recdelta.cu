@@ -546,12 +546,15 @@ static int launch_rec_bwd(const RecBwdParams& p, int nseq, cudaStream_t st) {
     return launch_dependent(kern, p, nseq / slots, D * SPLIT * slots, bytes * slots, st, "rec_bwd_kernel");
 }
 
-static int launch_rec_bwd_roles32(const RecBwdParams& p, int nseq, cudaStream_t st) {
+template <int SLOTS>
+static int launch_rec_bwd_roles32(const RecBwdParams& p, int nseq, int slots, cudaStream_t st) {
     constexpr int TC = 8;
-    auto kern = rec_bwd_roles32_kernel<TC>;
-    const int slots = spread_slots(4, nseq);
     const size_t bytes = (size_t)RecRolesSmem<TC>::kFloats * sizeof(float) * slots;
-    return launch_dependent(kern, p, nseq / slots, 64 * slots, bytes, st, "rec_bwd_roles32_kernel");
+    return launch_dependent(rec_bwd_roles32_kernel<TC, SLOTS>, p, nseq / slots, 96 * slots, bytes, st, "rec_bwd_roles32_kernel");
+}
+static int launch_rec_bwd_roles32(const RecBwdParams& p, int nseq, cudaStream_t st) {
+    const int slots = spread_slots(4, nseq);
+    return slots == 4 ? launch_rec_bwd_roles32<4>(p, nseq, 4, st) : launch_rec_bwd_roles32<2>(p, nseq, slots, st);
 }
 
 static int check_params(const fwp_tensor* Rq, const fwp_tensor* Rk, const fwp_tensor* Rv, const fwp_tensor* rb) {

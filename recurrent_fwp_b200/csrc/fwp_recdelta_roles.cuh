@@ -1,17 +1,20 @@
-// Backward of the recurrent delta net at d = 32: a chain warp and a trailing warp per sequence.
+// Backward of the recurrent delta net at d = 32: three warps per sequence.
 //
 // Everything but the parameter gradients sits on the chain here: the gradient handed back through tanh(y_{t-1})
-// needs dq, dk (both matrices G and S), their softmax backward and the three products with the rows of R.  A
-// hand-off between warps costs about 140 cycles against 33 for an exchange inside a warp, so one warp X runs the
-// whole chain with G by columns, G by rows and S by rows in registers (R by rows in shared memory), and prepares
-// whatever does not wait for the chain one step early:
-//   S is rewound first (that needs inputs only), so  dq = S_{t-1} g + k (u.g)  and  dk = G u + q (u.g) - S_{t-1} dv
-//   with G u, G^T k and q.k taken before g is known; r = G^T k + (q.k) g.
-// Vectors are fetched from shared memory where they are used instead of being kept across the step, so that the
-// three matrices and at most three vectors are live at a time (no spills).  The second warp Y trails one chunk of
-// steps behind, reads dq~, dk~, dv, db~ from a ring and does the three outer-product accumulations of the parameter
-// gradients and the four stores.
+// needs dq, dk (both matrices G and S), their softmax backward and the three products with the rows of R.  What G takes part
+// in, though, is known a step early but for a rank-one term, so G lives in a warp of its own:
+//   warp P   holds G (8 x 4 pieces, fwp_trail.cuh).  For step t it posts  r0 = G^T k,  G u  and  q . k  before g_t is known,
+//            then takes g_t and dv_t:  G += q (x) g - k (x) dv;
+//   warp X   the chain, two rows and half the columns of S and of the three R per lane:  r = r0 + (q.k) g,  dv = beta r,
+//            dq = S_{t-1} g + k (u.g),  dk = G u + q (u.g) - S_{t-1} dv,  softmax backward, the products with R, tanh.
+//            The sums over features come from products of vectors that the lane reads anyway: u.g = beta (w.g),
+//            db = (w.dv) (1 - beta), and  k . dk = r.u - v_old.dv = w.dv - v_old.dv  (v_old = S_{t-1}^T k, dv.w = r.u);
+//   warp Y   turns v into w = v - v_old for the chunk that X takes next, and two chunks later accumulates the three parameter
+//            gradients (8 x 4 pieces) and stores.
+// X and P hand over twice per step at named barriers: P has X's step to answer in.  The warps meet once per chunk of steps.
+// With four sequences per SM (504 of 512 registers of a scheduler's four threads: 208 X, 120 P, 176 Y) 512 sequences are resident.
 #pragma once
+#include "fwp_trail.cuh"
 
 namespace fwp {
 
@@ -19,37 +22,32 @@ template <int TC>
 struct RecRolesSmem {
     static constexpr int D = 32;
     using Stage = RecBwdStage<D, TC>;
-    static constexpr int kStages = 3;                 // X on chunk j, Y on chunk j - 1, chunk j + 1 in flight
-    static constexpr int kStep = 4 * D;               // per step: dq~, dk~, dv, db~ (lane 0)
+    static constexpr int kStages = 4;                 // chunk j + 1 in flight, w of chunk j, X and P on j - 1, Y on j - 2
+    static constexpr int kStep = 4 * D + 4;           // per step: g, dv, dq~, dk~, db~
     static constexpr int kRing = TC * kStep;
-    static constexpr int kRS = D + 4;                 // padded row stride of the R copies
-    static constexpr int kR = 3 * D * kRS + D;        // Rq, Rk, Rv rows + rb
-    static constexpr int kX = 2 * D;                  // X's exchange vectors: g, u
+    static constexpr int kMail = 2 * D + 4;           // r0, G u, q.k
     static constexpr int kTable = (sizeof(StageTable) + 15) / 16 * 4;
-    static constexpr int kFloats = kStages * Stage::kFloats + 2 * kRing + kR + kX + kTable;
+    static constexpr int kFloats = kStages * Stage::kFloats + 2 * kRing + 2 * kMail + kTable;
 };
 
-template <int TC>
-__global__ void __launch_bounds__(256, 1) rec_bwd_roles32_kernel(const RecBwdParams p) {
+template <int TC, int SLOTS>
+__global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const RecBwdParams p) {
     griddep_wait();               // launched as a dependent: global memory is touched from here on
     griddep_launch_dependents();
-    constexpr int D = 32, NP = 16, NT = 64;
+    constexpr int D = 32, NT = 96;
     using SM = RecRolesSmem<TC>;
     using Stage = typename SM::Stage;
-    const int nslots = blockDim.x / NT;
+    const int nslots = SLOTS == 4 ? 4 : blockDim.x / NT;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int slot = warp % nslots, role = warp / nslots;
+    const int slot = warp % nslots, role = warp / nslots;       // 0: X, 1: P, 2: Y
     const int stid = role * 32 + lane;
     const int seq = blockIdx.x * nslots + slot;
     const int n = seq / p.H, h = seq - n * p.H;
     extern __shared__ __align__(16) float smem_all[];
     float* smem = smem_all + (size_t)slot * SM::kFloats;
-    for (int i = stid; i < SM::kFloats - SM::kTable; i += NT) smem[i] = 0.f;
     float* ring = smem + SM::kStages * Stage::kFloats;
-    float* rmem = ring + 2 * SM::kRing;             // R rows: [3][D][kRS], then rb[D]
-    float* xg = rmem + SM::kR;
-    float* xu = xg + D;
-    StageTable* tb = reinterpret_cast<StageTable*>(xu + D);
+    float* mail = ring + 2 * SM::kRing;
+    StageTable* tb = reinterpret_cast<StageTable*>(mail + 2 * SM::kMail);
     if (stid == 0) {                // tile order of RecBwdStage: q, k, v, v_old, od, gy
         stage_table_set(tb, 0, p.q, n, h);
         stage_table_set(tb, 1, p.k, n, h);
@@ -59,30 +57,7 @@ __global__ void __launch_bounds__(256, 1) rec_bwd_roles32_kernel(const RecBwdPar
         stage_table_set(tb, 5, p.gy, n, h);
         stage_table_set_col(tb, 0, p.beta, n, h);
     }
-    slot_barrier(slot, NT);         // the zero fill is complete
-    for (int i = stid; i < D * D; i += NT) {
-        const int e = i / D, m = i - e * D;
-        const long long src = h * p.rH + (long long)e * p.rE + m;
-        rmem[0 * D * SM::kRS + e * SM::kRS + m] = p.Rq[src];
-        rmem[1 * D * SM::kRS + e * SM::kRS + m] = p.Rk[src];
-        rmem[2 * D * SM::kRS + e * SM::kRS + m] = p.Rv[src];
-    }
-    if (stid < D) rmem[3 * D * SM::kRS + stid] = p.rb[h * p.rbH + stid];
-
-    float* W = p.W + n * p.wN + h * p.wH;
-    // X: A = G by columns, B = S by rows, C = G by rows.  Y: A, B, C = the partial gradients of Rq, Rk, Rv by columns.
-    f2 A[NP], B[NP], C[NP];
-#pragma unroll
-    for (int i = 0; i < NP; i++) { A[i] = 0ull; B[i] = 0ull; C[i] = 0ull; }
-    if (role == 0) {
-        float v[2];
-#pragma unroll
-        for (int i = 0; i < D; i++) {
-            v[i & 1] = W[(long long)lane * p.wE + i];
-            if (i & 1) B[i >> 1] = f2_pack(v[0], v[1]);
-        }
-    }
-    float arb = 0.f;
+    slot_barrier(slot, NT);         // the table is in place
 
     const int nchunks = (p.L + TC - 1) / TC;
     auto issue = [&](int j) {
@@ -90,160 +65,252 @@ __global__ void __launch_bounds__(256, 1) rec_bwd_roles32_kernel(const RecBwdPar
         const int t0 = c * TC, nt = min(TC, p.L - t0);
         stage_table_issue<TC, NT>(smem + (j % SM::kStages) * Stage::kFloats, tb, 6, 1, t0, nt, stid);
     };
-    issue(0);
-    float gh = 0.f;
-    for (int j = 0; j <= nchunks; j++) {
+    // top of the loop that every warp runs
+    auto advance = [&](int j) {
         cp_async_wait<0>();
-        slot_barrier(slot, NT);     // chunk j's tiles (and, first time, the R rows) are in place
+        slot_barrier(slot, NT);
         if (j + 1 < nchunks) issue(j + 1);
-        if (role == 0 && j < nchunks) {
-            // ------------------------------------------------------------ X: the chain
-            Stage s; s.bind(smem + (j % SM::kStages) * Stage::kFloats);
-            const int c = nchunks - 1 - j;
-            const int nt = min(TC, p.L - c * TC);
-            float* rg = ring + (j & 1) * SM::kRing;
-            const float* rrow = rmem + lane * SM::kRS;
-            const float rbl = rmem[3 * D * SM::kRS + lane];
-            float r0, qk, dk0, w, beta, qe, ke, ul;
-            // Everything of step t that does not wait for g_h, in two parts.  The scalars and the vector u go out
-            // first (u through shared memory, with whatever exchange comes next); the products follow a barrier:
-            // r0 = (G k) and q.k for the head of the step, the early rewind of S and dk0 = G u.  The step loop runs
-            // them for step t - 1 inside step t, without a branch: at t = 0 they repeat step 0 with `live` = 0 (the
-            // rewind then adds zero), so that the compiler may schedule them beside the end of the step.
-            auto prep_scalars = [&](int t) {
-                const int o = t * D + lane;
-                beta = s.b.f[t];
-                w = s.v.f[o] - s.vo.f[o];
-                qe = s.q.f[o];
-                ke = s.k.f[o];
-                ul = beta * w;
-                xu[lane] = ul;
-            };
-            auto prep_products = [&](int t, float live) {
-                f2 va[NP], vb[NP];
-                lds_slice<D>(va, s.q.f + t * D);
-                lds_slice<D>(vb, s.k.f + t * D);
-                r0 = dot2<NP>(A, vb);
-                qk = dot2<NP>(va, vb);
-                lds_slice<D>(va, xu);
-                axpy2<NP>(B, va, -ke * live);       // S_{t-1}
-                dk0 = dot2<NP>(C, va);
-            };
-            prep_scalars(nt - 1);
-            __syncwarp();
-            prep_products(nt - 1, 1.f);
-#pragma unroll 1
-            for (int t = nt - 1; t >= 0; t--) {
-                const int o = t * D + lane;
-                float* e = rg + t * SM::kStep;
-                const float hte = s.od.f[o];
-                const float gcol = s.gy.f[o] + gh;
-                const float r = fmaf(qk, gcol, r0);
-                const float dv = beta * r;
-                xg[lane] = gcol;
-                e[2 * D + lane] = dv;
-                // u.g and db from lane products, in one shuffle sequence beside the exchange
-                float pgu = gcol * ul, pdb = r * w;
-#pragma unroll
-                for (int sft = 16; sft >= 1; sft >>= 1) {
-                    pgu += __shfl_xor_sync(0xffffffffu, pgu, sft);
-                    pdb += __shfl_xor_sync(0xffffffffu, pdb, sft);
-                }
-                const float dbh = pdb * beta * (1.f - beta);
-                f2 gv[NP], dvv[NP];
-                // G by columns takes this step's own vectors: += q (x) g, -= k (x) dv (the vectors come back from the tiles)
-                lds_slice<D>(gv, s.q.f + t * D);
-                axpy2<NP>(A, gv, gcol);
-                lds_slice<D>(dvv, s.k.f + t * D);
-                axpy2<NP>(A, dvv, -dv);
-                __syncwarp();
-                lds_slice<D>(gv, xg);
-                lds_slice<D>(dvv, e + 2 * D);
-                const float sg = dot2<NP>(B, gv);
-                const float sdv = dot2<NP>(B, dvv);
-                const float dq = fmaf(ke, pgu, sg);
-                const float dk = fmaf(qe, pgu, dk0) - sdv;
-                // the two softmax backward maps: both sums in one shuffle sequence
-                float pq = qe * dq, pk = ke * dk;
-#pragma unroll
-                for (int sft = 16; sft >= 1; sft >>= 1) {
-                    pq += __shfl_xor_sync(0xffffffffu, pq, sft);
-                    pk += __shfl_xor_sync(0xffffffffu, pk, sft);
-                }
-                // the part of the feedback that needs dv only, and the two updates of G by rows: placed ahead of the
-                // stores below so that they may be scheduled inside the shuffle sequence above
-                f2 rr[NP];
-                lds_slice<D>(rr, rrow + 2 * D * SM::kRS);
-                float back = fmaf(rbl, dbh, dot2<NP>(rr, dvv));
-                axpy2<NP>(C, gv, qe);               // G by rows: += q (x) g, -= k (x) dv
-                axpy2<NP>(C, dvv, -ke);
-                const float dqh = qe * (dq - pq), dkh = ke * (dk - pk);
-                e[lane] = dqh;
-                e[D + lane] = dkh;
-                if (lane == 0) e[3 * D] = dbh;
-                const int tn = t > 0 ? t - 1 : 0;
-                prep_scalars(tn);                   // the next step's u travels with this exchange
-                __syncwarp();
-                lds_slice<D>(gv, e);                // dq~
-                lds_slice<D>(rr, rrow);
-                back += dot2<NP>(rr, gv);
-                lds_slice<D>(dvv, e + D);           // dk~
-                lds_slice<D>(rr, rrow + D * SM::kRS);
-                back += dot2<NP>(rr, dvv);
-                gh = (1.f - hte * hte) * back;
-                prep_products(tn, t > 0 ? 1.f : 0.f);
-            }
-        } else if (role == 1 && j > 0) {
-            // ------------------------------------------------------------ Y: one chunk behind
-            const int jj = j - 1;
-            Stage s; s.bind(smem + (jj % SM::kStages) * Stage::kFloats);
-            const int c = nchunks - 1 - jj;
-            const int t0 = c * TC, nt = min(TC, p.L - t0);
-            const float* rg = ring + (jj & 1) * SM::kRing;
-            const long long tl = t0 + nt - 1;
-            float* pgq = reinterpret_cast<float*>(p.gq.p) + n * p.gq.sN + h * p.gq.sH + tl * p.gq.sL + lane;
-            float* pgk = reinterpret_cast<float*>(p.gk.p) + n * p.gk.sN + h * p.gk.sH + tl * p.gk.sL + lane;
-            float* pgv = reinterpret_cast<float*>(p.gv.p) + n * p.gv.sN + h * p.gv.sH + tl * p.gv.sL + lane;
-            float* pgb = reinterpret_cast<float*>(p.gb.p) + n * p.gb.sN + h * p.gb.sH + tl * p.gb.sL;
-#pragma unroll 1
-            for (int t = nt - 1; t >= 0; t--) {
-                const float* e = rg + t * SM::kStep;
-                const float dqh = e[lane], dkh = e[D + lane], dv = e[2 * D + lane], dbh = e[3 * D];
-                const float hte = s.od.f[t * D + lane];
-                f2 hs[NP];
-                lds_slice<D>(hs, s.od.f + t * D);
-                axpy2<NP>(A, hs, dqh);
-                axpy2<NP>(B, hs, dkh);
-                axpy2<NP>(C, hs, dv);
-                arb += hte * dbh;
-                *pgq = dqh; *pgk = dkh; *pgv = dv;
-                if (lane == 0) *pgb = dbh;
-                pgq -= p.gq.sL; pgk -= p.gk.sL; pgv -= p.gv.sL; pgb -= p.gb.sL;
-            }
-        }
-    }
+    };
+    // hand-overs between X and P: one side arrives, the other waits, in strict alternation
+    auto arrive = [&](int id) { asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory"); };
+    auto await = [&](int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); };
+    const int given = 5 + slot, posted = 9 + slot;
+    float* const W = p.W + n * p.wN + h * p.wH;
+    issue(0);
+
     if (role == 0) {
+        // ---------------------------------------------------------------- X: the chain
+        if constexpr (SLOTS == 4) asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+        // lane (half, lp): rows 2 lp + half (finished here) and 2 lp + 1 - half (given away), columns 16 half .. 16 half + 15
+        const int half = lane >> 4, lp = lane & 15, own = 2 * lp + half, other = 2 * lp + 1 - half;
+        auto at = [&](int i) { return (i < 8 ? own : other); };
+        f2 S[16], Rq[16], Rk[16], Rv[16];
 #pragma unroll
-        for (int i = 0; i < D; i++) {
-            float lo, hi;
-            f2_unpack(B[i >> 1], lo, hi);
-            W[(long long)lane * p.wE + i] = (i & 1) ? hi : lo;
+        for (int i = 0; i < 16; i++) {
+            const int c = 16 * half + 2 * (i & 7);
+            const float* w = W + (long long)at(i) * p.wE + c;
+            S[i] = f2_pack(w[0], w[1]);
+            const long long r = h * p.rH + (long long)at(i) * p.rE + c;
+            Rq[i] = f2_pack(p.Rq[r], p.Rq[r + 1]);
+            Rk[i] = f2_pack(p.Rk[r], p.Rk[r + 1]);
+            Rv[i] = f2_pack(p.Rv[r], p.Rv[r + 1]);
         }
-    } else {
-        // partial parameter gradients of this (n, h): [3][d][d] then [d]; lane = column m, element (e, m) at e d + m
-        float* out = p.scratch + (long long)seq * (3 * D * D + D);
+        const float rbl = p.rb[h * p.rbH + own];
+        // a0 + a1, b0 + b1: M x for the rows `own` and `other`
+        auto dots = [&](const f2 (&M)[16], const f2 (&x)[8], f2& a, f2& b) {
 #pragma unroll
-        for (int i = 0; i < D; i++) {
-            float lo, hi;
-            f2_unpack(A[i >> 1], lo, hi);
-            out[i * D + lane] = (i & 1) ? hi : lo;
-            f2_unpack(B[i >> 1], lo, hi);
-            out[D * D + i * D + lane] = (i & 1) ? hi : lo;
-            f2_unpack(C[i >> 1], lo, hi);
-            out[2 * D * D + i * D + lane] = (i & 1) ? hi : lo;
+            for (int i = 0; i < 8; i++) {
+                a = ffma2(M[i], x[i], a);
+                b = ffma2(M[8 + i], x[i], b);
+            }
+        };
+        auto dot = [&](const f2 (&x)[8], const f2 (&y)[8]) {
+            f2 a = fmul2(x[0], y[0]), b = fmul2(x[1], y[1]);
+#pragma unroll
+            for (int i = 2; i < 8; i += 2) {
+                a = ffma2(x[i], y[i], a);
+                b = ffma2(x[i + 1], y[i + 1], b);
+            }
+            return f2_hsum(fadd2(a, b));
+        };
+        auto swap_halves = [&](float x) { return __shfl_xor_sync(0xffffffffu, x, 16); };
+        float gh = 0.f;
+        for (int j = 0; j <= nchunks + 1; j++) {
+            advance(j);
+            if (j == 0 || j > nchunks) continue;
+            Stage s; s.bind(smem + ((j - 1) % SM::kStages) * Stage::kFloats);
+            const int nt = min(TC, p.L - (nchunks - j) * TC);
+            float* rg = ring + ((j - 1) & 1) * SM::kRing;
+            f2 w[8];
+            float beta, qe, ke;
+            auto rewind = [&](int t, float live) {      // S_{t-1} = S_t - beta k (x) w; what step t does not wait for
+                beta = s.b.f[t];
+                qe = s.q.f[t * D + own];
+                ke = s.k.f[t * D + own];
+                lds_slice<16>(w, s.v.f + t * D + 16 * half);
+                const float nb = -beta * live;
+                const f2 k0 = f2_dup(nb * ke), k1 = f2_dup(nb * s.k.f[t * D + other]);
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    S[i] = ffma2(w[i], k0, S[i]);
+                    S[8 + i] = ffma2(w[i], k1, S[8 + i]);
+                }
+            };
+            rewind(nt - 1, 1.f);
+#pragma unroll 1
+            for (int t = nt - 1; t >= 0; t--) {
+                float* e = rg + t * SM::kStep;
+                const float* mb = mail + (t & 1) * SM::kMail;
+                const float gcol = s.gy.f[t * D + own] + gh, hte = s.od.f[t * D + own];
+                await(posted);
+                const float r = fmaf(mb[2 * D], gcol, mb[own]), gu = mb[D + own];
+                e[own] = gcol;
+                e[D + own] = beta * r;
+                __syncwarp();
+                arrive(given);
+                f2 x[8], y[8];
+                lds_slice<16>(x, e + 16 * half);
+                lds_slice<16>(y, e + D + 16 * half);
+                float wg = dot(w, x), wdv = dot(w, y), vdv;
+                f2 a = 0ull, b = 0ull, c = 0ull, d = 0ull;
+                dots(S, x, a, b);
+                dots(S, y, c, d);
+                {
+                    f2 z[8];
+                    lds_slice<16>(z, s.vo.f + t * D + 16 * half);
+                    vdv = dot(z, y);
+                }
+                const float sg = f2_hsum(a) + swap_halves(f2_hsum(b));
+                const float sdv = f2_hsum(c) + swap_halves(f2_hsum(d));
+                wg += swap_halves(wg);
+                wdv += swap_halves(wdv);
+                vdv += swap_halves(vdv);
+                const float ug = beta * wg;
+                const float dq = fmaf(ke, ug, sg), dk = fmaf(qe, ug, gu) - sdv;
+                const float dbh = wdv * (1.f - beta);
+                float pq = qe * dq;
+#pragma unroll
+                for (int o = 16; o >= 1; o >>= 1) pq += __shfl_xor_sync(0xffffffffu, pq, o);
+                a = b = 0ull;
+                dots(Rv, y, a, b);                      // beside the reduction: the part of the feedback that needs dv only
+                const float dqh = qe * (dq - pq), dkh = ke * (dk - (wdv - vdv));
+                e[2 * D + own] = dqh;
+                e[3 * D + own] = dkh;
+                if (lane == 0) e[4 * D] = dbh;
+                __syncwarp();
+                lds_slice<16>(x, e + 2 * D + 16 * half);
+                lds_slice<16>(y, e + 3 * D + 16 * half);
+                c = d = 0ull;
+                dots(Rq, x, a, b);
+                dots(Rk, y, c, d);
+                gh = (1.f - hte * hte) * (fmaf(rbl, dbh, f2_hsum(fadd2(a, c))) + swap_halves(f2_hsum(fadd2(b, d))));
+                rewind(t > 0 ? t - 1 : 0, t > 0 ? 1.f : 0.f);       // at t = 0 repeated with nothing to subtract: no branch
+            }
         }
-        out[3 * D * D + lane] = arb;
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            float* w = W + (long long)at(i) * p.wE + 16 * half + 2 * (i & 7);
+            f2_unpack(S[i], w[0], w[1]);
+        }
+        return;
     }
+    if (role == 1) {
+        // ---------------------------------------------------------------- P: G
+        if constexpr (SLOTS == 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 120;");
+        const Tile32 tile(lane);
+        f2 G[16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) G[i] = 0ull;
+        for (int j = 0; j <= nchunks + 1; j++) {
+            advance(j);
+            if (j == 0 || j > nchunks) continue;
+            Stage s; s.bind(smem + ((j - 1) % SM::kStages) * Stage::kFloats);
+            const int nt = min(TC, p.L - (nchunks - j) * TC);
+            const float* rg = ring + ((j - 1) & 1) * SM::kRing;
+#pragma unroll 1
+            for (int t = nt - 1; t >= 0; t--) {
+                float* mb = mail + (t & 1) * SM::kMail;
+                f2 qq[4], kk[4], x[4], acc[4];
+                tile.rows(qq, s.q.f + t * D);
+                tile.rows(kk, s.k.f + t * D);
+                tile.cols(x, s.v.f + t * D);            // w
+                float r[4];
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    f2 d = 0ull;
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        d = i == 0 ? fmul2(G[4 * c], kk[0]) : ffma2(G[4 * c + i], kk[i], d);
+                        acc[i] = c == 0 ? fmul2(G[i], x[0]) : ffma2(G[4 * c + i], x[c], acc[i]);
+                    }
+                    r[c] = f2_hsum(d);
+                }
+                f2 d = fmul2(qq[0], kk[0]);
+#pragma unroll
+                for (int i = 1; i < 4; i++) d = ffma2(qq[i], kk[i], d);
+                float qk = f2_hsum(d);
+                qk += __shfl_xor_sync(0xffffffffu, qk, 8);
+                qk += __shfl_xor_sync(0xffffffffu, qk, 16);
+                mb[tile.own] = tile.sum_rows(r);
+                mb[D + lane] = s.b.f[t] * tile.sum_cols(acc);
+                if (lane == 0) mb[2 * D] = qk;
+                __syncwarp();
+                arrive(posted);
+                await(given);
+                const float* e = rg + t * SM::kStep;
+                f2 y[4];
+                tile.cols(x, e);
+                {
+                    const float2 a = *reinterpret_cast<const float2*>(e + D + tile.col0), b = *reinterpret_cast<const float2*>(e + D + tile.col1);
+                    y[0] = f2_dup(-a.x); y[1] = f2_dup(-a.y); y[2] = f2_dup(-b.x); y[3] = f2_dup(-b.y);
+                }
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) G[4 * c + i] = ffma2(kk[i], y[c], ffma2(qq[i], x[c], G[4 * c + i]));
+            }
+        }
+        return;
+    }
+    // -------------------------------------------------------------------- Y: w for X and P, then parameter gradients and stores
+    if constexpr (SLOTS == 4) asm volatile("setmaxnreg.inc.sync.aligned.u32 176;");
+    const Tile32 tile(lane);
+    f2 A[16], B[16], C[16];             // the partial gradients of Rq, Rk, Rv
+#pragma unroll
+    for (int i = 0; i < 16; i++) { A[i] = 0ull; B[i] = 0ull; C[i] = 0ull; }
+    float arb = 0.f;
+    const long long last = p.L - 1;
+    float* pgq = reinterpret_cast<float*>(p.gq.p) + n * p.gq.sN + h * p.gq.sH + lane + last * p.gq.sL;
+    float* pgk = reinterpret_cast<float*>(p.gk.p) + n * p.gk.sN + h * p.gk.sH + lane + last * p.gk.sL;
+    float* pgv = reinterpret_cast<float*>(p.gv.p) + n * p.gv.sN + h * p.gv.sH + lane + last * p.gv.sL;
+    float* pgb = reinterpret_cast<float*>(p.gb.p) + n * p.gb.sN + h * p.gb.sH + last * p.gb.sL;
+    for (int j = 0; j <= nchunks + 1; j++) {
+        advance(j);
+        if (j < nchunks) {
+            Stage s; s.bind(smem + (j % SM::kStages) * Stage::kFloats);
+            const int nt = min(TC, p.L - (nchunks - 1 - j) * TC);
+#pragma unroll 4
+            for (int t = 0; t < nt; t++) s.v.f[t * D + lane] -= s.vo.f[t * D + lane];
+        }
+        if (j < 2) continue;
+        Stage s; s.bind(smem + ((j - 2) % SM::kStages) * Stage::kFloats);
+        const int nt = min(TC, p.L - (nchunks + 1 - j) * TC);
+        const float* rg = ring + (j & 1) * SM::kRing;
+#pragma unroll 2
+        for (int t = nt - 1; t >= 0; t--) {
+            const float* e = rg + t * SM::kStep;
+            f2 hs[4], x[4], y[4], z[4];
+            tile.rows(hs, s.od.f + t * D);
+            tile.cols(x, e + 2 * D);
+            tile.cols(y, e + 3 * D);
+            tile.cols(z, e + D);
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    A[4 * c + i] = ffma2(hs[i], x[c], A[4 * c + i]);
+                    B[4 * c + i] = ffma2(hs[i], y[c], B[4 * c + i]);
+                    C[4 * c + i] = ffma2(hs[i], z[c], C[4 * c + i]);
+                }
+            const float dbh = e[4 * D];
+            arb += s.od.f[t * D + lane] * dbh;
+            *pgq = e[2 * D + lane]; *pgk = e[3 * D + lane]; *pgv = e[D + lane];
+            if (lane == 0) *pgb = dbh;
+            pgq -= p.gq.sL; pgk -= p.gk.sL; pgv -= p.gv.sL; pgb -= p.gb.sL;
+        }
+    }
+    // partial parameter gradients of this (n, h): [3][d][d] then [d]; element (e, m) at e d + m
+    float* out = p.scratch + (long long)seq * (3 * D * D + D);
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            float* o = out + tile.row(i) * D + tile.col(c);
+            f2_unpack(A[4 * c + i], o[0], o[D]);
+            f2_unpack(B[4 * c + i], o[D * D], o[D * D + D]);
+            f2_unpack(C[4 * c + i], o[2 * D * D], o[2 * D * D + D]);
+        }
+    out[3 * D * D + lane] = arb;
 }
 
 }  // namespace fwp
