@@ -245,6 +245,23 @@ int fwp_rec_update_fwm_tanh_backward(int N, int H, int L, int D,
                                      const fwp_tensor* grad_Rv, const fwp_tensor* grad_rb,
                                      float* scratch, int64_t scratch_floats,
                                      int io_dtype, void* stream, int device);
+/* The same from what the forward left: its outputs `out` and the vector `start` (N,H,1,D) that the first step was fed, instead
+ * of a tensor of their delayed tanh.  FWP_ERR_UNSUPPORTED, with nothing launched, where no kernel takes them (head sizes other
+ * than 32; rows that are not 16-byte aligned below 64 steps): the entry point above serves every case. */
+int fwp_rec_update_fwm_tanh_backward_from_outputs(int N, int H, int L, int D,
+                                     const fwp_tensor* q, const fwp_tensor* k,
+                                     const fwp_tensor* v, const fwp_tensor* beta,
+                                     const fwp_tensor* v_old, const fwp_tensor* out, const fwp_tensor* start,
+                                     const fwp_tensor* grad_out,
+                                     const fwp_tensor* Rq, const fwp_tensor* Rk,
+                                     const fwp_tensor* Rv, const fwp_tensor* rb,
+                                     const fwp_tensor* fw_mem,
+                                     const fwp_tensor* grad_q, const fwp_tensor* grad_k,
+                                     const fwp_tensor* grad_v, const fwp_tensor* grad_beta,
+                                     const fwp_tensor* grad_Rq, const fwp_tensor* grad_Rk,
+                                     const fwp_tensor* grad_Rv, const fwp_tensor* grad_rb,
+                                     float* scratch, int64_t scratch_floats,
+                                     int io_dtype, void* stream, int device);
 int64_t fwp_rec_update_fwm_tanh_scratch_floats(int N, int H, int D);
 
 /* Same backward for callers that cannot allocate device memory when they call it
@@ -314,6 +331,16 @@ int fwp_fast_rnn_backward(int N, int H, int L, int D,
                           const fwp_tensor* grad_Z, const fwp_tensor* grad_K,
                           const fwp_tensor* grad_V, const fwp_tensor* grad_beta,
                           int io_dtype, void* stream, int device);
+/* The same with the vector before the first output, (N,H,1,D), instead of the delayed outputs.  FWP_ERR_UNSUPPORTED as for
+ * fwp_rec_update_fwm_tanh_backward_from_outputs. */
+int fwp_fast_rnn_backward_from_outputs(int N, int H, int L, int D,
+                          const fwp_tensor* K, const fwp_tensor* V, const fwp_tensor* beta,
+                          const fwp_tensor* v_old, const fwp_tensor* grad_out,
+                          const fwp_tensor* out, const fwp_tensor* start,
+                          const fwp_tensor* fw_mem,
+                          const fwp_tensor* grad_Z, const fwp_tensor* grad_K,
+                          const fwp_tensor* grad_V, const fwp_tensor* grad_beta,
+                          int io_dtype, void* stream, int device);
 
 /* ---- delta LSTM v1..v4 -----------------------------------------------------
  * One entry point for the four variants (variant = 1..4).  The twelve streamed
@@ -345,6 +372,19 @@ int fwp_fast_lstm_backward(int variant, int N, int H, int L, int D,
                            const fwp_tensor v_old[3],
                            const fwp_tensor* out, const fwp_tensor* out_delayed,
                            const fwp_tensor* cell_out, const fwp_tensor* u_minus_c,
+                           const fwp_tensor gates[3], const fwp_tensor kv[3],
+                           const fwp_tensor grad_Z[3], const fwp_tensor grad_K[3],
+                           const fwp_tensor grad_V[3], const fwp_tensor grad_beta[3],
+                           int io_dtype, void* stream, int device);
+/* The same with `fed_back` = the vector before the first output, (N,H,1,D), in variant 1 and the forward's out_del_nmz in the
+ * others, and `cell_start` = the cell before the first, (N,H,1,D).  FWP_ERR_UNSUPPORTED as for
+ * fwp_rec_update_fwm_tanh_backward_from_outputs. */
+int fwp_fast_lstm_backward_from_outputs(int variant, int N, int H, int L, int D,
+                           const fwp_tensor* grad_out,
+                           const fwp_tensor K[3], const fwp_tensor V[3], const fwp_tensor beta[3],
+                           const fwp_tensor v_old[3],
+                           const fwp_tensor* out, const fwp_tensor* fed_back,
+                           const fwp_tensor* cell_out, const fwp_tensor* cell_start,
                            const fwp_tensor gates[3], const fwp_tensor kv[3],
                            const fwp_tensor grad_Z[3], const fwp_tensor grad_K[3],
                            const fwp_tensor grad_V[3], const fwp_tensor grad_beta[3],

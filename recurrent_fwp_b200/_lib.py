@@ -54,11 +54,13 @@ SIGNATURES = {
     'fwp_causal_dot_backward': [_i] * 5 + [_T] * 7 + [_i, _vp, _i],
     'fwp_rec_update_fwm_tanh_forward': [_i] * 4 + [_T] * 16 + [_i, _vp, _i],
     'fwp_rec_update_fwm_tanh_backward': [_i] * 4 + [_T] * 20 + [ctypes.POINTER(ctypes.c_float), _i64, _i, _vp, _i],
+    'fwp_rec_update_fwm_tanh_backward_from_outputs': [_i] * 4 + [_T] * 21 + [ctypes.POINTER(ctypes.c_float), _i64, _i, _vp, _i],
     'fwp_rec_update_fwm_tanh_backward_noalloc': [_i] * 4 + [_T] * 20 + [_i, _vp, _i],
     'fwp_fast_rnn_v2_forward': [_i] * 4 + [_T] * 9 + [_i, _vp, _i],
     'fwp_fast_rnn_v2_backward': [_i] * 4 + [_T] * 12 + [_i, _vp, _i],
     'fwp_fast_rnn_forward': [_i] * 4 + [_T] * 8 + [_i, _vp, _i],
     'fwp_fast_rnn_backward': [_i] * 4 + [_T] * 12 + [_i, _vp, _i],
+    'fwp_fast_rnn_backward_from_outputs': [_i] * 4 + [_T] * 12 + [_i, _vp, _i],
     'fwp_fast_lstm_forward': [_i] * 5 + [_T3] * 4 + [_T, _T, _T3, _T, _T, _T, _T3, _T3] + [_i, _vp, _i],
     'fwp_delta_layer_prologue_forward': [_i] * 4 + [ctypes.c_void_p] * 5 + [_vp, _i],
     'fwp_delta_layer_prologue_backward': [_i] * 4 + [ctypes.c_void_p] * 6 + [_vp, _i],
@@ -68,6 +70,7 @@ SIGNATURES = {
     'fwp_debug_bounded_wait_probe': [_i, _vp, _i],
     'fwp_delayed': [_i] * 4 + [_T] * 4 + [_i, _vp, _i],
     'fwp_fast_lstm_backward': [_i] * 5 + [_T] + [_T3] * 4 + [_T] * 4 + [_T3] * 6 + [_i, _vp, _i],
+    'fwp_fast_lstm_backward_from_outputs': [_i] * 5 + [_T] + [_T3] * 4 + [_T] * 4 + [_T3] * 6 + [_i, _vp, _i],
 }
 OTHER_SYMBOLS = ['fwp_status_string', 'fwp_last_cuda_error', 'fwp_version', 'fwp_max_head_dim',
                  'fwp_launch_count', 'fwp_tune', 'fwp_rec_update_fwm_tanh_scratch_floats', 'fwp_delta_device_fault',

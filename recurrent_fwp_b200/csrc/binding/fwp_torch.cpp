@@ -366,18 +366,26 @@ struct RecNode final : public OpNode {
         const Tensor &q = o[0], &k = o[1], &v = o[2], &beta = o[3], &v_old = o[4], &h0 = o[5];
         const Tensor gy = incoming(g[0], out, {d.N, d.H, d.L, d.M});
         Tensor gq = empty(d, d.M, out), gk = empty(d, d.M, out), gv = empty(d, d.M, out), gb = empty(d, 1, out);
-        Tensor gR[3], delayed = empty(d, d.M, out);
+        Tensor gR[3];
         for (auto& x : gR) x = empty({1, d.H, d.M, d.M}, at::kFloat, out);
         Tensor grb = empty({1, d.H, 1, d.M}, at::kFloat, out);
         const int64_t nscratch = fwp_rec_update_fwm_tanh_scratch_floats(d.N, d.H, d.M);
         Tensor scratch = empty({nscratch}, at::kFloat, out);
         void* st = stream_of(out);
         const int dev = out.device().index();
-        check(fwp_delayed(d.N, d.H, d.L, d.M, Desc(out), Desc(h0), Desc(Tensor()), Desc(delayed), 1, st, dev), "delayed");
-        check(fwp_rec_update_fwm_tanh_backward(d.N, d.H, d.L, d.M, Desc(q), Desc(k), Desc(v), Desc(beta), Desc(v_old), Desc(delayed),
-                                               Desc(gy), Desc(R[0]), Desc(R[1]), Desc(R[2]), Desc(R[3]), Desc(W), Desc(gq), Desc(gk),
-                                               Desc(gv), Desc(gb), Desc(gR[0]), Desc(gR[1]), Desc(gR[2]), Desc(grb),
-                                               scratch.data_ptr<float>(), nscratch, FWP_F32, st, dev), "rec_update_fwm_tanh_backward");
+        int rc = fwp_rec_update_fwm_tanh_backward_from_outputs(
+            d.N, d.H, d.L, d.M, Desc(q), Desc(k), Desc(v), Desc(beta), Desc(v_old), Desc(out), Desc(h0), Desc(gy), Desc(R[0]), Desc(R[1]),
+            Desc(R[2]), Desc(R[3]), Desc(W), Desc(gq), Desc(gk), Desc(gv), Desc(gb), Desc(gR[0]), Desc(gR[1]), Desc(gR[2]), Desc(grb),
+            scratch.data_ptr<float>(), nscratch, FWP_F32, st, dev);
+        if (rc == FWP_ERR_UNSUPPORTED) {
+            Tensor delayed = empty(d, d.M, out);
+            check(fwp_delayed(d.N, d.H, d.L, d.M, Desc(out), Desc(h0), Desc(Tensor()), Desc(delayed), 1, st, dev), "delayed");
+            rc = fwp_rec_update_fwm_tanh_backward(
+                d.N, d.H, d.L, d.M, Desc(q), Desc(k), Desc(v), Desc(beta), Desc(v_old), Desc(delayed), Desc(gy), Desc(R[0]), Desc(R[1]),
+                Desc(R[2]), Desc(R[3]), Desc(W), Desc(gq), Desc(gk), Desc(gv), Desc(gb), Desc(gR[0]), Desc(gR[1]), Desc(gR[2]), Desc(grb),
+                scratch.data_ptr<float>(), nscratch, FWP_F32, st, dev);
+        }
+        check(rc, "rec_update_fwm_tanh_backward");
         return {gq, gk, gv, gb, gR[0], gR[1], gR[2], grb, Tensor(), Tensor()};
     }
 };
@@ -430,17 +438,20 @@ struct RnnNode final : public OpNode {
         const Tensor &K = t[0], &V = t[1], &beta = t[2], &W = t[3], &out = t[4], &v_old = o[0];
         const Tensor gy = incoming(g[0], out, {d.N, d.H, d.L, d.M});
         Tensor gZ = empty(d, d.M, out), gK = empty(d, d.M, out), gV = empty(d, d.M, out), gb = empty(d, 1, out);
-        Tensor delayed = o[1];        // v2: the normalised delayed outputs of the forward; v1: the start vector
+        const Tensor& aux = o[1];     // v2: the normalised delayed outputs of the forward; v1: the start vector
         void* st = stream_of(out);
         const int dev = out.device().index();
-        if (VERSION == 1) {
-            delayed = empty(d, d.M, out);
-            check(fwp_delayed(d.N, d.H, d.L, d.M, Desc(out), Desc(o[1]), Desc(Tensor()), Desc(delayed), 0, st, dev), "delayed");
+        auto run = [&](auto backward, const Tensor& fed_back) {
+            return backward(d.N, d.H, d.L, d.M, Desc(K), Desc(V), Desc(beta), Desc(v_old), Desc(gy), Desc(out), Desc(fed_back), Desc(W),
+                            Desc(gZ), Desc(gK), Desc(gV), Desc(gb), FWP_F32, st, dev);
+        };
+        int rc = run(VERSION == 1 ? fwp_fast_rnn_backward_from_outputs : fwp_fast_rnn_v2_backward, aux);
+        if (VERSION == 1 && rc == FWP_ERR_UNSUPPORTED) {
+            Tensor delayed = empty(d, d.M, out);
+            check(fwp_delayed(d.N, d.H, d.L, d.M, Desc(out), Desc(aux), Desc(Tensor()), Desc(delayed), 0, st, dev), "delayed");
+            rc = run(fwp_fast_rnn_backward, delayed);
         }
-        const auto backward = VERSION == 1 ? fwp_fast_rnn_backward : fwp_fast_rnn_v2_backward;
-        check(backward(d.N, d.H, d.L, d.M, Desc(K), Desc(V), Desc(beta), Desc(v_old), Desc(gy), Desc(out), Desc(delayed), Desc(W),
-                       Desc(gZ), Desc(gK), Desc(gV), Desc(gb), FWP_F32, st, dev),
-              VERSION == 1 ? "fast_rnn_backward" : "fast_rnn_v2_backward");
+        check(rc, VERSION == 1 ? "fast_rnn_backward" : "fast_rnn_v2_backward");
         return {gZ, gK, gV, Tensor(), gb, Tensor()};
     }
 };
@@ -501,12 +512,6 @@ struct LstmNode final : public OpNode {
         const Tensor gy = incoming(g[0], out, {d.N, d.H, d.L, d.M});        // the cell's gradient is ignored, as in the reference
         void* st = stream_of(out);
         const int dev = out.device().index();
-        Tensor delayed = o[6], u_minus_c = empty(d, d.M, out);            // v1: h0, v2-v4: the normalised delayed outputs
-        if (variant == 1) {
-            delayed = empty(d, d.M, out);
-            check(fwp_delayed(d.N, d.H, d.L, d.M, Desc(out), Desc(o[6]), Desc(Tensor()), Desc(delayed), 0, st, dev), "delayed");
-        }
-        check(fwp_delayed(d.N, d.H, d.L, d.M, Desc(cell), Desc(o[7]), Desc(gates[1]), Desc(u_minus_c), 0, st, dev), "delayed");
         Tensor gZ[3], gK[3], gV[3], gb[3];
         for (int i = 0; i < 3; i++) {
             gZ[i] = empty(d, d.M, out);
@@ -514,9 +519,22 @@ struct LstmNode final : public OpNode {
             gV[i] = empty(d, d.M, out);
             gb[i] = empty(d, 1, out);
         }
-        check(fwp_fast_lstm_backward(variant, d.N, d.H, d.L, d.M, Desc(gy), Desc3(&t[0]), Desc3(&t[3]), Desc3(&t[6]), Desc3(v_old), Desc(out),
-                                     Desc(delayed), Desc(cell), Desc(u_minus_c), Desc3(gates), Desc3(&t[9]), Desc3(gZ), Desc3(gK),
-                                     Desc3(gV), Desc3(gb), FWP_F32, st, dev), "fast_lstm_backward");
+        auto run = [&](auto backward, const Tensor& fed_back, const Tensor& cells) {      // o[6]: h0 (v1) or the normalised delayed outputs
+            return backward(variant, d.N, d.H, d.L, d.M, Desc(gy), Desc3(&t[0]), Desc3(&t[3]), Desc3(&t[6]), Desc3(v_old), Desc(out),
+                            Desc(fed_back), Desc(cell), Desc(cells), Desc3(gates), Desc3(&t[9]), Desc3(gZ), Desc3(gK), Desc3(gV), Desc3(gb),
+                            FWP_F32, st, dev);
+        };
+        int rc = run(fwp_fast_lstm_backward_from_outputs, o[6], o[7]);
+        if (rc == FWP_ERR_UNSUPPORTED) {
+            Tensor delayed = o[6], u_minus_c = empty(d, d.M, out);
+            if (variant == 1) {
+                delayed = empty(d, d.M, out);
+                check(fwp_delayed(d.N, d.H, d.L, d.M, Desc(out), Desc(o[6]), Desc(Tensor()), Desc(delayed), 0, st, dev), "delayed");
+            }
+            check(fwp_delayed(d.N, d.H, d.L, d.M, Desc(cell), Desc(o[7]), Desc(gates[1]), Desc(u_minus_c), 0, st, dev), "delayed");
+            rc = run(fwp_fast_lstm_backward, delayed, u_minus_c);
+        }
+        check(rc, "fast_lstm_backward");
         variable_list r;
         r.reserve(17);
         for (int i = 0; i < 3; i++)

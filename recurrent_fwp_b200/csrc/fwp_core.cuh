@@ -542,14 +542,24 @@ struct StageTable {
     long long sL[kMaxTiles];
     int words[kMaxTiles];               // 1: rows are not 16-byte aligned
     int any_words;                      // 1: some tile is so; the others keep the shorter loop
+    const float* head[kMaxTiles];       // of a stream that lags one step behind: what stands in row 0
     const float* csrc[kMaxCols];
     long long csL[kMaxCols];
 };
 __device__ __forceinline__ void stage_table_set(StageTable* tb, int i, const Row4& r, int n, int h) {
     tb->src[i] = r.p ? reinterpret_cast<const float*>(r.p) + n * r.sN + h * r.sH : nullptr;
     tb->sL[i] = r.sL;
+    tb->head[i] = nullptr;
     tb->words[i] = ((reinterpret_cast<uintptr_t>(tb->src[i]) & 15) != 0 || r.sL % 4 != 0) ? 1 : 0;
     tb->any_words = (i == 0 ? 0 : tb->any_words) | tb->words[i];
+}
+// row t of the tile is row t - 1 of the stream, and row 0 the vector `first` (N, H, 1, 32)
+__device__ __forceinline__ void stage_table_set_lagging(StageTable* tb, int i, const Row4& r, const Row4& first, int n, int h) {
+    stage_table_set(tb, i, r, n, h);
+    tb->src[i] -= r.sL;
+    tb->head[i] = reinterpret_cast<const float*>(first.p) + n * first.sN + h * first.sH;
+    tb->words[i] |= (reinterpret_cast<uintptr_t>(tb->head[i]) & 15) != 0 ? 1 : 0;
+    tb->any_words |= tb->words[i];
 }
 __device__ __forceinline__ void stage_table_set_col(StageTable* tb, int i, const Row4& r, int n, int h) {
     tb->csrc[i] = reinterpret_cast<const float*>(r.p) + n * r.sN + h * r.sH;
@@ -561,20 +571,22 @@ __device__ __forceinline__ void stage_table_issue(float* stage, const StageTable
     static_assert((TC & (TC - 1)) == 0 && TC >= 4, "rows per chunk: a power of two");
     constexpr int D = 32;
     const int total = ntile * TC * 8;
-    if (!tb->any_words) {
+    if (!tb->any_words && t0 > 0) {
 #pragma unroll 1
         for (int i = tid; i < total; i += NT) {
             const int piece = i & 7, r = (i >> 3) & (TC - 1), tile = i / (8 * TC);
             const float* sp = tb->src[tile];
             if (r < nt && sp) cp_async16(stage + i * 4, sp + (long long)(t0 + r) * tb->sL[tile] + piece * 4);
         }
-    } else {
+    } else {                        // words, or the chunk in which a lagging stream has its first row from elsewhere
 #pragma unroll 1
         for (int i = tid; i < total; i += NT) {
             const int piece = i & 7, r = (i >> 3) & (TC - 1), tile = i / (8 * TC);
             const float* sp = tb->src[tile];
             if (r >= nt || !sp) continue;
-            sp += (long long)(t0 + r) * tb->sL[tile] + piece * 4;
+            sp += (long long)(t0 + r) * tb->sL[tile];
+            if (t0 + r == 0 && tb->head[tile]) sp = tb->head[tile];
+            sp += piece * 4;
             if (!tb->words[tile]) {
                 cp_async16(stage + i * 4, sp);
                 continue;

@@ -177,6 +177,7 @@ __global__ void __launch_bounds__(D * SPLIT * slots_for(D * SPLIT)) lstm_fwd_ker
 struct LstmBwdParams {
     Row4 k[3], v[3], beta[3], v_old[3], gate[3];
     Row4 gy, out, od, cell, umc;
+    Row4 start, cell_start;         // where od (v1) and umc are not given: the vector before the first output and the cell before the first
     Row4 gz[3], gk[3], gv[3], gb[3];
     float* W[3]; long long wN[3], wH[3], wE[3];
     int H, L, D;
@@ -428,15 +429,17 @@ static int dispatch_lstm_fwd(const LstmFwdParams& p, int nseq, cudaStream_t st) 
 
 template <int VAR>
 static int dispatch_lstm_bwd(const LstmBwdParams& p, int nseq, cudaStream_t st) {
+    if (!p.umc.p && p.D != 32) return FWP_ERR_UNSUPPORTED;
     switch (pad_dim(p.D)) {
         case 16: return launch_lstm_bwd<16, 2, 8, VAR>(p, nseq, st);
         case 32: {
-            bool aligned = rows_16B_aligned(p.gy) && rows_16B_aligned(p.od) && rows_16B_aligned(p.cell) &&
-                           rows_16B_aligned(p.umc) && (VAR != 1 || rows_16B_aligned(p.out));
+            bool aligned = rows_16B_aligned(p.gy) && rows_16B_aligned(p.cell) && (VAR != 1 || rows_16B_aligned(p.out)) &&
+                           (!p.od.p || rows_16B_aligned(p.od)) && (!p.umc.p || rows_16B_aligned(p.umc));
             for (int a = 0; a < 3; a++)
                 aligned = aligned && rows_16B_aligned(p.k[a]) && rows_16B_aligned(p.v[a]) && rows_16B_aligned(p.v_old[a]) &&
                           rows_16B_aligned(p.gate[a]);
             if (p.D == 32 && tune_get(T_LSTM_BWD_ROLES32, 1) && (aligned || p.L >= 64)) return launch_lstm_bwd_roles32<VAR>(p, nseq, st);
+            if (!p.umc.p) return FWP_ERR_UNSUPPORTED;
             const int sp = tune_get(T_LSTM_BWD_SPLIT32, 2);
             // measured: 2 -> 1.37 ms, 4 -> 2.14 ms
             if (sp == 4) return launch_lstm_bwd<32, 4, 4, VAR>(p, nseq, st);
@@ -505,12 +508,13 @@ FWP_API int fwp_fast_lstm_forward(int variant, int N, int H, int L, int D,
     }
 }
 
-FWP_API int fwp_fast_lstm_backward(int variant, int N, int H, int L, int D,
+static int lstm_backward(int variant, int N, int H, int L, int D,
                                    const fwp_tensor* grad_out,
                                    const fwp_tensor K[3], const fwp_tensor V[3], const fwp_tensor beta[3],
                                    const fwp_tensor v_old[3],
                                    const fwp_tensor* out, const fwp_tensor* out_delayed,
                                    const fwp_tensor* cell_out, const fwp_tensor* u_minus_c,
+                                   const fwp_tensor* start, const fwp_tensor* cell_start,
                                    const fwp_tensor gates[3], const fwp_tensor kv[3],
                                    const fwp_tensor grad_Z[3], const fwp_tensor grad_K[3],
                                    const fwp_tensor grad_V[3], const fwp_tensor grad_beta[3],
@@ -523,8 +527,9 @@ FWP_API int fwp_fast_lstm_backward(int variant, int N, int H, int L, int D,
     if ((rc = check3(K)) || (rc = check3(V)) || (rc = check3(beta)) || (rc = check3(v_old)) || (rc = check3(gates)) ||
         (rc = check3(kv)) || (rc = check3(grad_Z)) || (rc = check3(grad_K)) || (rc = check3(grad_V)) ||
         (rc = check3(grad_beta)) || (rc = check_tensor(grad_out, 4, true)) ||
-        (rc = check_tensor(out, 4, variant == 1)) || (rc = check_tensor(out_delayed, 4, true)) ||
-        (rc = check_tensor(cell_out, 4, true)) || (rc = check_tensor(u_minus_c, 4, true)))
+        (rc = check_tensor(out, 4, variant == 1)) || (rc = check_tensor(out_delayed, 4, !start)) ||
+        (rc = check_tensor(cell_out, 4, true)) || (rc = check_tensor(u_minus_c, 4, !cell_start)) ||
+        (rc = check_tensor(start, 4, false)) || (rc = check_tensor(cell_start, 4, false)))
         return rc;
     DeviceGuard guard(device);
     if (guard.status) return guard.status;
@@ -535,6 +540,7 @@ FWP_API int fwp_fast_lstm_backward(int variant, int N, int H, int L, int D,
         p.gz[a] = row4(grad_Z + a); p.gk[a] = row4(grad_K + a); p.gv[a] = row4(grad_V + a); p.gb[a] = row4(grad_beta + a);
     }
     p.gy = row4(grad_out); p.out = row4(out); p.od = row4(out_delayed); p.cell = row4(cell_out); p.umc = row4(u_minus_c);
+    p.start = row4(start); p.cell_start = row4(cell_start);
     set_w(p.W, p.wN, p.wH, p.wE, kv);
     p.H = H; p.L = L; p.D = D;
     cudaStream_t st = (cudaStream_t)stream;
@@ -544,4 +550,35 @@ FWP_API int fwp_fast_lstm_backward(int variant, int N, int H, int L, int D,
         case 3: return dispatch_lstm_bwd<3>(p, N * H, st);
         default: return dispatch_lstm_bwd<4>(p, N * H, st);
     }
+}
+
+FWP_API int fwp_fast_lstm_backward(int variant, int N, int H, int L, int D,
+                                   const fwp_tensor* grad_out,
+                                   const fwp_tensor K[3], const fwp_tensor V[3], const fwp_tensor beta[3],
+                                   const fwp_tensor v_old[3],
+                                   const fwp_tensor* out, const fwp_tensor* out_delayed,
+                                   const fwp_tensor* cell_out, const fwp_tensor* u_minus_c,
+                                   const fwp_tensor gates[3], const fwp_tensor kv[3],
+                                   const fwp_tensor grad_Z[3], const fwp_tensor grad_K[3],
+                                   const fwp_tensor grad_V[3], const fwp_tensor grad_beta[3],
+                                   int io_dtype, void* stream, int device) {
+    if (!out_delayed || !u_minus_c) return FWP_ERR_NULL;
+    return lstm_backward(variant, N, H, L, D, grad_out, K, V, beta, v_old, out, out_delayed, cell_out, u_minus_c, nullptr, nullptr, gates, kv,
+                         grad_Z, grad_K, grad_V, grad_beta, io_dtype, stream, device);
+}
+
+FWP_API int fwp_fast_lstm_backward_from_outputs(int variant, int N, int H, int L, int D,
+                                   const fwp_tensor* grad_out,
+                                   const fwp_tensor K[3], const fwp_tensor V[3], const fwp_tensor beta[3],
+                                   const fwp_tensor v_old[3],
+                                   const fwp_tensor* out, const fwp_tensor* fed_back,
+                                   const fwp_tensor* cell_out, const fwp_tensor* cell_start,
+                                   const fwp_tensor gates[3], const fwp_tensor kv[3],
+                                   const fwp_tensor grad_Z[3], const fwp_tensor grad_K[3],
+                                   const fwp_tensor grad_V[3], const fwp_tensor grad_beta[3],
+                                   int io_dtype, void* stream, int device) {
+    if (!fed_back || !fed_back->data || !cell_start || !cell_start->data) return FWP_ERR_NULL;
+    const bool lag = variant == 1;
+    return lstm_backward(variant, N, H, L, D, grad_out, K, V, beta, v_old, out, lag ? nullptr : fed_back, cell_out, nullptr,
+                         lag ? fed_back : nullptr, cell_start, gates, kv, grad_Z, grad_K, grad_V, grad_beta, io_dtype, stream, device);
 }

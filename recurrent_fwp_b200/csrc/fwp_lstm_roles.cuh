@@ -51,6 +51,7 @@ __global__ void __launch_bounds__(128 * SLOTS, 1) lstm_bwd_roles32_kernel(const 
     float* ring = smem + SM::kStages * Stage::kFloats;
     float* hown = ring + 2 * SM::kRing;
 
+    const bool lagging = !p.umc.p;      // tile 16 has the cell of the step before instead of u - that cell
     StageTable* tb = reinterpret_cast<StageTable*>(hown + 3 * SM::kOwn);
     if (stid == 0) {                // tile order of LstmBwdStage: k, v, v_old, gate of each gate, then gy, out, od, cell, umc
         for (int a = 0; a < 3; a++) {
@@ -63,9 +64,11 @@ __global__ void __launch_bounds__(128 * SLOTS, 1) lstm_bwd_roles32_kernel(const 
         stage_table_set(tb, 12, p.gy, n, h);
         stage_table_set(tb, 13, p.out, n, h);
         if (VAR != 1) tb->src[13] = nullptr;
-        stage_table_set(tb, 14, p.od, n, h);
+        if (VAR == 1 && !p.od.p) stage_table_set_lagging(tb, 14, p.out, p.start, n, h);
+        else stage_table_set(tb, 14, p.od, n, h);
         stage_table_set(tb, 15, p.cell, n, h);
-        stage_table_set(tb, 16, p.umc, n, h);
+        if (lagging) stage_table_set_lagging(tb, 16, p.cell, p.cell_start, n, h);
+        else stage_table_set(tb, 16, p.umc, n, h);
     }
     slot_barrier(slot, NT);      // the zero fill is complete before the first copies land
 
@@ -128,7 +131,8 @@ __global__ void __launch_bounds__(128 * SLOTS, 1) lstm_bwd_roles32_kernel(const 
                 float dz[3];
                 dz[2] = (s.cell.f[o] * a) * (1.f - go) * go;
                 gc += go * a;
-                dz[0] = (gc * s.umc.f[o]) * (1.f - gi) * gi;
+                const float before = s.umc.f[o];
+                dz[0] = (gc * (lagging ? uu - before : before)) * (1.f - gi) * gi;
                 dz[1] = gc * gi;
                 if constexpr (VAR != 4) dz[1] = dz[1] * (1.f - uu) * uu;
                 gc *= (1.f - gi);

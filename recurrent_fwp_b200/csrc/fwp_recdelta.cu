@@ -278,6 +278,7 @@ struct RecBwdParams {
     long long rH, rE, rbH;
     float* W; long long wN, wH, wE;
     float* scratch;          // [N*H][3*d*d + d] partial parameter gradients
+    Row4 out, start;         // the forward's outputs and the vector before the first, where od is not given
     int H, L, D;
 };
 
@@ -546,15 +547,16 @@ static int launch_rec_bwd(const RecBwdParams& p, int nseq, cudaStream_t st) {
     return launch_dependent(kern, p, nseq / slots, D * SPLIT * slots, bytes * slots, st, "rec_bwd_kernel");
 }
 
-template <int SLOTS>
+template <int SLOTS, bool OUT>
 static int launch_rec_bwd_roles32(const RecBwdParams& p, int nseq, int slots, cudaStream_t st) {
     constexpr int TC = 8;
-    const size_t bytes = (size_t)RecRolesSmem<TC>::kFloats * sizeof(float) * slots;
-    return launch_dependent(rec_bwd_roles32_kernel<TC, SLOTS>, p, nseq / slots, 96 * slots, bytes, st, "rec_bwd_roles32_kernel");
+    const size_t bytes = (size_t)RecRolesSmem<TC, OUT>::kFloats * sizeof(float) * slots;
+    return launch_dependent(rec_bwd_roles32_kernel<TC, SLOTS, OUT>, p, nseq / slots, 96 * slots, bytes, st, "rec_bwd_roles32_kernel");
 }
+template <bool OUT>
 static int launch_rec_bwd_roles32(const RecBwdParams& p, int nseq, cudaStream_t st) {
     const int slots = spread_slots(4, nseq);
-    return slots == 4 ? launch_rec_bwd_roles32<4>(p, nseq, 4, st) : launch_rec_bwd_roles32<2>(p, nseq, slots, st);
+    return slots == 4 ? launch_rec_bwd_roles32<4, OUT>(p, nseq, 4, st) : launch_rec_bwd_roles32<2, OUT>(p, nseq, slots, st);
 }
 
 static int check_params(const fwp_tensor* Rq, const fwp_tensor* Rk, const fwp_tensor* Rv, const fwp_tensor* rb) {
@@ -627,10 +629,10 @@ FWP_API int fwp_rec_update_fwm_tanh_forward(int N, int H, int L, int D,
     return FWP_ERR_UNSUPPORTED;
 }
 
-FWP_API int fwp_rec_update_fwm_tanh_backward(int N, int H, int L, int D,
+static int rec_backward(int N, int H, int L, int D,
                                              const fwp_tensor* q, const fwp_tensor* k,
                                              const fwp_tensor* v, const fwp_tensor* beta,
-                                             const fwp_tensor* v_old, const fwp_tensor* o_delayed,
+                                             const fwp_tensor* v_old, const fwp_tensor* o_delayed, const fwp_tensor* out, const fwp_tensor* start,
                                              const fwp_tensor* grad_out,
                                              const fwp_tensor* Rq, const fwp_tensor* Rk,
                                              const fwp_tensor* Rv, const fwp_tensor* rb,
@@ -648,7 +650,8 @@ FWP_API int fwp_rec_update_fwm_tanh_backward(int N, int H, int L, int D,
     int rc;
     if ((rc = check_tensor(q, 4, true)) || (rc = check_tensor(k, 4, true)) || (rc = check_tensor(v, 4, true)) ||
         (rc = check_tensor(beta, 4, true)) || (rc = check_tensor(v_old, 4, true)) ||
-        (rc = check_tensor(o_delayed, 4, true)) || (rc = check_tensor(grad_out, 4, true)) ||
+        (rc = o_delayed ? check_tensor(o_delayed, 4, true) : check_tensor(out, 4, true)) ||
+        (!o_delayed && (rc = check_tensor(start, 4, true))) || (rc = check_tensor(grad_out, 4, true)) ||
         (rc = check_params(Rq, Rk, Rv, rb)) || (rc = check_tensor(fw_mem, 4, true)) ||
         (rc = check_tensor(grad_q, 4, true)) || (rc = check_tensor(grad_k, 4, true)) ||
         (rc = check_tensor(grad_v, 4, true)) || (rc = check_tensor(grad_beta, 4, true)) ||
@@ -661,7 +664,7 @@ FWP_API int fwp_rec_update_fwm_tanh_backward(int N, int H, int L, int D,
     if (guard.status) return guard.status;
     RecBwdParams p;
     p.q = row4(q); p.k = row4(k); p.v = row4(v); p.beta = row4(beta); p.v_old = row4(v_old);
-    p.od = row4(o_delayed); p.gy = row4(grad_out);
+    p.od = row4(o_delayed); p.out = row4(out); p.start = row4(start); p.gy = row4(grad_out);
     p.gq = row4(grad_q); p.gk = row4(grad_k); p.gv = row4(grad_v); p.gb = row4(grad_beta);
     p.Rq = (const float*)Rq->data; p.Rk = (const float*)Rk->data; p.Rv = (const float*)Rv->data;
     p.rb = (const float*)rb->data;
@@ -670,13 +673,15 @@ FWP_API int fwp_rec_update_fwm_tanh_backward(int N, int H, int L, int D,
     p.scratch = scratch;
     p.H = H; p.L = L; p.D = D;
     cudaStream_t st = (cudaStream_t)stream;
+    const bool aligned = rows_16B_aligned(p.q) && rows_16B_aligned(p.k) && rows_16B_aligned(p.v) && rows_16B_aligned(p.v_old) &&
+                         rows_16B_aligned(o_delayed ? p.od : p.out) && rows_16B_aligned(p.gy);
+    const bool roles = p.D == 32 && tune_get(T_REC_BWD_ROLES32, 1) && (aligned || p.L >= 64);
+    if (!o_delayed && !roles) return FWP_ERR_UNSUPPORTED;
     switch (DP) {
         case 16: rc = launch_rec_bwd<16, 2, 16>(p, N * H, st); break;
         case 32: {
-            const bool aligned = rows_16B_aligned(p.q) && rows_16B_aligned(p.k) && rows_16B_aligned(p.v) && rows_16B_aligned(p.v_old) &&
-                                 rows_16B_aligned(p.od) && rows_16B_aligned(p.gy);
-            if (p.D == 32 && tune_get(T_REC_BWD_ROLES32, 1) && (aligned || p.L >= 64)) {
-                rc = launch_rec_bwd_roles32(p, N * H, st);
+            if (roles) {
+                rc = o_delayed ? launch_rec_bwd_roles32<false>(p, N * H, st) : launch_rec_bwd_roles32<true>(p, N * H, st);
                 break;
             }
             const int sp = tune_get(T_REC_BWD_SPLIT32, 2);
@@ -697,6 +702,43 @@ FWP_API int fwp_rec_update_fwm_tanh_backward(int N, int H, int L, int D,
     return launch_dependent(rec_param_reduce_kernel, r, (total + 31) / 32, 32 * kReduceParts, 0, st, nullptr);
 }
 
+
+FWP_API int fwp_rec_update_fwm_tanh_backward(int N, int H, int L, int D,
+                                             const fwp_tensor* q, const fwp_tensor* k,
+                                             const fwp_tensor* v, const fwp_tensor* beta,
+                                             const fwp_tensor* v_old, const fwp_tensor* o_delayed,
+                                             const fwp_tensor* grad_out,
+                                             const fwp_tensor* Rq, const fwp_tensor* Rk,
+                                             const fwp_tensor* Rv, const fwp_tensor* rb,
+                                             const fwp_tensor* fw_mem,
+                                             const fwp_tensor* grad_q, const fwp_tensor* grad_k,
+                                             const fwp_tensor* grad_v, const fwp_tensor* grad_beta,
+                                             const fwp_tensor* grad_Rq, const fwp_tensor* grad_Rk,
+                                             const fwp_tensor* grad_Rv, const fwp_tensor* grad_rb,
+                                             float* scratch, int64_t scratch_floats,
+                                             int io_dtype, void* stream, int device) {
+    if (!o_delayed || !o_delayed->data) return FWP_ERR_NULL;
+    return rec_backward(N, H, L, D, q, k, v, beta, v_old, o_delayed, nullptr, nullptr, grad_out, Rq, Rk, Rv, rb, fw_mem, grad_q, grad_k,
+                        grad_v, grad_beta, grad_Rq, grad_Rk, grad_Rv, grad_rb, scratch, scratch_floats, io_dtype, stream, device);
+}
+
+FWP_API int fwp_rec_update_fwm_tanh_backward_from_outputs(int N, int H, int L, int D,
+                                             const fwp_tensor* q, const fwp_tensor* k,
+                                             const fwp_tensor* v, const fwp_tensor* beta,
+                                             const fwp_tensor* v_old, const fwp_tensor* out, const fwp_tensor* start,
+                                             const fwp_tensor* grad_out,
+                                             const fwp_tensor* Rq, const fwp_tensor* Rk,
+                                             const fwp_tensor* Rv, const fwp_tensor* rb,
+                                             const fwp_tensor* fw_mem,
+                                             const fwp_tensor* grad_q, const fwp_tensor* grad_k,
+                                             const fwp_tensor* grad_v, const fwp_tensor* grad_beta,
+                                             const fwp_tensor* grad_Rq, const fwp_tensor* grad_Rk,
+                                             const fwp_tensor* grad_Rv, const fwp_tensor* grad_rb,
+                                             float* scratch, int64_t scratch_floats,
+                                             int io_dtype, void* stream, int device) {
+    return rec_backward(N, H, L, D, q, k, v, beta, v_old, nullptr, out, start, grad_out, Rq, Rk, Rv, rb, fw_mem, grad_q, grad_k, grad_v,
+                        grad_beta, grad_Rq, grad_Rk, grad_Rv, grad_rb, scratch, scratch_floats, io_dtype, stream, device);
+}
 
 // ---------------------------------------------------------------------------
 // Backward of the recurrent delta net for callers that cannot allocate.

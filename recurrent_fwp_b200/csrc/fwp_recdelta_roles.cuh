@@ -8,20 +8,34 @@
 //   warp X   the chain, two rows and half the columns of S and of the three R per lane:  r = r0 + (q.k) g,  dv = beta r,
 //            dq = S_{t-1} g + k (u.g),  dk = G u + q (u.g) - S_{t-1} dv,  softmax backward, the products with R, tanh.
 //            The sums over features come from products of vectors that the lane reads anyway: u.g = beta (w.g),
-//            db = (w.dv) (1 - beta), and  k . dk = r.u - v_old.dv = w.dv - v_old.dv  (v_old = S_{t-1}^T k, dv.w = r.u);
-//   warp Y   turns v into w = v - v_old for the chunk that X takes next, and two chunks later accumulates the three parameter
+//            db = (w.dv) (1 - beta),  k . dk = r.u - v_old.dv = w.dv - v_old.dv  (v_old = S_{t-1}^T k, dv.w = r.u)  and, where the forward's
+//            outputs are given, q . dq = y . g  (y = S_t^T q);
+//   warp Y   turns v into w = v - v_old (and the outputs into their tanh) for the chunk that X takes next, and two chunks later accumulates the three parameter
 //            gradients (8 x 4 pieces) and stores.
 // X and P hand over twice per step at named barriers: P has X's step to answer in.  The warps meet once per chunk of steps.
+// Alone, X takes 131 us for 512 sequences x 256 steps (250 instructions a step, 128 of them packed multiply-adds at 2.7 cycles), with
+// P 160, with both 177; 230 us with one warp for all but the parameter gradients.  Not worth their instructions: P posting from a
+// G one step older, corrected by scalars (180).
 // With four sequences per SM (504 of 512 registers of a scheduler's four threads: 208 X, 120 P, 176 Y) 512 sequences are resident.
 #pragma once
 #include "fwp_trail.cuh"
 
 namespace fwp {
 
-template <int TC>
+template <int TC, bool OUT>
 struct RecRolesSmem {
     static constexpr int D = 32;
-    using Stage = RecBwdStage<D, TC>;
+    struct Stage : RecBwdStage<D, TC> {
+        using Base = RecBwdStage<D, TC>;
+        const float* y;                               // the forward's outputs, if given (between the tiles and beta)
+        static constexpr int kTiles = OUT ? 7 : 6;
+        static constexpr int kFloats = Base::kFloats + (OUT ? TC * D : 0);
+        __device__ __forceinline__ void bind(float* mem) {
+            Base::bind(mem);
+            y = mem + 6 * TC * D;
+            this->b.f = mem + kTiles * TC * D;
+        }
+    };
     static constexpr int kStages = 4;                 // chunk j + 1 in flight, w of chunk j, X and P on j - 1, Y on j - 2
     static constexpr int kStep = 4 * D + 4;           // per step: g, dv, dq~, dk~, db~
     static constexpr int kRing = TC * kStep;
@@ -30,12 +44,12 @@ struct RecRolesSmem {
     static constexpr int kFloats = kStages * Stage::kFloats + 2 * kRing + 2 * kMail + kTable;
 };
 
-template <int TC, int SLOTS>
+template <int TC, int SLOTS, bool OUT>
 __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const RecBwdParams p) {
     griddep_wait();               // launched as a dependent: global memory is touched from here on
     griddep_launch_dependents();
     constexpr int D = 32, NT = 96;
-    using SM = RecRolesSmem<TC>;
+    using SM = RecRolesSmem<TC, OUT>;
     using Stage = typename SM::Stage;
     const int nslots = SLOTS == 4 ? 4 : blockDim.x / NT;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -48,12 +62,17 @@ __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const Re
     float* ring = smem + SM::kStages * Stage::kFloats;
     float* mail = ring + 2 * SM::kRing;
     StageTable* tb = reinterpret_cast<StageTable*>(mail + 2 * SM::kMail);
-    if (stid == 0) {                // tile order of RecBwdStage: q, k, v, v_old, od, gy
+    if (stid == 0) {                // tile order: q, k, v, v_old, od, gy, (y)
         stage_table_set(tb, 0, p.q, n, h);
         stage_table_set(tb, 1, p.k, n, h);
         stage_table_set(tb, 2, p.v, n, h);
         stage_table_set(tb, 3, p.v_old, n, h);
-        stage_table_set(tb, 4, p.od, n, h);
+        if constexpr (OUT) {
+            stage_table_set_lagging(tb, 4, p.out, p.start, n, h);
+            stage_table_set(tb, 6, p.out, n, h);
+        } else {
+            stage_table_set(tb, 4, p.od, n, h);
+        }
         stage_table_set(tb, 5, p.gy, n, h);
         stage_table_set_col(tb, 0, p.beta, n, h);
     }
@@ -63,7 +82,7 @@ __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const Re
     auto issue = [&](int j) {
         const int c = nchunks - 1 - j;
         const int t0 = c * TC, nt = min(TC, p.L - t0);
-        stage_table_issue<TC, NT>(smem + (j % SM::kStages) * Stage::kFloats, tb, 6, 1, t0, nt, stid);
+        stage_table_issue<TC, NT>(smem + (j % SM::kStages) * Stage::kFloats, tb, Stage::kTiles, 1, t0, nt, stid);
     };
     // top of the loop that every warp runs
     auto advance = [&](int j) {
@@ -122,14 +141,14 @@ __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const Re
             const int nt = min(TC, p.L - (nchunks - j) * TC);
             float* rg = ring + ((j - 1) & 1) * SM::kRing;
             f2 w[8];
-            float beta, qe, ke;
+            float nbeta, nqe, nke;
             auto rewind = [&](int t, float live) {      // S_{t-1} = S_t - beta k (x) w; what step t does not wait for
-                beta = s.b.f[t];
-                qe = s.q.f[t * D + own];
-                ke = s.k.f[t * D + own];
+                nbeta = s.b.f[t];
+                nqe = s.q.f[t * D + own];
+                nke = s.k.f[t * D + own];
                 lds_slice<16>(w, s.v.f + t * D + 16 * half);
-                const float nb = -beta * live;
-                const f2 k0 = f2_dup(nb * ke), k1 = f2_dup(nb * s.k.f[t * D + other]);
+                const float nb = -nbeta * live;
+                const f2 k0 = f2_dup(nb * nke), k1 = f2_dup(nb * s.k.f[t * D + other]);
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
                     S[i] = ffma2(w[i], k0, S[i]);
@@ -140,6 +159,7 @@ __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const Re
 #pragma unroll 1
             for (int t = nt - 1; t >= 0; t--) {
                 float* e = rg + t * SM::kStep;
+                const float beta = nbeta, qe = nqe, ke = nke;
                 const float* mb = mail + (t & 1) * SM::kMail;
                 const float gcol = s.gy.f[t * D + own] + gh, hte = s.od.f[t * D + own];
                 await(posted);
@@ -155,10 +175,16 @@ __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const Re
                 f2 a = 0ull, b = 0ull, c = 0ull, d = 0ull;
                 dots(S, x, a, b);
                 dots(S, y, c, d);
+                float pq = 0.f;
                 {
                     f2 z[8];
                     lds_slice<16>(z, s.vo.f + t * D + 16 * half);
                     vdv = dot(z, y);
+                    if constexpr (OUT) {                // q . dq = y . g
+                        lds_slice<16>(z, s.y + t * D + 16 * half);
+                        pq = dot(z, x);
+                        pq += swap_halves(pq);
+                    }
                 }
                 const float sg = f2_hsum(a) + swap_halves(f2_hsum(b));
                 const float sdv = f2_hsum(c) + swap_halves(f2_hsum(d));
@@ -168,11 +194,10 @@ __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const Re
                 const float ug = beta * wg;
                 const float dq = fmaf(ke, ug, sg), dk = fmaf(qe, ug, gu) - sdv;
                 const float dbh = wdv * (1.f - beta);
-                float pq = qe * dq;
-#pragma unroll
-                for (int o = 16; o >= 1; o >>= 1) pq += __shfl_xor_sync(0xffffffffu, pq, o);
+                if constexpr (!OUT) pq = warp_sum_idx<1>(qe * dq);
                 a = b = 0ull;
-                dots(Rv, y, a, b);                      // beside the reduction: the part of the feedback that needs dv only
+                dots(Rv, y, a, b);                      // beside the sums: the part of the feedback that needs dv only, and
+                rewind(t > 0 ? t - 1 : 0, t > 0 ? 1.f : 0.f);       // the next step's state (at t = 0 nothing is subtracted: no branch)
                 const float dqh = qe * (dq - pq), dkh = ke * (dk - (wdv - vdv));
                 e[2 * D + own] = dqh;
                 e[3 * D + own] = dkh;
@@ -184,7 +209,6 @@ __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const Re
                 dots(Rq, x, a, b);
                 dots(Rk, y, c, d);
                 gh = (1.f - hte * hte) * (fmaf(rbl, dbh, f2_hsum(fadd2(a, c))) + swap_halves(f2_hsum(fadd2(b, d))));
-                rewind(t > 0 ? t - 1 : 0, t > 0 ? 1.f : 0.f);       // at t = 0 repeated with nothing to subtract: no branch
             }
         }
 #pragma unroll
@@ -270,7 +294,10 @@ __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const Re
             Stage s; s.bind(smem + (j % SM::kStages) * Stage::kFloats);
             const int nt = min(TC, p.L - (nchunks - 1 - j) * TC);
 #pragma unroll 4
-            for (int t = 0; t < nt; t++) s.v.f[t * D + lane] -= s.vo.f[t * D + lane];
+            for (int t = 0; t < nt; t++) {
+                s.v.f[t * D + lane] -= s.vo.f[t * D + lane];
+                if constexpr (OUT) s.od.f[t * D + lane] = tanh_fast(s.od.f[t * D + lane]);      // as the forward took it
+            }
         }
         if (j < 2) continue;
         Stage s; s.bind(smem + ((j - 2) % SM::kStages) * Stage::kFloats);

@@ -144,6 +144,7 @@ __global__ void __launch_bounds__(D * SPLIT * slots_for(D * SPLIT)) rnn_fwd_kern
 // ------------------------------------------------------------------ backward
 struct RnnBwdParams {
     Row4 k, v, beta, v_old, gy, out, od, gz, gk, gv, gb;
+    Row4 start;             // v1 where od is not given: the vector before the first output
     float* W; long long wN, wH, wE;
     int H, L, D;
 };
@@ -356,7 +357,7 @@ template <bool V1>
 static int rnn_backward(int N, int H, int L, int D,
                         const fwp_tensor* K, const fwp_tensor* V, const fwp_tensor* beta,
                         const fwp_tensor* v_old, const fwp_tensor* grad_out,
-                        const fwp_tensor* out, const fwp_tensor* out_delayed,
+                        const fwp_tensor* out, const fwp_tensor* out_delayed, const fwp_tensor* start,
                         const fwp_tensor* fw_mem,
                         const fwp_tensor* grad_Z, const fwp_tensor* grad_K,
                         const fwp_tensor* grad_V, const fwp_tensor* grad_beta,
@@ -368,7 +369,7 @@ static int rnn_backward(int N, int H, int L, int D,
     int rc;
     if ((rc = check_tensor(K, 4, true)) || (rc = check_tensor(V, 4, true)) || (rc = check_tensor(beta, 4, true)) ||
         (rc = check_tensor(v_old, 4, true)) || (rc = check_tensor(grad_out, 4, true)) ||
-        (rc = check_tensor(out, 4, V1)) || (rc = check_tensor(out_delayed, 4, true)) ||
+        (rc = check_tensor(out, 4, V1)) || (rc = check_tensor(out_delayed, 4, !start)) || (rc = check_tensor(start, 4, false)) ||
         (rc = check_tensor(fw_mem, 4, true)) || (rc = check_tensor(grad_Z, 4, true)) ||
         (rc = check_tensor(grad_K, 4, true)) || (rc = check_tensor(grad_V, 4, true)) ||
         (rc = check_tensor(grad_beta, 4, true)))
@@ -377,11 +378,12 @@ static int rnn_backward(int N, int H, int L, int D,
     if (guard.status) return guard.status;
     RnnBwdParams p;
     p.k = row4(K); p.v = row4(V); p.beta = row4(beta); p.v_old = row4(v_old); p.gy = row4(grad_out);
-    p.out = row4(out); p.od = row4(out_delayed);
+    p.out = row4(out); p.od = row4(out_delayed); p.start = row4(start);
     p.gz = row4(grad_Z); p.gk = row4(grad_K); p.gv = row4(grad_V); p.gb = row4(grad_beta);
     p.W = (float*)fw_mem->data; p.wN = fw_mem->stride[0]; p.wH = fw_mem->stride[1]; p.wE = fw_mem->stride[2];
     p.H = H; p.L = L; p.D = D;
     cudaStream_t st = (cudaStream_t)stream;
+    if (!out_delayed && DP != 32) return FWP_ERR_UNSUPPORTED;
     switch (DP) {
         case 16: return launch_rnn_bwd<16, 2, 16, V1>(p, N * H, st);
         case 32: {
@@ -389,10 +391,11 @@ static int rnn_backward(int N, int H, int L, int D,
             // the role kernel wants full rows; rows at odd offsets (the layers' slices) go word by word, which a short call
             // does not earn back
             const bool aligned = rows_16B_aligned(p.k) && rows_16B_aligned(p.v) && rows_16B_aligned(p.gy) && rows_16B_aligned(p.v_old) &&
-                                 rows_16B_aligned(p.od) && (!V1 || rows_16B_aligned(p.out));
+                                 (!out_delayed || rows_16B_aligned(p.od)) && (!V1 || rows_16B_aligned(p.out));
             if (p.D != 32 || (!aligned && p.L < 64)) roles = 0;
             if (roles == 1) return launch_rnn_bwd_roles32<8, V1>(p, N * H, st);
             if (roles == 2) return launch_rnn_bwd_roles32<4, V1>(p, N * H, st);
+            if (!out_delayed) return FWP_ERR_UNSUPPORTED;
             const int sp = tune_get(T_RNN_BWD_SPLIT32, 1);
             // measured (512 sequences x 512 steps): 1 -> 0.34 ms, 2 -> 0.39 ms, 4 -> 0.42 ms
             if (sp == 2) return launch_rnn_bwd<32, 2, 8, V1>(p, N * H, st);
@@ -425,7 +428,8 @@ FWP_API int fwp_fast_rnn_v2_backward(int N, int H, int L, int D,
                                      const fwp_tensor* grad_Z, const fwp_tensor* grad_K,
                                      const fwp_tensor* grad_V, const fwp_tensor* grad_beta,
                                      int io_dtype, void* stream, int device) {
-    return rnn_backward<false>(N, H, L, D, K, V, beta, v_old, grad_out, out, out_delayed, fw_mem,
+    if (!out_delayed) return FWP_ERR_NULL;
+    return rnn_backward<false>(N, H, L, D, K, V, beta, v_old, grad_out, out, out_delayed, nullptr, fw_mem,
                                grad_Z, grad_K, grad_V, grad_beta, io_dtype, stream, device);
 }
 
@@ -446,6 +450,20 @@ FWP_API int fwp_fast_rnn_backward(int N, int H, int L, int D,
                                   const fwp_tensor* grad_Z, const fwp_tensor* grad_K,
                                   const fwp_tensor* grad_V, const fwp_tensor* grad_beta,
                                   int io_dtype, void* stream, int device) {
-    return rnn_backward<true>(N, H, L, D, K, V, beta, v_old, grad_out, out, out_delayed, fw_mem,
+    if (!out_delayed) return FWP_ERR_NULL;
+    return rnn_backward<true>(N, H, L, D, K, V, beta, v_old, grad_out, out, out_delayed, nullptr, fw_mem,
+                              grad_Z, grad_K, grad_V, grad_beta, io_dtype, stream, device);
+}
+
+FWP_API int fwp_fast_rnn_backward_from_outputs(int N, int H, int L, int D,
+                                  const fwp_tensor* K, const fwp_tensor* V, const fwp_tensor* beta,
+                                  const fwp_tensor* v_old, const fwp_tensor* grad_out,
+                                  const fwp_tensor* out, const fwp_tensor* start,
+                                  const fwp_tensor* fw_mem,
+                                  const fwp_tensor* grad_Z, const fwp_tensor* grad_K,
+                                  const fwp_tensor* grad_V, const fwp_tensor* grad_beta,
+                                  int io_dtype, void* stream, int device) {
+    if (!start || !start->data) return FWP_ERR_NULL;
+    return rnn_backward<true>(N, H, L, D, K, V, beta, v_old, grad_out, out, nullptr, start, fw_mem,
                               grad_Z, grad_K, grad_V, grad_beta, io_dtype, stream, device);
 }

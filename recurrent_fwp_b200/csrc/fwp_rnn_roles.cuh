@@ -52,7 +52,8 @@ __global__ void __launch_bounds__(256, 1) rnn_bwd_roles32_kernel(const RnnBwdPar
         stage_table_set(tb, 1, p.v, n, h);
         stage_table_set(tb, 2, p.gy, n, h);
         stage_table_set(tb, 3, p.v_old, n, h);
-        stage_table_set(tb, 4, p.od, n, h);
+        if (V1 && !p.od.p) stage_table_set_lagging(tb, 4, p.out, p.start, n, h);
+        else stage_table_set(tb, 4, p.od, n, h);
         if (V1) stage_table_set(tb, 5, p.out, n, h);
         stage_table_set_col(tb, 0, p.beta, n, h);
     }
