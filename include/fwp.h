@@ -104,7 +104,8 @@ unsigned long long fwp_launch_count(void);
  * in the forward only, or not at all),
  * "delta.wy" (-1 automatic / 1 / 0: the chunkwise split-product plan wherever it is the faster one, wherever it has an
  * instance, or never), "delta.wy.helpers" (0 automatic / 4 / 2: preparing warps per sequence of that plan),
- * "delta_bwd.phases" (-1 automatic / 1 / 0: the three-launch backward over scratch, see below).  Returns 0 if accepted, FWP_ERR_UNSUPPORTED for an unknown key. */
+ * "delta_bwd.phases" (-1 automatic / 1 / 0: the three-launch backward over scratch, see below), "delta_bwd.32.tile" (1 / 0: the
+ * fp32 backward at E = M = 32 step by step over four warps a sequence, or the four-step blocked kernel).  Returns 0 if accepted, FWP_ERR_UNSUPPORTED for an unknown key. */
 int fwp_tune(const char* key, int value);
 /* Name of the kernel this host thread launched last through the library ("" before the
  * first launch): lets a benchmark label its numbers with the plan the dispatch picked. */

@@ -68,6 +68,7 @@ enum TuneKey {
     T_DELTA_WY,             // "delta.wy": -1 automatic, 1 / 0 the chunkwise split-product plan (fwp_delta_wy.cuh) wherever it has an instance, or never
     T_DELTA_WY_HELPERS,     // "delta.wy.helpers": preparing warps per sequence of that plan (2 or 4), 0 automatic
     T_DELTA_PHASES,         // "delta_bwd.phases": -1 automatic, 1 / 0 the three-launch backward wherever it has an instance and scratch, or never
+    T_DELTA_BWD_TILE32,     // "delta_bwd.32.tile": 1 the backward at E = M = 32 (fp32) step by step over four warps, 0 the blocked kernel
     T_COUNT
 };
 int tune_get(TuneKey key, int fallback);

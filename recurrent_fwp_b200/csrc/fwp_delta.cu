@@ -586,15 +586,15 @@ static int dispatch_fwd(const DeltaFwdParams& p, int nseq, cudaStream_t st) {
 // Where the three-launch backward is the faster one, from measurements on B200 (fp32, 256 steps, us, one-launch kernel ->
 // three launches):
 //   d = 16: 16 sequences 37 -> 13, 128 37 -> 25, 256 38 -> 37, 512 38 -> 65; with rows of 12 128 65 -> 27, 256 66 -> 52, 512 67 -> 76
-//   d = 32: 128 63 -> 48, 256 64 -> 92; with rows of 20 128 139 -> 51, 512 283 -> 174
+//   d = 32 with rows of 20: 128 139 -> 51, 512 283 -> 174.  Rows of 32 (training pass, one launch over four warps a sequence -> three launches):
+//           16 sequences x 64 27 -> 29, x 128 41 -> 35, x 256 71 -> 49, x 1024 248 -> 183; 64 x 128 43 -> 46, x 256 74 -> 68,
+//           x 1024 250 -> 233; 96 x 256 74 -> 76, x 1024 253 -> 269; 128 x 256 74 -> 85
 //   d = 64: 64 114 -> 76, 128 116 -> 125; with rows of 55 512 1789 -> 557;  d = 48: 512 1128 -> 354
 //   E, M = 96, 32: 128 951 -> 120, 1024 2777 -> 930;  128, 128: 128 2826 -> 676
 // and by length (time of the one-launch kernel over that of the three): d = 16, 80 sequences: 0.9 at 24 steps, 1.1 at 40, 1.8 at 250;
-//   d = 32: 80 0.7 (24), 0.9 (40), 1.2 (64), 1.4 (500), 144 0.9 (100), 1.1 (250), 304 (a second wave of the blocked kernel, which
-//   holds two sequences per SM) 1.1 (40), 1.2 (100), 400 0.9;
 //   d = 64: 80 0.8 (24), 1.2 (40), 1.6 (64); from there on against the blocked kernel (one per SM) 1.0, 144 0.8, 160 1.3, 208 1.0;
 //   rows of 55: 736 0.8 up to 64 steps, then 2.1;  304 1.1 (24), 1.5, 3.3
-// The four-step blocked kernels are at their best with rows of exactly 16, 32 or 64 elements and a sequence for every SM;
+// The four-step blocked kernels are at their best with rows of exactly 16 or 64 elements and a sequence for every SM;
 // short rows cost them a division per copied piece, and states above 64 have no register-resident kernel at all.
 // bf16 streams (1024 steps) need a third of the operand parts:
 //   d = 16: 16 sequences 187 -> 37, 128 189 -> 102, 288 190 -> 188, 512 191 -> 270; with rows of 12 (256 steps) 512 166 -> 75
@@ -618,10 +618,7 @@ static bool bwd_phases_pay(const DeltaBwdParams& p, int nseq, int io_dtype) {
     }
     if (p.L <= 2 * kShortSeq) return false;
     if (d == 16) return nseq <= sms;
-    if (d == 32) {
-        if (nseq > 2 * sms) return wave_fill(nseq, 2) < 0.6f && nseq <= 4 * sms;
-        return nseq <= sms && p.L >= (nseq <= sms * 3 / 4 ? 4 : 10) * kShortSeq;
-    }
+    if (d == 32) return nseq <= sms / 2 && p.L >= (nseq <= sms / 4 ? 6 : 12) * kShortSeq;
     if (p.L <= 3 * kShortSeq) return nseq <= sms * 3 / 4;
     if (p.L <= 4 * kShortSeq) return nseq <= 3 * sms;
     return nseq <= sms / 2 || (nseq > sms && nseq <= sms * 5 / 4);
@@ -644,8 +641,11 @@ static int dispatch_bwd(const DeltaBwdParams& p0, int nseq, cudaStream_t st) {
             return launch_bwd<16, 2, 32, float, 1>(p, nseq, st);
         }
         case 32: {
-            // fp32 streams: blocked 138 us vs per-step 175 us; bf16 streams: per-step 201 us vs blocked 207 us
+            // fp32 streams, 256 steps of 128 / 512 / 1536 sequences: step by step over four warps 46 / 93 / 271 us, four-step blocked 66 /
+            // 136 / 380 us (which serves rows shorter than 32 where there is no scratch for the three launches); bf16 streams: per-step
+            // 201 us vs blocked 207 us
             if constexpr (sizeof(T) == 4) {
+                if (force == -1 && p.L > kShortSeq && p.E == 32 && p.M == 32 && tune_get(T_DELTA_BWD_TILE32, 1)) return launch_bwd_tile32(p, nseq, st);
                 if (force == 1 || (force == -1 && p.L > kShortSeq))
                     return tune_get(T_DELTA_BWD_SPLIT32, 2) == 4 ? launch_bwd<32, 4, 8, T>(p, nseq, st) : launch_bwd<32, 2, 8, T>(p, nseq, st);
             }

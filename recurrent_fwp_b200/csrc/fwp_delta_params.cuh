@@ -37,6 +37,8 @@ template <typename T, bool SUM> int launch_fwd_wy(const DeltaFwdParams& p, int n
 // three-launch backward over a workspace (fwp_delta_phases.cuh): floats of scratch it needs (run = false) or the launches; -1
 // when the sizes have no instance
 template <typename T> int64_t bwd_phases(bool run, const DeltaBwdParams& p, int nseq, float* scratch, cudaStream_t st);
+// step by step over four warps a sequence, E = M = 32, fp32 streams (fwp_delta_tile.cuh)
+int launch_bwd_tile32(const DeltaBwdParams& p, int nseq, cudaStream_t st);
 int tc_fault_read_clear();
 int launch_wait_probe(int polls, cudaStream_t st);
 // the sum rule's backward as three forwards of the plan above; -1 when the sizes have no instance
