@@ -244,7 +244,8 @@ __global__ void __launch_bounds__(WARPS * 32) delta_bwd_prepare_kernel(const __g
     };
     float bt[2][2];
     load_beta(bt, stream_at<T>(p.beta, n, h) + t0 * p.beta.sL, p.beta.sL, nt, t);
-    constexpr bool kAhead = KS <= 4;
+    constexpr bool kAhead = KS <= 4, kRolled = KS > 4;    // loops over the blocks of a large state stay rolled: instruction fetch
+    constexpr int kUnroll = kRolled ? 1 : KS;
     if (kAhead) streams(0);
     if (g == 0) {
 #pragma unroll
@@ -256,7 +257,7 @@ __global__ void __launch_bounds__(WARPS * 32) delta_bwd_prepare_kernel(const __g
         const T* qp = stream_at<T>(p.q, n, h) + (t0 + g) * p.q.sL + 2 * t;
         auto even = [&](const T* q, long long sL) { return p.E == E && (reinterpret_cast<uintptr_t>(q) & (2 * sizeof(T) - 1)) == 0 && (sL & 1) == 0; };
         const bool kpair = even(kp, p.k.sL), qpair = even(qp, p.q.sL);
-        constexpr int AHEAD = KS < 2 ? KS : 2;
+        constexpr int AHEAD = KS < 2 ? KS : kRolled ? 1 : 2;
         float x[AHEAD][2][4], y[AHEAD][2][4];
         auto fetch = [&](int k) {
             load_block<T>(x[k % AHEAD], kp + 16 * k, p.k.sL, nt, p.E - 16 * k, kpair, g, t);
@@ -264,7 +265,11 @@ __global__ void __launch_bounds__(WARPS * 32) delta_bwd_prepare_kernel(const __g
         };
 #pragma unroll
         for (int k = 0; k < AHEAD; k++) fetch(k);
-#pragma unroll
+        if (kRolled) {
+            zero(kk);
+            zero(z);
+        }
+#pragma unroll kUnroll
         for (int k = 0; k < KS; k++) {
             Frag<NP> fk, fq;
             from_c(fk, x[k % AHEAD][0], x[k % AHEAD][1]);
@@ -272,8 +277,8 @@ __global__ void __launch_bounds__(WARPS * 32) delta_bwd_prepare_kernel(const __g
             if (k + AHEAD < KS) fetch(k + AHEAD);
             store(aK + 32 * k, kPart, fk);
             store(aQ + 32 * k, kPart, fq);
-            sum_product<BY_ROWS>(k, kk, fk, fk);
-            sum_product<BY_ROWS>(k, z, fk, fq);
+            sum_product<BY_ROWS>(kRolled ? 1 : k, kk, fk, fk);
+            sum_product<BY_ROWS>(kRolled ? 1 : k, z, fk, fq);
         }
     }
 #pragma unroll
@@ -297,7 +302,7 @@ __global__ void __launch_bounds__(WARPS * 32) delta_bwd_prepare_kernel(const __g
         product<BY_COLS>(x, ta, by_cols(fz));           // T' triu(K Q^T)
         from_c(tz, x[0], x[1]);
     }
-#pragma unroll
+#pragma unroll kUnroll
     for (int k = 0; k < KS; k++) {
         Frag<NP> r;
         Frag<3> f;
@@ -323,7 +328,7 @@ __global__ void __launch_bounds__(WARPS * 32) delta_bwd_prepare_kernel(const __g
         if (j + 1 < MS) streams(j + 1);
         product<BY_ROWS>(x, fy, tz);                    // Tv^T = gY^T (T' Z)^T
         put_block(ws + Sp::R + j * 64, x, lane);
-#pragma unroll
+#pragma unroll kUnroll
         for (int k = 0; k < KS; k++) {
             Frag<NP> r;
             load_cols(r, aQ + 32 * k, kPart);
