@@ -868,7 +868,8 @@ FWP_API int fwp_debug_bounded_wait_probe(int polls, void* stream, int device) {
 // (the affected launch produced wrong numbers instead of hanging), 0 if not, -1 on a CUDA error.
 // Synchronises the device; reading clears the flag.
 FWP_API int fwp_delta_device_fault(void) {
-    const int v = fwp::flag_read_clear(fwp::g_delta_fault), t = fwp::tc_fault_read_clear(), w = fwp::wy_fault_read_clear(), u = fwp::sum_wy_fault_read_clear();
-    if (v < 0 || t < 0 || w < 0 || u < 0) return -1;
-    return (v || t || w || u) ? 1 : 0;
+    const int v = fwp::flag_read_clear(fwp::g_delta_fault), t = fwp::tc_fault_read_clear(), w = fwp::wy_fault_read_clear(), f = fwp::wy_few_fault_read_clear(),
+              u = fwp::sum_wy_fault_read_clear();
+    if (v < 0 || t < 0 || w < 0 || f < 0 || u < 0) return -1;
+    return (v || t || w || f || u) ? 1 : 0;
 }

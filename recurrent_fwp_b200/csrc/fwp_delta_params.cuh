@@ -32,7 +32,10 @@ bool chunk_bf16_applies(const DeltaBwdParams& p);
 int launch_bwd_chunk_bf16(const DeltaBwdParams& p, int nseq, cudaStream_t st);
 // chunkwise plan on split fp32 products (fwp_delta_wy.cuh); -1 when the sizes have no instance
 int wy_fault_read_clear();
+int wy_few_fault_read_clear();
 int sum_wy_fault_read_clear();
+// its form for few sequences, fp32; -1 where the other is the better one or has the only instance
+template <bool SUM> int launch_fwd_wy_few(const DeltaFwdParams& p, int nseq, cudaStream_t st);
 template <typename T, bool SUM> int launch_fwd_wy(const DeltaFwdParams& p, int nseq, cudaStream_t st);
 // three-launch backward over a workspace (fwp_delta_phases.cuh): floats of scratch it needs (run = false) or the launches; -1
 // when the sizes have no instance

@@ -11,11 +11,6 @@ static int run_fwd(const DeltaFwdParams& p, int nseq, cudaStream_t st) {
     return launch_dependent(wy::delta_fwd_wy_kernel<E, M, NB, CTAS, T, SUM>, p, nseq, (M / 16 + NB) * 32,
                             NB * sizeof(wy::FwdBuf<E, wy::stream_parts<T>()>), st, "delta_fwd_wy_kernel");
 }
-template <int E, int M, int NB, typename T, bool SUM>
-static int run_fwd_few(const DeltaFwdParams& p, int nseq, cudaStream_t st) {
-    return launch_dependent(wy::delta_fwd_wy_few_kernel<E, M, NB, T, SUM>, p, nseq, (M / 16 + NB) * 32,
-                            NB * sizeof(wy::FewBuf<E, M, wy::stream_parts<T>()>), st, "delta_fwd_wy_few_kernel");
-}
 // How many preparing warps a sequence gets and how many sequences an SM holds.  With no more sequences than SMs
 // (FEW_CTAS = 1; two per SM where registers and shared memory allow it without spilling) four warps keep a chain
 // supplied; with more, shared latency replaces them and residency counts.
@@ -30,16 +25,11 @@ static int pick_fwd(const DeltaFwdParams& p, int nseq, cudaStream_t st) {
 template <typename T, bool SUM>
 int launch_fwd_wy(const DeltaFwdParams& p, int nseq, cudaStream_t st) {
     const int d = p.E > p.M ? p.E : p.M;
+    if constexpr (sizeof(T) == 4) {
+        const int rc = launch_fwd_wy_few<SUM>(p, nseq, st);
+        if (rc >= 0) return rc;
+    }
     if (d <= 16) {
-        // at d = 16 a chain waits more than it works: up to two sequences per SM the form with the short chain wins once
-        // its longer start (about 5 us) is paid for: 11.6 against 14.5 us at 16 sequences of 256 steps, 7.7 against 3.9 at 20 steps.
-        // Rows shorter than 16 cost its staging copies a loop per row: 20.6 us, where the other form takes 17
-        if constexpr (sizeof(T) == 4) {
-            const int force = tune_get(T_DELTA_WY_HELPERS, 0);
-            const bool few = force ? force == 4 : p.E == 16 && p.M == 16 && p.L >= 7 * wy::C;
-            if (few && nseq <= sm_count()) return run_fwd_few<16, 16, 6, T, SUM>(p, nseq, st);
-            if (few && (force || nseq <= 2 * sm_count())) return run_fwd_few<16, 16, 4, T, SUM>(p, nseq, st);
-        }
         return run_fwd<16, 16, 2, 5, T, SUM>(p, nseq, st);
     }
     if (d <= 32) return pick_fwd<32, 32, 2, 2, 4, T, SUM>(p, nseq, st);

@@ -61,43 +61,44 @@ struct Stream {
     const T* at;            // this lane's first element of row 0 of a sweep
     long long sL;
     int width, off;         // off: that element's place in the tile
-    bool vec;
+    bool vec, full;         // 16-byte pieces; whole rows of W elements
     static constexpr int PPR = W / 4, RS = PPR <= 32 ? 32 / PPR : 1;                // 16-byte pieces per row, rows per sweep
-    static constexpr int RS1 = W < 32 ? 32 / W : 1, CS1 = W < 32 ? 1 : W / 32;      // 4-byte copies: rows and columns per sweep
-    static constexpr bool kVec = PPR <= 32 && 32 % PPR == 0, kWord = W < 32 ? 32 % W == 0 : W % 32 == 0;
+    static constexpr int CS1 = (W + 31) / 32;                                       // 4-byte copies: column groups
+    static constexpr bool kVec = PPR <= 32 && 32 % PPR == 0;
     __device__ __forceinline__ void init(const Row4& r, int n, int h, int w, int lane) {
-        Src<T> s;
-        s.init(r, n, h, w);
-        base = s.base;
-        sL = s.sL;
+        base = reinterpret_cast<const T*>(r.p) + n * r.sN + h * r.sH;
+        sL = r.sL;
         width = w;
-        vec = kVec && s.vec && w == W;
-        at = base + (vec ? (lane / PPR) * sL + (lane % PPR) * 4 : W < 32 ? (lane / W) * sL + lane % W : lane);
-        off = vec ? (lane / PPR) * P + (lane % PPR) * 4 : W < 32 ? (lane / W) * P + lane % W : lane;
+        vec = sizeof(T) == 4 && (reinterpret_cast<uintptr_t>(base) & 15) == 0 && sL % 4 == 0 && w % 4 == 0;
+        full = kVec && w == W;
+        at = base + (vec ? (full ? (lane / PPR) * sL + (lane % PPR) * 4 : 4 * lane) : lane);
+        off = vec ? (full ? (lane / PPR) * P + (lane % PPR) * 4 : 4 * lane) : lane;
     }
     // rows past the end are zeroed
     __device__ __forceinline__ void copy(float* tile, int t0, int nt, int lane) const {
         if (nt < C)
             for (int i = lane; i < (C - nt) * P; i += 32) tile[nt * P + i] = 0.f;
         if constexpr (sizeof(T) == 4) {
-            if (nt == C && vec) {
-                const T* g = at + t0 * sL;
+            const T* g = at + t0 * sL;
+            tile += off;
+            if (vec && full && nt == C) {
 #pragma unroll
-                for (int r = 0; r < C; r += RS, g += RS * sL) cp_async16(tile + off + r * P, g);
-                return;
-            }
-            if (kWord && nt == C && width == W) {
-                const T* g = at + t0 * sL;
-#pragma unroll
-                for (int r = 0; r < C; r += RS1, g += RS1 * sL)
-#pragma unroll
-                    for (int c = 0; c < CS1; c++) cp_async4(tile + off + r * P + 32 * c, g + 32 * c);
-                return;
-            }
-            const T* g = base + t0 * sL;
+                for (int r = 0; r < C; r += RS, g += RS * sL) cp_async16(tile + r * P, g);
+            } else if (vec && !full) {                  // a row at a time
+                if (4 * lane < width)
 #pragma unroll 4
-            for (int r = 0; r < nt; r++, g += sL)
-                for (int c = lane; c < width; c += 32) cp_async4(tile + r * P + c, g + c);
+                    for (int r = 0; r < nt; r++, g += sL) cp_async16(tile + r * P, g);
+            } else {
+                g = base + lane + t0 * sL;
+                tile += lane - off;
+#pragma unroll
+                for (int c = 0; c < CS1; c++)
+                    if (lane + 32 * c < width) {
+                        const T* gc = g + 32 * c;
+#pragma unroll 4
+                        for (int r = 0; r < nt; r++, gc += sL) cp_async4(tile + r * P + 32 * c, gc);
+                    }
+            }
         } else {
             const T* g = base + t0 * sL;
 #pragma unroll 4
@@ -350,7 +351,8 @@ __device__ __forceinline__ void fwd_few(const DeltaFwdParams& p) {
         return;
     }
 
-    // ---- helper: chunks b, b + NB, ...
+    // ---- helper: chunks b, b + NB, ...  Its loops over blocks stay rolled: with as many helpers as chunks in flight, each in a place of
+    // its own, instruction fetch was the largest stall (E, M = 96, 32, 128 x 256: 72 us unrolled, 50 rolled)
     const int b = warp - NCW;
     Buf& buf = bufs[b];
     Stream<E, PR, T> sk, sq;
@@ -381,7 +383,7 @@ __device__ __forceinline__ void fwd_few(const DeltaFwdParams& p) {
         cp_async_wait<0>();
         __syncwarp();
         float kk[2][4] = {}, qk[2][4] = {};
-#pragma unroll
+#pragma unroll 1
         for (int k = 0; k < KS; k++) {
             Frag<NP> fk, fq;
             float x[2][4];
@@ -391,8 +393,8 @@ __device__ __forceinline__ void fwd_few(const DeltaFwdParams& p) {
             tile_block<PR>(x, &buf.qraw[g][2 * t + 16 * k]);
             from_c(fq, x[0], x[1]);
             store(aQ + 32 * k, kPart, fq);
-            if (!SUM) sum_product<BY_ROWS>(k, kk, fk, fk);
-            sum_product<BY_ROWS>(k, qk, fq, fk);
+            if (!SUM) add_product<BY_ROWS>(kk, fk, fk);
+            add_product<BY_ROWS>(qk, fq, fk);
         }
 #pragma unroll
         for (int nn = 0; nn < 2; nn++) {
@@ -430,7 +432,7 @@ __device__ __forceinline__ void fwd_few(const DeltaFwdParams& p) {
                 ta.r[i][2] = tt.r[i][1];
                 ta.r[i][3] = tt.r[i][3];
             }
-#pragma unroll
+#pragma unroll 1
             for (int k = 0; k < KS; k++) {            // X = T K
                 Frag<NP> r;
                 float x[2][4] = {};
@@ -440,7 +442,7 @@ __device__ __forceinline__ void fwd_few(const DeltaFwdParams& p) {
                 store(aX + 32 * k, kPart, f);
             }
         }
-#pragma unroll
+#pragma unroll 1
         for (int j = 0; j < NCW; j++) {               // (T V)^T = V^T T^T
             float x[2][4];
             tile_block_t<PV>(x, &buf.v[st][2 * t][16 * j + g]);
@@ -459,7 +461,7 @@ __device__ __forceinline__ void fwd_few(const DeltaFwdParams& p) {
         Frag<3> ra;
         load_rows(ra, aA, kPartC);
         wait(&done[b], phase);
-#pragma unroll
+#pragma unroll 1
         for (int j = 0; j < NCW; j++) {
             float y[2][4], w[2][4], u[2][4];
             Frag<3> us;
@@ -475,7 +477,7 @@ __device__ __forceinline__ void fwd_few(const DeltaFwdParams& p) {
 #pragma unroll
             for (int i = 0; i < 8; i++) y[i >> 2][i & 3] = 0.f;
             product<BY_ROWS>(y, us, ra);
-#pragma unroll
+#pragma unroll 1
             for (int k = 0; k < KS; k++) {
                 Frag<3> s;
                 Frag<NP> r;
@@ -493,8 +495,8 @@ __device__ __forceinline__ void fwd_few(const DeltaFwdParams& p) {
     }
     slot_barrier(0, (NCW + NB) * 32);
 }
-template <int E, int M, int NB, typename T, bool SUM>
-__global__ void __launch_bounds__((M / 16 + NB) * 32, 2) delta_fwd_wy_few_kernel(const __grid_constant__ DeltaFwdParams p) {
+template <int E, int M, int NB, int CTAS, typename T, bool SUM>
+__global__ void __launch_bounds__((M / 16 + NB) * 32, CTAS) delta_fwd_wy_few_kernel(const __grid_constant__ DeltaFwdParams p) {
     fwd_few<E, M, NB, T, SUM>(p);
     if (redo()) stepwise_forward<T, SUM>(p, nullptr);
 }
