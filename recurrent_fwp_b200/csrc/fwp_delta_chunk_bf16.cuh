@@ -9,7 +9,7 @@
 //   Akk = strict_lower(K K^T), Aqk = lower(Q K^T)                          (bf16 products)
 //   [Cv | Ck] = T [V | K],  T = (I + Akk diag(b))^-1   (the unit triangular solve
 //               c_t = rhs_t - sum_{i<t} Akk[t,i] b_i c_i as an explicit inverse, see the forward kernel)
-//   w = Cv - Ck S0  (= v - v_old),  u = b w,  v_old = (V - Cv) + Ck S0
+//   w = Cv - Ck S0  (= v - v_old),  u = b w,  v_old = V - w
 //   y = Q S0 + Aqk u,   S1 = S0 + K^T u
 //
 // (the same recurrence as algorithmic/fast_weight/fast_weight_cuda.cu:107-180, regrouped).
@@ -46,9 +46,17 @@ __device__ __forceinline__ void ldsm4t(unsigned (&r)[4], const void* p) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)) : "memory");
 }
+__device__ __forceinline__ void stsm4(void* p, const unsigned (&r)[4]) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};"
+                 ::"r"(smem_u32(p)), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
+}
+__device__ __forceinline__ void stsm4t(void* p, const unsigned (&r)[4]) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};"
+                 ::"r"(smem_u32(p)), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
+}
 // d += a b, a: 16 x 16 (row), b: 16 x 8 (col), bf16 operands, fp32 accumulation.  volatile, like movm: the products stay in
 // the order of the source, which interleaves them with the loads of their operands.  Left to the compiler the forward of 4096
-// sequences x 4096 steps took 4.15 ms instead of 3.92; the backward does not care (9.08 ms either way)
+// sequences x 4096 steps took 6 % longer; the backward does not care
 __device__ __forceinline__ void mma_bf16(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
@@ -244,7 +252,7 @@ __global__ void __launch_bounds__(cb::NT, 4) delta_fwd_chunk_bf16_inv_kernel(con
         const float* bs = s.b[cur];
 
         // (1) per warp: Akk, Aqk, T; the warp's 16 columns of Ck = T K
-        unsigned th[4], tl[4], yh[4], yl[4], qk[4];     // right operands T^T, (T - I)^T (two parts each), Aqk^T
+        unsigned th[4], tl[4], qk[4];                   // right operands T^T (two parts), Aqk^T
         {
             float akk[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
             float aqk[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
@@ -327,7 +335,6 @@ __global__ void __launch_bounds__(cb::NT, 4) delta_fwd_chunk_bf16_inv_kernel(con
 #pragma unroll
                 for (int i = 0; i < 4; i++) T[j][i] = Y[j][i] + ((8 * j + 2 * t4 + (i & 1)) == (g + 8 * (i >> 1)) ? 1.f : 0.f);
             bt_of(th, tl, T);
-            bt_of(yh, yl, Y);
             unsigned ah[4], al[4], bK[4];
             split_bf16(T[0][0], T[0][1], ah[0], al[0]); split_bf16(T[0][2], T[0][3], ah[1], al[1]);
             split_bf16(T[1][0], T[1][1], ah[2], al[2]); split_bf16(T[1][2], T[1][3], ah[3], al[3]);
@@ -363,24 +370,21 @@ __global__ void __launch_bounds__(cb::NT, 4) delta_fwd_chunk_bf16_inv_kernel(con
                 mm(Yo, sa[ks], bq);
             }
             float cv[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-            float py[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-            {
-                unsigned va[4];
-                lda_trans(va, s.v[cur] + m0, LDT, lane);
-                mm(cv, va, th);
-                mm(cv, va, tl);
-                mm(py, va, yh);
-                mm(py, va, yl);
-            }
+            unsigned va[4];
+            lda_trans(va, s.v[cur] + m0, LDT, lane);
+            mm(cv, va, th);
+            mm(cv, va, tl);
             float u[2][4];
 #pragma unroll
             for (int j = 0; j < 2; j++)
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
                     const int m = m0 + g + 8 * (i >> 1), t = 8 * j + 2 * t4 + (i & 1);
-                    u[j][i] = bs[t] * (cv[j][i] - P[j][i]);
+                    const unsigned v2 = va[2 * j + (i >> 1)];
+                    const float w = cv[j][i] - P[j][i], v = __uint_as_float((i & 1) ? v2 & 0xffff0000u : v2 << 16);
+                    u[j][i] = bs[t] * w;
                     if (t < nt) {
-                        if (vob) vob[(long long)(t0 + t) * p.v_old.sL + m] = P[j][i] - py[j][i];
+                        if (vob) vob[(long long)(t0 + t) * p.v_old.sL + m] = v - w;
                         if (uib) uib[(long long)(t0 + t) * p.v_ins.sL + m] = u[j][i];
                     }
                 }
@@ -424,8 +428,8 @@ __global__ void __launch_bounds__(cb::NT, 4) delta_fwd_chunk_bf16_inv_kernel(con
 // Everything of a chunk that does not involve the state -- the Gram tiles, the inverse T, Aqk^T and Ck = T K -- is
 // the same for the four chain warps and does not wait for the previous chunk.  In the kernel above every warp
 // computes it for itself, between two CTA-wide barriers, on the critical path of the chunk.  Here a fifth warp
-// prepares it one chunk ahead (and issues all the copies): it leaves the five right-operand fragment sets
-// (T^T and (T - I)^T as two bf16 parts each, Aqk^T) in shared memory in fragment order, one 16-byte piece per lane,
+// prepares it one chunk ahead (and issues all the copies): it leaves the three right-operand fragment sets
+// (T^T as two bf16 parts, Aqk^T) in shared memory in fragment order, one 16-byte piece per lane,
 // and Ck as a row-major tile.  The chain warps wait for that package, run the state-dependent products and hand the
 // buffers back.  Two named barriers per package buffer: FULL (the preparing warp arrives, the chain warps wait) and
 // EMPTY (the chain warps arrive after their last read of the package and of the input stage, the preparing warp
@@ -437,20 +441,22 @@ constexpr int NTP = 160;                // four chain warps and the preparing wa
 
 struct SmemP {
     __nv_bfloat16 k[3][C * LDT], v[3][C * LDT], q[3][C * LDT];    // input stages
-    uint4 frag[2][5][32];               // per package: T^T hi, lo; (T - I)^T hi, lo; Aqk^T -- in fragment order
+    uint4 frag[2][3][32];               // per package: T^T hi, lo; Aqk^T -- in fragment order
     __nv_bfloat16 ck[2][C * LDT];       // per package: Ck, [t][e]
-    __nv_bfloat16 ys[2][C * LDT];       // y, [t][m]
+    __nv_bfloat16 ys[4][C * LDQ];       // per chain warp: y, [t][m of the warp]
     float b[3][C];
 };
 
-enum { BAR_FULL = 1, BAR_EMPTY = 3, BAR_CHAIN = 5 };     // FULL, EMPTY: + (chunk & 1)
+enum { BAR_FULL = 1, BAR_EMPTY = 3 };     // FULL, EMPTY: + (chunk & 1)
 
 __device__ __forceinline__ void nbar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 __device__ __forceinline__ void nbar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 
 }  // namespace cb
 
-// SAVE: v_old is asked for.  A test per store instead costs 1 % (3.96 against 3.92 ms, the kernel is at its register limit)
+// SAVE: v_old is asked for (a test per store instead costs 1 %, the kernel is at its register limit).  4096 sequences x 4096 steps:
+// 3.58 ms, against 3.91 with v_old from a product of its own with (T - I), stores of y through a tile that the four warps shared
+// behind a barrier, and an address per v_old store.  Its DRAM traffic alone takes 2.0.
 template <bool SAVE>
 __global__ void __launch_bounds__(cb::NTP, 4) delta_fwd_chunk_bf16_pipe_kernel(const DeltaFwdParams p) {
     griddep_wait();               // launched as a dependent: global memory is touched from here on
@@ -527,7 +533,7 @@ __global__ void __launch_bounds__(cb::NTP, 4) delta_fwd_chunk_bf16_pipe_kernel(c
                     aqk[j][i] = cc <= r ? aqk[j][i] : 0.f;
                     Y[j][i] = -N1[j][i];
                 }
-            unsigned th[4], tl[4], yh[4], yl[4], qk[4];
+            unsigned th[4], tl[4], qk[4];
             {
                 unsigned lo[4];
                 bt_of(qk, lo, aqk);
@@ -580,12 +586,9 @@ __global__ void __launch_bounds__(cb::NTP, 4) delta_fwd_chunk_bf16_pipe_kernel(c
 #pragma unroll
                 for (int i = 0; i < 4; i++) T[j][i] = Y[j][i] + ((8 * j + 2 * t4 + (i & 1)) == (g + 8 * (i >> 1)) ? 1.f : 0.f);
             bt_of(th, tl, T);
-            bt_of(yh, yl, Y);
             s.frag[pk][0][lane] = make_uint4(th[0], th[1], th[2], th[3]);
             s.frag[pk][1][lane] = make_uint4(tl[0], tl[1], tl[2], tl[3]);
-            s.frag[pk][2][lane] = make_uint4(yh[0], yh[1], yh[2], yh[3]);
-            s.frag[pk][3][lane] = make_uint4(yl[0], yl[1], yl[2], yl[3]);
-            s.frag[pk][4][lane] = make_uint4(qk[0], qk[1], qk[2], qk[3]);
+            s.frag[pk][2][lane] = make_uint4(qk[0], qk[1], qk[2], qk[3]);
             unsigned ah[4], al[4];
             split_bf16(T[0][0], T[0][1], ah[0], al[0]); split_bf16(T[0][2], T[0][3], ah[1], al[1]);
             split_bf16(T[1][0], T[1][1], ah[2], al[2]); split_bf16(T[1][2], T[1][3], ah[3], al[3]);
@@ -609,10 +612,11 @@ __global__ void __launch_bounds__(cb::NTP, 4) delta_fwd_chunk_bf16_pipe_kernel(c
 
     // ---------------------------------------------------------------- the chain warps
     bf16* yb = reinterpret_cast<bf16*>(p.out.p) + n * p.out.sN + h * p.out.sH;
-    float* vob = reinterpret_cast<float*>(p.v_old.p) + n * p.v_old.sN + h * p.v_old.sH;
     float* uib = p.v_ins.p ? reinterpret_cast<float*>(p.v_ins.p) + n * p.v_ins.sN + h * p.v_ins.sH : nullptr;
     float* W = p.W + n * p.wN + h * p.wH;
     const int m0 = 16 * warp;
+    float* vp = reinterpret_cast<float*>(p.v_old.p) + n * p.v_old.sN + h * p.v_old.sH + 2 * t4 * p.v_old.sL + m0 + g;     // v_old: this lane's rows and columns
+    bf16* yp = yb + (lane >> 1) * p.out.sL + m0 + 8 * (lane & 1);
     float S[8][4];
 #pragma unroll
     for (int j = 0; j < 8; j++)
@@ -626,15 +630,12 @@ __global__ void __launch_bounds__(cb::NTP, 4) delta_fwd_chunk_bf16_pipe_kernel(c
         const bf16* Qs = s.q[st];
         const float* bs = s.b[st];
         const bf16* cks = s.ck[pk];
-        unsigned th[4], tl[4], yh[4], yl[4], qk[4];
+        unsigned th[4], tl[4], qk[4];
         {
-            const uint4 f0 = s.frag[pk][0][lane], f1 = s.frag[pk][1][lane], f2 = s.frag[pk][2][lane],
-                        f3 = s.frag[pk][3][lane], f4 = s.frag[pk][4][lane];
+            const uint4 f0 = s.frag[pk][0][lane], f1 = s.frag[pk][1][lane], f2 = s.frag[pk][2][lane];
             th[0] = f0.x; th[1] = f0.y; th[2] = f0.z; th[3] = f0.w;
             tl[0] = f1.x; tl[1] = f1.y; tl[2] = f1.z; tl[3] = f1.w;
-            yh[0] = f2.x; yh[1] = f2.y; yh[2] = f2.z; yh[3] = f2.w;
-            yl[0] = f3.x; yl[1] = f3.y; yl[2] = f3.z; yl[3] = f3.w;
-            qk[0] = f4.x; qk[1] = f4.y; qk[2] = f4.z; qk[3] = f4.w;
+            qk[0] = f2.x; qk[1] = f2.y; qk[2] = f2.z; qk[3] = f2.w;
         }
         unsigned sa[4][4];
 #pragma unroll
@@ -655,27 +656,41 @@ __global__ void __launch_bounds__(cb::NTP, 4) delta_fwd_chunk_bf16_pipe_kernel(c
             mm(Yo, sa[ks], bq);
         }
         float cv[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-        float py[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-        {
-            unsigned va[4];
-            lda_trans(va, s.v[st] + m0, LDT, lane);
-            mm(cv, va, th);
-            mm(cv, va, tl);
-            mm(py, va, yh);
-            mm(py, va, yl);
-        }
-        float u[2][4];
+        unsigned va[4];                 // V^T as left operand: the same elements, lane for lane, as the products' results
+        lda_trans(va, s.v[st] + m0, LDT, lane);
+        mm(cv, va, th);
+        mm(cv, va, tl);
+        float u[2][4], vo[2][4];
 #pragma unroll
-        for (int j = 0; j < 2; j++)
+        for (int j = 0; j < 2; j++) {
+            const float2 b2 = *reinterpret_cast<const float2*>(bs + 8 * j + 2 * t4);
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                const int m = m0 + g + 8 * (i >> 1), t = 8 * j + 2 * t4 + (i & 1);
-                u[j][i] = bs[t] * (cv[j][i] - P[j][i]);
-                if (t < nt) {
-                    if (SAVE) vob[(long long)(t0 + t) * p.v_old.sL + m] = P[j][i] - py[j][i];
-                    if (uib) uib[(long long)(t0 + t) * p.v_ins.sL + m] = u[j][i];
-                }
+                const unsigned v2 = va[2 * j + (i >> 1)];
+                const float w = cv[j][i] - P[j][i], v = __uint_as_float((i & 1) ? v2 & 0xffff0000u : v2 << 16);
+                u[j][i] = ((i & 1) ? b2.y : b2.x) * w;
+                vo[j][i] = v - w;
             }
+        }
+        if (SAVE) {
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    float* q = vp + (8 * j + i) * p.v_old.sL;
+                    if (nt == C || 8 * j + 2 * t4 + i < nt) { q[0] = vo[j][i]; q[8] = vo[j][2 + i]; }
+                }
+            vp += C * p.v_old.sL;
+        }
+        if (uib) {
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int m = m0 + g + 8 * (i >> 1), t = 8 * j + 2 * t4 + (i & 1);
+                    if (t < nt) uib[(long long)(t0 + t) * p.v_ins.sL + m] = u[j][i];
+                }
+        }
         unsigned ua[4], ul[4];
         split_bf16(u[0][0], u[0][1], ua[0], ul[0]); split_bf16(u[0][2], u[0][3], ua[1], ul[1]);
         split_bf16(u[1][0], u[1][1], ua[2], ul[2]); split_bf16(u[1][2], u[1][3], ua[3], ul[3]);
@@ -690,19 +705,16 @@ __global__ void __launch_bounds__(cb::NTP, 4) delta_fwd_chunk_bf16_pipe_kernel(c
             mma_bf16(S[2 * jp + 1], ul, bk[2], bk[3]);
         }
         if (c + 2 < nchunks) nbar_arrive(BAR_EMPTY + pk, NTP);      // last read of the package and of the stage is behind us
-        bf16* ys = s.ys[pk];
-#pragma unroll
-        for (int j = 0; j < 2; j++)
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-                ys[(8 * j + 2 * t4 + (i & 1)) * LDT + m0 + g + 8 * (i >> 1)] = __float2bfloat16_rn(Yo[j][i]);
-        nbar_sync(BAR_CHAIN, NT);
-        {   // y: 16-byte row pieces
-            const int row = tid >> 3, part = (tid & 7) * 8;
-            if (row < nt)
-                *reinterpret_cast<uint4*>(yb + (long long)(t0 + row) * p.out.sL + part) =
-                    *reinterpret_cast<const uint4*>(ys + row * LDT + part);
-        }
+        // y: this warp's sixteen columns, two 16-byte pieces to a row (a whole sector)
+        bf16* ys = s.ys[warp];
+        const unsigned y4[4] = {pack_bf16(Yo[0][0], Yo[0][1]), pack_bf16(Yo[0][2], Yo[0][3]), pack_bf16(Yo[1][0], Yo[1][1]), pack_bf16(Yo[1][2], Yo[1][3])};
+        stsm4t(ys + ((lane & 7) + 8 * (lane >> 4)) * LDQ + 8 * ((lane >> 3) & 1), y4);
+        __syncwarp();
+        const int row = lane >> 1, part = 8 * (lane & 1);
+        const uint4 piece = *reinterpret_cast<const uint4*>(ys + row * LDQ + part);
+        if (row < nt) *reinterpret_cast<uint4*>(yp) = piece;
+        yp += C * p.out.sL;
+        __syncwarp();
     }
 #pragma unroll
     for (int j = 0; j < 8; j++)

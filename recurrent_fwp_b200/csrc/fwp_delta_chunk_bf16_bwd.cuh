@@ -48,14 +48,6 @@ __device__ __forceinline__ void bwd_arrive(unsigned long long* bar, int lane) {
     __syncwarp();
     if (lane == 0) asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ void stsm4(void* p, const unsigned (&r)[4]) {
-    asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};"
-                 ::"r"(smem_u32(p)), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
-}
-__device__ __forceinline__ void stsm4t(void* p, const unsigned (&r)[4]) {
-    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};"
-                 ::"r"(smem_u32(p)), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
-}
 
 }  // namespace cb
 
@@ -320,24 +312,24 @@ __global__ void __launch_bounds__((12 + PW) * 32, 1) delta_bwd_chunk_bf16_pipe_k
 #pragma unroll
             for (int j = 0; j < 2; j++) {
                 const int t = 8 * j + 2 * t4;
-                const float b0 = sg.b[t], b1 = sg.b[t + 1];
+                const float2 b2 = *reinterpret_cast<const float2*>(sg.b + t);
 #pragma unroll
                 for (int hr = 0; hr < 2; hr++) {
                     const float* w = sg.vo + t * LDO + m0 + g + 8 * hr;
                     const float l0 = lm[j][2 * hr], l1 = lm[j][2 * hr + 1];
                     db[j][0] = fmaf(l0, w[0], db[j][0]);
                     db[j][1] = fmaf(l1, w[LDO], db[j][1]);
-                    la[2 * j + hr] = pack_bf16(b0 * l0, b1 * l1);
+                    la[2 * j + hr] = pack_bf16(b2.x * l0, b2.y * l1);
                 }
             }
             stsm4t(s.bl[it & 1] + ((lane & 7) + 8 * (lane >> 4)) * LDT + m0 + 8 * ((lane >> 3) & 1), la);
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                float x = db[i >> 1][i & 1];
-                x += __shfl_xor_sync(0xffffffffu, x, 4);
-                x += __shfl_xor_sync(0xffffffffu, x, 8);
+            {   // four sums over the eight lanes that share t4: a lane gives half of its values away at a time
+                const bool h2 = lane & 4, h3 = lane & 8;
+                const float x0 = (h2 ? db[1][0] : db[0][0]) + __shfl_xor_sync(0xffffffffu, h2 ? db[0][0] : db[1][0], 4);
+                const float x1 = (h2 ? db[1][1] : db[0][1]) + __shfl_xor_sync(0xffffffffu, h2 ? db[0][1] : db[1][1], 4);
+                float x = (h3 ? x1 : x0) + __shfl_xor_sync(0xffffffffu, h3 ? x0 : x1, 8);
                 x += __shfl_xor_sync(0xffffffffu, x, 16);
-                if (g == 0) s.dbp[it & 1][warp][8 * (i >> 1) + 2 * t4 + (i & 1)] = x;
+                if (lane < 16) s.dbp[it & 1][warp][(h2 ? 8 : 0) + 2 * t4 + (h3 ? 1 : 0)] = x;
             }
             bwd_arrive(&s.blfull[it & 1], lane);
             neg4(la, la);
