@@ -604,6 +604,55 @@ __device__ __forceinline__ void stage_table_issue(float* stage, const StageTable
     cp_async_commit();
 }
 
+// The same copies for kernels with registers to spare, walking backwards from the last chunk: each of WARPS warps has its groups of
+// four rows of a tile to itself, by running pointers -- a 16-byte piece per lane, or a row at a time word by word where the stream's
+// rows are not 16-byte aligned (WORDS; the test costs 7 %, so callers that know better have an instance without).  The loop above cost
+// the tiled delta backward a tenth of its time.  Streams that lag have their first row elsewhere: their users take the loop for it.
+template <int TC, int WARPS, int NTILE, bool WORDS>
+struct RowStager {
+    static constexpr int D = 32, ITEMS = NTILE * TC / 4, MINE = (ITEMS + WARPS - 1) / WARPS;
+    const float* from[MINE];
+    long long sL[MINE];
+    int to[MINE];
+    bool words[MINE];
+    const float* bfrom;
+    long long bsL;
+    int warp, lane;
+    __device__ __forceinline__ RowStager(const StageTable* tb, int t0, int tid) : warp(tid >> 5), lane(tid & 31) {
+#pragma unroll
+        for (int i = 0; i < MINE; i++) {
+            const int item = warp + WARPS * i < ITEMS ? warp + WARPS * i : 0, tile = item / (TC / 4), r0 = item % (TC / 4) * 4;
+            words[i] = WORDS && tb->words[tile];
+            sL[i] = tb->sL[tile];
+            from[i] = tb->src[tile] + (t0 + r0) * sL[i] + (words[i] ? lane : (lane >> 3) * sL[i] + 4 * (lane & 7));
+            to[i] = (tile * TC + r0) * D + (words[i] ? lane : 4 * lane);
+        }
+        bfrom = tb->csrc[0] + (t0 + tid) * tb->csL[0];
+        bsL = tb->csL[0];
+    }
+    // rows [0, nt) of the chunk the pointers stand at; they move on to the chunk before it
+    __device__ __forceinline__ void issue(float* stage, int nt) {
+#pragma unroll
+        for (int i = 0; i < MINE; i++) {
+            const int rows = nt - (warp + WARPS * i) % (TC / 4) * 4;       // of this group that exist
+            if (ITEMS % WARPS == 0 || warp + WARPS * i < ITEMS) {
+                if (!words[i]) {
+                    if ((lane >> 3) < rows) cp_async16(stage + to[i], from[i]);
+                } else {
+#pragma unroll
+                    for (int r = 0; r < 4; r++)
+                        if (r < rows) cp_async4(stage + to[i] + r * D, from[i] + r * sL[i]);
+                }
+            }
+            from[i] -= TC * sL[i];
+        }
+        const int t = warp * 32 + lane;
+        if (t < nt) cp_async4(stage + NTILE * TC * D + t, bfrom);
+        bfrom -= TC * bsL;
+        cp_async_commit();
+    }
+};
+
 // shared-memory tile of one streamed tensor: fp32 rows the compute loop reads,
 // plus (for 16-bit inputs) the raw rows cp.async lands in.
 template <int D, int TC, typename T>

@@ -587,8 +587,8 @@ static int dispatch_fwd(const DeltaFwdParams& p, int nseq, cudaStream_t st) {
 // three launches):
 //   d = 16: 16 sequences 37 -> 13, 128 37 -> 25, 256 38 -> 37, 512 38 -> 65; with rows of 12 128 65 -> 27, 256 66 -> 52, 512 67 -> 76
 //   d = 32 with rows of 20: 128 139 -> 51, 512 283 -> 174.  Rows of 32 (training pass, one launch over four warps a sequence -> three launches):
-//           16 sequences x 64 27 -> 29, x 128 41 -> 35, x 256 71 -> 49, x 1024 248 -> 183; 64 x 128 43 -> 46, x 256 74 -> 68,
-//           x 1024 250 -> 233; 96 x 256 74 -> 76, x 1024 253 -> 269; 128 x 256 74 -> 85
+//           16 sequences x 64 25 -> 29, x 128 37 -> 35, x 256 64 -> 49, x 1024 220 -> 183; 32 x 256 65 -> 57, x 1024 221 -> 178; 64 x 128 39 -> 46,
+//           x 256 66 -> 68, x 1024 222 -> 233
 //   d = 64: 64 114 -> 76, 128 116 -> 125; with rows of 55 512 1789 -> 557;  d = 48: 512 1128 -> 354
 //   E, M = 96, 32: 128 951 -> 120, 1024 2777 -> 930;  128, 128: 128 2826 -> 676
 // and by length (time of the one-launch kernel over that of the three): d = 16, 80 sequences: 0.9 at 24 steps, 1.1 at 40, 1.8 at 250;
@@ -618,7 +618,7 @@ static bool bwd_phases_pay(const DeltaBwdParams& p, int nseq, int io_dtype) {
     }
     if (p.L <= 2 * kShortSeq) return false;
     if (d == 16) return nseq <= sms;
-    if (d == 32) return nseq <= sms / 2 && p.L >= (nseq <= sms / 4 ? 6 : 12) * kShortSeq;
+    if (d == 32) return nseq <= sms / 4 && p.L >= 8 * kShortSeq;
     if (p.L <= 3 * kShortSeq) return nseq <= sms * 3 / 4;
     if (p.L <= 4 * kShortSeq) return nseq <= 3 * sms;
     return nseq <= sms / 2 || (nseq > sms && nseq <= sms * 5 / 4);
@@ -641,7 +641,7 @@ static int dispatch_bwd(const DeltaBwdParams& p0, int nseq, cudaStream_t st) {
             return launch_bwd<16, 2, 32, float, 1>(p, nseq, st);
         }
         case 32: {
-            // fp32 streams, 256 steps of 128 / 512 / 1536 sequences: step by step over four warps 46 / 93 / 271 us, four-step blocked 66 /
+            // fp32 streams, 256 steps of 128 / 512 / 1536 sequences: step by step over four warps 39 / 88 / 253 us, four-step blocked 66 /
             // 136 / 380 us (which serves rows shorter than 32 where there is no scratch for the three launches); bf16 streams: per-step
             // 201 us vs blocked 207 us
             if constexpr (sizeof(T) == 4) {

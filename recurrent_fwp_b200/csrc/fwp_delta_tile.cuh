@@ -8,10 +8,10 @@
 //   warps B0, B1    one chunk of steps behind, sixteen rows of S each, pieces of four rows and four columns: dq, the S part of dk,
 //                   the rewind, dv and dbeta.  And one chunk ahead they turn v and v_old of a chunk into w and -u.
 // The four meet once per chunk of eight steps.  A lane reads 4 to 8 operands per product where a line per lane takes 32; its sums
-// over other lanes are reduce-scatters.  Bound by the latency of an A step with one sequence per SM (340 cycles; 46 us for 128
-// sequences x 256 steps, 89 for x 512), by issue and shared memory (53 and 65 % with two per SM: 114 us for 256 x 512; 93 for 512 x
-// 256).  The four-step blocked kernel took 66, 126, 132 and 136 us.  Other splits were slower where it counts: G over four
-// warps 53 and 113 us (128 and 512 x 256), S over four 53 and 113, three chunks in flight instead of one 49 and 92.
+// over other lanes are reduce-scatters.  Bound by the latency of an A step with one sequence per SM (39 us for 128 sequences x
+// 256 steps, 75 for x 512), by issue and shared memory with more (256 x 512: 101 us; 512 x 256: 88).  The four-step blocked kernel took
+// 66, 126, 132 and 136 us.  Other splits were slower where it counts: G over four warps or S over four 11 and 22 % (128 and 512 x
+// 256), three chunks in flight instead of one the same.
 #pragma once
 #include "fwp_delta_params.cuh"
 #include "fwp_trail.cuh"
@@ -29,7 +29,7 @@ struct DeltaTileSmem {
     static constexpr int kFloats = kStages * kStage + 2 * (kR + kDk) + kTable;
 };
 
-template <int TC, int SLOTS>
+template <int TC, int SLOTS, bool WORDS>
 __global__ void __launch_bounds__(128 * SLOTS, 1) delta_bwd_tile32_kernel(const __grid_constant__ DeltaBwdParams p) {
     constexpr int D = 32, NT = 128;
     using SM = DeltaTileSmem<TC>;
@@ -56,9 +56,9 @@ __global__ void __launch_bounds__(128 * SLOTS, 1) delta_bwd_tile32_kernel(const 
     }
     slot_barrier(slot, NT);
     const int nchunks = (p.L + TC - 1) / TC;
-    auto issue = [&](int j) {
-        const int t0 = (nchunks - 1 - j) * TC, nt = min(TC, p.L - t0);
-        stage_table_issue<TC, NT>(smem + (j % SM::kStages) * SM::kStage, tb, 5, 1, t0, nt, stid);
+    RowStager<TC, 4, 5, WORDS> rows_in(tb, (nchunks - 1) * TC, stid);
+    auto issue = [&](int j) {           // called for j = 0, 1, 2, ...
+        rows_in.issue(smem + (j % SM::kStages) * SM::kStage, min(TC, p.L - (nchunks - 1 - j) * TC));
     };
     auto advance = [&](int j) {
         cp_async_wait<0>();

@@ -308,8 +308,8 @@ static int launch_rnn_bwd(const RnnBwdParams& p, int nseq, cudaStream_t st) {
 }
 
 template <int TC, bool V1>
-static int launch_rnn_bwd_roles32(const RnnBwdParams& p, int nseq, cudaStream_t st) {
-    auto kern = rnn_bwd_roles32_kernel<TC, V1>;
+static int launch_rnn_bwd_roles32(const RnnBwdParams& p, int nseq, bool aligned, cudaStream_t st) {
+    const auto kern = aligned ? rnn_bwd_roles32_kernel<TC, V1, false> : rnn_bwd_roles32_kernel<TC, V1, true>;
     const int slots = spread_slots(4, nseq);
     const size_t bytes = (size_t)RnnRolesSmem<TC, V1>::kFloats * sizeof(float) * slots;
     return launch_dependent(kern, p, nseq / slots, 64 * slots, bytes, st, "rnn_bwd_roles32_kernel");
@@ -393,8 +393,8 @@ static int rnn_backward(int N, int H, int L, int D,
             const bool aligned = rows_16B_aligned(p.k) && rows_16B_aligned(p.v) && rows_16B_aligned(p.gy) && rows_16B_aligned(p.v_old) &&
                                  (!out_delayed || rows_16B_aligned(p.od)) && (!V1 || rows_16B_aligned(p.out));
             if (p.D != 32 || (!aligned && p.L < 64)) roles = 0;
-            if (roles == 1) return launch_rnn_bwd_roles32<8, V1>(p, N * H, st);
-            if (roles == 2) return launch_rnn_bwd_roles32<4, V1>(p, N * H, st);
+            if (roles == 1) return launch_rnn_bwd_roles32<8, V1>(p, N * H, aligned, st);
+            if (roles == 2) return launch_rnn_bwd_roles32<4, V1>(p, N * H, aligned, st);
             if (!out_delayed) return FWP_ERR_UNSUPPORTED;
             const int sp = tune_get(T_RNN_BWD_SPLIT32, 1);
             // measured (512 sequences x 512 steps): 1 -> 0.34 ms, 2 -> 0.39 ms, 4 -> 0.42 ms

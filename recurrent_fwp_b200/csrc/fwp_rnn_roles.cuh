@@ -8,9 +8,10 @@
 //   warp X (chain)      S, two rows and half the columns per lane: dz, w = v - v_old and -u of every step into a ring;
 //   warp T (one chunk behind)  the other gradients, from G and its own S (fwp_trail.cuh), the chunk unrolled.
 // The two meet once per chunk on a named barrier; that is also where staged input tiles change hands.  Each alone would take
-// about 490 (X) and 600 (T) cycles per step with four sequences per SM; a scheduler with one sequence issues for both in 720.
-// 512 sequences x 512 steps: 194 us, against 222 us with T's work in two warps that held G by columns and by rows, and 222 us
-// with T's columns split over two warps (a third more instructions).
+// about 490 (X) and 600 (T) cycles per step with four sequences per SM; a scheduler with one sequence issues for both.
+// 512 sequences x 512 steps: 169 us, 181 with one stream whose rows are not 16-byte aligned (194 when a loop over single pieces
+// staged the tiles), against 222 us with T's work in two warps that held G by columns and by rows, and 222 us with T's columns split
+// over two warps (a third more instructions).
 #pragma once
 #include "fwp_trail.cuh"
 
@@ -28,7 +29,7 @@ struct RnnRolesSmem {
     static constexpr int kFloats = kStages * Stage::kFloats + 2 * kRing + kOwn + kTable;
 };
 
-template <int TC, bool V1>
+template <int TC, bool V1, bool WORDS>
 __global__ void __launch_bounds__(256, 1) rnn_bwd_roles32_kernel(const RnnBwdParams p) {
     griddep_wait();               // launched as a dependent: global memory is touched from here on
     griddep_launch_dependents();
@@ -61,10 +62,13 @@ __global__ void __launch_bounds__(256, 1) rnn_bwd_roles32_kernel(const RnnBwdPar
     slot_barrier(slot, NT);         // the table is in place
 
     const int nchunks = (p.L + TC - 1) / TC;
-    auto issue = [&](int j) {
-        const int c = nchunks - 1 - j;
-        const int t0 = c * TC, nt = min(TC, p.L - t0);
-        stage_table_issue<TC, NT>(smem + (j % SM::kStages) * Stage::kFloats, tb, V1 ? 6 : 5, 1, t0, nt, stid);
+    constexpr int TILES = V1 ? 6 : 5;
+    RowStager<TC, 2, TILES, WORDS> rows_in(tb, (nchunks - 1) * TC, stid);
+    auto issue = [&](int j) {           // called for j = 0, 1, 2, ...
+        const int t0 = (nchunks - 1 - j) * TC, nt = min(TC, p.L - t0);
+        float* const st = smem + (j % SM::kStages) * Stage::kFloats;
+        if (V1 && t0 == 0) stage_table_issue<TC, NT>(st, tb, TILES, 1, t0, nt, stid);
+        else rows_in.issue(st, nt);
     };
     // top of the loop both warps run: chunk j's tiles have landed, X is through chunk j - 1, T through j - 2
     auto advance = [&](int j) {
