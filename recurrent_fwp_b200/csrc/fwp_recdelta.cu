@@ -547,16 +547,14 @@ static int launch_rec_bwd(const RecBwdParams& p, int nseq, cudaStream_t st) {
     return launch_dependent(kern, p, nseq / slots, D * SPLIT * slots, bytes * slots, st, "rec_bwd_kernel");
 }
 
-template <int SLOTS, bool OUT>
-static int launch_rec_bwd_roles32(const RecBwdParams& p, int nseq, int slots, cudaStream_t st) {
-    constexpr int TC = 8;
-    const size_t bytes = (size_t)RecRolesSmem<TC, OUT>::kFloats * sizeof(float) * slots;
-    return launch_dependent(rec_bwd_roles32_kernel<TC, SLOTS, OUT>, p, nseq / slots, 96 * slots, bytes, st, "rec_bwd_roles32_kernel");
-}
 template <bool OUT>
-static int launch_rec_bwd_roles32(const RecBwdParams& p, int nseq, cudaStream_t st) {
+static int launch_rec_bwd_roles32(const RecBwdParams& p, int nseq, bool aligned, cudaStream_t st) {
+    constexpr int TC = 8;
     const int slots = spread_slots(4, nseq);
-    return slots == 4 ? launch_rec_bwd_roles32<4, OUT>(p, nseq, 4, st) : launch_rec_bwd_roles32<2, OUT>(p, nseq, slots, st);
+    const size_t bytes = (size_t)RecRolesSmem<TC, OUT>::kFloats * sizeof(float) * slots;
+    const auto kern = slots == 4 ? (aligned ? rec_bwd_roles32_kernel<TC, 4, OUT, false> : rec_bwd_roles32_kernel<TC, 4, OUT, true>)
+                                 : (aligned ? rec_bwd_roles32_kernel<TC, 2, OUT, false> : rec_bwd_roles32_kernel<TC, 2, OUT, true>);
+    return launch_dependent(kern, p, nseq / slots, 96 * slots, bytes, st, "rec_bwd_roles32_kernel");
 }
 
 static int check_params(const fwp_tensor* Rq, const fwp_tensor* Rk, const fwp_tensor* Rv, const fwp_tensor* rb) {
@@ -681,7 +679,7 @@ static int rec_backward(int N, int H, int L, int D,
         case 16: rc = launch_rec_bwd<16, 2, 16>(p, N * H, st); break;
         case 32: {
             if (roles) {
-                rc = o_delayed ? launch_rec_bwd_roles32<false>(p, N * H, st) : launch_rec_bwd_roles32<true>(p, N * H, st);
+                rc = o_delayed ? launch_rec_bwd_roles32<false>(p, N * H, aligned, st) : launch_rec_bwd_roles32<true>(p, N * H, aligned, st);
                 break;
             }
             const int sp = tune_get(T_REC_BWD_SPLIT32, 2);

@@ -13,9 +13,9 @@
 //   warp Y   turns v into w = v - v_old (and the outputs into their tanh) for the chunk that X takes next, and two chunks later accumulates the three parameter
 //            gradients (8 x 4 pieces) and stores.
 // X and P hand over twice per step at named barriers: P has X's step to answer in.  The warps meet once per chunk of steps.
-// Alone, X takes 131 us for 512 sequences x 256 steps (250 instructions a step, 128 of them packed multiply-adds at 2.7 cycles), with
-// P 160, with both 177; 230 us with one warp for all but the parameter gradients.  Not worth their instructions: P posting from a
-// G one step older, corrected by scalars (180).
+// With Y staging the tiles by running pointers 512 sequences x 256 steps take 167 us (177 when all three ran a loop over single pieces;
+// of those X alone 131 -- 250 instructions a step, 128 of them packed multiply-adds at 2.7 cycles -- and P alone 160), 230 us with one
+// warp for all but the parameter gradients.  Not worth its instructions: P posting from a G one step older, corrected by scalars.
 // With four sequences per SM (504 of 512 registers of a scheduler's four threads: 208 X, 120 P, 176 Y) 512 sequences are resident.
 #pragma once
 #include "fwp_trail.cuh"
@@ -44,7 +44,7 @@ struct RecRolesSmem {
     static constexpr int kFloats = kStages * Stage::kFloats + 2 * kRing + 2 * kMail + kTable;
 };
 
-template <int TC, int SLOTS, bool OUT>
+template <int TC, int SLOTS, bool OUT, bool WORDS>
 __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const RecBwdParams p) {
     griddep_wait();               // launched as a dependent: global memory is touched from here on
     griddep_launch_dependents();
@@ -79,13 +79,9 @@ __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const Re
     slot_barrier(slot, NT);         // the table is in place
 
     const int nchunks = (p.L + TC - 1) / TC;
-    auto issue = [&](int j) {
-        const int c = nchunks - 1 - j;
-        const int t0 = c * TC, nt = min(TC, p.L - t0);
-        stage_table_issue<TC, NT>(smem + (j % SM::kStages) * Stage::kFloats, tb, Stage::kTiles, 1, t0, nt, stid);
-    };
-    // top of the loop that every warp runs
-    auto advance = [&](int j) {
+    // top of the loop that every warp runs; Y stages the tiles
+    auto issue = [&](int) {};
+    auto advance = [&](int j, auto&& issue) {
         cp_async_wait<0>();
         slot_barrier(slot, NT);
         if (j + 1 < nchunks) issue(j + 1);
@@ -95,8 +91,6 @@ __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const Re
     auto await = [&](int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); };
     const int given = 5 + slot, posted = 9 + slot;
     float* const W = p.W + n * p.wN + h * p.wH;
-    issue(0);
-
     if (role == 0) {
         // ---------------------------------------------------------------- X: the chain
         if constexpr (SLOTS == 4) asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
@@ -135,7 +129,7 @@ __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const Re
         auto swap_halves = [&](float x) { return __shfl_xor_sync(0xffffffffu, x, 16); };
         float gh = 0.f;
         for (int j = 0; j <= nchunks + 1; j++) {
-            advance(j);
+            advance(j, issue);
             if (j == 0 || j > nchunks) continue;
             Stage s; s.bind(smem + ((j - 1) % SM::kStages) * Stage::kFloats);
             const int nt = min(TC, p.L - (nchunks - j) * TC);
@@ -226,7 +220,7 @@ __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const Re
 #pragma unroll
         for (int i = 0; i < 16; i++) G[i] = 0ull;
         for (int j = 0; j <= nchunks + 1; j++) {
-            advance(j);
+            advance(j, issue);
             if (j == 0 || j > nchunks) continue;
             Stage s; s.bind(smem + ((j - 1) % SM::kStages) * Stage::kFloats);
             const int nt = min(TC, p.L - (nchunks - j) * TC);
@@ -288,8 +282,16 @@ __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const Re
     float* pgk = reinterpret_cast<float*>(p.gk.p) + n * p.gk.sN + h * p.gk.sH + lane + last * p.gk.sL;
     float* pgv = reinterpret_cast<float*>(p.gv.p) + n * p.gv.sN + h * p.gv.sH + lane + last * p.gv.sL;
     float* pgb = reinterpret_cast<float*>(p.gb.p) + n * p.gb.sN + h * p.gb.sH + last * p.gb.sL;
+    RowStager<TC, 1, Stage::kTiles, WORDS> rows_in(tb, (nchunks - 1) * TC, lane);
+    auto stage = [&](int j) {           // called for j = 0, 1, 2, ...
+        const int t0 = (nchunks - 1 - j) * TC, nt = min(TC, p.L - t0);
+        float* const st = smem + (j % SM::kStages) * Stage::kFloats;
+        if (OUT && t0 == 0) stage_table_issue<TC, 32>(st, tb, Stage::kTiles, 1, t0, nt, lane);
+        else rows_in.issue(st, nt);
+    };
+    stage(0);
     for (int j = 0; j <= nchunks + 1; j++) {
-        advance(j);
+        advance(j, stage);
         if (j < nchunks) {
             Stage s; s.bind(smem + (j % SM::kStages) * Stage::kFloats);
             const int nt = min(TC, p.L - (nchunks - 1 - j) * TC);
