@@ -398,12 +398,12 @@ static int launch_lstm_bwd_roles32(const LstmBwdParams& p, int nseq, cudaStream_
 }
 
 template <int VAR>
-static int launch_lstm_fwd_gates32(const LstmFwdParams& p, int nseq, cudaStream_t st) {
+static int launch_lstm_fwd_gates32(const LstmFwdParams& p, int nseq, bool aligned, cudaStream_t st) {
     constexpr int TC = 16;
-    auto kern = lstm_fwd_gates32_kernel<TC, VAR>;
     const int slots = spread_slots(4, nseq);
     const size_t bytes = (size_t)LstmGatesSmem<TC>::kFloats * sizeof(float) * slots;
-    return launch_dependent(kern, p, nseq / slots, 96 * slots, bytes, st, "lstm_fwd_gates32_kernel");
+    return launch_dependent(aligned ? lstm_fwd_gates32_kernel<TC, VAR, false> : lstm_fwd_gates32_kernel<TC, VAR, true>, p, nseq / slots, 96 * slots,
+                            bytes, st, "lstm_fwd_gates32_kernel");
 }
 
 template <int VAR>
@@ -415,7 +415,7 @@ static int dispatch_lstm_fwd(const LstmFwdParams& p, int nseq, cudaStream_t st) 
             bool aligned = true;
             for (int a = 0; a < 3; a++)
                 aligned = aligned && rows_16B_aligned(p.z[a]) && rows_16B_aligned(p.k[a]) && rows_16B_aligned(p.v[a]);
-            if (p.D == 32 && tune_get(T_LSTM_FWD_GATES32, 1) && (aligned || p.L >= 64)) return launch_lstm_fwd_gates32<VAR>(p, nseq, st);
+            if (p.D == 32 && tune_get(T_LSTM_FWD_GATES32, 1) && (aligned || p.L >= 64)) return launch_lstm_fwd_gates32<VAR>(p, nseq, aligned, st);
             const int sp = tune_get(T_LSTM_FWD_SPLIT32, 1);
             // measured (512 sequences x 512 steps): 1 -> 0.78 ms, 4 -> 0.83 ms, 2 -> 0.85 ms
             if (sp == 2) return launch_lstm_fwd<32, 2, 8, VAR>(p, nseq, st);
