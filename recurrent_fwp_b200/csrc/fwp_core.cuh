@@ -653,6 +653,35 @@ struct RowStager {
     }
 };
 
+// One stream of rows of 32 floats as a single warp copies it, TC rows at a time, forwards: four rows at a time, a 16-byte piece per
+// lane, or (WORDS, where its rows are not 16-byte aligned) row by row word by word.
+template <int TC, bool WORDS>
+struct WarpRows32 {
+    const float* from;
+    long long sL;
+    bool words;
+    int lane;
+    __device__ __forceinline__ void init(const Row4& r, int n, int h, int lane_) {
+        lane = lane_;
+        const float* at = reinterpret_cast<const float*>(r.p) + n * r.sN + h * r.sH;
+        sL = r.sL;
+        words = WORDS && ((reinterpret_cast<uintptr_t>(at) & 15) != 0 || sL % 4 != 0);
+        from = at + (words ? lane : (lane >> 3) * sL + 4 * (lane & 7));
+    }
+    __device__ __forceinline__ void issue(float* tile, int nt) {
+        if (!words) {
+#pragma unroll
+            for (int r = 0; r < TC; r += 4)
+                if (r + (lane >> 3) < nt) cp_async16(tile + 32 * r + 4 * lane, from + r * sL);
+        } else {
+#pragma unroll
+            for (int r = 0; r < TC; r++)
+                if (r < nt) cp_async4(tile + 32 * r + lane, from + r * sL);
+        }
+        from += TC * sL;
+    }
+};
+
 // shared-memory tile of one streamed tensor: fp32 rows the compute loop reads,
 // plus (for 16-bit inputs) the raw rows cp.async lands in.
 template <int D, int TC, typename T>

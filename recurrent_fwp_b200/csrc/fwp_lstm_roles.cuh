@@ -304,38 +304,19 @@ __global__ void __launch_bounds__(384, 1) lstm_fwd_gates32_kernel(const LstmFwdP
     // a warp copies z, k, v and beta of its own gate, by running pointers: four rows at a time, a 16-byte piece per lane, or row by
     // row word by word (12 rolled iterations over a table of all nine tiles: 512 sequences x 512 steps
     // 286 us, now 255; 32 sequences 192, now 151)
-    const float* from[3];
-    long long sL[3];
-    bool words[3];
-    auto source = [&](int i, const Row4& r) {
-        const float* at = reinterpret_cast<const float*>(r.p) + n * r.sN + h * r.sH;
-        sL[i] = r.sL;
-        words[i] = WORDS && ((reinterpret_cast<uintptr_t>(at) & 15) != 0 || r.sL % 4 != 0);
-        from[i] = at + (words[i] ? lane : (lane >> 3) * r.sL + 4 * (lane & 7));
-    };
-    source(0, q == 0 ? p.z[0] : (q == 1 ? p.z[1] : p.z[2]));
-    source(1, q == 0 ? p.k[0] : (q == 1 ? p.k[1] : p.k[2]));
-    source(2, q == 0 ? p.v[0] : (q == 1 ? p.v[1] : p.v[2]));
+    WarpRows32<TC, WORDS> rz, rk, rv;
+    rz.init(q == 0 ? p.z[0] : (q == 1 ? p.z[1] : p.z[2]), n, h, lane);
+    rk.init(q == 0 ? p.k[0] : (q == 1 ? p.k[1] : p.k[2]), n, h, lane);
+    rv.init(q == 0 ? p.v[0] : (q == 1 ? p.v[1] : p.v[2]), n, h, lane);
     const Row4& rbeta = q == 0 ? p.beta[0] : (q == 1 ? p.beta[1] : p.beta[2]);
     const long long sb = rbeta.sL;
     const float* bfrom = reinterpret_cast<const float*>(rbeta.p) + n * rbeta.sN + h * rbeta.sH + lane * sb;
     auto issue = [&](int c) {           // called for c = 0, 1, 2, ...
         const int nt = min(TC, p.L - c * TC);
         float* const base = smem + (c & 1) * Stage::kFloats;
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-            float* dst = base + (3 * q + i) * kTile + (words[i] ? lane : 4 * lane);
-            if (!words[i]) {
-#pragma unroll
-                for (int r = 0; r < TC; r += 4)
-                    if (r + (lane >> 3) < nt) cp_async16(dst + r * D, from[i] + r * sL[i]);
-            } else {
-#pragma unroll
-                for (int r = 0; r < TC; r++)
-                    if (r < nt) cp_async4(dst + r * D, from[i] + r * sL[i]);
-            }
-            from[i] += TC * sL[i];
-        }
+        rz.issue(base + 3 * q * kTile, nt);
+        rk.issue(base + (3 * q + 1) * kTile, nt);
+        rv.issue(base + (3 * q + 2) * kTile, nt);
         if (lane < nt) cp_async4(base + 9 * kTile + q * r4(TC) + lane, bfrom);
         bfrom += TC * sb;
         cp_async_commit();
