@@ -981,9 +981,9 @@ __global__ void __launch_bounds__(cb::NT, 3) delta_bwd_chunk_bf16_inv_kernel(con
 #pragma unroll
                 for (int par = 0; par < 2; par++) {
                     float x = db[j][par];
-                    x += __shfl_xor_sync(0xffffffffu, x, 4);
-                    x += __shfl_xor_sync(0xffffffffu, x, 8);
                     x += __shfl_xor_sync(0xffffffffu, x, 16);
+                    x += __shfl_xor_sync(0xffffffffu, x, 8);
+                    x += __shfl_xor_sync(0xffffffffu, x, 4);
                     if (g == 0) s.dbp[warp][8 * j + 2 * t4 + par] = x;
                 }
         }
