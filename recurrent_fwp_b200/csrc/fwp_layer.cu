@@ -10,7 +10,8 @@
 // copies); the backward pass recomputes the normalisation from the same row and writes the gradient row once.
 // All kernels are plain streaming kernels.  The prologue kernels give 8, 16 or 32 lanes to a (len, batch, head) row,
 // visit rows in the order of the projected tensor so that reads are fully contiguous and writes are whole aligned
-// rows, and issue every load before the first use; the transpose moves 16-byte pieces, four per thread.
+// rows, and issue every load before the first use; the tile forms below move the same rows by 16-byte accesses.  The
+// transpose moves 16-byte pieces, four per thread.
 #include "fwp_core.cuh"
 
 namespace fwp {
@@ -182,6 +183,153 @@ __global__ void __launch_bounds__(kLayerWarps * 32) layer_prologue_bwd_kernel(co
     }
 }
 
+// The same two passes for D % 4 == 0 and 16-byte aligned tensors.  A warp takes a span of 32/LPR projected rows (4 or 8):
+// (3D+1) * 32/LPR floats that start on a 16-byte boundary, although the rows in the span do not.  It goes to shared memory by
+// 16-byte copies; LPR lanes share a row, lane `sub` holding elements 4 (sub + LPR m) + j (j < 4) of each of q, k, v, so that
+// rows of the (B, H, len, .) tensors move by 16-byte accesses and with LPR = 8 a warp's reads of the span (four rows, each
+// 1 mod 4 floats after the one before) meet every bank once.  What bounded the 4-byte kernels was the
+// load/store unit (71 %) and issue (69 %).  The backward does not load what only the gradient of v replaces and writes the
+// gradient row over the row it was computed from.  Warps never wait for one another.
+template <int LPR, int MP>
+struct LayerTile {
+    static constexpr int kWarps = MP == 4 ? 4 : 8;
+    static constexpr int kRows = 32 / LPR;                  // a warp's rows; 6 KB of shared memory for D = 128, 1.6 KB for 16, 32
+    static constexpr int kThreads = kWarps * 32;
+};
+
+// the warp's rows of the projected tensor -> its part of shared memory, without the 16-byte pieces that hold nothing but
+// values if SKIP_V; returns how many rows there are (<= 0: none)
+template <int ROWS, int SKIP_V>
+__device__ __forceinline__ int load_span(float* xs, const float* qkvb, long long r0, const LayerDims& d) {
+    const int W = 3 * d.D + 1, lane = threadIdx.x & 31;
+    const int n = (int)(d.rows - r0 < ROWS ? d.rows - r0 : ROWS), len = n * W;
+    const float* src = qkvb + r0 * W;
+    for (int i = 4 * lane; i + 3 < len; i += 128) {
+        if (SKIP_V) {
+            int c = i;
+#pragma unroll
+            for (int r = 1; r < ROWS; r++) c -= i >= r * W ? W : 0;
+            if (c >= 2 * d.D && c + 3 < 3 * d.D) continue;
+        }
+        cp_async16(xs + i, src + i);
+    }
+    const int rest = (len & ~3) + lane;
+    if (rest < len) xs[rest] = src[rest];
+    cp_async_commit();
+    return n;
+}
+
+__device__ __forceinline__ float4 f4(const float* x) { return make_float4(x[0], x[1], x[2], x[3]); }
+
+template <int LPR, int MP>
+__global__ void __launch_bounds__(LayerTile<LPR, MP>::kThreads) layer_prologue_fwd_tile_kernel(const PrologueParams p) {
+    using T = LayerTile<LPR, MP>;
+    extern __shared__ float4 span4[];
+    griddep_wait();
+    griddep_launch_dependents();
+    const LayerDims& d = p.d;
+    const int D = d.D, W = 3 * D + 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane % LPR, row = lane / LPR;
+    const long long r0 = ((long long)blockIdx.x * T::kWarps + warp) * T::kRows;
+    float* xs = reinterpret_cast<float*>(span4) + warp * T::kRows * W;
+    const int n = load_span<T::kRows, 0>(xs, p.qkvb, r0, d);
+    const bool live = row < n;
+    const long long o = live ? bhl_row(d, r0 + row) : 0;
+    cp_async_wait<0>();
+    __syncwarp();
+    const float* x = xs + row * W;
+    float pq[MP][4], pk[MP][4];
+    float sq = 0.f, sk = 0.f;
+#pragma unroll
+    for (int m = 0; m < MP; m++) {
+        const int i = 4 * (sub + LPR * m);
+        const bool ok = live && i < D;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            pq[m][j] = ok ? elu_p1(x[i + j]) : 0.f;
+            pk[m][j] = ok ? elu_p1(x[D + i + j]) : 0.f;
+            sq += pq[m][j];
+            sk += pk[m][j];
+        }
+    }
+    const float iq = p.scale / row_sum<LPR>(sq), ik = 1.f / row_sum<LPR>(sk);
+    if (!live) return;
+#pragma unroll
+    for (int m = 0; m < MP; m++) {
+        const int i = 4 * (sub + LPR * m);
+        if (i < D) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                pq[m][j] *= iq;
+                pk[m][j] *= ik;
+            }
+            *reinterpret_cast<float4*>(p.q + o * D + i) = f4(pq[m]);
+            *reinterpret_cast<float4*>(p.k + o * D + i) = f4(pk[m]);
+            *reinterpret_cast<float4*>(p.v + o * D + i) = f4(x + 2 * D + i);
+        }
+    }
+    if (sub == 0) p.beta[o] = 1.f / (1.f + expf(-x[3 * D]));
+}
+
+// D <= 16 only: a lane's piece of each tensor is one 16-byte access.
+__global__ void __launch_bounds__(LayerTile<4, 1>::kThreads) layer_prologue_bwd_tile_kernel(const PrologueGradParams p) {
+    using T = LayerTile<4, 1>;
+    extern __shared__ float4 span4[];
+    griddep_wait();
+    griddep_launch_dependents();
+    const LayerDims& d = p.d;
+    const int D = d.D, W = 3 * D + 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & 3, row = lane >> 2, i = 4 * sub;
+    const long long r0 = ((long long)blockIdx.x * T::kWarps + warp) * T::kRows;
+    float* xs = reinterpret_cast<float*>(span4) + warp * T::kRows * W;
+    const int n = load_span<T::kRows, 1>(xs, p.qkvb, r0, d);
+    const bool live = row < n, ok = live && i < D;
+    const long long o = live ? bhl_row(d, r0 + row) : 0;
+    float4 gq = make_float4(0.f, 0.f, 0.f, 0.f), gk = gq, gv = gq;
+    if (ok) {
+        gq = *reinterpret_cast<const float4*>(p.gq + o * D + i);
+        gk = *reinterpret_cast<const float4*>(p.gk + o * D + i);
+        gv = *reinterpret_cast<const float4*>(p.gv + o * D + i);
+    }
+    const float gb = (live && sub == 0) ? p.gbeta[o] : 0.f;
+    cp_async_wait<0>();
+    __syncwarp();
+    float* x = xs + row * W;
+    const float aq[4] = {p.scale * gq.x, p.scale * gq.y, p.scale * gq.z, p.scale * gq.w};
+    const float ak[4] = {gk.x, gk.y, gk.z, gk.w}, av[4] = {gv.x, gv.y, gv.z, gv.w};
+    float xq[4], xk[4], pq[4], pk[4];
+    float sq = 0.f, sk = 0.f, dq = 0.f, dk = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        xq[j] = ok ? x[i + j] : 0.f;
+        xk[j] = ok ? x[D + i + j] : 0.f;
+        pq[j] = ok ? elu_p1(xq[j]) : 0.f;
+        pk[j] = ok ? elu_p1(xk[j]) : 0.f;
+        sq += pq[j];
+        sk += pk[j];
+        dq = fmaf(aq[j], pq[j], dq);
+        dk = fmaf(ak[j], pk[j], dk);
+    }
+    const float iq = 1.f / row_sum<4>(sq), ik = 1.f / row_sum<4>(sk);
+    dq = row_sum<4>(dq) * iq;       // sum_j g_j y_j
+    dk = row_sum<4>(dk) * ik;
+    if (ok) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            x[i + j] = (aq[j] - dq) * iq * (xq[j] > 0.f ? 1.f : pq[j]);
+            x[D + i + j] = (ak[j] - dk) * ik * (xk[j] > 0.f ? 1.f : pk[j]);
+            x[2 * D + i + j] = av[j];
+        }
+    }
+    if (live && sub == 0) {
+        const float sg = 1.f / (1.f + expf(-x[3 * D]));
+        x[3 * D] = gb * sg * (1.f - sg);
+    }
+    __syncwarp();
+    const int len = n * W, rest = (len & ~3) + lane;
+    float* y = p.gx + r0 * W;
+    for (int e = 4 * lane; e + 3 < len; e += 128) *reinterpret_cast<float4*>(y + e) = *reinterpret_cast<const float4*>(xs + e);
+    if (rest < len) y[rest] = xs[rest];
+}
+
 // (B, H, len, D) <-> (len, B, H, D) with a scale: dst row of one side = scale * src row of the other.
 // One thread per 16-byte piece (4-byte piece when D is not a multiple of 4), kLayerRows pieces per thread.
 template <typename V>
@@ -268,6 +416,19 @@ __global__ void __launch_bounds__(256) delayed_kernel(const DelayedParams p) {
     *reinterpret_cast<V*>(p.dst + n * p.dN + h * p.dH + (long long)t * p.dL + c) = x;
 }
 
+// the tile kernels: every piece of 16 bytes lies in one row of q, k, v and on a boundary of 16
+static bool layer_tile_ok(const LayerDims& d, const void* a, const void* b, const void* c, const void* e, const void* f = nullptr) {
+    return d.D % 4 == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c) |
+                             reinterpret_cast<uintptr_t>(e) | reinterpret_cast<uintptr_t>(f)) & 15) == 0;
+}
+template <int LPR, int MP, class K, class P>
+static int launch_layer_tile(K kern, const P& p, cudaStream_t st) {
+    using T = LayerTile<LPR, MP>;
+    constexpr int rows = T::kWarps * T::kRows;
+    return launch_dependent(kern, p, (int)((p.d.rows + rows - 1) / rows), T::kThreads, sizeof(float) * rows * (3 * p.d.D + 1), st,
+                            nullptr);
+}
+
 static int layer_dims(int L, int B, int H, int D, LayerDims& d) {
     if (L <= 0 || B <= 0 || H <= 0 || D <= 0) return FWP_ERR_SHAPE;
     if (D > kLayerMaxD) return FWP_ERR_UNSUPPORTED;
@@ -291,6 +452,14 @@ FWP_API int fwp_delta_layer_prologue_forward_scaled(int L, int B, int H, int D, 
     DeviceGuard guard(device);
     if (guard.status) return guard.status;
     cudaStream_t st = (cudaStream_t)stream;
+    // L2 flushed before, 4-byte kernel and this: (512, 96, 8) rows of 16 45.8 and 32.8 us, (512, 32, 8) rows of 32 28.7 and 24.6,
+    // of 64 41.8 and 39.0, (256, 32, 8) of 128 41.0 and 40.8, of 96 36.9 and 32.8; (16, 1, 8) the same 6 to 8 us.
+    if (layer_tile_ok(p.d, qkvb, q, k, v)) {
+        if (D <= 16) return launch_layer_tile<4, 1>(layer_prologue_fwd_tile_kernel<4, 1>, p, st);
+        if (D <= 32) return launch_layer_tile<8, 1>(layer_prologue_fwd_tile_kernel<8, 1>, p, st);
+        if (D <= 64) return launch_layer_tile<8, 2>(layer_prologue_fwd_tile_kernel<8, 2>, p, st);
+        return launch_layer_tile<8, 4>(layer_prologue_fwd_tile_kernel<8, 4>, p, st);
+    }
     auto grid = [&](int rows_per_warp) { return (int)((p.d.rows + kLayerWarps * rows_per_warp - 1) / (kLayerWarps * rows_per_warp)); };
     if (D <= 32) return launch_dependent(layer_prologue_fwd_kernel<8, 2>, p, grid(8), kLayerWarps * 32, 0, st, nullptr);
     if (D <= 64) return launch_dependent(layer_prologue_fwd_kernel<16, 2>, p, grid(4), kLayerWarps * 32, 0, st, nullptr);
@@ -314,6 +483,10 @@ FWP_API int fwp_delta_layer_prologue_backward_scaled(int L, int B, int H, int D,
     DeviceGuard guard(device);
     if (guard.status) return guard.status;
     cudaStream_t st = (cudaStream_t)stream;
+    // L2 flushed before, 4-byte kernel and this form: (512, 96, 8) rows of 16 65.5 and 59.4 us, but (512, 32, 8) rows of 32
+    // 36.8 and 40.9, of 64 58.1 and 68.2, (256, 32, 8) of 128 58.1 and 72.4.
+    if (D <= 16 && layer_tile_ok(p.d, qkvb, grad_q, grad_k, grad_v, grad_qkvb))
+        return launch_layer_tile<4, 1>(layer_prologue_bwd_tile_kernel, p, st);
     auto grid = [&](int rows_per_warp) { return (int)((p.d.rows + kLayerWarps * rows_per_warp - 1) / (kLayerWarps * rows_per_warp)); };
     if (D <= 32) return launch_dependent(layer_prologue_bwd_kernel<8>, p, grid(4), kLayerWarps * 32, 0, st, nullptr);
     if (D <= 64) return launch_dependent(layer_prologue_bwd_kernel<16>, p, grid(2), kLayerWarps * 32, 0, st, nullptr);

@@ -38,6 +38,28 @@ def test_prologue_matches_the_elementwise_chain(fwp, L, B, H, d):
     assert util.scaled_rel(res['fused'][1], res['chain'][1]) <= 1e-5
 
 
+# a span of 64, 32, 16 rows (d up to 32, 64, 128) and one row more or less; off=1: rows that only the 4-byte kernels can take
+@pytest.mark.parametrize('off', [0, 1])
+@pytest.mark.parametrize('rows,d', [(63, 32), (64, 4), (65, 32), (131, 28), (31, 64), (33, 36), (15, 128), (17, 100)])
+def test_prologue_spans_and_their_remainders(fwp, rows, d, off):
+    from recurrent_fwp_b200.delta_layer_io import delta_layer_prologue
+    g = util.gen(6)
+    W = 3 * d + 1
+    x = (torch.randn(rows * W + off, generator=g) * 2).to(DEV)[off:].view(rows, 1, 1, W)
+    grads = [torch.randn(1, 1, rows, w, generator=g).to(DEV) for w in (d, d, d, 1)]
+    leaf = x.detach().requires_grad_()
+    outs = delta_layer_prologue(leaf)
+    got = torch.autograd.grad(outs, leaf, grads)[0]
+    ref = x.double().requires_grad_()
+    want = chain(ref, d)
+    grad = torch.autograd.grad(want, ref, [t.double() for t in grads])[0]
+    # a sum of d positive terms is off by d roundings of 2^-24 at most, and 16 cover expf, the division and the products;
+    # a gradient is the difference of two such values, each up to twice the largest gradient
+    for a, b in zip(outs, want):
+        assert torch.allclose(a.double(), b, rtol=(d + 16) * 2.0 ** -24, atol=1e-9)
+    assert (got.double() - grad).abs().max() <= (d + 16) * 2.0 ** -22 * grad.abs().max()
+
+
 @pytest.mark.parametrize('L,B,H,d', [(37, 3, 2, 16), (5, 2, 8, 32), (3, 2, 2, 21)])
 def test_epilogue_matches_scale_transpose_reshape(fwp, L, B, H, d):
     from recurrent_fwp_b200.delta_layer_io import delta_layer_epilogue
