@@ -198,11 +198,12 @@ struct LayerTile {
 };
 
 // the warp's rows of the projected tensor -> its part of shared memory, without the 16-byte pieces that hold nothing but
-// values if SKIP_V; returns how many rows there are (<= 0: none)
+// values if SKIP_V; returns how many rows there are.  A warp past the last row has none, not a negative count: the remainder of a
+// negative length would lie in the span of the last warp that has rows.
 template <int ROWS, int SKIP_V>
 __device__ __forceinline__ int load_span(float* xs, const float* qkvb, long long r0, const LayerDims& d) {
     const int W = 3 * d.D + 1, lane = threadIdx.x & 31;
-    const int n = (int)(d.rows - r0 < ROWS ? d.rows - r0 : ROWS), len = n * W;
+    const int n = max(0, (int)min(d.rows - r0, (long long)ROWS)), len = n * W;
     const float* src = qkvb + r0 * W;
     for (int i = 4 * lane; i + 3 < len; i += 128) {
         if (SKIP_V) {

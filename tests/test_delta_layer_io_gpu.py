@@ -60,6 +60,31 @@ def test_prologue_spans_and_their_remainders(fwp, rows, d, off):
     assert (got.double() - grad).abs().max() <= (d + 16) * 2.0 ** -22 * grad.abs().max()
 
 
+# Warps of the last block without a row of their own, and a last row at every residue modulo four of the floats before it: nothing
+# but the live warps may write, so repeats agree bit for bit and the floats beside the result stay as they were.
+@pytest.mark.parametrize('d', [4, 8, 12, 16])
+@pytest.mark.parametrize('rows', [217, 222, 75, 200, 1])
+def test_prologue_backward_of_a_partly_filled_block(fwp, rows, d):
+    from recurrent_fwp_b200 import _lib
+    g = util.gen(7)
+    W = 3 * d + 1
+    x = (torch.randn(rows, 1, 1, W, generator=g) * 2).to(DEV)
+    grads = [torch.randn(1, 1, rows, w, generator=g).to(DEV) for w in (d, d, d, 1)]
+    ref = x.double().requires_grad_()
+    want = torch.autograd.grad(chain(ref, d), ref, [t.double() for t in grads])[0]
+    stream, dev = _lib.stream_and_device(x)
+    first = None
+    for _ in range(20):
+        wide = torch.full((rows * W + 64,), 7., device=DEV)
+        got = wide[32:32 + rows * W].view(x.shape)
+        _lib.check(_lib.lib.fwp_delta_layer_prologue_backward(rows, 1, 1, d, x.data_ptr(), *(t.data_ptr() for t in grads),
+                                                              got.data_ptr(), stream, dev), 'prologue backward')
+        assert (wide[:32] == 7.).all() and (wide[32 + rows * W:] == 7.).all()
+        first = got if first is None else first
+        assert torch.equal(got, first)
+    assert (first.double() - want).abs().max() <= (d + 16) * 2.0 ** -22 * want.abs().max()      # as above
+
+
 @pytest.mark.parametrize('L,B,H,d', [(37, 3, 2, 16), (5, 2, 8, 32), (3, 2, 2, 21)])
 def test_epilogue_matches_scale_transpose_reshape(fwp, L, B, H, d):
     from recurrent_fwp_b200.delta_layer_io import delta_layer_epilogue
