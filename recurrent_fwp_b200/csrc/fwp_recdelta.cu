@@ -571,7 +571,7 @@ template <bool OUT>
 static int launch_rec_bwd_roles32(const RecBwdParams& p, int nseq, bool aligned, cudaStream_t st) {
     constexpr int TC = 8;
     const int slots = spread_slots(4, nseq);
-    const size_t bytes = (size_t)RecRolesSmem<TC, OUT>::kFloats * sizeof(float) * slots;
+    const size_t bytes = (size_t)RecRolesSmem<TC>::kFloats * sizeof(float) * slots;
     const auto kern = slots == 4 ? (aligned ? rec_bwd_roles32_kernel<TC, 4, OUT, false> : rec_bwd_roles32_kernel<TC, 4, OUT, true>)
                                  : (aligned ? rec_bwd_roles32_kernel<TC, 2, OUT, false> : rec_bwd_roles32_kernel<TC, 2, OUT, true>);
     return launch_dependent(kern, p, nseq / slots, 96 * slots, bytes, st, "rec_bwd_roles32_kernel");

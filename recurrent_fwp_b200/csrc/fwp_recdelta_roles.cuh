@@ -7,35 +7,29 @@
 //            then takes g_t and dv_t:  G += q (x) g - k (x) dv;
 //   warp X   the chain, two rows and half the columns of S and of the three R per lane:  r = r0 + (q.k) g,  dv = beta r,
 //            dq = S_{t-1} g + k (u.g),  dk = G u + q (u.g) - S_{t-1} dv,  softmax backward, the products with R, tanh.
-//            The sums over features come from products of vectors that the lane reads anyway: u.g = beta (w.g),
-//            db = (w.dv) (1 - beta),  k . dk = r.u - v_old.dv = w.dv - v_old.dv  (v_old = S_{t-1}^T k, dv.w = r.u)  and, where the forward's
-//            outputs are given, q . dq = y . g  (y = S_t^T q);
+//            Two of the sums over features come from products of vectors that the lane reads anyway: u.g = beta (w.g) and
+//            db = (w.dv) (1 - beta).  Those of the softmax, q . dq and k . dk, are taken over the dq and dk that they are subtracted from:
+//            y . g and w.dv - v_old.dv are the same numbers by the forward's saved values, but those and the rewound S part by the
+//            rewind's rounding, and the gradients through the softmax then sum to that instead of to zero;
 //   warp Y   turns v into w = v - v_old (and the outputs into their tanh) for the chunk that X takes next, and two chunks later accumulates the three parameter
 //            gradients (8 x 4 pieces) and stores.
 // X and P hand over twice per step at named barriers: P has X's step to answer in.  The warps meet once per chunk of steps.
-// With Y staging the tiles by running pointers 512 sequences x 256 steps take 167 us (177 when all three ran a loop over single pieces;
-// of those X alone 131 -- 250 instructions a step, 128 of them packed multiply-adds at 2.7 cycles -- and P alone 160), 230 us with one
-// warp for all but the parameter gradients.  Not worth its instructions: P posting from a G one step older, corrected by scalars.
+// 512 sequences x 256 steps take 161 us, 32 sequences 105 (230 us for 512 with one warp for all but the parameter gradients; 10 more when
+// all three ran a loop over single pieces instead of Y staging by running pointers).  X alone took 131 -- 250 instructions a step, 128 of
+// them packed multiply-adds at 2.7 cycles -- and P alone 160, when q . dq and k . dk came from the saved values: that form's seventh tile
+// cost 6 us of 167 with 512 sequences, its shorter chain gave 10 of 105 with 32.  Not worth its instructions: P posting from a G one step
+// older, corrected by scalars, and the two sums over the parts of dq and dk before the halves of the warp meet (164 us and 104).
 // With four sequences per SM (504 of 512 registers of a scheduler's four threads: 208 X, 120 P, 176 Y) 512 sequences are resident.
 #pragma once
 #include "fwp_trail.cuh"
 
 namespace fwp {
 
-template <int TC, bool OUT>
+template <int TC>
 struct RecRolesSmem {
     static constexpr int D = 32;
-    struct Stage : RecBwdStage<D, TC> {
-        using Base = RecBwdStage<D, TC>;
-        const float* y;                               // the forward's outputs, if given (between the tiles and beta)
-        static constexpr int kTiles = OUT ? 7 : 6;
-        static constexpr int kFloats = Base::kFloats + (OUT ? TC * D : 0);
-        __device__ __forceinline__ void bind(float* mem) {
-            Base::bind(mem);
-            y = mem + 6 * TC * D;
-            this->b.f = mem + kTiles * TC * D;
-        }
-    };
+    using Stage = RecBwdStage<D, TC>;
+    static constexpr int kTiles = 6;
     static constexpr int kStages = 4;                 // chunk j + 1 in flight, w of chunk j, X and P on j - 1, Y on j - 2
     static constexpr int kStep = 4 * D + 4;           // per step: g, dv, dq~, dk~, db~
     static constexpr int kRing = TC * kStep;
@@ -49,7 +43,7 @@ __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const Re
     griddep_wait();               // launched as a dependent: global memory is touched from here on
     griddep_launch_dependents();
     constexpr int D = 32, NT = 96;
-    using SM = RecRolesSmem<TC, OUT>;
+    using SM = RecRolesSmem<TC>;
     using Stage = typename SM::Stage;
     const int nslots = SLOTS == 4 ? 4 : blockDim.x / NT;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -62,17 +56,13 @@ __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const Re
     float* ring = smem + SM::kStages * Stage::kFloats;
     float* mail = ring + 2 * SM::kRing;
     StageTable* tb = reinterpret_cast<StageTable*>(mail + 2 * SM::kMail);
-    if (stid == 0) {                // tile order: q, k, v, v_old, od, gy, (y)
+    if (stid == 0) {                // tile order: q, k, v, v_old, od, gy
         stage_table_set(tb, 0, p.q, n, h);
         stage_table_set(tb, 1, p.k, n, h);
         stage_table_set(tb, 2, p.v, n, h);
         stage_table_set(tb, 3, p.v_old, n, h);
-        if constexpr (OUT) {
-            stage_table_set_lagging(tb, 4, p.out, p.start, n, h);
-            stage_table_set(tb, 6, p.out, n, h);
-        } else {
-            stage_table_set(tb, 4, p.od, n, h);
-        }
+        if constexpr (OUT) stage_table_set_lagging(tb, 4, p.out, p.start, n, h);
+        else stage_table_set(tb, 4, p.od, n, h);
         stage_table_set(tb, 5, p.gy, n, h);
         stage_table_set_col(tb, 0, p.beta, n, h);
     }
@@ -165,34 +155,27 @@ __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const Re
                 f2 x[8], y[8];
                 lds_slice<16>(x, e + 16 * half);
                 lds_slice<16>(y, e + D + 16 * half);
-                float wg = dot(w, x), wdv = dot(w, y), vdv;
+                float wg = dot(w, x), wdv = dot(w, y);
                 f2 a = 0ull, b = 0ull, c = 0ull, d = 0ull;
                 dots(S, x, a, b);
                 dots(S, y, c, d);
-                float pq = 0.f;
-                {
-                    f2 z[8];
-                    lds_slice<16>(z, s.vo.f + t * D + 16 * half);
-                    vdv = dot(z, y);
-                    if constexpr (OUT) {                // q . dq = y . g
-                        lds_slice<16>(z, s.y + t * D + 16 * half);
-                        pq = dot(z, x);
-                        pq += swap_halves(pq);
-                    }
-                }
                 const float sg = f2_hsum(a) + swap_halves(f2_hsum(b));
                 const float sdv = f2_hsum(c) + swap_halves(f2_hsum(d));
                 wg += swap_halves(wg);
                 wdv += swap_halves(wdv);
-                vdv += swap_halves(vdv);
                 const float ug = beta * wg;
                 const float dq = fmaf(ke, ug, sg), dk = fmaf(qe, ug, gu) - sdv;
                 const float dbh = wdv * (1.f - beta);
-                if constexpr (!OUT) pq = warp_sum_idx<1>(qe * dq);
+                float pq = qe * dq, pk = ke * dk;       // both softmax sums in one shuffle sequence
+#pragma unroll
+                for (int o = 16; o >= 1; o >>= 1) {
+                    pq += __shfl_xor_sync(0xffffffffu, pq, o);
+                    pk += __shfl_xor_sync(0xffffffffu, pk, o);
+                }
                 a = b = 0ull;
                 dots(Rv, y, a, b);                      // beside the sums: the part of the feedback that needs dv only, and
                 rewind(t > 0 ? t - 1 : 0, t > 0 ? 1.f : 0.f);       // the next step's state (at t = 0 nothing is subtracted: no branch)
-                const float dqh = qe * (dq - pq), dkh = ke * (dk - (wdv - vdv));
+                const float dqh = qe * (dq - pq), dkh = ke * (dk - pk);
                 e[2 * D + own] = dqh;
                 e[3 * D + own] = dkh;
                 if (lane == 0) e[4 * D] = dbh;
@@ -282,11 +265,11 @@ __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const Re
     float* pgk = reinterpret_cast<float*>(p.gk.p) + n * p.gk.sN + h * p.gk.sH + lane + last * p.gk.sL;
     float* pgv = reinterpret_cast<float*>(p.gv.p) + n * p.gv.sN + h * p.gv.sH + lane + last * p.gv.sL;
     float* pgb = reinterpret_cast<float*>(p.gb.p) + n * p.gb.sN + h * p.gb.sH + last * p.gb.sL;
-    RowStager<TC, 1, Stage::kTiles, WORDS> rows_in(tb, (nchunks - 1) * TC, lane);
+    RowStager<TC, 1, SM::kTiles, WORDS> rows_in(tb, (nchunks - 1) * TC, lane);
     auto stage = [&](int j) {           // called for j = 0, 1, 2, ...
         const int t0 = (nchunks - 1 - j) * TC, nt = min(TC, p.L - t0);
         float* const st = smem + (j % SM::kStages) * Stage::kFloats;
-        if (OUT && t0 == 0) stage_table_issue<TC, 32>(st, tb, Stage::kTiles, 1, t0, nt, lane);
+        if (OUT && t0 == 0) stage_table_issue<TC, 32>(st, tb, SM::kTiles, 1, t0, nt, lane);
         else rows_in.issue(st, nt);
     };
     stage(0);

@@ -82,3 +82,27 @@ def test_config3_shape_slice_and_determinism(fwp):
                 y_cpu32=util.max_abs(out32, out))
     assert util.max_abs(runs[0][0], out) <= 1e-4
     util.check_grads('rec_delta recurrent-delta-net shape slice', NAMES, runs[0][1:], g32, g)
+
+
+@pytest.mark.parametrize('L', [256, 4096])
+def test_gradients_through_the_softmax_sum_to_zero(fwp, L):
+    """Each step's gradients of q and k before their softmax sum to zero over the features up to the rounding of that sum, however long
+    the sequence: the three-warp backward must not put the rewind's rounding there.  The general kernel sums the same 32 products in
+    another order, so the largest sum of either is within a factor of two of the other's."""
+    from recurrent_fwp_b200 import _lib
+    from recurrent_fwp_b200.rec_update_fwm_tanh import rec_update_fwm_tanh
+    B, H, d = 2, 4, 32
+    *ins, gy = util.rec_inputs(2, B, H, L, d)
+    W0 = torch.randn(B, H, d, d, generator=util.gen(52)) * 0.1
+    h0 = torch.randn(B, H, 1, d, generator=util.gen(62)) * 0.1
+    sums = {}
+    try:
+        for roles in (1, 0):
+            _lib.tune('rec_bwd.32.roles', roles)
+            leaves = [t.clone().to(DEV).requires_grad_() for t in ins]
+            rec_update_fwm_tanh(*leaves, W0.to(DEV), h0.to(DEV)).backward(gy.to(DEV))
+            sums[roles] = [leaf.grad.double().sum(-1).abs().amax().item() for leaf in leaves[:2]]
+    finally:
+        _lib.tune('rec_bwd.32.roles', 1)
+    for fast, general in zip(sums[1], sums[0]):
+        assert fast <= 2 * general, sums
