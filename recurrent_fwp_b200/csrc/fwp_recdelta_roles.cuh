@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const Re
 #pragma unroll 4
             for (int t = 0; t < nt; t++) {
                 s.v.f[t * D + lane] -= s.vo.f[t * D + lane];
-                if constexpr (OUT) s.od.f[t * D + lane] = tanh_fast(s.od.f[t * D + lane]);      // as the forward took it
+                if constexpr (OUT) s.od.f[t * D + lane] = tanhf(s.od.f[t * D + lane]);       // the accuracy of fwp_delayed
             }
         }
         if (j < 2) continue;

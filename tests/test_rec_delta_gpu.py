@@ -106,3 +106,24 @@ def test_gradients_through_the_softmax_sum_to_zero(fwp, L):
         _lib.tune('rec_bwd.32.roles', 1)
     for fast, general in zip(sums[1], sums[0]):
         assert fast <= 2 * general, sums
+
+
+@pytest.mark.parametrize('roles', [1, 0])
+def test_delayed_output_enters_the_backward_by_an_accurate_tanh(fwp, roles):
+    """With one step the gradient of r_b is tanh(h0) times the gradient of beta, one rounded product, so the tanh can be read off:
+    2 ulp for tanhf as CUDA documents it and half an ulp for the product, an ulp being 2^-23 of the value at most."""
+    from recurrent_fwp_b200 import _lib
+    from recurrent_fwp_b200.rec_update_fwm_tanh import rec_update_fwm_tanh
+    B, H, L, d = 1, 64, 1, 32
+    *ins, gy = util.rec_inputs(3, B, H, L, d)
+    W0 = torch.randn(B, H, d, d, generator=util.gen(4)) * 0.1
+    h0 = torch.linspace(-3, 3, H * d).view(B, H, 1, d)
+    leaves = [t.clone().to(DEV).requires_grad_() for t in ins]
+    try:
+        _lib.tune('rec_bwd.32.roles', roles)
+        rec_update_fwm_tanh(*leaves, W0.to(DEV), h0.to(DEV)).backward(gy.to(DEV))
+    finally:
+        _lib.tune('rec_bwd.32.roles', 1)
+    got = leaves[7].grad.double() / leaves[3].grad.double()
+    want = torch.tanh(h0.double()).to(DEV)
+    assert ((got - want) / want).abs().max().item() <= 2.5 * 2.0 ** -23
