@@ -9,7 +9,7 @@
 //   Akk = strict_lower(K K^T), Aqk = lower(Q K^T)                          (bf16 products)
 //   [Cv | Ck] = T [V | K],  T = (I + Akk diag(b))^-1   (the unit triangular solve
 //               c_t = rhs_t - sum_{i<t} Akk[t,i] b_i c_i as an explicit inverse, see the forward kernel)
-//   w = Cv - Ck S0  (= v - v_old),  u = b w,  v_old = V - w
+//   v_old = (V - Cv) + Ck S0,  w = V - v_old,  u = b w    ((V - Cv) from T - I: of the size of v_old, not of v)
 //   y = Q S0 + Aqk u,   S1 = S0 + K^T u
 //
 // (the same recurrence as algorithmic/fast_weight/fast_weight_cuda.cu:107-180, regrouped).
@@ -156,7 +156,7 @@ __device__ __forceinline__ void load_tile_f32(float* tile, const float* base, lo
 //   T = (I - N)(I + N^2)(I + N^4)(I + N^8)
 // Every warp builds Akk, Aqk and T for itself in accumulator fragments (six 16 x 16 x 16 products whose right
 // operands are transposed in registers with movmatrix), so the Gram tiles, the solve and Cv never touch shared
-// memory: Cv^T = V^T T^T and (V - Cv)^T = -V^T (T - I)^T are two products of the chain warp with T taken from
+// memory: (V - Cv)^T = -V^T (T - I)^T is one product of the chain warp with T taken from
 // its own fragments, and only Ck = T K (16 columns per warp) is exchanged through shared memory.
 namespace cb {
 
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(cb::NT, 4) delta_fwd_chunk_bf16_inv_kernel(con
         const float* bs = s.b[cur];
 
         // (1) per warp: Akk, Aqk, T; the warp's 16 columns of Ck = T K
-        unsigned th[4], tl[4], qk[4];                   // right operands T^T (two parts), Aqk^T
+        unsigned yh[4], yl[4], qk[4];                   // right operands (T - I)^T (two parts), Aqk^T
         {
             float akk[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
             float aqk[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(cb::NT, 4) delta_fwd_chunk_bf16_inv_kernel(con
             for (int j = 0; j < 2; j++)
 #pragma unroll
                 for (int i = 0; i < 4; i++) T[j][i] = Y[j][i] + ((8 * j + 2 * t4 + (i & 1)) == (g + 8 * (i >> 1)) ? 1.f : 0.f);
-            bt_of(th, tl, T);
+            bt_of(yh, yl, Y);
             unsigned ah[4], al[4], bK[4];
             split_bf16(T[0][0], T[0][1], ah[0], al[0]); split_bf16(T[0][2], T[0][3], ah[1], al[1]);
             split_bf16(T[1][0], T[1][1], ah[2], al[2]); split_bf16(T[1][2], T[1][3], ah[3], al[3]);
@@ -369,11 +369,11 @@ __global__ void __launch_bounds__(cb::NT, 4) delta_fwd_chunk_bf16_inv_kernel(con
                 mm(P, sa[ks], bc);
                 mm(Yo, sa[ks], bq);
             }
-            float cv[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+            float py[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
             unsigned va[4];
             lda_trans(va, s.v[cur] + m0, LDT, lane);
-            mm(cv, va, th);
-            mm(cv, va, tl);
+            mm(py, va, yh);
+            mm(py, va, yl);
             float u[2][4];
 #pragma unroll
             for (int j = 0; j < 2; j++)
@@ -381,10 +381,10 @@ __global__ void __launch_bounds__(cb::NT, 4) delta_fwd_chunk_bf16_inv_kernel(con
                 for (int i = 0; i < 4; i++) {
                     const int m = m0 + g + 8 * (i >> 1), t = 8 * j + 2 * t4 + (i & 1);
                     const unsigned v2 = va[2 * j + (i >> 1)];
-                    const float w = cv[j][i] - P[j][i], v = __uint_as_float((i & 1) ? v2 & 0xffff0000u : v2 << 16);
-                    u[j][i] = bs[t] * w;
+                    const float vo = P[j][i] - py[j][i], v = __uint_as_float((i & 1) ? v2 & 0xffff0000u : v2 << 16);
+                    u[j][i] = bs[t] * (v - vo);
                     if (t < nt) {
-                        if (vob) vob[(long long)(t0 + t) * p.v_old.sL + m] = v - w;
+                        if (vob) vob[(long long)(t0 + t) * p.v_old.sL + m] = vo;
                         if (uib) uib[(long long)(t0 + t) * p.v_ins.sL + m] = u[j][i];
                     }
                 }
@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(cb::NT, 4) delta_fwd_chunk_bf16_inv_kernel(con
 // the same for the four chain warps and does not wait for the previous chunk.  In the kernel above every warp
 // computes it for itself, between two CTA-wide barriers, on the critical path of the chunk.  Here a fifth warp
 // prepares it one chunk ahead (and issues all the copies): it leaves the three right-operand fragment sets
-// (T^T as two bf16 parts, Aqk^T) in shared memory in fragment order, one 16-byte piece per lane,
+// ((T - I)^T as two bf16 parts, Aqk^T) in shared memory in fragment order, one 16-byte piece per lane,
 // and Ck as a row-major tile.  The chain warps wait for that package, run the state-dependent products and hand the
 // buffers back.  Two named barriers per package buffer: FULL (the preparing warp arrives, the chain warps wait) and
 // EMPTY (the chain warps arrive after their last read of the package and of the input stage, the preparing warp
@@ -441,7 +441,7 @@ constexpr int NTP = 160;                // four chain warps and the preparing wa
 
 struct SmemP {
     __nv_bfloat16 k[3][C * LDT], v[3][C * LDT], q[3][C * LDT];    // input stages
-    uint4 frag[2][3][32];               // per package: T^T hi, lo; Aqk^T -- in fragment order
+    uint4 frag[2][3][32];               // per package: (T - I)^T hi, lo; Aqk^T -- in fragment order
     __nv_bfloat16 ck[2][C * LDT];       // per package: Ck, [t][e]
     __nv_bfloat16 ys[4][C * LDQ];       // per chain warp: y, [t][m of the warp]
     float b[3][C];
@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(cb::NTP, 4) delta_fwd_chunk_bf16_pipe_kernel(c
                     aqk[j][i] = cc <= r ? aqk[j][i] : 0.f;
                     Y[j][i] = -N1[j][i];
                 }
-            unsigned th[4], tl[4], qk[4];
+            unsigned yh[4], yl[4], qk[4];
             {
                 unsigned lo[4];
                 bt_of(qk, lo, aqk);
@@ -585,9 +585,9 @@ __global__ void __launch_bounds__(cb::NTP, 4) delta_fwd_chunk_bf16_pipe_kernel(c
             for (int j = 0; j < 2; j++)
 #pragma unroll
                 for (int i = 0; i < 4; i++) T[j][i] = Y[j][i] + ((8 * j + 2 * t4 + (i & 1)) == (g + 8 * (i >> 1)) ? 1.f : 0.f);
-            bt_of(th, tl, T);
-            s.frag[pk][0][lane] = make_uint4(th[0], th[1], th[2], th[3]);
-            s.frag[pk][1][lane] = make_uint4(tl[0], tl[1], tl[2], tl[3]);
+            bt_of(yh, yl, Y);
+            s.frag[pk][0][lane] = make_uint4(yh[0], yh[1], yh[2], yh[3]);
+            s.frag[pk][1][lane] = make_uint4(yl[0], yl[1], yl[2], yl[3]);
             s.frag[pk][2][lane] = make_uint4(qk[0], qk[1], qk[2], qk[3]);
             unsigned ah[4], al[4];
             split_bf16(T[0][0], T[0][1], ah[0], al[0]); split_bf16(T[0][2], T[0][3], ah[1], al[1]);
@@ -630,11 +630,11 @@ __global__ void __launch_bounds__(cb::NTP, 4) delta_fwd_chunk_bf16_pipe_kernel(c
         const bf16* Qs = s.q[st];
         const float* bs = s.b[st];
         const bf16* cks = s.ck[pk];
-        unsigned th[4], tl[4], qk[4];
+        unsigned yh[4], yl[4], qk[4];
         {
             const uint4 f0 = s.frag[pk][0][lane], f1 = s.frag[pk][1][lane], f2 = s.frag[pk][2][lane];
-            th[0] = f0.x; th[1] = f0.y; th[2] = f0.z; th[3] = f0.w;
-            tl[0] = f1.x; tl[1] = f1.y; tl[2] = f1.z; tl[3] = f1.w;
+            yh[0] = f0.x; yh[1] = f0.y; yh[2] = f0.z; yh[3] = f0.w;
+            yl[0] = f1.x; yl[1] = f1.y; yl[2] = f1.z; yl[3] = f1.w;
             qk[0] = f2.x; qk[1] = f2.y; qk[2] = f2.z; qk[3] = f2.w;
         }
         unsigned sa[4][4];
@@ -655,11 +655,11 @@ __global__ void __launch_bounds__(cb::NTP, 4) delta_fwd_chunk_bf16_pipe_kernel(c
             mm(P, sa[ks], bc);
             mm(Yo, sa[ks], bq);
         }
-        float cv[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        float py[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
         unsigned va[4];                 // V^T as left operand: the same elements, lane for lane, as the products' results
         lda_trans(va, s.v[st] + m0, LDT, lane);
-        mm(cv, va, th);
-        mm(cv, va, tl);
+        mm(py, va, yh);
+        mm(py, va, yl);
         float u[2][4], vo[2][4];
 #pragma unroll
         for (int j = 0; j < 2; j++) {
@@ -667,9 +667,9 @@ __global__ void __launch_bounds__(cb::NTP, 4) delta_fwd_chunk_bf16_pipe_kernel(c
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 const unsigned v2 = va[2 * j + (i >> 1)];
-                const float w = cv[j][i] - P[j][i], v = __uint_as_float((i & 1) ? v2 & 0xffff0000u : v2 << 16);
-                u[j][i] = ((i & 1) ? b2.y : b2.x) * w;
-                vo[j][i] = v - w;
+                const float v = __uint_as_float((i & 1) ? v2 & 0xffff0000u : v2 << 16);
+                vo[j][i] = P[j][i] - py[j][i];
+                u[j][i] = ((i & 1) ? b2.y : b2.x) * (v - vo[j][i]);
             }
         }
         if (SAVE) {

@@ -618,6 +618,33 @@ def test_preparing_warp_kernels_equal_the_self_preparing_ones_bit_for_bit(fwp, B
         assert torch.equal(a, r)
 
 
+@pytest.mark.parametrize('pipe', [1, 0])
+def test_small_old_values_keep_their_own_precision(fwp, pipe):
+    """With an empty memory and small write strengths the first chunk's old values are some hundred times smaller than v.  They come
+    from products of V with (T - I) in two bf16 parts, 16 bits, so their error is 2^-16 of their own norm at most, not of v's."""
+    from recurrent_fwp_b200 import _lib
+    B, H, L, d = 2, 8, 16 + 7, 64
+    q, k, v, _, _ = util.delta_inputs(505, B, H, L, d)
+    b = torch.sigmoid(torch.randn(B, H, L, 1, generator=util.gen(506)) - 4)
+    q, k, v, b = (t.to(torch.bfloat16) for t in (q, k, v, b))
+    S, ref = torch.zeros(B, H, d, d, dtype=torch.float64), []
+    for t in range(16):
+        kt = k[:, :, t].double()
+        ref.append(torch.einsum('nhem,nhe->nhm', S, kt))
+        S = S + kt[..., None] * (b[:, :, t].double() * (v[:, :, t].double() - ref[-1]))[:, :, None]
+    D, (y, vo, vi) = _lib.desc, [torch.empty(B, H, L, d, device=DEV, dtype=t) for t in (torch.bfloat16, torch.float32, torch.float32)]
+    streams, W = [t.to(DEV) for t in (q, k, v, b)], torch.zeros(B, H, d, d, device=DEV)
+    stream, dev = _lib.stream_and_device(W)
+    try:
+        _lib.tune('delta.pipe64', pipe)
+        _lib.check(_lib.lib.fwp_fast_weight_forward(B, H, L, d, d, *map(D, streams), D(vo), D(vi), D(W), D(y), _lib.BF16, stream, dev), 'forward')
+    finally:
+        _lib.tune('delta.pipe64', 1)
+    assert _lib.last_kernel() == 'delta_fwd_chunk_bf16_%s_kernel' % ('pipe' if pipe else 'inv')
+    ref = torch.stack(ref, 2)
+    assert ((vo[:, :, :16].double().cpu() - ref).norm() / ref.norm()).item() <= 2 ** -16
+
+
 def test_tcgen05_forward_is_the_kernel_that_ran(fwp):
     """With the switch on, an eligible call runs delta_fwd_tc_kernel; a caller that asks for v_insert, or whose
     state is not 8-byte aligned, gets the warp-level kernel (the tcgen05 plan does not apply), never an error."""
