@@ -859,6 +859,17 @@ static int set_smem(K kernel, size_t bytes) {
     return FWP_OK;
 }
 
+// Warpgroups that change their register counts (setmaxnreg) share what the block was launched with, and a share that is not there is
+// waited for without end.  Launch bounds only cap that number, so the launcher asks: do `groups` warpgroups of `kern` start with `sum`
+// registers per thread of each?
+template <typename K>
+static bool registers_cover(K kern, int groups, int sum) {
+    cudaFuncAttributes a;
+    if (cudaFuncGetAttributes(&a, kern) == cudaSuccess) return groups * a.numRegs >= sum;
+    cudaGetLastError();
+    return false;
+}
+
 // `name` (a string literal) is what fwp_last_kernel() reports for the calling thread afterwards; nullptr leaves that as it is.
 template <typename K, typename P>
 static int launch(K kern, const P& p, dim3 grid, int threads, size_t bytes, cudaStream_t st, const char* name) {

@@ -393,8 +393,9 @@ template <int VAR>
 static int launch_lstm_bwd_roles32(const LstmBwdParams& p, int nseq, cudaStream_t st) {
     // four sequences per SM leave shared memory for chunks of four steps; fewer keep chunks of eight and registers to spare
     const int slots = spread_slots(4, nseq);
-    if (slots == 4) return launch_lstm_bwd_roles32<4, VAR, 4>(p, nseq, 4, st);
-    return launch_lstm_bwd_roles32<8, VAR, 2>(p, nseq, slots, st);
+    if (slots == 4 && registers_cover(lstm_bwd_roles32_kernel<4, VAR, 4>, 4, LstmRolesRegs::kSum))
+        return launch_lstm_bwd_roles32<4, VAR, 4>(p, nseq, 4, st);
+    return launch_lstm_bwd_roles32<8, VAR, 2>(p, nseq, slots < 2 ? slots : 2, st);
 }
 
 template <int VAR>

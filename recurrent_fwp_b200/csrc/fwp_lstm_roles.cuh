@@ -32,6 +32,11 @@ struct LstmRolesSmem {
     static constexpr int kFloats = kStages * Stage::kFloats + 2 * kRing + 3 * kOwn + kTable;
 };
 
+// registers a thread of X and of each H_q with four sequences per SM (a warpgroup each)
+struct LstmRolesRegs {
+    static constexpr int X = 152, H = 120, kSum = X + 3 * H;
+};
+
 template <int TC, int VAR, int SLOTS>
 __global__ void __launch_bounds__(128 * SLOTS, 1) lstm_bwd_roles32_kernel(const LstmBwdParams p) {
     griddep_wait();               // launched as a dependent: global memory is touched from here on
@@ -89,7 +94,7 @@ __global__ void __launch_bounds__(128 * SLOTS, 1) lstm_bwd_roles32_kernel(const 
 
     if (role == 0) {
         // ---------------------------------------------------------------- X: the chain
-        if constexpr (SLOTS == 4) asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
+        if constexpr (SLOTS == 4) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(LstmRolesRegs::X));
         // lane (half, lp): rows 2 lp + half (finished here) and 2 lp + 1 - half (given away), columns 16 half .. 16 half + 15
         const int half = lane >> 4, lp = lane & 15, own = 2 * lp + half, other = 2 * lp + 1 - half;
         f2 M[3][16];
@@ -188,7 +193,7 @@ __global__ void __launch_bounds__(128 * SLOTS, 1) lstm_bwd_roles32_kernel(const 
     }
 
     // -------------------------------------------------------------------- H_q: one chunk behind
-    if constexpr (SLOTS == 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 120;");
+    if constexpr (SLOTS == 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(LstmRolesRegs::H));
     const int q = role - 1;
     // this gate's gradient streams, picked once (by value: a reference chosen at run time would make every
     // later field access an indexed load from the parameter bank)

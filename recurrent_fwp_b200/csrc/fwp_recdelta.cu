@@ -570,10 +570,13 @@ static int launch_rec_bwd(const RecBwdParams& p, int nseq, cudaStream_t st) {
 template <bool OUT>
 static int launch_rec_bwd_roles32(const RecBwdParams& p, int nseq, bool aligned, cudaStream_t st) {
     constexpr int TC = 8;
-    const int slots = spread_slots(4, nseq);
+    int slots = spread_slots(4, nseq);
+    auto kern = aligned ? rec_bwd_roles32_kernel<TC, 4, OUT, false> : rec_bwd_roles32_kernel<TC, 4, OUT, true>;
+    if (slots != 4 || !registers_cover(kern, 3, RecRolesRegs::kSum)) {
+        slots = slots < 2 ? slots : 2;
+        kern = aligned ? rec_bwd_roles32_kernel<TC, 2, OUT, false> : rec_bwd_roles32_kernel<TC, 2, OUT, true>;
+    }
     const size_t bytes = (size_t)RecRolesSmem<TC>::kFloats * sizeof(float) * slots;
-    const auto kern = slots == 4 ? (aligned ? rec_bwd_roles32_kernel<TC, 4, OUT, false> : rec_bwd_roles32_kernel<TC, 4, OUT, true>)
-                                 : (aligned ? rec_bwd_roles32_kernel<TC, 2, OUT, false> : rec_bwd_roles32_kernel<TC, 2, OUT, true>);
     return launch_dependent(kern, p, nseq / slots, 96 * slots, bytes, st, "rec_bwd_roles32_kernel");
 }
 

@@ -38,6 +38,11 @@ struct RecRolesSmem {
     static constexpr int kFloats = kStages * Stage::kFloats + 2 * kRing + 2 * kMail + kTable;
 };
 
+// registers a thread of X, P and Y with four sequences per SM (a warpgroup each)
+struct RecRolesRegs {
+    static constexpr int X = 208, P = 120, Y = 176, kSum = X + P + Y;
+};
+
 template <int TC, int SLOTS, bool OUT, bool WORDS>
 __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const RecBwdParams p) {
     griddep_wait();               // launched as a dependent: global memory is touched from here on
@@ -83,7 +88,7 @@ __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const Re
     float* const W = p.W + n * p.wN + h * p.wH;
     if (role == 0) {
         // ---------------------------------------------------------------- X: the chain
-        if constexpr (SLOTS == 4) asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+        if constexpr (SLOTS == 4) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(RecRolesRegs::X));
         // lane (half, lp): rows 2 lp + half (finished here) and 2 lp + 1 - half (given away), columns 16 half .. 16 half + 15
         const int half = lane >> 4, lp = lane & 15, own = 2 * lp + half, other = 2 * lp + 1 - half;
         auto at = [&](int i) { return (i < 8 ? own : other); };
@@ -197,7 +202,7 @@ __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const Re
     }
     if (role == 1) {
         // ---------------------------------------------------------------- P: G
-        if constexpr (SLOTS == 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 120;");
+        if constexpr (SLOTS == 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(RecRolesRegs::P));
         const Tile32 tile(lane);
         f2 G[16];
 #pragma unroll
@@ -254,7 +259,7 @@ __global__ void __launch_bounds__(96 * SLOTS, 1) rec_bwd_roles32_kernel(const Re
         return;
     }
     // -------------------------------------------------------------------- Y: w for X and P, then parameter gradients and stores
-    if constexpr (SLOTS == 4) asm volatile("setmaxnreg.inc.sync.aligned.u32 176;");
+    if constexpr (SLOTS == 4) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(RecRolesRegs::Y));
     const Tile32 tile(lane);
     f2 A[16], B[16], C[16];             // the partial gradients of Rq, Rk, Rv
 #pragma unroll
