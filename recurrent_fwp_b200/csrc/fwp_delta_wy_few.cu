@@ -23,15 +23,20 @@ int launch_fwd_wy_few(const DeltaFwdParams& p, int nseq, cudaStream_t st) {
         if (few && (force || nseq <= 2 * sm_count())) return run_fwd_few<16, 16, 4, 2, SUM>(p, nseq, st);
         return -1;
     }
-    // One sequence per SM (evaluation, us; the other form -> this one): d = 32, 64 sequences: 20 steps 8.4 -> 9.9, 64 10.4 -> 10.6, 112 13.2 -> 12.7,
-    // 512 41 -> 31; 40 x 243, rows of 20 in any layout 26.8 -> 22.9; 144 x 512, rows of 24 46 -> 40.  E, M = 96, 32, 128 x 256: 64 -> 50; 80, 32 64 -> 50;
-    // 77, 32 64 -> 57; 80, 32 x 64 18.7 -> 20.7, x 128 28.9 -> 28.9; 96, 16 52 -> 41.  Buffers of larger sizes leave too few helpers: d = 48 51 -> 78,
-    // 64 63 -> 88, E, M = 128, 32 64 -> 78
+    // Up to one sequence per SM, evaluation, time of this form over the other's (packed rows, rows as layers slice them; 1 to 148 sequences):
+    //   E = M = 32     96 steps 1.00-1.05, 112 0.96-1.02, 128 0.91-0.98, 256 0.84-0.90
+    //   other sizes up to 32 (17, 20, 24; 25, 31; 16, 32; 32, 12)   112 1.00-1.12, 120 0.94-1.02, 128 0.94-1.03, 160 0.90-1.00, 256 0.84-0.94
+    //   E up to 96, M = 12, 16     128 0.71-0.96, 144 0.66-0.92, 384 0.52-0.88
+    //   E, M = 66, 32; 77, 30; 80, 32; 96, 20; 96, 32, from 144 steps: up to 64 sequences 0.99-1.19, 96 0.89-1.07, 128 0.76-0.97, 148 0.70-0.93.
+    //     There the other form's loops, unrolled, are fetched by many SMs at once; with few it has the shorter chunk
+    // Buffers of larger sizes leave too few helpers: 128 x 256, d = 48 51 -> 78 us, 64 63 -> 88, E, M = 128, 32 64 -> 78
     if constexpr (!SUM) {
-        const bool few = force ? force == 6 : nseq <= sm_count();
-        if (d <= 32 && few && (force || p.L >= 7 * wy::C)) return run_fwd_few<32, 32, 6, 1, SUM>(p, nseq, st);
-        if (d > 64 && d <= 96 && p.M <= 32 && few && (force || p.L >= 9 * wy::C))
-            return p.M <= 16 ? run_fwd_few<96, 16, 3, 1, SUM>(p, nseq, st) : run_fwd_few<96, 32, 3, 1, SUM>(p, nseq, st);
+        const int sms = sm_count(), least = d > 32 ? 9 * wy::C : p.E == 32 && p.M == 32 ? 7 * wy::C : 7 * wy::C + 1;
+        if (force ? force != 6 : nseq > sms || p.L < least) return -1;
+        if (d <= 32) return run_fwd_few<32, 32, 6, 1, SUM>(p, nseq, st);
+        if (d <= 64 || d > 96 || p.M > 32) return -1;
+        if (p.M <= 16) return run_fwd_few<96, 16, 3, 1, SUM>(p, nseq, st);
+        if (force || nseq >= sms * 3 / 4) return run_fwd_few<96, 32, 3, 1, SUM>(p, nseq, st);
     }
     return -1;
 }

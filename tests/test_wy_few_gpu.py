@@ -21,8 +21,8 @@ def run(ins, W0, grad):
 
 
 @pytest.mark.parametrize('E,M,L,form,few', [(32, 32, 112, 'packed', True), (20, 20, 113, 'views', True), (17, 25, 127, 'packed', True),
-                                            (24, 32, 240, 'offset', True), (32, 32, 111, 'packed', False), (96, 32, 144, 'views', True),
-                                            (80, 29, 161, 'packed', True), (77, 32, 150, 'offset', True), (65, 16, 145, 'packed', True),
+                                            (24, 32, 240, 'offset', True), (32, 32, 111, 'packed', False), (96, 32, 144, 'views', 'forced'),
+                                            (80, 29, 161, 'packed', 'forced'), (77, 32, 150, 'offset', 'forced'), (65, 16, 145, 'packed', True),
                                             (96, 32, 143, 'packed', False), (97, 32, 160, 'packed', False)])
 def test_few_sequences(fwp, E, M, L, form, few):
     from recurrent_fwp_b200 import _lib
@@ -40,8 +40,12 @@ def test_few_sequences(fwp, E, M, L, form, few):
             return wide[..., 1:]
         return t
     ins = [lay_out(t) for t in ins]
-    y, W, kf = run(ins, W0, True)
-    assert (kf == 'delta_fwd_wy_few_kernel') == few
+    try:                        # so few sequences take it by themselves up to 16 values only
+        _lib.tune('delta.wy.helpers', 6 if few == 'forced' else 0)
+        y, W, kf = run(ins, W0, True)
+    finally:
+        _lib.tune('delta.wy.helpers', 0)
+    assert (kf == 'delta_fwd_wy_few_kernel') == bool(few)
     try:
         _lib.tune('delta.wy', 0)
         yr, Wr, kr = run(ins, W0, False)
@@ -50,3 +54,12 @@ def test_few_sequences(fwp, E, M, L, form, few):
     assert 'wy' not in kr
     for a, r in ((y, yr), (W, Wr)):
         assert (a - r).abs().max().item() <= 1e-5 * r.abs().max().item()
+
+
+@pytest.mark.parametrize('E,M,n,L,few', [(96, 32, 111, 144, True), (96, 32, 110, 144, False), (77, 20, 6, 384, False), (96, 16, 6, 144, True),
+                                         (24, 24, 6, 112, False), (24, 24, 6, 113, True), (32, 32, 149, 160, False)])
+def test_where_it_is_taken(fwp, E, M, n, L, few):
+    """By the numbers of a B200's SMs (148): up to one sequence each, from three quarters of them on where M is above 16."""
+    *ins, _ = (t.to(DEV) for t in util.delta_inputs(83, n, 1, L, E, M))
+    _, _, kf = run(ins, torch.zeros(n, 1, E, M, device=DEV), False)
+    assert kf == ('delta_fwd_wy_few_kernel' if few else 'delta_fwd_wy_kernel')
