@@ -586,9 +586,11 @@ static int dispatch_fwd(const DeltaFwdParams& p, int nseq, cudaStream_t st) {
 // Where the three-launch backward is the faster one, from measurements on B200 (fp32, 256 steps, us, one-launch kernel ->
 // three launches):
 //   d = 16: 16 sequences 37 -> 13, 128 37 -> 25, 256 38 -> 37, 512 38 -> 65; with rows of 12 128 65 -> 27, 256 66 -> 52, 512 67 -> 76
-//   d = 32 with rows of 20: 128 139 -> 51, 512 283 -> 174.  Rows of 32 (training pass, one launch over four warps a sequence -> three launches):
-//           16 sequences x 64 25 -> 29, x 128 37 -> 35, x 256 64 -> 49, x 1024 220 -> 183; 32 x 256 65 -> 57, x 1024 221 -> 178; 64 x 128 39 -> 46,
-//           x 256 66 -> 68, x 1024 222 -> 233
+//   d = 32 with rows of 20: 128 139 -> 51, 512 283 -> 174.  Rows of 32, three launches over one launch of four warps a sequence, whole training
+//           pass: 64 steps 1.07-1.38, 80 0.98-1.04 (1 to 64 sequences), 96 0.92-0.99 (1 to 56; 1.07 at 64), 128 0.85-0.93 (1 to 48; 1.01 at 56, 1.16 at
+//           64), 256 0.68-0.98 (1 to 37; 1.02 to 72, 1.14 at 80), 1024 0.51-0.95 (1 to 52; 1.03 at 56, 1.17 at 96).  Where some rows are
+//           not 16-byte aligned: 64 1.00-1.06, 80 0.93-0.99 (1 to 64), 128 0.79-0.94 (1 to 56; 1.06 at 64), 256 0.62-0.93 (1 to 72; 1.05 at
+//           96), 1024 0.47-0.94 (1 to 72; 1.07 at 96)
 //   d = 64: 64 114 -> 76, 128 116 -> 125; with rows of 55 512 1789 -> 557;  d = 48: 512 1128 -> 354
 //   E, M = 96, 32: 128 951 -> 120, 1024 2777 -> 930;  128, 128: 128 2826 -> 676
 // and by length (time of the one-launch kernel over that of the three): d = 16, 80 sequences: 0.9 at 24 steps, 1.1 at 40, 1.8 at 250;
@@ -600,7 +602,8 @@ static int dispatch_fwd(const DeltaFwdParams& p, int nseq, cudaStream_t st) {
 //   d = 16: 16 sequences 187 -> 37, 128 189 -> 102, 288 190 -> 188, 512 191 -> 270; with rows of 12 (256 steps) 512 166 -> 75
 //   d = 32: 16 653 -> 55, 128 679 -> 215, 512 775 -> 714, 1024 1092 -> 1432;  d = 48 (256 steps): 512 648 -> 306, 1600 1766 -> 1235
 //   rows of 56 (256 steps): 512 651 -> 603.  Rows of 64 have a one-launch kernel on tensor cores.
-static bool bwd_phases_pay(const DeltaBwdParams& p, int nseq, int io_dtype) {
+// words: some stream's rows are not 16-byte aligned.  It widens the range, so it is what the size of the scratch is asked with.
+static bool bwd_phases_pay(const DeltaBwdParams& p, int nseq, int io_dtype, bool words) {
     if (tune_get(T_DELTA_BLOCKED, -1) != -1) return false;
     const int force = tune_get(T_DELTA_PHASES, -1);
     if (force != -1) return force == 1;
@@ -618,7 +621,7 @@ static bool bwd_phases_pay(const DeltaBwdParams& p, int nseq, int io_dtype) {
     }
     if (p.L <= 2 * kShortSeq) return false;
     if (d == 16) return nseq <= sms;
-    if (d == 32) return nseq <= sms / 4 && p.L >= 8 * kShortSeq;
+    if (d == 32) return words ? nseq <= sms / 2 && p.L > 72 : nseq <= sms * 3 / 8 && p.L > (nseq <= sms / 4 ? 88 : 95);
     if (p.L <= 3 * kShortSeq) return nseq <= sms * 3 / 4;
     if (p.L <= 4 * kShortSeq) return nseq <= 3 * sms;
     return nseq <= sms / 2 || (nseq > sms && nseq <= sms * 5 / 4);
@@ -768,7 +771,7 @@ static int fast_weight_backward_impl(int N, int H, int L, int E, int M,
     p.H = H; p.L = L; p.E = E; p.M = M; p.NH = N * H;
     cudaStream_t st = (cudaStream_t)stream;
     const auto phases = io_dtype == FWP_F32 ? bwd_phases<float> : bwd_phases<__nv_bfloat16>;
-    if (scratch && bwd_phases_pay(p, N * H, io_dtype)) {
+    if (scratch && bwd_phases_pay(p, N * H, io_dtype, !rows_16B_aligned(p))) {
         if (reinterpret_cast<uintptr_t>(scratch) & 15) return FWP_ERR_SCRATCH;
         const int64_t need = phases(false, p, N * H, nullptr, st);
         if (need > 0) return scratch_floats < need ? FWP_ERR_SCRATCH : (int)phases(true, p, N * H, scratch, st);
@@ -793,7 +796,7 @@ FWP_API int64_t fwp_fast_weight_backward_scratch_floats(int N, int H, int L, int
     if (check_common(N, H, L, E, M, io_dtype)) return 0;
     DeltaBwdParams p;
     p.H = H; p.L = L; p.E = E; p.M = M; p.NH = N * H;
-    if (!bwd_phases_pay(p, N * H, io_dtype)) return 0;
+    if (!bwd_phases_pay(p, N * H, io_dtype, true)) return 0;
     const int64_t need = (io_dtype == FWP_F32 ? bwd_phases<float> : bwd_phases<__nv_bfloat16>)(false, p, N * H, nullptr, nullptr);
     return need > 0 ? need : 0;
 }

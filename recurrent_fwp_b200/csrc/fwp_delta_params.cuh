@@ -40,6 +40,9 @@ template <typename T, bool SUM> int launch_fwd_wy(const DeltaFwdParams& p, int n
 // three-launch backward over a workspace (fwp_delta_phases.cuh): floats of scratch it needs (run = false) or the launches; -1
 // when the sizes have no instance
 template <typename T> int64_t bwd_phases(bool run, const DeltaBwdParams& p, int nseq, float* scratch, cudaStream_t st);
+static inline bool rows_16B_aligned(const DeltaBwdParams& p) {        // of fp32 streams
+    return rows_16B_aligned(p.k) && rows_16B_aligned(p.q) && rows_16B_aligned(p.v) && rows_16B_aligned(p.v_old) && rows_16B_aligned(p.gy);
+}
 // step by step over four warps a sequence, E = M = 32, fp32 streams (fwp_delta_tile.cuh)
 int launch_bwd_tile32(const DeltaBwdParams& p, int nseq, cudaStream_t st);
 int tc_fault_read_clear();

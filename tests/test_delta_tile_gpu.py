@@ -66,3 +66,15 @@ def test_four_warp_backward(fwp, B, H, L, form):
     grads = torch.autograd.grad(torch.stack(y, 2), leaves, g64)
     for a, r in zip(got, grads):
         assert close(a[:1].cpu(), r)
+
+
+@pytest.mark.parametrize('B,H,L,form,tile', [(1, 4, 88, 'packed', True), (1, 4, 89, 'packed', False), (5, 8, 96, 'packed', False),
+                                             (5, 8, 256, 'packed', False), (7, 8, 160, 'packed', True), (1, 4, 72, 'offset', True),
+                                             (1, 4, 73, 'offset', False), (9, 8, 112, 'offset', False), (10, 8, 160, 'offset', True)])
+def test_few_long_sequences_take_the_three_launches(fwp, B, H, L, form, tile):
+    """Up to 3/8 (rows off a 16-byte boundary: half) as many sequences as the SMs of a B200, from the length on where they win."""
+    *ins, gy = util.delta_inputs(73, B, H, L, D)
+    W0 = torch.randn(B, H, D, D, generator=util.gen(74)) * 0.1
+    got, kb = run(ins, gy, W0, form)
+    assert kb == ('delta_bwd_tile32_kernel' if tile else 'delta_bwd_finish_kernel')
+    assert (got[-1].cpu() - W0).abs().max().item() <= 1e-5      # rewound
