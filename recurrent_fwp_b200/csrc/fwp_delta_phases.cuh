@@ -244,7 +244,9 @@ __global__ void __launch_bounds__(WARPS * 32) delta_bwd_prepare_kernel(const __g
     };
     float bt[2][2];
     load_beta(bt, stream_at<T>(p.beta, n, h) + t0 * p.beta.sL, p.beta.sL, nt, t);
-    constexpr bool kAhead = KS <= 4, kRolled = KS > 4;    // loops over the blocks of a large state stay rolled: instruction fetch
+    constexpr bool kAhead = KS <= 4, kRolled = KS > 4 && KS <= 6 && MS <= 2;
+    // rolled loops over the blocks: less to fetch, slower to run.  Training pass, rolled over unrolled: E up to 96, M up to 32 0.95-1.00 (4 to
+    // 320 sequences); 128, 32 0.97-0.99 up to 144 sequences, 1.01 with 320; 128, 64 0.98-1.04; 128, 128 1.03-1.08
     constexpr int kUnroll = kRolled ? 1 : KS;
     if (kAhead) streams(0);
     if (g == 0) {
