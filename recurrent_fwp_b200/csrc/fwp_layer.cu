@@ -422,6 +422,16 @@ static bool layer_tile_ok(const LayerDims& d, const void* a, const void* b, cons
     return d.D % 4 == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c) |
                              reinterpret_cast<uintptr_t>(e) | reinterpret_cast<uintptr_t>(f)) & 15) == 0;
 }
+// Where the forward's is the faster one (us, 4-byte kernel and this, everything in L2):
+//   D = 4, 8     4 rows 2.09 and 2.22, 2.02 and 2.22; 128 2.57 and 2.21; 12800 3.3 and 2.9; 65536 7.0 and 5.6;  D = 12, 16 at any size
+//   D = 24       4 rows 2.4 and 2.2, 12800 3.9 and 3.3, but 25600 5.5 and 5.7, 65536 8.7 and 9.1 (a quarter of the lanes idle); D = 32 at any size
+//   D = 96       4 rows 3.0 and 3.4, 3200 3.9 and 4.3; 6400 6.4 and 4.8, 25600 12.2 and 10.2;  D = 48, 64 at any size
+//   D = 128      4 rows 3.2 and 3.9, 3200 4.2 and 5.1, 12800 8.3 and 8.9; 25600 13.5 and 12.6
+static bool fwd_tile_pays(int D, long long rows) {
+    if (D <= 8) return rows >= 128;
+    if (D > 16 && D < 32) return rows < 16384;
+    return D <= 64 || rows >= (D <= 96 ? 6144 : 16384);
+}
 template <int LPR, int MP, class K, class P>
 static int launch_layer_tile(K kern, const P& p, cudaStream_t st) {
     using T = LayerTile<LPR, MP>;
@@ -454,8 +464,8 @@ FWP_API int fwp_delta_layer_prologue_forward_scaled(int L, int B, int H, int D, 
     if (guard.status) return guard.status;
     cudaStream_t st = (cudaStream_t)stream;
     // L2 flushed before, 4-byte kernel and this: (512, 96, 8) rows of 16 45.8 and 32.8 us, (512, 32, 8) rows of 32 28.7 and 24.6,
-    // of 64 41.8 and 39.0, (256, 32, 8) of 128 41.0 and 40.8, of 96 36.9 and 32.8; (16, 1, 8) the same 6 to 8 us.
-    if (layer_tile_ok(p.d, qkvb, q, k, v)) {
+    // of 64 41.8 and 39.0, (256, 32, 8) of 128 41.0 and 40.8, of 96 36.9 and 32.8.
+    if (layer_tile_ok(p.d, qkvb, q, k, v) && fwd_tile_pays(D, p.d.rows)) {
         if (D <= 16) return launch_layer_tile<4, 1>(layer_prologue_fwd_tile_kernel<4, 1>, p, st);
         if (D <= 32) return launch_layer_tile<8, 1>(layer_prologue_fwd_tile_kernel<8, 1>, p, st);
         if (D <= 64) return launch_layer_tile<8, 2>(layer_prologue_fwd_tile_kernel<8, 2>, p, st);
@@ -485,8 +495,9 @@ FWP_API int fwp_delta_layer_prologue_backward_scaled(int L, int B, int H, int D,
     if (guard.status) return guard.status;
     cudaStream_t st = (cudaStream_t)stream;
     // L2 flushed before, 4-byte kernel and this form: (512, 96, 8) rows of 16 65.5 and 59.4 us, but (512, 32, 8) rows of 32
-    // 36.8 and 40.9, of 64 58.1 and 68.2, (256, 32, 8) of 128 58.1 and 72.4.
-    if (D <= 16 && layer_tile_ok(p.d, qkvb, grad_q, grad_k, grad_v, grad_qkvb))
+    // 36.8 and 40.9, of 64 58.1 and 68.2, (256, 32, 8) of 128 58.1 and 72.4.  In L2, D = 4 and 16: 4 rows 1.8 and 2.4, 1.9 and 2.5 us;
+    // 12800 3.1 and 3.3, 3.4 and 4.0; 25600 4.3 and 4.4, 4.8 and 5.9; 65536 8.3 and 6.9, 9.3 and 9.1; 393216 42 and 33, 57 and 51.
+    if (D <= 16 && p.d.rows >= 65536 && layer_tile_ok(p.d, qkvb, grad_q, grad_k, grad_v, grad_qkvb))
         return launch_layer_tile<4, 1>(layer_prologue_bwd_tile_kernel, p, st);
     auto grid = [&](int rows_per_warp) { return (int)((p.d.rows + kLayerWarps * rows_per_warp - 1) / (kLayerWarps * rows_per_warp)); };
     if (D <= 32) return launch_dependent(layer_prologue_bwd_kernel<8>, p, grid(4), kLayerWarps * 32, 0, st, nullptr);

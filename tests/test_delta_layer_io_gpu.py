@@ -38,9 +38,11 @@ def test_prologue_matches_the_elementwise_chain(fwp, L, B, H, d):
     assert util.scaled_rel(res['fused'][1], res['chain'][1]) <= 1e-5
 
 
-# a span of 64, 32, 16 rows (d up to 32, 64, 128) and one row more or less; off=1: rows that only the 4-byte kernels can take
+# a span of 64, 32, 16 rows (d up to 32, 64, 128) and one row more or less, and the row counts from which the kernels change (forward
+# at d = 4, 24, 96 and above, backward at d up to 16); off=1: rows that only the 4-byte kernels can take
 @pytest.mark.parametrize('off', [0, 1])
-@pytest.mark.parametrize('rows,d', [(63, 32), (64, 4), (65, 32), (131, 28), (31, 64), (33, 36), (15, 128), (17, 100)])
+@pytest.mark.parametrize('rows,d', [(63, 32), (64, 4), (65, 32), (131, 28), (31, 64), (33, 36), (15, 128), (17, 100),
+                                    (127, 8), (129, 4), (16383, 24), (16387, 24), (6145, 96), (16387, 100), (16383, 128), (65537, 4), (65559, 16)])
 def test_prologue_spans_and_their_remainders(fwp, rows, d, off):
     from recurrent_fwp_b200.delta_layer_io import delta_layer_prologue
     g = util.gen(6)
@@ -63,7 +65,7 @@ def test_prologue_spans_and_their_remainders(fwp, rows, d, off):
 # Warps of the last block without a row of their own, and a last row at every residue modulo four of the floats before it: nothing
 # but the live warps may write, so repeats agree bit for bit and the floats beside the result stay as they were.
 @pytest.mark.parametrize('d', [4, 8, 12, 16])
-@pytest.mark.parametrize('rows', [217, 222, 75, 200, 1])
+@pytest.mark.parametrize('rows', [217, 222, 75, 200, 1, 65536 + 25, 65536 + 30, 65536 + 11, 65536 + 8])
 def test_prologue_backward_of_a_partly_filled_block(fwp, rows, d):
     from recurrent_fwp_b200 import _lib
     g = util.gen(7)
