@@ -410,6 +410,17 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
 }
+// predicated, never a branch
+__device__ __forceinline__ void cp_async4_if(bool on, void* smem, const void* gmem) {
+    unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p cp.async.ca.shared.global [%0], [%1], 4;\n\t}"
+                 ::"r"(sa), "l"(gmem), "r"((int)on) : "memory");
+}
+__device__ __forceinline__ void cp_async16_if(bool on, void* smem, const void* gmem) {
+    unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p cp.async.cg.shared.global [%0], [%1], 16;\n\t}"
+                 ::"r"(sa), "l"(gmem), "r"((int)on) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
@@ -606,7 +617,8 @@ __device__ __forceinline__ void stage_table_issue(float* stage, const StageTable
 
 // The same copies for kernels with registers to spare, walking backwards from the last chunk: each of WARPS warps has its groups of
 // four rows of a tile to itself, by running pointers -- a 16-byte piece per lane, or a row at a time word by word where the stream's
-// rows are not 16-byte aligned (WORDS; the test costs 7 %, so callers that know better have an instance without).  The loop above cost
+// rows are not 16-byte aligned (WORDS; the test costs 7 %, so callers that know better have an instance without).  A branch per
+// group cost the chain warp of the RNN's backward 13 to 25 us of 256 steps (v2 and v1, up to a sequence per SM).  The loop above cost
 // the tiled delta backward a tenth of its time.  Streams that lag have their first row elsewhere: their users take the loop for it.
 template <int TC, int WARPS, int NTILE, bool WORDS>
 struct RowStager {
@@ -636,12 +648,10 @@ struct RowStager {
         for (int i = 0; i < MINE; i++) {
             const int rows = nt - (warp + WARPS * i) % (TC / 4) * 4;       // of this group that exist
             if (ITEMS % WARPS == 0 || warp + WARPS * i < ITEMS) {
-                if (!words[i]) {
-                    if ((lane >> 3) < rows) cp_async16(stage + to[i], from[i]);
-                } else {
+                cp_async16_if(!words[i] && (lane >> 3) < rows, stage + to[i], from[i]);
+                if constexpr (WORDS) {
 #pragma unroll
-                    for (int r = 0; r < 4; r++)
-                        if (r < rows) cp_async4(stage + to[i] + r * D, from[i] + r * sL[i]);
+                    for (int r = 0; r < 4; r++) cp_async4_if(words[i] && r < rows, stage + to[i] + r * D, from[i] + r * sL[i]);
                 }
             }
             from[i] -= TC * sL[i];
@@ -654,8 +664,10 @@ struct RowStager {
 };
 
 // One stream of rows of 32 floats as a single warp copies it, TC rows at a time, forwards: four rows at a time, a 16-byte piece per
-// lane, or (WORDS, where its rows are not 16-byte aligned) row by row word by word.
-template <int TC, bool WORDS>
+// lane, or (WORDS, where its rows are not 16-byte aligned) row by row word by word.  A last chunk's rows go one by one (a single step:
+// rows that are tested for instead cost the recurrent delta net 0.3 us of 8.3); ONE has the chunk once in code, each row tested for,
+// for a kernel without registers to spare (the LSTM's forward 82 us against 88 with 32 sequences x 256 steps, where the RNN's took 50 against 46).
+template <int TC, bool WORDS, bool ONE = false>
 struct WarpRows32 {
     const float* from;
     long long sL;
@@ -673,10 +685,13 @@ struct WarpRows32 {
 #pragma unroll
             for (int r = 0; r < TC; r += 4)
                 if (r + (lane >> 3) < nt) cp_async16(tile + 32 * r + 4 * lane, from + r * sL);
-        } else {
+        } else if (ONE || nt == TC) {
 #pragma unroll
             for (int r = 0; r < TC; r++)
-                if (r < nt) cp_async4(tile + 32 * r + lane, from + r * sL);
+                if (!ONE || r < nt) cp_async4(tile + 32 * r + lane, from + r * sL);
+        } else {
+#pragma unroll 1
+            for (int r = 0; r < nt; r++) cp_async4(tile + 32 * r + lane, from + r * sL);
         }
         from += TC * sL;
     }

@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(384, 1) lstm_fwd_gates32_kernel(const LstmFwdP
     // a warp copies z, k, v and beta of its own gate, by running pointers: four rows at a time, a 16-byte piece per lane, or row by
     // row word by word (12 rolled iterations over a table of all nine tiles: 512 sequences x 512 steps
     // 286 us, now 255; 32 sequences 192, now 151)
-    WarpRows32<TC, WORDS> rz, rk, rv;
+    WarpRows32<TC, WORDS, true> rz, rk, rv;
     rz.init(q == 0 ? p.z[0] : (q == 1 ? p.z[1] : p.z[2]), n, h, lane);
     rk.init(q == 0 ? p.k[0] : (q == 1 ? p.k[1] : p.k[2]), n, h, lane);
     rv.init(q == 0 ? p.v[0] : (q == 1 ? p.v[1] : p.v[2]), n, h, lane);

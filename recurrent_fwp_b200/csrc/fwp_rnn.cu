@@ -35,7 +35,8 @@ struct RnnFwdStage {
 };
 
 // ROWS: how the streams are copied -- 0 any size and alignment; at a head size of exactly 32, by one warp and running pointers, 1 rows on
-// 16-byte boundaries, 2 any rows (512 sequences x 512 steps, v2: 108 us with 0, 104 with 2, packed rows less; 32 sequences 94, 92)
+// 16-byte boundaries, 2 any rows (512 sequences x 512 steps, v2: 108 us with 0, 104 with 2, packed rows less; 32 sequences 94, 92).  A call
+// of one chunk keeps 0: a single step takes 2.9 us with it and 3.2 with the others
 template <int D, int SPLIT, int TC, bool V1, int ROWS>
 __global__ void __launch_bounds__(D * SPLIT * slots_for(D * SPLIT)) rnn_fwd_kernel(const RnnFwdParams p) {
     griddep_wait();               // launched as a dependent: global memory is touched from here on
@@ -316,7 +317,7 @@ static int launch_rnn_fwd(const RnnFwdParams& p, int nseq, cudaStream_t st) {
     auto kern = rnn_fwd_kernel<D, SPLIT, TC, V1, 0>;
     if constexpr (D == 32 && SPLIT == 1) {
         const bool aligned = rows_16B_aligned(p.z) && rows_16B_aligned(p.k) && rows_16B_aligned(p.v);
-        if (p.D == 32) kern = aligned ? rnn_fwd_kernel<D, SPLIT, TC, V1, 1> : rnn_fwd_kernel<D, SPLIT, TC, V1, 2>;
+        if (p.D == 32 && p.L > TC) kern = aligned ? rnn_fwd_kernel<D, SPLIT, TC, V1, 1> : rnn_fwd_kernel<D, SPLIT, TC, V1, 2>;
     }
     const size_t bytes = (2 * RnnFwdStage<D, TC>::kFloats + 2 * (D + 16)) * sizeof(float);
     const int slots = spread_slots(slots_for(D * SPLIT), nseq);
