@@ -62,6 +62,8 @@ struct Stream {
     long long sL;
     int width, off;         // off: that element's place in the tile
     bool vec, full;         // 16-byte pieces; whole rows of W elements
+    static constexpr bool kNarrow = W > 16;     // 16-byte pieces of narrower rows too (in tiles of 16 the test costs more)
+    static constexpr int RS1 = W < 32 ? 32 / W : 1;                                 // 4-byte copies of whole rows: rows per sweep
     static constexpr int PPR = W / 4, RS = PPR <= 32 ? 32 / PPR : 1;                // 16-byte pieces per row, rows per sweep
     static constexpr int CS1 = (W + 31) / 32;                                       // 4-byte copies: column groups
     static constexpr bool kVec = PPR <= 32 && 32 % PPR == 0;
@@ -69,10 +71,10 @@ struct Stream {
         base = reinterpret_cast<const T*>(r.p) + n * r.sN + h * r.sH;
         sL = r.sL;
         width = w;
-        vec = sizeof(T) == 4 && (reinterpret_cast<uintptr_t>(base) & 15) == 0 && sL % 4 == 0 && w % 4 == 0;
         full = kVec && w == W;
-        at = base + (vec ? (full ? (lane / PPR) * sL + (lane % PPR) * 4 : 4 * lane) : lane);
-        off = vec ? (full ? (lane / PPR) * P + (lane % PPR) * 4 : 4 * lane) : lane;
+        vec = sizeof(T) == 4 && (reinterpret_cast<uintptr_t>(base) & 15) == 0 && sL % 4 == 0 && (kNarrow ? w % 4 == 0 : full);
+        at = base + (vec ? (full ? (lane / PPR) * sL + (lane % PPR) * 4 : 4 * lane) : W < 32 ? (lane / W) * sL + lane % W : lane);
+        off = vec ? (full ? (lane / PPR) * P + (lane % PPR) * 4 : 4 * lane) : W < 32 ? (lane / W) * P + lane % W : lane;
     }
     // rows past the end are zeroed
     __device__ __forceinline__ void copy(float* tile, int t0, int nt, int lane) const {
@@ -84,7 +86,10 @@ struct Stream {
             if (vec && full && nt == C) {
 #pragma unroll
                 for (int r = 0; r < C; r += RS, g += RS * sL) cp_async16(tile + r * P, g);
-            } else if (vec && !full) {                  // a row at a time
+            } else if (W < 32 && full && nt == C) {
+#pragma unroll
+                for (int r = 0; r < C; r += RS1, g += RS1 * sL) cp_async4(tile + r * P, g);
+            } else if (kNarrow && vec && !full) {       // a row at a time
                 if (4 * lane < width)
 #pragma unroll 4
                     for (int r = 0; r < nt; r++, g += sL) cp_async16(tile + r * P, g);
@@ -353,6 +358,7 @@ __device__ __forceinline__ void fwd_few(const DeltaFwdParams& p) {
 
     // ---- helper: chunks b, b + NB, ...  Its loops over blocks stay rolled: with as many helpers as chunks in flight, each in a place of
     // its own, instruction fetch was the largest stall (E, M = 96, 32, 128 x 256: 72 us unrolled, 50 rolled)
+    constexpr int kUnroll = KS == 1 ? 16 : 1;   // at d = 16 they are single blocks, and the chain waits for every instruction
     const int b = warp - NCW;
     Buf& buf = bufs[b];
     Stream<E, PR, T> sk, sq;
@@ -383,7 +389,7 @@ __device__ __forceinline__ void fwd_few(const DeltaFwdParams& p) {
         cp_async_wait<0>();
         __syncwarp();
         float kk[2][4] = {}, qk[2][4] = {};
-#pragma unroll 1
+#pragma unroll kUnroll
         for (int k = 0; k < KS; k++) {
             Frag<NP> fk, fq;
             float x[2][4];
@@ -393,8 +399,8 @@ __device__ __forceinline__ void fwd_few(const DeltaFwdParams& p) {
             tile_block<PR>(x, &buf.qraw[g][2 * t + 16 * k]);
             from_c(fq, x[0], x[1]);
             store(aQ + 32 * k, kPart, fq);
-            if (!SUM) add_product<BY_ROWS>(kk, fk, fk);
-            add_product<BY_ROWS>(qk, fq, fk);
+            if (!SUM) sum_product<BY_ROWS>(KS == 1 ? 0 : 1, kk, fk, fk);
+            sum_product<BY_ROWS>(KS == 1 ? 0 : 1, qk, fq, fk);
         }
 #pragma unroll
         for (int nn = 0; nn < 2; nn++) {
@@ -432,7 +438,7 @@ __device__ __forceinline__ void fwd_few(const DeltaFwdParams& p) {
                 ta.r[i][2] = tt.r[i][1];
                 ta.r[i][3] = tt.r[i][3];
             }
-#pragma unroll 1
+#pragma unroll kUnroll
             for (int k = 0; k < KS; k++) {            // X = T K
                 Frag<NP> r;
                 float x[2][4] = {};
@@ -442,7 +448,7 @@ __device__ __forceinline__ void fwd_few(const DeltaFwdParams& p) {
                 store(aX + 32 * k, kPart, f);
             }
         }
-#pragma unroll 1
+#pragma unroll kUnroll
         for (int j = 0; j < NCW; j++) {               // (T V)^T = V^T T^T
             float x[2][4];
             tile_block_t<PV>(x, &buf.v[st][2 * t][16 * j + g]);
@@ -461,7 +467,7 @@ __device__ __forceinline__ void fwd_few(const DeltaFwdParams& p) {
         Frag<3> ra;
         load_rows(ra, aA, kPartC);
         wait(&done[b], phase);
-#pragma unroll 1
+#pragma unroll kUnroll
         for (int j = 0; j < NCW; j++) {
             float y[2][4], w[2][4], u[2][4];
             Frag<3> us;
@@ -477,7 +483,7 @@ __device__ __forceinline__ void fwd_few(const DeltaFwdParams& p) {
 #pragma unroll
             for (int i = 0; i < 8; i++) y[i >> 2][i & 3] = 0.f;
             product<BY_ROWS>(y, us, ra);
-#pragma unroll 1
+#pragma unroll kUnroll
             for (int k = 0; k < KS; k++) {
                 Frag<3> s;
                 Frag<NP> r;
