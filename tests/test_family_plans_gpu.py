@@ -1,13 +1,13 @@
 """The d = 32 execution plans of the recurrent families against the general kernels on the same inputs.
 
 The short-chain / multi-warp kernels (``rec_fwd_warp32_kernel``, ``rec_bwd_roles32_kernel``, ``rnn_bwd_roles32_kernel``,
-``lstm_fwd_gates32_kernel``, ``lstm_bwd_roles32_kernel``) are the default at a head dimension of exactly 32 with
-16-byte aligned rows.  Each test runs the op twice, with the plan on and switched off through ``fwp_tune``, checks
+``lstm_fwd_gates32_kernel``, ``lstm_bwd_roles32_kernel``) are the default at a head dimension of exactly 32.  Each test runs the op twice, with the plan on and switched off through ``fwp_tune``, checks
 which kernel ran (``fwp_last_kernel``) and that outputs, end states, rewound states and gradients agree to 2e-5 of
 the tensor's scale (both paths are fp32 and differ in summation order and in the exp / tanh forms); sequence counts
 that are not multiples of the sequences per CTA and lengths on both sides of the chunk boundaries are covered.
-Rows that are not 16-byte aligned must take the general kernel and still give the same numbers.  Parity with the
-fp64 oracle is in test_rnn_gpu.py, test_lstm_gpu.py and test_rec_delta_gpu.py (their d = 32 cases run these plans)."""
+Rows that are not 16-byte aligned take the general kernel below 64 steps (from there on the plans copy them word by
+word) and still give the same numbers.  Parity with the fp64 oracle is in test_rnn_gpu.py, test_lstm_gpu.py and
+test_rec_delta_gpu.py (their d = 32 cases run these plans)."""
 import importlib
 
 import pytest
@@ -194,6 +194,35 @@ def test_recurrent_delta_backward_plans_agree(fwp, B, H, L):
     assert fast['kb'] == 'rec_bwd_roles32_kernel' and ref['kb'] == 'rec_bwd_kernel'
     assert close(fast['W_back'], ref['W_back'])
     for a, r in zip(fast['g'], ref['g']):
+        assert close(a, r)
+
+
+@pytest.mark.parametrize('B', [111, 74])
+@pytest.mark.parametrize('L,mis', [(1, False), (8, False), (9, False), (19, False), (70, False), (70, True)])
+def test_recurrent_delta_backward_with_several_sequences_per_sm(fwp, B, L, mis):
+    """111 x 4 sequences fill an SM with four (warps that change their register counts, a set of hand-over barriers per
+    sequence); 74 x 4 take two."""
+    from recurrent_fwp_b200 import _lib
+    from recurrent_fwp_b200.rec_update_fwm_tanh import rec_update_fwm_tanh
+    H = 4
+    *ins, gy = util.rec_inputs(71, B, H, L, D)
+    W0 = torch.randn(B, H, D, D, generator=util.gen(72)) * 0.1
+    h0 = torch.randn(B, H, 1, D, generator=util.gen(73))
+    got = {}
+    try:
+        for roles in (1, 0):
+            _lib.tune('rec_bwd.32.roles', roles)
+            off = mis and roles == 1
+            leaves = [(misalign(t.to(DEV)) if off and i < 4 else t.clone().to(DEV)).requires_grad_() for i, t in enumerate(ins)]
+            W, hs, kb = W0.clone().to(DEV), h0.clone().to(DEV), []
+            y = rec_update_fwm_tanh(*leaves, W, hs)
+            note_backward_kernel(leaves[0], kb)
+            y.backward(misalign(gy.to(DEV)) if off else gy.to(DEV))     # the backward's other streams are the forward's own
+            got[roles] = [W] + [l.grad for l in leaves]
+            assert kb == ['rec_bwd_roles32_kernel' if roles else 'rec_bwd_kernel']
+    finally:
+        _lib.tune('rec_bwd.32.roles', 1)
+    for a, r in zip(got[1], got[0]):
         assert close(a, r)
 
 

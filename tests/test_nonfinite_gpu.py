@@ -13,7 +13,7 @@ from tests import util
 pytestmark = pytest.mark.gpu
 DEV = 'cuda:0'
 INF, NAN = math.inf, math.nan
-SIZES = [(16, 16), (9, 14), (32, 32), (48, 48), (50, 33), (96, 32), (32, 97), (128, 128)]
+SIZES = [(16, 16), (9, 14), (32, 32), (20, 31), (48, 48), (50, 33), (96, 32), (77, 12), (32, 97), (128, 128)]
 B, H, L = 2, 3, 45
 
 
@@ -58,6 +58,7 @@ def forward(rule, x, W, plan):
                                         ('W', NAN)])
 def test_forward_is_causal_for_any_value(fwp, E, M, dtype, name, value):
     """One bad element at step 21 (chunk 2 of 3, row 5) of one sequence, or in its start state."""
+    from recurrent_fwp_b200 import _lib
     q, k, v, b, _ = util.delta_inputs(71, B, H, L, E, M, dtype=dtype)
     W0 = torch.randn(B, H, E, M, generator=util.gen(72)) * 0.1
     clean = dict(q=q, k=k, v=v, beta=b, W=W0)
@@ -75,9 +76,10 @@ def test_forward_is_causal_for_any_value(fwp, E, M, dtype, name, value):
         else:
             K.causal_dot_product(*[bad[n].float() for n in x], kv, refs[0])
             refs = [refs[0], kv]
-        for helpers in (2, 4):
+        for helpers in (2, 4, 6):
             plan = {'delta.wy': 1, 'delta.wy.helpers': helpers}
             got = forward(rule, [bad[n].to(DEV) for n in x], bad['W'].to(DEV), plan)
+            assert _lib.last_kernel() == ('delta_fwd_wy_few_kernel' if util.few_form(rule, E, M, dtype, helpers) else 'delta_fwd_wy_kernel')
             ref = forward(rule, [clean[n].to(DEV) for n in x], W0.to(DEV), plan)
             for i, (a, c, r) in enumerate(zip(got, ref, refs)):
                 # bf16 outputs are rounded to 8 bits; everything else is fp32 on both sides, sums in another order

@@ -49,9 +49,9 @@ def test_forward_meets_the_oracle(fwp, E, M, L):
             ref[:, :, t] = torch.einsum('bhem,bhe->bhm', S, q[:, :, t].double())
         dev = [t.to(DEV) for t in x]
         for streams in (dev, sliced(dev)):
-            for helpers in (2, 4):
+            for helpers in (2, 4, 6):
                 y, W, kernel = run(fwp, rule, streams, W0.to(DEV), {'delta.wy': 1, 'delta.wy.helpers': helpers})
-                assert kernel.startswith('delta_fwd_wy')
+                assert kernel == ('delta_fwd_wy_few_kernel' if util.few_form(rule, E, M, q.dtype, helpers) else 'delta_fwd_wy_kernel')
                 # fp32 accuracy: three-part products keep every bit of the operands
                 assert util.max_abs(y, ref) <= 2e-6 * max(1., ref.abs().max().item()), (rule, helpers)
                 assert util.max_abs(W, S) <= 2e-6 * max(1., S.abs().max().item()), (rule, helpers)
@@ -62,7 +62,7 @@ def test_forward_with_more_sequences_than_the_gpu_holds(fwp, B, H, L, d):
     q, k, v, b, _ = (t.to(DEV) for t in util.delta_inputs(9, B, H, L, d))
     W0 = torch.randn(B, H, d, d, generator=util.gen(10)).to(DEV) * 0.1
     y, W, _ = run(fwp, 'delta', [q, k, v, b], W0, {'delta.wy': 0})
-    for helpers in (0, 2, 4):
+    for helpers in (0, 2, 4, 6):
         y2, W2, _ = run(fwp, 'delta', [q, k, v, b], W0, {'delta.wy': 1, 'delta.wy.helpers': helpers})
         assert util.max_abs(y, y2) <= 5e-6 and util.max_abs(W, W2) <= 5e-6
     from recurrent_fwp_b200 import _lib

@@ -59,6 +59,14 @@ def lstm_inputs(seed, B, H, L, d):
     return gates, gy
 
 
+def few_form(rule, E, M, dtype, helpers):
+    """Whether the chunkwise forward has a form for few sequences at these sizes that ``delta.wy.helpers`` selects."""
+    d = max(E, M)
+    if dtype != torch.float32:
+        return False
+    return helpers == 4 if d <= 16 else helpers == 6 and rule == 'delta' and (d <= 32 or (64 < d <= 96 and M <= 32))
+
+
 def max_abs(a, b):
     return (a.double().cpu() - b.double().cpu()).abs().max().item()
 
