@@ -648,8 +648,10 @@ struct RowStager {
         for (int i = 0; i < MINE; i++) {
             const int rows = nt - (warp + WARPS * i) % (TC / 4) * 4;       // of this group that exist
             if (ITEMS % WARPS == 0 || warp + WARPS * i < ITEMS) {
-                cp_async16_if(!words[i] && (lane >> 3) < rows, stage + to[i], from[i]);
-                if constexpr (WORDS) {
+                if constexpr (!WORDS) {
+                    if ((lane >> 3) < rows) cp_async16(stage + to[i], from[i]);
+                } else {
+                    cp_async16_if(!words[i] && (lane >> 3) < rows, stage + to[i], from[i]);
 #pragma unroll
                     for (int r = 0; r < 4; r++) cp_async4_if(words[i] && r < rows, stage + to[i] + r * D, from[i] + r * sL[i]);
                 }
