@@ -83,7 +83,7 @@ struct Stream {
         if constexpr (sizeof(T) == 4) {
             const T* g = at + t0 * sL;
             tile += off;
-            if (vec && full && nt == C) {
+            if (vec && (full || !kNarrow) && nt == C) {
 #pragma unroll
                 for (int r = 0; r < C; r += RS, g += RS * sL) cp_async16(tile + r * P, g);
             } else if (W < 32 && full && nt == C) {
