@@ -103,7 +103,10 @@ unsigned long long fwp_launch_count(void);
  * "delta.pipe64" (1 / 2 / 0: chunkwise bf16 kernels with a preparing warp one chunk ahead in both directions,
  * in the forward only, or not at all),
  * "delta.wy" (-1 automatic / 1 / 0: the chunkwise split-product plan wherever it is the faster one, wherever it has an
- * instance, or never), "delta.wy.helpers" (0 automatic / 4 / 2: preparing warps per sequence of that plan),
+ * instance, or never), "delta.wy.helpers" (0 automatic; 2 or 4: preparing warps per sequence of its general form,
+ * where an instance has the choice; the form for few sequences, fp32: 4 asks for it at sizes up to 16 (six preparing warps up to one
+ * sequence per SM, four beyond), 6 for the delta rule at sizes up to 32 and at E up to 96 with M up to 32; any of the three keeps the
+ * general form where it is not asked for),
  * "delta_bwd.phases" (-1 automatic / 1 / 0: the three-launch backward over scratch, see below), "delta_bwd.32.tile" (1 / 0: the
  * fp32 backward at E = M = 32 step by step over four warps a sequence, or the four-step blocked kernel).  Returns 0 if accepted, FWP_ERR_UNSUPPORTED for an unknown key. */
 int fwp_tune(const char* key, int value);
@@ -248,7 +251,8 @@ int fwp_rec_update_fwm_tanh_backward(int N, int H, int L, int D,
                                      int io_dtype, void* stream, int device);
 /* The same from what the forward left: its outputs `out` and the vector `start` (N,H,1,D) that the first step was fed, instead
  * of a tensor of their delayed tanh.  FWP_ERR_UNSUPPORTED, with nothing launched, where no kernel takes them (head sizes other
- * than 32; rows that are not 16-byte aligned below 64 steps): the entry point above serves every case. */
+ * than 32; rows that are not 16-byte aligned below 64 steps; "rec_bwd.32.roles" = 0, for the RNN and the LSTM "rnn_bwd.32.roles" and
+ * "lstm_bwd.32.roles" = 0): the entry point above serves every case. */
 int fwp_rec_update_fwm_tanh_backward_from_outputs(int N, int H, int L, int D,
                                      const fwp_tensor* q, const fwp_tensor* k,
                                      const fwp_tensor* v, const fwp_tensor* beta,

@@ -66,7 +66,7 @@ enum TuneKey {
     T_LAUNCH_DEPENDENT,     // "launch.dependent": 1 the register-resident delta-rule kernels (blocked and per-step) are launched with programmatic stream serialisation (their prologue overlaps the tail of the kernel before), 0 plain launches
     T_STEP_SPREAD,          // "step.spread": 1 the per-step forward packs fewer sequences into a CTA while that puts CTAs on more SMs, 0 always four warps per CTA
     T_DELTA_WY,             // "delta.wy": -1 automatic, 1 / 0 the chunkwise split-product plan (fwp_delta_wy.cuh) wherever it has an instance, or never
-    T_DELTA_WY_HELPERS,     // "delta.wy.helpers": preparing warps per sequence of that plan (2, 4, or 6: the form for few sequences above d = 16), 0 automatic
+    T_DELTA_WY_HELPERS,     // "delta.wy.helpers": 2, 4: preparing warps per sequence of that plan's general form; 4 up to d = 16 and 6 above: its form for few sequences; 0 automatic
     T_DELTA_PHASES,         // "delta_bwd.phases": -1 automatic, 1 / 0 the three-launch backward wherever it has an instance and scratch, or never
     T_DELTA_BWD_TILE32,     // "delta_bwd.32.tile": 1 the backward at E = M = 32 (fp32) step by step over four warps, 0 the blocked kernel
     T_COUNT

@@ -455,7 +455,7 @@ __device__ __forceinline__ void nbar_arrive(int id, int n) { asm volatile("bar.a
 }  // namespace cb
 
 // SAVE: v_old is asked for (a test per store instead costs 1 %, the kernel is at its register limit).  4096 sequences x 4096 steps:
-// 3.58 ms, against 3.91 with v_old from a product of its own with (T - I), stores of y through a tile that the four warps shared
+// 3.58 ms, against 3.91 with products with both T and (T - I), stores of y through a tile that the four warps shared
 // behind a barrier, and an address per v_old store.  Its DRAM traffic alone takes 2.0.
 template <bool SAVE>
 __global__ void __launch_bounds__(cb::NTP, 4) delta_fwd_chunk_bf16_pipe_kernel(const DeltaFwdParams p) {

@@ -14,7 +14,8 @@
 //   warp Y   turns v into w = v - v_old (and the outputs into their tanh) for the chunk that X takes next, and two chunks later accumulates the three parameter
 //            gradients (8 x 4 pieces) and stores.
 // X and P hand over twice per step at named barriers: P has X's step to answer in.  The warps meet once per chunk of steps.
-// 512 sequences x 256 steps take 161 us, 32 sequences 105 (230 us for 512 with one warp for all but the parameter gradients; 10 more when
+// 512 sequences x 256 steps take 161 us, 32 sequences 105, and 171 and 105 where gy's rows are off a 16-byte boundary (320 bytes of
+// spills with four sequences per SM) (230 us for 512 with one warp for all but the parameter gradients; 10 more when
 // all three ran a loop over single pieces instead of Y staging by running pointers).  X alone took 131 -- 250 instructions a step, 128 of
 // them packed multiply-adds at 2.7 cycles -- and P alone 160, when q . dq and k . dk came from the saved values: that form's seventh tile
 // cost 6 us of 167 with 512 sequences, its shorter chain gave 10 of 105 with 32.  Not worth its instructions: P posting from a G one step

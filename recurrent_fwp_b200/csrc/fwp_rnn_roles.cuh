@@ -9,8 +9,8 @@
 //   warp T (one chunk behind)  the other gradients, from G and its own S (fwp_trail.cuh), the chunk unrolled.
 // The two meet once per chunk on a named barrier; that is also where staged input tiles change hands.  Each alone would take
 // about 490 (X) and 600 (T) cycles per step with four sequences per SM; a scheduler with one sequence issues for both.
-// 512 sequences x 512 steps: 169 us, 181 with one stream whose rows are not 16-byte aligned (194 when a loop over single pieces
-// staged the tiles), against 222 us with T's work in two warps that held G by columns and by rows, and 222 us with T's columns split
+// 512 sequences x 512 steps: 167 us, 180 with one stream whose rows are not 16-byte aligned (194 when a loop over single pieces
+// staged the tiles); 32 sequences x 256 65 and 70 us, against 222 us with T's work in two warps that held G by columns and by rows, and 222 us with T's columns split
 // over two warps (a third more instructions).
 #pragma once
 #include "fwp_trail.cuh"
